@@ -38,14 +38,16 @@ __global__ void __launch_bounds__(NT) k_shift_dots(unsigned n, const double *__r
     if (threadIdx.x == 0) part[(size_t)j * gridDim.x + blockIdx.x] = acc;
 }
 
-// out[j] = scale * w_j * sum_b part[j][b] (in block order)
-__global__ void k_sum_parts(int m, int g, const double *__restrict__ part, const double *__restrict__ w, double scale,
-                            double *out) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
+// out[j] = scale * w_j * sum_b part[j][b], one warp per shift, in a fixed order
+// (one thread per shift: 512 dependent adds of 64 clocks, 42 us; a warp: 5 us)
+__global__ void __launch_bounds__(NT) k_sum_parts(int m, int g, const double *__restrict__ part,
+                                                  const double *__restrict__ w, double scale, double *out) {
+    const int j = blockIdx.x * NW + (threadIdx.x >> 5);
     if (j >= m) return;
     double s = 0.0;
-    for (int b = 0; b < g; ++b) s += part[(size_t)j * g + b];
-    out[j] = scale * (w ? w[j] : 1.0) * s;
+    for (int b = threadIdx.x & 31; b < g; b += 32) s += part[(size_t)j * g + b];
+    s = warp_sum(s);
+    if ((threadIdx.x & 31) == 0) out[j] = scale * (w ? w[j] : 1.0) * s;
 }
 
 // db[i] = sum_j w_j Y[j][i]
@@ -55,6 +57,46 @@ __global__ void __launch_bounds__(NT) k_grad_b(unsigned n, int m, const double *
         double s = 0.0;
         for (int j = 0; j < m; ++j) s = fma(w ? w[j] : 1.0, Y[(size_t)j * ldy + i], s);
         db[i] = s;
+    }
+}
+
+// The same as k_grad_val for rows of few entries: one thread per row, up to
+// GRAD_E entries at a time in registers.  The sum is bound by the FP64 pipe:
+// w_j Y[j][row] is formed once per row and shift instead of once per entry (a
+// seven-point stencil: 8 instead of 14 operations per row and shift), Y is
+// read once and coalesced, and two shifts have their loads in flight together
+// (one or four: 2 % slower; more than two blocks per SM: up to 5 %).  128^3,
+// 32 shifts: 2062 -> 1110 us, without the map from entries to rows (47 us);
+// floor 740 us (one FMA per entry and shift).
+constexpr int GRAD_E = 8;
+__global__ void __launch_bounds__(NT, 2) k_grad_val_rows(unsigned n, const unsigned *__restrict__ ptr,
+                                                      const unsigned *__restrict__ col, int m,
+                                                      const double *__restrict__ X, size_t ldx,
+                                                      const double *__restrict__ Y, size_t ldy,
+                                                      const double *__restrict__ w, double *__restrict__ dval) {
+    for (size_t i = blockIdx.x * (size_t)NT + threadIdx.x; i < n; i += (size_t)gridDim.x * NT) {
+        const unsigned e1 = ptr[i + 1];
+        for (unsigned e0 = ptr[i]; e0 < e1; e0 += GRAD_E) {
+            const unsigned cnt = e1 - e0;
+            unsigned c[GRAD_E];
+            double s[GRAD_E];
+#pragma unroll
+            for (int e = 0; e < GRAD_E; ++e) {
+                c[e] = (unsigned)e < cnt ? col[e0 + e] : 0u;
+                s[e] = 0.0;
+            }
+            const double *xj = X, *yj = Y + i;
+#pragma unroll 2
+            for (int j = 0; j < m; ++j, xj += ldx, yj += ldy) {
+                const double y = (w ? w[j] : 1.0) * *yj;
+#pragma unroll
+                for (int e = 0; e < GRAD_E; ++e)
+                    if ((unsigned)e < cnt) s[e] = fma(y, xj[c[e]], s[e]);
+            }
+#pragma unroll
+            for (int e = 0; e < GRAD_E; ++e)
+                if ((unsigned)e < cnt) dval[e0 + e] = -s[e];
+        }
     }
 }
 
@@ -88,12 +130,20 @@ int hbk_shift_dots(unsigned n, int m, const double *X, size_t ldx, const double 
                    const double *w, double scale, double *out, void *tmp, cudaStream_t st) {
     if (m <= 0) return 0;
     k_shift_dots<<<dim3(DOT_GRID, m), NT, 0, st>>>(n, X, ldx, a, lda, a_shared, (double *)tmp);
-    k_sum_parts<<<(m + 63) / 64, 64, 0, st>>>(m, DOT_GRID, (const double *)tmp, w, scale, out);
+    k_sum_parts<<<(m + NW - 1) / NW, NT, 0, st>>>(m, DOT_GRID, (const double *)tmp, w, scale, out);
     return (int)cudaGetLastError();
 }
 
 int hbk_grad_b(unsigned n, int m, const double *Y, size_t ldy, const double *w, double *db, cudaStream_t st) {
     k_grad_b<<<grid_for(n ? n : 1, 2), NT, 0, st>>>(n, m, Y, ldy, w, db);
+    return (int)cudaGetLastError();
+}
+
+int hbk_grad_val_rows(unsigned n, const unsigned *ptr, const unsigned *col, int m, const double *X, size_t ldx,
+                      const double *Y, size_t ldy, const double *w, double *dval, cudaStream_t st) {
+    if (!n) return 0;
+    k_grad_val_rows<<<wave_grid<k_grad_val_rows>((int)(((size_t)n + NT - 1) / NT)), NT, 0, st>>>(n, ptr, col, m, X, ldx, Y,
+                                                                                              ldy, w, dval);
     return (int)cudaGetLastError();
 }
 

@@ -262,6 +262,9 @@ int hbk_shift_dots(unsigned n, int m, const double *X, size_t ldx, const double 
 int hbk_grad_b(unsigned n, int m, const double *Y, size_t ldy, const double *w, double *db, cudaStream_t st);
 int hbk_grad_val(unsigned nnz, const unsigned *rows, const unsigned *col, int m, const double *X, size_t ldx,
                  const double *Y, size_t ldy, const double *w, double *dval, cudaStream_t st);
+/* the same without the entries' rows, one thread per row (rows of few entries) */
+int hbk_grad_val_rows(unsigned n, const unsigned *ptr, const unsigned *col, int m, const double *X, size_t ldx,
+                      const double *Y, size_t ldy, const double *w, double *dval, cudaStream_t st);
 size_t hbk_flush_tc_workspace_bytes(int m);
 int hbk_flush_tc_max_slots(void);
 int hbk_flush_tc_run(const double *V, size_t ld, unsigned n, int L, const double *Xc, const double *Pc, int cap,
