@@ -24,11 +24,13 @@ extern "C" {
 #define HBK_MAX_GRID 4096    /* upper bound on persistent grids (partial-sum slots) */
 #define HBK_TILE_NNZ 2048    /* nonzeros staged in shared memory per SpMV row block */
 #define HBK_NCOEF 8          /* coefficients per shift per iteration */
+#define HBK_NPART 6          /* sets of partial sums of an iteration */
 
 /* status bits (device and host) */
 #define HBK_ST_BREAKDOWN 1   /* a scalar of the recurrence became 0, inf or nan */
 #define HBK_ST_BASIS_FULL 2  /* deferred mode: the basis needs a flush */
 #define HBK_ST_SHIFT_FAIL 4  /* a non-seed shift broke down (its conv_k is -k) and stopped */
+#define HBK_ST_NEED_PS 8     /* deferred mode: paused after a seed switch, the host has the new seed's p formed */
 
 /* SpMV row-block kinds (bits 30..31 of blk_row entries are not used; kinds
  * are a separate byte array) */
@@ -79,23 +81,30 @@ typedef struct {
     unsigned nmlong;
 } hbk_matrix;
 
+/* The scalars that the kernels of one iteration after K1 read: K1's block 0
+ * copies them from hbk_scalars, whose own fields the iteration's end (K5)
+ * advances while other blocks of K5 still read this copy. */
+typedef struct {
+    int k, seed, slots, slot_r_old;
+    int active;         /* 0: the solve had stopped when K1 ran, or broke down since */
+    int rr_pend;        /* (r^, r) is still in partial sums (the iteration before ended with a switch) */
+    int n_done, max_sigma;
+} hbk_cur;
+
 /* Device-resident scalars of one solve. */
 typedef struct {
+    hbk_cur cur;        /* first: read as two 16-byte words */
     double rr_hat;      /* (r^, r) */
     double rr_hat_old;
     double rr;          /* (r, r) at the end of the current iteration */
     double bb;          /* (b, b) */
     double rs, qq, qy;  /* raw reductions of the current iteration */
     double alpha, omega, beta;
-    double r_scale;     /* 1 / (zeta_t pi_t) when the iteration ends with a switch */
     double tol;
     int k;              /* current iteration, 1-based */
     int seed;           /* seed of the current iteration */
-    int next_seed;
     int n_done;         /* converged systems */
     int finished;       /* set once n_done == m or k == kcap */
-    int switched;       /* this iteration ends with a seed switch */
-    int n_active;       /* entries in act_list for the shift update */
     int status;         /* HBK_ST_* */
     int n_sw;           /* seed switches so far */
     int max_sigma;      /* the argmax of the last convergence test */
@@ -105,7 +114,10 @@ typedef struct {
     int slot_r_old;     /* deferred mode: slot of r_{k-1} */
     int slot_cap;
     int need_ps;        /* deferred mode: the new seed's p must be formed from the basis */
-    double rs_switch;   /* (r^, r_k) after the switch rescale */
+    int rr_pend;        /* the iteration ended with a switch: (r^, r) of the rescaled r is in K5's partial sums */
+    int inline_ps;      /* 1: the launch that runs the iterations forms the new seed's p itself (shared launches) */
+    double aw;          /* alpha_k / omega_k */
+    double ba;          /* beta_{k-1} / alpha_{k-1} */
     int loops;          /* bodies of the device-side iteration loop run in this solve (bound on the loop) */
 } hbk_scalars;
 
@@ -116,11 +128,11 @@ typedef struct {
     double *pi;                 /* [m][kcap] */
     double *eta, *zeta;         /* [m] */
     int *done, *conv_k;         /* [m]; conv_k: iteration of convergence, -k for a shift that broke down at k */
-    int *act_list;              /* [m] shifts updated this iteration */
-    double *coef;               /* [m][HBK_NCOEF] their coefficients */
+    double *coef;               /* [m][HBK_NCOEF] their coefficients (entry 4: (pi_{k-1} / pi_k)^2, times beta in use) */
+    int *live;                  /* [m] this iteration: 0 stopped before, 1 running, 2 its recurrence just broke down */
     int *sw_k, *sw_seed;        /* [m] switch log */
     int *act_hist;              /* [kcap] active non-seed shifts per iteration */
-    double *partials;           /* [4][HBK_MAX_GRID] */
+    double *partials;           /* [HBK_NPART][HBK_MAX_GRID] */
     unsigned *counters;         /* [8] last-block tickets */
     double *ratio;              /* [kcap] scratch for the switch replay */
     int *lslot;                 /* [m] deferred mode: basis slots in use at a system's last update */
@@ -210,8 +222,14 @@ int hbk_sell_fill(unsigned n, const unsigned *ptr, const unsigned *col, const do
 
 /* ---- fused solver ---- */
 int hbk_fused_init(const hbk_matrix *A, const hbk_vectors *v, const hbk_shifts *sh, const double *b, int seed,
-                   double tol, cudaStream_t st);
-int hbk_fused_iteration(const hbk_matrix *A, const hbk_vectors *v, const hbk_shifts *sh, cudaStream_t st);
+                   double tol, int switching, int inline_ps, cudaStream_t st);
+/* early: 0: the iteration's kernels one after the other; 1: each but the
+ * first may start before the one before it ends (programmatic dependent
+ * launch); 2: the first too (the stream's previous kernel was an iteration's) */
+int hbk_fused_iteration(const hbk_matrix *A, const hbk_vectors *v, const hbk_shifts *sh, int early, cudaStream_t st);
+/* deferred mode, after a switch (HBK_ST_NEED_PS): form the new seed's p from
+ * the basis and let the solve run on */
+int hbk_materialize_ps(const hbk_matrix *A, const hbk_vectors *v, const hbk_shifts *sh, cudaStream_t st);
 /* end of one body of a CUDA graph's conditional while loop over iterations:
  * sets the loop's condition to "not finished", and to 0 once the solve has run
  * loop_cap bodies (a bound on the loop whatever the scalars say) */

@@ -22,11 +22,24 @@ constexpr int NT = HBK_THREADS;
 #ifndef HBK_HYB_MINB
 #define HBK_HYB_MINB 8
 #endif
+// blocks per SM of the SELL-32 kernels: their slice pipeline holds 80 registers
+#define HBK_SELL_MINB 3
 constexpr int NW = NT / 32;
 
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
     for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+// sums over the warp of x (lanes 0..15) and of y (lanes 16..31), in the FP64
+// adds of one sum: the halves swap what they do not keep
+__device__ __forceinline__ double warp_sum_pair(double x, double y) {
+    const bool up = threadIdx.x & 16;
+    const double other = __shfl_xor_sync(0xffffffffu, up ? x : y, 16);
+    double v = (up ? y : x) + other;
+#pragma unroll
+    for (int o = 8; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
 }
 
@@ -90,6 +103,19 @@ struct HwGrid {
     template <class T>
     __device__ static __forceinline__ T ldv(const T *p) { return __ldg(p); }
 };
+// the launch's grid behind `x` extra blocks: block 0 for the scalars, blocks
+// 1 .. x - 1 for the coefficient update
+struct HwGridX {
+    static constexpr bool hw = true;
+    unsigned x;
+    __device__ __forceinline__ unsigned b() const { return blockIdx.x - x; }
+    __device__ __forceinline__ unsigned nb() const { return gridDim.x - x; }
+    __device__ __forceinline__ bool extra() const { return blockIdx.x == 0; }
+    __device__ __forceinline__ bool coef_only() const { return blockIdx.x != 0 && blockIdx.x < x; }
+    __device__ __forceinline__ bool does_coef() const { return coef_only(); }
+    __device__ __forceinline__ unsigned cb() const { return blockIdx.x - 1; }
+    __device__ __forceinline__ unsigned ncb() const { return x - 1; }
+};
 // element i of a vector the launch also writes (p indexed directly in a
 // one-step kernel, so its code is what it was without grid views)
 #define HBK_LD(G, p, i) ((G::hw) ? (p)[i] : __ldcg((p) + (i)))
@@ -105,8 +131,14 @@ struct is_hw_grid<HwGrid> {
 struct VGrid {
     static constexpr bool hw = false;
     unsigned vb, vnb;
+    bool ex;  // the family's extra block
     __device__ __forceinline__ unsigned b() const { return vb; }
     __device__ __forceinline__ unsigned nb() const { return vnb; }
+    __device__ __forceinline__ bool extra() const { return ex; }
+    __device__ __forceinline__ bool coef_only() const { return false; }
+    __device__ __forceinline__ bool does_coef() const { return true; }
+    __device__ __forceinline__ unsigned cb() const { return vb; }
+    __device__ __forceinline__ unsigned ncb() const { return vnb; }
     template <class T>
     __device__ static __forceinline__ T ld(const T *p) { return __ldcg(p); }
     template <class T>
@@ -124,12 +156,23 @@ __device__ __forceinline__ double sum_partials(const double *partials, int npart
     return block_sum(acc, sh);
 }
 
-__device__ __forceinline__ bool fin(double v) { return isfinite(v) != 0; }
+// on the integer pipe: an FP64 compare costs a warp 64 clocks like any other
+// FP64 instruction, and these tests run in every warp
+__device__ __forceinline__ bool fin(double v) {
+    return (__double2hiint(v) & 0x7ff00000) != 0x7ff00000;
+}
+__device__ __forceinline__ bool is_zero(double v) { return (__double2hiint(v) << 1 | __double2loint(v)) == 0; }
+
+// Programmatic dependent launch: a kernel lets the next one of its stream
+// start early, and waits for the one before it (both do nothing in a launch
+// without the attribute).
+__device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // max of v over the block (every thread calls), then one atomicMax into
 // out[blockIdx.x % HBK_SLOT_SPREAD] when it is nonzero (bits of non-negative
 // doubles order as unsigned integers; spreading the blocks over entries keeps
-// the atomics from queueing on one address); `sh` needs NW values
+// the atomics from queueing on one address); `sh` needs a value per warp
 __device__ __forceinline__ void block_max_to(unsigned long long v, unsigned long long *sh, unsigned long long *out) {
 #pragma unroll
     for (int o = 16; o; o >>= 1) {
@@ -142,7 +185,7 @@ __device__ __forceinline__ void block_max_to(unsigned long long v, unsigned long
     __syncthreads();
     if (threadIdx.x == 0) {
         unsigned long long m = 0;
-        for (int i = 0; i < NW; ++i) m = sh[i] > m ? sh[i] : m;
+        for (int i = 0; i < (int)(blockDim.x >> 5); ++i) m = sh[i] > m ? sh[i] : m;
         if (m) atomicMax(out + blockIdx.x % HBK_SLOT_SPREAD, m);
     }
 }
@@ -180,14 +223,94 @@ struct SpmvSmem {
 // of column indices, so every load is coalesced and no shared memory or
 // barrier is needed; each row is still summed in stored order with FMAs from
 // 0, exactly as in the TILE path (padding entries are skipped by row length).
-template <class Epi, class G = HwGrid>
-__device__ __forceinline__ void spmv_rows_sell(const hbk_matrix &A, const double *__restrict__ x, Epi &epi,
-                                               const G &g = G()) {
-    const unsigned *__restrict__ ptr = A.ptr;
-    const double *__restrict__ sval = A.sval;
-    const unsigned *__restrict__ scol = A.scol;
-    const unsigned n = A.n;
-    const unsigned ns = (n + 31) / 32;
+//
+// Three loads follow one another for a slice: its offset and row lengths, its
+// columns and values, the x they name; and FP64 FMAs take 64 clocks per warp
+// and SM quarter.  So a warp keeps three slices going: it sums one while the
+// columns and values of the next and the offset of the one after are on their
+// way, up to SELL_AHEAD entries per row ahead (7 or 8: a seven-point stencil's
+// whole row), and `pre(row)` loads what the row's epilogue needs beside the x.
+// start() issues the first slice's loads, so that a caller can wait for x to
+// be ready behind them.  256^3 stencil, measured alone: y = A x 300 -> 261 us
+// (6.7 TB/s) with 7 ahead (8: 275 us), with a dot product 330 -> 312 us; the
+// 256^3 solve 765 ms with 7 ahead in its products, 755 ms with 8; at 80
+// registers, three blocks per SM (64 registers, four blocks: 597 us).  Values and columns through
+// bulk copies into shared memory, two to four slices deep, were slower
+// (275..339 us).
+template <int SELL_AHEAD>
+struct SellRows {
+    const hbk_matrix &A;
+    unsigned stride, r0;    // first row of the block's next NT rows
+    unsigned off, off1;     // of the slices at r0 and r0 + stride: their first entry / 32,
+    unsigned wl, wl1;       // their width (entries per row) and, in the low byte, this lane's row length
+    unsigned cc[SELL_AHEAD];
+    double vv[SELL_AHEAD];
+
+    __device__ __forceinline__ explicit SellRows(const hbk_matrix &a)
+        : A(a), stride(gridDim.x * NT), r0(blockIdx.x * NT) {}
+    __device__ __forceinline__ void head(unsigned at, unsigned &of, unsigned &width_len) const {
+        const unsigned r = at + threadIdx.x;
+        of = width_len = 0;
+        if (r / 32 < (A.n + 31) / 32) {
+            of = (unsigned)(__ldg(A.sptr + r / 32) >> 5);
+            width_len = ((unsigned)(__ldg(A.sptr + r / 32 + 1) >> 5) - of) << 8;
+        }
+        if (r < A.n) width_len |= __ldg(A.ptr + r + 1) - __ldg(A.ptr + r);
+    }
+    __device__ __forceinline__ size_t entry(unsigned of, unsigned e) const {
+        return (size_t)(of + e) * 32 + (threadIdx.x & 31);
+    }
+    __device__ __forceinline__ void entries(unsigned of, unsigned width_len, unsigned (&c)[SELL_AHEAD],
+                                            double (&v)[SELL_AHEAD]) const {
+        const unsigned ln = width_len & 255u;
+        const unsigned *__restrict__ pc = A.scol + entry(of, 0);
+        const double *__restrict__ pv = A.sval + entry(of, 0);
+#pragma unroll
+        for (unsigned e = 0; e < SELL_AHEAD; ++e) {
+            c[e] = e < ln ? __ldg(pc + 32 * e) : 0u;
+            v[e] = e < ln ? __ldg(pv + 32 * e) : 0.0;
+        }
+    }
+    // rows of the block's next step (n: none left)
+    __device__ __forceinline__ unsigned after(unsigned at) const { return A.n - at > stride ? at + stride : A.n; }
+    __device__ __forceinline__ void start() {
+        if (r0 >= A.n) return;
+        head(r0, off, wl);
+        entries(off, wl, cc, vv);
+        head(after(r0), off1, wl1);
+    }
+    template <class Pre, class Epi>
+    __device__ __forceinline__ void run(const double *__restrict__ x, const Pre &pre, Epi &epi) {
+        while (r0 < A.n) {
+            const unsigned r = r0 + threadIdx.x, len = wl & 255u;
+            double xv[SELL_AHEAD], vn[SELL_AHEAD];
+#pragma unroll
+            for (unsigned e = 0; e < SELL_AHEAD; ++e) xv[e] = e < len ? __ldg(x + cc[e]) : 0.0;
+            const double own = r < A.n ? pre(r) : 0.0;
+            entries(off1, wl1, cc, vn);
+            r0 = after(r0);
+            unsigned off2, wl2;
+            head(r0 < A.n ? after(r0) : r0, off2, wl2);
+            double acc = 0.0;
+#pragma unroll
+            for (unsigned e = 0; e < SELL_AHEAD; ++e)
+                if (e < wl >> 8 && e < len) acc = fma(vv[e], xv[e], acc);
+            for (unsigned e = SELL_AHEAD; e < wl >> 8; ++e)
+                if (e < len) acc = fma(__ldg(A.sval + entry(off, e)), __ldg(x + __ldg(A.scol + entry(off, e))), acc);
+            if (r < A.n) epi(r, acc, own);
+#pragma unroll
+            for (unsigned e = 0; e < SELL_AHEAD; ++e) vv[e] = vn[e];
+            off = off1, wl = wl1;
+            off1 = off2, wl1 = wl2;
+        }
+    }
+};
+// the same on a virtual grid (a persistent launch's families are small and
+// their matrices in L2; the x may have been written by the same launch)
+template <class Pre, class Epi>
+__device__ __forceinline__ void spmv_rows_sell(const hbk_matrix &A, const double *__restrict__ x, const Pre &pre,
+                                               Epi &epi, const VGrid &g) {
+    const unsigned n = A.n, ns = (n + 31) / 32;
     const unsigned stride = g.nb() * NT;
     for (unsigned r0 = g.b() * NT; r0 < n; r0 += stride) {
         const unsigned r = r0 + threadIdx.x;
@@ -198,20 +321,21 @@ __device__ __forceinline__ void spmv_rows_sell(const hbk_matrix &A, const double
             base = __ldg(A.sptr + s);
             w = (unsigned)((__ldg(A.sptr + s + 1) - base) >> 5);
         }
-        const unsigned len = r < n ? __ldg(ptr + r + 1) - __ldg(ptr + r) : 0;
-        const double *__restrict__ vv = sval + base + lane;
-        const unsigned *__restrict__ cc = scol + base + lane;
+        const unsigned len = r < n ? __ldg(A.ptr + r + 1) - __ldg(A.ptr + r) : 0;
+        const double *__restrict__ vv = A.sval + base + lane;
+        const unsigned *__restrict__ cc = A.scol + base + lane;
+        const double own = r < n ? pre(r) : 0.0;
         double acc = 0.0;
 #pragma unroll 4
         for (unsigned e = 0; e < w; ++e) {
-            if (e < len) acc = fma(G::ldv(vv + 32 * (size_t)e), G::ldx(x + __ldg(cc + 32 * (size_t)e)), acc);
+            if (e < len) acc = fma(VGrid::ldv(vv + 32 * (size_t)e), VGrid::ldx(x + __ldg(cc + 32 * (size_t)e)), acc);
         }
-        if (r < n) epi(r, acc);
+        if (r < n) epi(r, acc, own);
     }
 }
 
-template <class Epi>
-__device__ __forceinline__ void spmv_rows_tile(const hbk_matrix &A, const double *__restrict__ x, Epi &epi,
+template <class Pre, class Epi>
+__device__ __forceinline__ void spmv_rows_tile(const hbk_matrix &A, const double *__restrict__ x, const Pre &pre, Epi &epi,
                                                SpmvSmem &sm) {
     const unsigned *__restrict__ ptr = A.ptr;
     const unsigned *__restrict__ col = A.col;
@@ -223,7 +347,7 @@ __device__ __forceinline__ void spmv_rows_tile(const hbk_matrix &A, const double
             double acc = 0.0;
             for (unsigned e = e0 + threadIdx.x; e < e1; e += NT) acc = fma(__ldg(val + e), __ldg(x + __ldg(col + e)), acc);
             acc = block_sum(acc, sm.red);
-            if (threadIdx.x == 0) epi(r0, acc);
+            if (threadIdx.x == 0) epi(r0, acc, pre(r0));
             __syncthreads();
             continue;
         }
@@ -239,7 +363,7 @@ __device__ __forceinline__ void spmv_rows_tile(const hbk_matrix &A, const double
             const unsigned a = __ldg(ptr + r) - e0, z = __ldg(ptr + r + 1) - e0;
             double acc = 0.0;
             for (unsigned e = a; e < z; ++e) acc = fma(sm.val[e], sm.xv[e], acc);
-            epi(r, acc);
+            epi(r, acc, pre(r));
         }
         __syncthreads();
     }
@@ -261,8 +385,9 @@ __device__ __forceinline__ void spmv_rows_tile(const hbk_matrix &A, const double
 // a slice, and the tree), so no warp is left with several of the longest
 // rows; warp w of the grid runs lists w, w + (warps of the grid), ...  A row's
 // arithmetic does not depend on the list it is in.
-template <class Epi>
-__device__ __forceinline__ void spmv_rows_hyb(const hbk_matrix &A, const double *__restrict__ x, Epi &epi) {
+template <class Pre, class Epi>
+__device__ __forceinline__ void spmv_rows_hyb(const hbk_matrix &A, const double *__restrict__ x, const Pre &pre,
+                                              Epi &epi) {
     const unsigned lane = threadIdx.x & 31;
     const unsigned nw = (gridDim.x * NT) >> 5;
     for (unsigned w = (blockIdx.x * NT + threadIdx.x) >> 5; w < A.hnw; w += nw) {
@@ -295,7 +420,7 @@ __device__ __forceinline__ void spmv_rows_hyb(const hbk_matrix &A, const double 
                 for (unsigned e = rg.x + (lane & (g - 1)); e < rg.y; e += g)
                     acc = fma(__ldg(A.val + e), __ldg(x + __ldg(A.col + e)), acc);
                 for (unsigned o = g >> 1; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-                if (valid && (lane & (g - 1)) == 0) epi(r, acc);
+                if (valid && (lane & (g - 1)) == 0) epi(r, acc, pre(r));
             } else {
                 const unsigned s = it - A.hitl;
                 const unsigned long long base = __ldg(A.sptr + s);
@@ -308,7 +433,7 @@ __device__ __forceinline__ void spmv_rows_hyb(const hbk_matrix &A, const double 
 #pragma unroll 4
                 for (unsigned e = 0; e < wd; ++e)
                     if (e < len) acc = fma(__ldg(vv + 32 * (size_t)e), __ldg(x + __ldg(cc + 32 * (size_t)e)), acc);
-                if (r < A.n) epi(r, acc);
+                if (r < A.n) epi(r, acc, pre(r));
             }
         }
     }
@@ -348,9 +473,9 @@ struct MergeSmem {
 
 constexpr unsigned kNoRow = 0x80000000u;
 
-template <class Epi>
-__device__ __forceinline__ void spmv_rows_merge(const hbk_matrix &A, const double *__restrict__ x, Epi &epi,
-                                                MergeSmem &sm) {
+template <class Pre, class Epi>
+__device__ __forceinline__ void spmv_rows_merge(const hbk_matrix &A, const double *__restrict__ x, const Pre &pre,
+                                                Epi &epi, MergeSmem &sm) {
     constexpr int IPT = HBK_MERGE_IPT;
     const unsigned *__restrict__ ptr = A.ptr;
     const unsigned *__restrict__ col = A.col;
@@ -378,7 +503,7 @@ __device__ __forceinline__ void spmv_rows_merge(const hbk_matrix &A, const doubl
                 if (h3) a3 = fma(v3, x3, a3);
             }
             const double acc = warp_sum((a0 + a1) + (a2 + a3));
-            if (lane == 0) epi(r, acc);
+            if (lane == 0) epi(r, acc, pre(r));
             continue;
         }
         const unsigned b = u - A.nmlong;
@@ -472,7 +597,7 @@ __device__ __forceinline__ void spmv_rows_merge(const hbk_matrix &A, const doubl
             if (rr[q] != kNoRow) ws.xv[merge_pad(rr[q])] = rv[q];
         if (head_row != kNoRow) ws.xv[merge_pad(head_row)] = ((lane > 0 && pk == head_row) ? ps : 0.0) + head_v;
         __syncwarp();
-        for (unsigned q = lane; q < nr; q += 32) epi(r0 + q, ws.xv[merge_pad(q)]);
+        for (unsigned q = lane; q < nr; q += 32) epi(r0 + q, ws.xv[merge_pad(q)], pre(r0 + q));
         __syncwarp();  // before the next unit overwrites this warp's staging
     }
 }
@@ -480,31 +605,47 @@ __device__ __forceinline__ void spmv_rows_merge(const hbk_matrix &A, const doubl
 // Format chosen at compile time so the SELL kernels carry no shared-memory
 // tile (full occupancy); launchers pick the instantiation from A.fmt.
 // (the virtual grids of a persistent launch take the SELL-32 form only)
-template <int FMT, class Epi, class G = HwGrid>
-__device__ __forceinline__ void spmv_rows(const hbk_matrix &A, const double *__restrict__ x, Epi &epi,
-                                          const G &g = G()) {
-    static_assert(FMT == HBK_FMT_SELL || is_hw_grid<G>::value, "virtual grids take the SELL-32 form only");
-    if constexpr (FMT == HBK_FMT_SELL) {
-        spmv_rows_sell(A, x, epi, g);
-    } else if constexpr (FMT == HBK_FMT_HYB) {
-        spmv_rows_hyb(A, x, epi);
-    } else if constexpr (FMT == HBK_FMT_MERGE) {
-        __shared__ MergeSmem sm;
-        spmv_rows_merge(A, x, epi, sm);
-    } else {
-        __shared__ SpmvSmem sm;
-        spmv_rows_tile(A, x, epi, sm);
+// start() reads the matrix alone, so it may run before x is ready.
+template <int FMT, class G, int AHEAD = 8>
+struct SpmvRows {
+    static_assert(is_hw_grid<G>::value, "virtual grids take the SELL-32 form only");
+    const hbk_matrix &A;
+    __device__ __forceinline__ SpmvRows(const hbk_matrix &a, const G &) : A(a) {}
+    __device__ __forceinline__ void start() {}
+    template <class Pre, class Epi>
+    __device__ __forceinline__ void run(const double *__restrict__ x, const Pre &pre, Epi &epi) {
+        if constexpr (FMT == HBK_FMT_HYB) {
+            spmv_rows_hyb(A, x, pre, epi);
+        } else if constexpr (FMT == HBK_FMT_MERGE) {
+            __shared__ MergeSmem sm;
+            spmv_rows_merge(A, x, pre, epi, sm);
+        } else {
+            __shared__ SpmvSmem sm;
+            spmv_rows_tile(A, x, pre, epi, sm);
+        }
     }
+};
+template <int AHEAD>
+struct SpmvRows<HBK_FMT_SELL, HwGrid, AHEAD> : SellRows<AHEAD> {
+    __device__ __forceinline__ SpmvRows(const hbk_matrix &a, const HwGrid &) : SellRows<AHEAD>(a) {}
+};
+template <int AHEAD>
+struct SpmvRows<HBK_FMT_SELL, VGrid, AHEAD> {
+    const hbk_matrix &A;
+    const VGrid &g;
+    __device__ __forceinline__ SpmvRows(const hbk_matrix &a, const VGrid &v) : A(a), g(v) {}
+    __device__ __forceinline__ void start() {}
+    template <class Pre, class Epi>
+    __device__ __forceinline__ void run(const double *__restrict__ x, const Pre &pre, Epi &epi) {
+        spmv_rows_sell(A, x, pre, epi, g);
+    }
+};
+template <int FMT, int AHEAD = 8, class Pre, class Epi>
+__device__ __forceinline__ void spmv_rows(const hbk_matrix &A, const double *__restrict__ x, const Pre &pre, Epi &epi) {
+    SpmvRows<FMT, HwGrid, AHEAD> rows(A, HwGrid());
+    rows.start();
+    rows.run(x, pre, epi);
 }
-
-// launch helper: kernel<FMT> for the matrix's format
-#define HBK_LAUNCH_FMT(A, kern, grid, block, stream, ...)                                   \
-    do {                                                                                    \
-        if ((A).fmt == HBK_FMT_SELL) kern<HBK_FMT_SELL><<<grid, block, 0, stream>>>(__VA_ARGS__); \
-        else if ((A).fmt == HBK_FMT_HYB) kern<HBK_FMT_HYB><<<grid, block, 0, stream>>>(__VA_ARGS__); \
-        else if ((A).fmt == HBK_FMT_MERGE) kern<HBK_FMT_MERGE><<<grid, block, 0, stream>>>(__VA_ARGS__); \
-        else kern<HBK_FMT_TILE><<<grid, block, 0, stream>>>(__VA_ARGS__);                  \
-    } while (0)
 
 // number of SMs of the current device (cached: one device type per process)
 inline int sm_count() {
@@ -528,6 +669,15 @@ inline int wave_grid(int want) {
     }();
     return want < one_wave ? want : one_wave;
 }
+
+// launch helper: kernel<FMT> for the matrix's format
+#define HBK_LAUNCH_FMT(A, kern, grid, block, stream, ...)                                   \
+    do {                                                                                    \
+        if ((A).fmt == HBK_FMT_SELL) kern<HBK_FMT_SELL><<<grid, block, 0, stream>>>(__VA_ARGS__); \
+        else if ((A).fmt == HBK_FMT_HYB) kern<HBK_FMT_HYB><<<grid, block, 0, stream>>>(__VA_ARGS__); \
+        else if ((A).fmt == HBK_FMT_MERGE) kern<HBK_FMT_MERGE><<<grid, block, 0, stream>>>(__VA_ARGS__); \
+        else kern<HBK_FMT_TILE><<<grid, block, 0, stream>>>(__VA_ARGS__);                  \
+    } while (0)
 
 inline int grid_for(unsigned n, int per_thread) {
     static int sms = 0;

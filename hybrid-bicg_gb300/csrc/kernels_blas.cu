@@ -48,25 +48,36 @@ struct EpiStore {
     const double *x;
     double sigma;
     int add;
-    __device__ void operator()(unsigned r, double acc) const { y[r] = add ? fma(sigma, x[r], acc) : acc; }
+    __device__ void operator()(unsigned r, double acc, double xr) const { y[r] = add ? fma(sigma, xr, acc) : acc; }
 };
 
 struct EpiAccum {
     double *y;
-    __device__ void operator()(unsigned r, double acc) const { y[r] += acc; }
+    __device__ void operator()(unsigned r, double acc, double yr) const { y[r] = yr + acc; }
 };
 
 template <int FMT>
 __global__ void __launch_bounds__(NT) k_spmv(hbk_matrix A, const double *__restrict__ x, double *__restrict__ y,
                                              double sigma, int add) {
     EpiStore epi{y, x, sigma, add};
-    spmv_rows<FMT>(A, x, epi);
+    auto pre = [&](unsigned r) { return add ? x[r] : 0.0; };
+    spmv_rows<FMT>(A, x, pre, epi);
+}
+
+template <>
+__global__ void __launch_bounds__(NT, HBK_SELL_MINB) k_spmv<HBK_FMT_SELL>(hbk_matrix A, const double *__restrict__ x,
+                                                                         double *__restrict__ y, double sigma,
+                                                                         int add) {
+    EpiStore epi{y, x, sigma, add};
+    auto pre = [&](unsigned r) { return add ? x[r] : 0.0; };
+    spmv_rows<HBK_FMT_SELL, 7>(A, x, pre, epi);
 }
 
 template <int FMT>
 __global__ void __launch_bounds__(NT) k_spmv_acc(hbk_matrix A, const double *__restrict__ x, double *__restrict__ y) {
     EpiAccum epi{y};
-    spmv_rows<FMT>(A, x, epi);
+    auto pre = [&](unsigned r) { return y[r]; };
+    spmv_rows<FMT>(A, x, pre, epi);
 }
 
 // out[j] = ||b - (A + sigma_j I) x_j||^2 ; one launch per shift block (grid.y = shift)
@@ -79,11 +90,12 @@ __device__ __forceinline__ void true_res_body(const hbk_matrix &A, const double 
     const double *xj = X + (size_t)j * ld;
     const double sg = sigma[j];
     double acc = 0.0;
-    auto epi = [&](unsigned r, double ax) {
-        const double res = b[r] - fma(sg, xj[r], ax);
+    auto pre = [&](unsigned r) { return b[r]; };
+    auto epi = [&](unsigned r, double ax, double br) {
+        const double res = br - fma(sg, xj[r], ax);
         acc = fma(res, res, acc);
     };
-    spmv_rows<FMT>(A, xj, epi);
+    spmv_rows<FMT>(A, xj, pre, epi);
     acc = block_sum(acc, sh);
     double *pj = partials + (size_t)j * gridDim.x;
     if (threadIdx.x == 0) pj[blockIdx.x] = acc;
@@ -107,6 +119,12 @@ __global__ void __launch_bounds__(NT) k_true_res(hbk_matrix A, const double *__r
                                                  const double *__restrict__ b, const double *__restrict__ sigma,
                                                  double *partials, unsigned *counters, double *out) {
     true_res_body<FMT>(A, X, ld, b, sigma, partials, counters, out);
+}
+template <>
+__global__ void __launch_bounds__(NT, HBK_SELL_MINB) k_true_res<HBK_FMT_SELL>(
+    hbk_matrix A, const double *__restrict__ X, size_t ld, const double *__restrict__ b,
+    const double *__restrict__ sigma, double *partials, unsigned *counters, double *out) {
+    true_res_body<HBK_FMT_SELL>(A, X, ld, b, sigma, partials, counters, out);
 }
 template <>
 __global__ void __launch_bounds__(NT, HBK_HYB_MINB) k_true_res<HBK_FMT_HYB>(
@@ -310,15 +328,21 @@ int hbk_merge_grid(unsigned units) {
     return g < 1 ? 1 : g;
 }
 
+// blocks of a product: SELL-32 at most one wave (a second, partial wave cost
+// 340 against 261 us on the 256^3 stencil), the other forms as planned
+static int product_grid(const hbk_matrix *A) {
+    return A->fmt == HBK_FMT_SELL ? wave_grid<k_spmv<HBK_FMT_SELL>>(A->grid) : A->grid;
+}
+
 int hbk_spmv(const hbk_matrix *A, const double *x, double *y, double sigma, int sigma_add, cudaStream_t st) {
     if (!A->n) return 0;
-    HBK_LAUNCH_FMT(*A, k_spmv, A->grid, NT, st, *A, x, y, sigma, sigma_add);
+    HBK_LAUNCH_FMT(*A, k_spmv, product_grid(A), NT, st, *A, x, y, sigma, sigma_add);
     return (int)cudaGetLastError();
 }
 
 int hbk_spmv_accumulate(const hbk_matrix *A, const double *x, double *y, cudaStream_t st) {
     if (!A->n) return 0;
-    HBK_LAUNCH_FMT(*A, k_spmv_acc, A->grid, NT, st, *A, x, y);
+    HBK_LAUNCH_FMT(*A, k_spmv_acc, product_grid(A), NT, st, *A, x, y);
     return (int)cudaGetLastError();
 }
 
@@ -326,7 +350,7 @@ int hbk_true_residuals(const hbk_matrix *A, const double *X, const double *b, co
                        double *partials, unsigned *counters, double *out, cudaStream_t st) {
     if (!A->n || m <= 0) return 0;
     size_t ld = ((size_t)A->n + 31) / 32 * 32;
-    dim3 grid(A->grid, m);
+    dim3 grid(product_grid(A), m);
     HBK_LAUNCH_FMT(*A, k_true_res, grid, NT, st, *A, X, ld, b, sigma, partials, counters, out);
     return (int)cudaGetLastError();
 }
@@ -334,7 +358,7 @@ int hbk_true_residuals(const hbk_matrix *A, const double *X, const double *b, co
 int hbk_true_residuals_ld(const hbk_matrix *A, const double *X, size_t ldx, const double *b, const double *sigma,
                           int m, int grid_cap, double *partials, unsigned *counters, double *out, cudaStream_t st) {
     if (!A->n || m <= 0) return 0;
-    const int g = A->grid < grid_cap ? A->grid : grid_cap;
+    const int w = product_grid(A), g = w < grid_cap ? w : grid_cap;
     dim3 grid(g, m);
     HBK_LAUNCH_FMT(*A, k_true_res, grid, NT, st, *A, X, ldx, b, sigma, partials, counters, out);
     return (int)cudaGetLastError();

@@ -1,18 +1,20 @@
 // Fused shifted BiCGStab iteration with on-device scalars and seed switching.
 //
-// One iteration is five launches (seven in deferred mode), each reading the
+// One iteration is five launches, each reading the
 // device-resident scalars, so an iteration (or a CUDA graph of many) needs no
 // host round trip:
-//   K1 seed_s     s = (A + sigma_s I) p_s, (r^,s) fused        -> alpha
-//   K2 seed_q     q = r_{k-1} - alpha s
-//   K3 seed_y     y = (A + sigma_s I) q, (q,q), (q,y) fused     -> omega
-//   K4 seed_upd   x_s += alpha p_s + omega q ; r_k = q - omega y ; (r,r), (r^,r)
-//                 last block: beta, every shift's recurrence and coefficients,
-//                 the convergence test, argmax and the seed switch
-//   K5 shifts     p_s and every unconverged shift's x_j, p_j in one pass
-//                 (incremental mode); r_k rescaled on a switch
-//   K6/K7         deferred mode only: coefficient update of every system in
-//                 the Krylov basis; materialise the new seed's p after a switch
+//   K1 seed_s     s = (A + sigma_s I) p_s, (r^,s) fused
+//   K2 seed_q     alpha; q = r_{k-1} - alpha s
+//   K3 seed_y     y = (A + sigma_s I) q, (q,q), (q,y) fused
+//   K4 seed_upd   omega; r_k = q - omega y ; (r,r), (r^,r); beside it every
+//                 shift's recurrence and coefficients
+//   K5 shifts     beta, the convergence test and the decision to switch; x_s,
+//                 p_s and every unconverged shift's x_j, p_j in one pass
+//                 (incremental mode) or the update of every system's
+//                 coefficients in the Krylov basis (deferred mode); r_k
+//                 rescaled on a switch
+// After a switch in the deferred mode the new seed's p is formed from the
+// basis by a launch of its own.
 // Reference: src/solver_dynamic.c:147-381 (seed step :156-210, shift loop
 // :239-256, convergence test :278-303, seed switch :312-359).
 #include <vector>
@@ -36,29 +38,139 @@ struct Ctx {
     hbk_matrix A;
     hbk_vectors v;
     hbk_shifts sh;
+    // partial sums that each step leaves behind (the blocks of K1, K3, K4, K5)
+    unsigned np_s, np_y, np_r, np_p;
 };
 
 __device__ __forceinline__ size_t ldn(unsigned n) { return ((size_t)n + 31) / 32 * 32; }
 
+// sets of partial sums: (r^,s); (q,q), (q,y); (r,r), (r^,r); (r^, rescaled r) after a switch
+enum { P_RS, P_QQ, P_QY, P_RR, P_RRH, P_RRS };
+__device__ __forceinline__ double *parts(const Ctx &c, int set) { return c.sh.partials + (size_t)set * HBK_MAX_GRID; }
+
 __device__ __forceinline__ const double *seed_p(const Ctx &c, int seed) {
     return c.v.deferred ? c.v.ps : c.v.P + (size_t)seed * ldn(c.v.n);
 }
-__device__ __forceinline__ double *vec_r_old(const Ctx &c, const hbk_scalars *sc) {
-    return c.v.deferred ? c.v.V + (size_t)sc->slot_r_old * ldn(c.v.n) : c.v.rbuf[(sc->k - 1) & 1];
+__device__ __forceinline__ double *vec_r_old(const Ctx &c, const hbk_cur &u) {
+    return c.v.deferred ? c.v.V + (size_t)u.slot_r_old * ldn(c.v.n) : c.v.rbuf[(u.k - 1) & 1];
 }
-__device__ __forceinline__ double *vec_r_new(const Ctx &c, const hbk_scalars *sc) {
-    return c.v.deferred ? c.v.V + (size_t)(sc->slots + 1) * ldn(c.v.n) : c.v.rbuf[sc->k & 1];
+__device__ __forceinline__ double *vec_r_new(const Ctx &c, const hbk_cur &u) {
+    return c.v.deferred ? c.v.V + (size_t)(u.slots + 1) * ldn(c.v.n) : c.v.rbuf[u.k & 1];
 }
-__device__ __forceinline__ double *vec_q(const Ctx &c, const hbk_scalars *sc) {
-    return c.v.deferred ? c.v.V + (size_t)sc->slots * ldn(c.v.n) : c.v.q;
+__device__ __forceinline__ double *vec_q(const Ctx &c, const hbk_cur &u) {
+    return c.v.deferred ? c.v.V + (size_t)u.slots * ldn(c.v.n) : c.v.q;
 }
-
-// (an L2 load: in a persistent launch another CTA may have set the flag
-// since this SM last read it)
-__device__ __forceinline__ bool stopped(const hbk_scalars *sc) { return __ldcg(&sc->finished) != 0; }
+// (an L2 load: in a persistent launch another CTA wrote it in an earlier step)
+__device__ __forceinline__ hbk_cur load_cur(const hbk_scalars *sc) {
+    const int4 a = __ldcg(reinterpret_cast<const int4 *>(&sc->cur));
+    const int4 b = __ldcg(reinterpret_cast<const int4 *>(&sc->cur) + 1);
+    hbk_cur u;
+    u.k = a.x, u.seed = a.y, u.slots = a.z, u.slot_r_old = a.w;
+    u.active = b.x, u.rr_pend = b.y, u.n_done = b.z, u.max_sigma = b.w;
+    return u;
+}
 
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(NT) k_init(Ctx c, int seed, double tol) {
+// Scalars between the steps.
+//
+// A kernel boundary inside a graph costs 0.5..1.3 us on GB300; a fence, a
+// ticket and a last block that sums and divides cost 4..8 us at the end of
+// every step, and the whole scalar stage of an iteration in one last block
+// 20 us.  (A grid barrier inside one persistent kernel costs 1..1.7 us too.)
+// So no step has a last block.  A step's blocks leave one partial sum each,
+// and every block of the next step sums them again in the same fixed order
+// (so all blocks get the same bits) while its first loads are in flight.  The
+// shifts' recurrences need alpha and omega only: one extra block of K4
+// computes them beside the vector work.  The decisions that need (r, r) and
+// beta (convergence, the switch) are made by every block of K5 for itself;
+// one extra block of K5 records them, replays the histories after a switch
+// and advances the iteration.  Measured, whole solves, with the slice pipeline
+// of SellRows and early launches: n = 512, 6 shifts 1788 -> 974 us; 32^3, 16
+// shifts 5.61 -> 3.22 ms; 97 k rows, 24 shifts 26.4 -> 18.2 ms; 128^3, 32
+// shifts 72.9 -> 61.1 ms; 256^3, 64 shifts 805 -> 711 ms.
+
+// The vector kernels (K2, K4, K5) run one block per SM, of as many threads as
+// that takes (blockDim.x, 128..1024): the sums at a block's start then cost an
+// SM one pass, not one per resident block.
+
+constexpr int MAXW = 32;  // warps of the largest block
+
+// Sum of np partials per set over the block, in a fixed order: the totals are
+// valid in warp 0 (every lane).  NA = 2: both sets at once.  FP64 adds cost 64
+// clocks per warp and SM quarter whatever the active lanes, so warps without
+// partials take no part.  `sh` needs 2 MAXW doubles.  One barrier.
+template <int NA>
+__device__ __forceinline__ double2 sum_parts(const double *p0, const double *p1, unsigned np, double *sh) {
+    const unsigned t = threadIdx.x, w = t >> 5, l = t & 31;
+    const unsigned nw = min(min(blockDim.x >> 5, 16u), (np + 31) >> 5);
+    double x = 0.0, y = 0.0;
+    if (w < nw) {
+        for (unsigned i = t; i < np; i += nw * 32) {
+            x += __ldcg(p0 + i);
+            if (NA == 2) y += __ldcg(p1 + i);
+        }
+        if (NA == 2) x = warp_sum_pair(x, y);
+        else x = warp_sum(x);
+        if (NA == 2 ? (l & 15) == 0 : l == 0) sh[(l >> 4) * MAXW + w] = x;
+    }
+    __syncthreads();
+    double2 r = make_double2(0.0, 0.0);
+    if (w == 0) {
+        double v = 0.0;
+        if ((l & 15) < nw && (NA == 2 || l < 16)) v = sh[(l >> 4) * MAXW + (l & 15)];
+#pragma unroll
+        for (unsigned k = 8; k; k >>= 1)
+            if (k < nw) v += __shfl_xor_sync(0xffffffffu, v, k);
+        r.x = __shfl_sync(0xffffffffu, v, 0);
+        if (NA == 2) r.y = __shfl_sync(0xffffffffu, v, 16);
+    }
+    return r;
+}
+
+// This block's share of one or two dot products into its partial-sum slot.
+__device__ __forceinline__ void store_part(double v, double *sh, double *out) {
+    v = warp_sum(v);
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        const unsigned nw = blockDim.x >> 5;
+        double t = threadIdx.x < nw ? sh[threadIdx.x] : 0.0;
+#pragma unroll
+        for (unsigned k = 16; k; k >>= 1)
+            if (k < nw) t += __shfl_xor_sync(0xffffffffu, t, k);
+        if (threadIdx.x == 0) *out = t;
+    }
+}
+__device__ __forceinline__ void store_part2(double2 v, double *sh, double *out_x, double *out_y) {
+    const unsigned w = threadIdx.x >> 5, l = threadIdx.x & 31, nw = blockDim.x >> 5;
+    const double x = warp_sum_pair(v.x, v.y);
+    if ((l & 15) == 0) sh[(l >> 4) * MAXW + w] = x;
+    __syncthreads();
+    if (w == 0) {
+        const double *p = sh + (l >> 4) * MAXW + (l & 15);
+        double t = (l & 15) < nw ? p[0] : 0.0;
+        if (nw > 16) t += (l & 15) + 16 < nw ? p[16] : 0.0;
+#pragma unroll
+        for (unsigned k = 8; k; k >>= 1)
+            if (k < nw) t += __shfl_xor_sync(0xffffffffu, t, k);
+        if (l == 0) *out_x = t;
+        if (l == 16) *out_y = t;
+    }
+}
+// shared memory of a body is used again by the next virtual block of the CTA
+template <class G>
+__device__ __forceinline__ void body_begin() {
+    if constexpr (!G::hw) __syncthreads();
+    else let_next_start();
+}
+// nothing that an earlier kernel of the iteration writes is read before this
+template <class G>
+__device__ __forceinline__ void body_ready() {
+    if constexpr (G::hw) wait_previous();
+}
+
+// ---------------------------------------------------------------------------
+__global__ void __launch_bounds__(NT) k_init(Ctx c, int seed, double tol, int switching, int inline_ps) {
     hbk_scalars *sc = c.sh.sc;
     const int m = c.sh.m, kcap = c.sh.kcap;
     for (int j = threadIdx.x; j < m; j += NT) {
@@ -80,14 +192,10 @@ __global__ void __launch_bounds__(NT) k_init(Ctx c, int seed, double tol) {
         sc->rr_hat_old = bb;
         sc->rr = bb;
         sc->alpha = sc->omega = sc->beta = 0.0;
-        sc->r_scale = 1.0;
         sc->tol = tol;
         sc->k = 1;
         sc->seed = seed;
-        sc->next_seed = seed;
         sc->n_done = 0;
-        sc->switched = 0;
-        sc->n_active = 0;
         sc->status = 0;
         sc->n_sw = 0;
         sc->loops = 0;
@@ -98,11 +206,15 @@ __global__ void __launch_bounds__(NT) k_init(Ctx c, int seed, double tol) {
         sc->slot_r_old = 0;
         sc->slot_cap = c.v.slot_cap;
         sc->need_ps = 0;
+        sc->rr_pend = 0;
+        sc->switching = switching;
+        sc->inline_ps = inline_ps;
         sc->finished = (m <= 0 || kcap <= 1) ? 1 : 0;
         if (bb == 0.0) {  // b = 0: x = 0 solves every system exactly
             sc->finished = 1;
             sc->n_done = m;
         }
+        sc->cur.active = 0;
     }
 }
 
@@ -122,246 +234,325 @@ __global__ void __launch_bounds__(NT) k_init_coef(Ctx c) {
 }
 
 // ---------------------------------------------------------------------------
-// K1: s = (A + sigma_s I) p_s and (r^, s)
+// K1: s = (A + sigma_s I) p_s and (r^, s).  Block 0 copies the scalars that
+// the iteration's other kernels read (hbk_cur).
 template <int FMT, class G>
 __device__ __forceinline__ void seed_s_body(const Ctx &c, const G &g) {
-    __shared__ double red[2 * NW];
+    __shared__ double red[MAXW];
     hbk_scalars *sc = c.sh.sc;
-    if (stopped(sc)) return;
-    const int seed = sc->seed;
+    body_begin<G>();
+    SpmvRows<FMT, G> rows(c.A, g);
+    rows.start();
+    body_ready<G>();
+    const int fin_flag = __ldcg(&sc->finished), seed = __ldcg(&sc->seed);
+    if (g.b() == 0 && threadIdx.x == 0) {
+        hbk_cur u;
+        u.k = __ldcg(&sc->k), u.seed = seed, u.slots = __ldcg(&sc->slots), u.slot_r_old = __ldcg(&sc->slot_r_old);
+        u.active = fin_flag == 0, u.rr_pend = __ldcg(&sc->rr_pend);
+        u.n_done = __ldcg(&sc->n_done), u.max_sigma = __ldcg(&sc->max_sigma);
+        sc->cur = u;
+    }
+    if (fin_flag) return;
     const double sig = c.sh.sigma[seed];
     const double *__restrict__ ps = seed_p(c, seed);
     const double *__restrict__ rh = c.v.r_hat;
     double *__restrict__ s = c.v.s;
     const bool folded = c.v.sval_shift != nullptr;  // the product already holds sigma p
     double acc = 0.0;
-    auto epi = [&](unsigned r, double ax) {
+    auto pre = [&](unsigned r) { return HBK_LD(G, rh, r); };
+    auto epi = [&](unsigned r, double ax, double hr) {
         const double sv = folded ? ax : fma(sig, HBK_LD(G, ps, r), ax);
         s[r] = sv;
-        acc = fma(HBK_LD(G, rh, r), sv, acc);
+        acc = fma(hr, sv, acc);
     };
-    spmv_rows<FMT>(c.A, ps, epi, g);
-    acc = block_sum(acc, red);
-    if (threadIdx.x == 0) c.sh.partials[g.b()] = acc;
-    if (take_ticket(c.sh.counters + 0, g.nb())) {
-        const double rs = sum_partials(c.sh.partials, g.nb(), red);
-        if (threadIdx.x == 0) {
-            const int k = sc->k;
-            const double a = dvd(sc->rr_hat, rs);
-            sc->rs = rs;
-            c.sh.a_hist[k] = a;
-            sc->alpha = a;
-            if (!fin(a)) {
-                sc->status |= HBK_ST_BREAKDOWN;
-                sc->finished = 1;
-            }
-            c.sh.counters[0] = 0;
-        }
-    }
+    rows.run(ps, pre, epi);
+    store_part(acc, red, parts(c, P_RS) + g.b());
 }
 template <int FMT>
 __global__ void __launch_bounds__(NT) k_seed_s(Ctx c) { seed_s_body<FMT>(c, HwGrid()); }
+template <>
+__global__ void __launch_bounds__(NT, HBK_SELL_MINB) k_seed_s<HBK_FMT_SELL>(Ctx c) {
+    seed_s_body<HBK_FMT_SELL>(c, HwGrid());
+}
 template <>
 __global__ void __launch_bounds__(NT, HBK_HYB_MINB) k_seed_s<HBK_FMT_HYB>(Ctx c) {
     seed_s_body<HBK_FMT_HYB>(c, HwGrid());
 }
 
-// K2: q = r_{k-1} - alpha s (deferred mode: q is a basis slot; its max |q| is
-// kept for the flush)
+// K2: alpha = (r^,r) / (r^,s); q = r_{k-1} - alpha s (deferred mode: q is a
+// basis slot; its max |q| is kept for the flush)
 template <class G>
 __device__ __forceinline__ void seed_q_body(const Ctx &c, const G &g) {
-    __shared__ unsigned long long smx[NW];
-    const hbk_scalars *sc = c.sh.sc;
-    if (stopped(sc)) return;
-    const double a = sc->alpha;
-    const double *__restrict__ ro = vec_r_old(c, sc);
-    const double *__restrict__ s = c.v.s;
-    double *__restrict__ q = vec_q(c, sc);
+    __shared__ double red[2 * MAXW], s_a;
+    __shared__ unsigned long long smx[MAXW];
+    hbk_scalars *sc = c.sh.sc;
+    body_begin<G>();
     const unsigned n = c.v.n;
+    const double *__restrict__ s = c.v.s;
+    size_t i = g.b() * (size_t)blockDim.x + threadIdx.x;
+    body_ready<G>();
+    const hbk_cur u = load_cur(sc);
+    double si = i < n ? HBK_LD(G, s, i) : 0.0;
+    if (!u.active) return;
+    const double *__restrict__ ro = vec_r_old(c, u);
+    double *__restrict__ q = vec_q(c, u);
+    double ri = i < n ? HBK_LD(G, ro, i) : 0.0;
+    double2 t;
+    if (u.rr_pend) {  // (np_p sums, not np_s: two passes)
+        const double rr = sum_parts<1>(parts(c, P_RRS), nullptr, c.np_p, red).x;
+        __syncthreads();
+        t = sum_parts<1>(parts(c, P_RS), nullptr, c.np_s, red);
+        t.y = rr;
+    } else {
+        t = sum_parts<1>(parts(c, P_RS), nullptr, c.np_s, red);
+        t.y = __ldcg(&sc->rr_hat);
+    }
+    if (threadIdx.x < 32) {
+        const double a = dvd(t.y, t.x);
+        if (threadIdx.x == 0) {
+            s_a = a;
+            if (g.b() == 0) {
+                sc->rs = t.x;
+                sc->rr_hat_old = t.y;
+                c.sh.a_hist[u.k] = a;
+                sc->alpha = a;
+                if (!fin(a)) {
+                    sc->status = __ldcg(&sc->status) | HBK_ST_BREAKDOWN;
+                    sc->finished = 1;
+                }
+            }
+        }
+    } else if (threadIdx.x == 32 && g.b() == 0) {  // for the recurrences in K4
+        sc->ba = dvd(__ldcg(c.sh.b_hist + u.k - 1), __ldcg(c.sh.a_hist + u.k - 1));
+    }
+    __syncthreads();
+    const double a = s_a;
+    if (!fin(a)) return;
     unsigned long long mx = 0;
-    for (size_t i = g.b() * (size_t)NT + threadIdx.x; i < n; i += (size_t)g.nb() * NT) {
-        const double qi = fma(-a, HBK_LD(G, s, i), HBK_LD(G, ro, i));
+    const size_t step = (size_t)g.nb() * blockDim.x;
+    while (i < n) {
+        const size_t in = i + step;  // the next element's loads go before this one's store
+        const double sn = in < n ? HBK_LD(G, s, in) : 0.0, rnx = in < n ? HBK_LD(G, ro, in) : 0.0;
+        const double qi = fma(-a, si, ri);
         q[i] = qi;
         const unsigned long long b = abs_bits(qi);
         mx = b > mx ? b : mx;
+        si = sn, ri = rnx, i = in;
     }
-    if (c.v.slot_max) block_max_to(mx, smx, c.v.slot_max + (size_t)sc->slots * HBK_SLOT_SPREAD);
+    if (c.v.slot_max) block_max_to(mx, smx, c.v.slot_max + (size_t)u.slots * HBK_SLOT_SPREAD);
 }
-__global__ void __launch_bounds__(NT) k_seed_q(Ctx c) { seed_q_body(c, HwGrid()); }
+__global__ void __launch_bounds__(1024) k_seed_q(Ctx c) { seed_q_body(c, HwGrid()); }
 
 // K3: y = (A + sigma_s I) q, (q,q) and (q,y)
 template <int FMT, class G>
 __device__ __forceinline__ void seed_y_body(const Ctx &c, const G &g) {
-    __shared__ double red[2 * NW];
-    hbk_scalars *sc = c.sh.sc;
-    if (stopped(sc)) return;
-    const double sig = c.sh.sigma[sc->seed];
-    const double *__restrict__ q = vec_q(c, sc);
+    __shared__ double red[2 * MAXW];
+    body_begin<G>();
+    SpmvRows<FMT, G> rows(c.A, g);
+    rows.start();
+    body_ready<G>();
+    const hbk_cur u = load_cur(c.sh.sc);
+    if (!u.active || !fin(__ldcg(&c.sh.sc->alpha))) return;
+    const double sig = c.sh.sigma[u.seed];
+    const double *__restrict__ q = vec_q(c, u);
     double *__restrict__ y = c.v.y;
     const bool folded = c.v.sval_shift != nullptr;  // the product already holds sigma q
     double2 acc = make_double2(0.0, 0.0);
-    auto epi = [&](unsigned r, double ax) {
-        const double qr = HBK_LD(G, q, r);
+    auto pre = [&](unsigned r) { return HBK_LD(G, q, r); };
+    auto epi = [&](unsigned r, double ax, double qr) {
         const double yv = folded ? ax : fma(sig, qr, ax);
         y[r] = yv;
         acc.x = fma(qr, qr, acc.x);
         acc.y = fma(qr, yv, acc.y);
     };
-    spmv_rows<FMT>(c.A, q, epi, g);
-    acc = block_sum2(acc, red);
-    if (threadIdx.x == 0) {
-        c.sh.partials[g.b()] = acc.x;
-        c.sh.partials[HBK_MAX_GRID + g.b()] = acc.y;
-    }
-    if (take_ticket(c.sh.counters + 1, g.nb())) {
-        const double qq = sum_partials(c.sh.partials, g.nb(), red);
-        const double qy = sum_partials(c.sh.partials + HBK_MAX_GRID, g.nb(), red);
-        if (threadIdx.x == 0) {
-            const int k = sc->k;
-            const double w = dvd(qq, qy);
-            sc->qq = qq;
-            sc->qy = qy;
-            c.sh.w_hist[k] = w;
-            sc->omega = w;
-            sc->rr_hat_old = sc->rr_hat;
-            if (!fin(w) || w == 0.0) {
-                sc->status |= HBK_ST_BREAKDOWN;
-                sc->finished = 1;
-            }
-            c.sh.counters[1] = 0;
-        }
-    }
+    rows.run(q, pre, epi);
+    store_part2(acc, red, parts(c, P_QQ) + g.b(), parts(c, P_QY) + g.b());
 }
 template <int FMT>
 __global__ void __launch_bounds__(NT) k_seed_y(Ctx c) { seed_y_body<FMT>(c, HwGrid()); }
+template <>
+__global__ void __launch_bounds__(NT, HBK_SELL_MINB) k_seed_y<HBK_FMT_SELL>(Ctx c) {
+    seed_y_body<HBK_FMT_SELL>(c, HwGrid());
+}
 template <>
 __global__ void __launch_bounds__(NT, HBK_HYB_MINB) k_seed_y<HBK_FMT_HYB>(Ctx c) {
     seed_y_body<HBK_FMT_HYB>(c, HwGrid());
 }
 
 // ---------------------------------------------------------------------------
-// End of the seed step, run by the last block of K4: beta, the shift
-// recurrences (src/solver_dynamic.c:243-253), the convergence test
-// (:278-303) and the seed switch (:312-359).
-__device__ void seed_step_scalars(const Ctx &c, double rr, double rrh) {
-    __shared__ double s_bk;
-    __shared__ int s_ok, s_sw, s_t, s_nconv, s_nfail;
-    __shared__ double s_best[NW];
-    __shared__ int s_bidx[NW];
+// One extra block of K4: every shift's recurrence (src/solver_dynamic.c:243-253)
+// and this iteration's vector coefficients but for the factor beta, which K5
+// multiplies in.  Four lanes per shift: FP64 division takes 573 clocks of a
+// warp, so a shift's independent quotients go side by side, in two rounds.
+__device__ void shift_recurrences(const Ctx &c, const hbk_cur &u, double wk) {
     hbk_scalars *sc = c.sh.sc;
     const hbk_shifts &S = c.sh;
-    const int k = sc->k, seed = sc->seed, m = S.m, kcap = S.kcap;
-    const int deferred = c.v.deferred;
-    if (threadIdx.x == 0) {
-        sc->rr = rr;
-        if (k < kcap) S.rr_hist[k] = rr;
-        const double bk = mul(dvd(S.a_hist[k], S.w_hist[k]), dvd(rrh, sc->rr_hat_old));
-        S.b_hist[k] = bk;
-        sc->beta = bk;
-        sc->rr_hat = rrh;
-        s_bk = bk;
-        s_ok = fin(bk);
-        s_nfail = 0;
-        if (!s_ok) {
-            sc->status |= HBK_ST_BREAKDOWN;
-            sc->finished = 1;
-        }
-    }
-    __syncthreads();
-    if (!s_ok) return;
-    const double ak = S.a_hist[k], wk = S.w_hist[k], bk = s_bk;
-    const double c_prev = mul(dvd(S.b_hist[k - 1], S.a_hist[k - 1]), ak);
+    const int k = u.k, seed = u.seed, m = S.m, kcap = S.kcap;
+    const double ak = __ldcg(&sc->alpha);
+    const double c_prev = mul(__ldcg(&sc->ba), ak);
     const double sig_s = S.sigma[seed];
-
-    // (1) per-shift recurrences and this iteration's vector coefficients
-    for (int j = threadIdx.x; j < m; j += NT) {
-        double *co = S.coef + (size_t)j * HBK_NCOEF;
-        if (j == seed) {
-            // the seed as a system of its own (deferred mode): pi = zeta = 1,
-            // shift 0.  Its x is not carried in coefficient form: K4 adds
-            // alpha p_s + omega q to its row of X directly, with the
-            // materialised p_s, as the reference's seed step does
-            // (src/solver_dynamic.c:156-210).  In coefficient form p_s would enter
-            // through s = (r_{k-1} - q) / alpha, which cancels when a step makes
-            // little progress; its p coefficients stay (needed after a switch).
-            co[0] = 0.0;
-            co[1] = 0.0;
-            co[2] = dvd(wk, ak);
-            co[3] = -dvd(wk, ak);
-            co[4] = bk;
-            co[5] = 1.0;
-            continue;
+    const unsigned l = threadIdx.x & 31, quad = l & ~3u, part = threadIdx.x & 3;
+    // (whole warps leave together: the shuffles below need all lanes)
+    for (int j0 = 0; j0 + (int)(threadIdx.x & ~31u) / 4 < m; j0 += (int)blockDim.x / 4) {
+        const int j = j0 + (int)(threadIdx.x / 4);
+        const bool here = j < m;
+        const bool is_seed = j == seed;
+        const bool run = here && (is_seed || !__ldcg(S.done + j));
+        double pik1 = 1.0, z = 1.0, e0 = 0.0, sj = sig_s;
+        if (run && !is_seed) {
+            pik1 = __ldcg(S.pi + (size_t)j * kcap + k - 1);
+            z = __ldcg(S.zeta + j);
+            e0 = __ldcg(S.eta + j);
+            sj = S.sigma[j];
         }
-        if (S.done[j]) continue;
-        double *pij = S.pi + (size_t)j * kcap;
-        const double d = sub(sig_s, S.sigma[j]);
-        const double pik1 = pij[k - 1];
-        const double eta = sub(mul(c_prev, S.eta[j]), mul(mul(d, ak), pik1));
+        const double d = sub(sig_s, sj);
+        const double eta = sub(mul(c_prev, e0), mul(mul(d, ak), pik1));
         const double pik = add(eta, pik1);
         const double den = sub(1.0, mul(wk, d));
-        const double aj = mul(dvd(pik1, pik), ak);
-        const double wj = dvd(wk, den);
-        const double z = S.zeta[j];
-        double cn[6];
-        cn[0] = dvd(wj, mul(pik, z));
-        cn[1] = aj;
-        cn[2] = dvd(wj, mul(mul(aj, z), pik));
-        cn[3] = dvd(-wj, mul(mul(aj, z), pik1));
         const double zn = mul(den, z);
-        const double rp = dvd(pik1, pik);
-        cn[4] = mul(mul(rp, rp), bk);
-        cn[5] = dvd(1.0, mul(pik, zn));
-        // Shift breakdown (the reference never tests for it and carries the
-        // inf or nan into x_j): pi_k = 0, 1 - omega_k d = 0, or any scalar of
-        // the update not finite.  The shift stops at its last finite iterate,
-        // counts as finished so the others run on, and records -k.
-        bool ok = pik != 0.0 && den != 0.0 && fin(eta) && fin(zn);
-#pragma unroll
-        for (int t = 0; t < 6; t++) ok = ok && fin(cn[t]);
-        if (!ok) {
-            S.done[j] = 1;
-            S.conv_k[j] = -k;
-            atomicAdd(&s_nfail, 1);
+        // round 1: pi_{k-1} / pi_k, omega_j, 1 / (pi_k zeta_k); the seed as a
+        // system of its own (deferred mode): omega / alpha, alpha / omega
+        double num, by;
+        if (is_seed) num = part == 0 ? wk : ak, by = part == 0 ? ak : wk;
+        else if (part == 0) num = pik1, by = pik;
+        else if (part == 1) num = wk, by = den;
+        else num = 1.0, by = mul(pik, zn);
+        const double q1 = dvd(num, by);
+        const double rp = __shfl_sync(0xffffffffu, q1, quad), wj = __shfl_sync(0xffffffffu, q1, quad + 1);
+        const double c5 = __shfl_sync(0xffffffffu, q1, quad + 2);
+        const double aj = mul(rp, ak);
+        // round 2: omega_j / (pi_k zeta_{k-1}), omega_j / (alpha_j zeta pi_k), -omega_j / (alpha_j zeta pi_{k-1})
+        const double azj = mul(aj, z);
+        const double q2 = dvd(part == 2 ? -wj : wj, part == 0 ? mul(pik, z) : mul(azj, part == 1 ? pik : pik1));
+        const double c0 = __shfl_sync(0xffffffffu, q2, quad), c2 = __shfl_sync(0xffffffffu, q2, quad + 1);
+        const double c3 = __shfl_sync(0xffffffffu, q2, quad + 2);
+        if (!here || part) continue;
+        double *co = S.coef + (size_t)j * HBK_NCOEF;
+        if (is_seed) {
+            // pi = zeta = 1, shift 0.  Its x is not carried in coefficient
+            // form: K5 adds alpha p_s + omega q to its row of X directly, with
+            // the materialised p_s, as the reference's seed step does
+            // (src/solver_dynamic.c:156-210).  In coefficient form p_s would
+            // enter through s = (r_{k-1} - q) / alpha, which cancels when a
+            // step makes little progress; its p coefficients stay (needed
+            // after a switch).
+            co[0] = co[1] = 0.0;
+            co[2] = rp;  // omega / alpha
+            co[3] = -rp;
+            co[4] = co[5] = 1.0;
+            sc->aw = wj;  // alpha / omega
+            S.live[j] = __ldcg(S.done + j) ? 0 : 1;
             continue;
         }
-        pij[k] = pik;
+        if (!run) {
+            S.live[j] = 0;
+            continue;
+        }
+        const double c4 = mul(rp, rp);
+        // Shift breakdown (the reference never tests for it and carries the
+        // inf or nan into x_j): pi_k = 0, 1 - omega_k d = 0, or any scalar of
+        // the update not finite (K5 tests beta c4).  The shift stops at its
+        // last finite iterate, counts as finished so the others run on, and
+        // records -k.
+        const bool ok = !is_zero(pik) && !is_zero(den) && fin(eta) && fin(zn) && fin(c0) && fin(aj) && fin(c2) && fin(c3) &&
+                        fin(c4) && fin(c5);
+        S.live[j] = ok ? 1 : 2;
+        if (!ok) continue;
+        S.pi[(size_t)j * kcap + k] = pik;
         S.eta[j] = eta;
         S.zeta[j] = zn;
-#pragma unroll
-        for (int t = 0; t < 6; t++) co[t] = cn[t];
+        co[0] = c0;
+        co[1] = aj;
+        co[2] = c2;
+        co[3] = c3;
+        co[4] = c4;
+        co[5] = c5;
+    }
+}
+
+// K4: omega = (q,q) / (q,y); r_k = q - omega y; (r,r), (r^,r); the extra block:
+// the shifts' recurrences
+template <class G>
+__device__ __forceinline__ void seed_update_body(const Ctx &c, const G &g) {
+    __shared__ double sh[2 * MAXW], s_w;
+    __shared__ unsigned long long smx[MAXW];
+    hbk_scalars *sc = c.sh.sc;
+    body_begin<G>();
+    const unsigned n = c.v.n;
+    const double *__restrict__ y = c.v.y;
+    const double *__restrict__ rh = c.v.r_hat;
+    const bool extra = g.extra();
+    size_t i = extra ? (size_t)n : g.b() * (size_t)blockDim.x + threadIdx.x;
+    double hi = i < n ? HBK_LD(G, rh, i) : 0.0;
+    body_ready<G>();
+    const hbk_cur u = load_cur(sc);
+    double yi = i < n ? HBK_LD(G, y, i) : 0.0;
+    if (!u.active || !fin(__ldcg(&sc->alpha))) return;
+    const double *__restrict__ q = vec_q(c, u);
+    double *__restrict__ rn = vec_r_new(c, u);
+    double qi = i < n ? HBK_LD(G, q, i) : 0.0;
+    const double2 t = sum_parts<2>(parts(c, P_QQ), parts(c, P_QY), c.np_y, sh);
+    if (threadIdx.x < 32) {
+        const double w = dvd(t.x, t.y);
+        if (threadIdx.x == 0) {
+            s_w = w;
+            if (extra) {
+                sc->qq = t.x;
+                sc->qy = t.y;
+                c.sh.w_hist[u.k] = w;
+                sc->omega = w;
+                if (!fin(w) || is_zero(w)) {
+                    sc->status = __ldcg(&sc->status) | HBK_ST_BREAKDOWN;
+                    sc->finished = 1;
+                }
+            }
+        }
     }
     __syncthreads();
-
-    // (2) the systems updated this iteration, in index order
-    if (threadIdx.x == 0) {
-        int na = 0;
-        if (deferred) S.act_list[na++] = seed;
-        for (int j = 0; j < m; j++)
-            if (j != seed && !S.done[j]) S.act_list[na++] = j;
-        sc->n_active = na;
-        if (k < kcap) S.act_hist[k] = na - deferred;
+    const double w = s_w;
+    if (!fin(w) || is_zero(w)) return;
+    if (extra) {
+        shift_recurrences(c, u, w);
+        return;
     }
-    __syncthreads();
+    double2 acc = make_double2(0.0, 0.0);
+    unsigned long long mx = 0;
+    const size_t step = (size_t)g.nb() * blockDim.x;
+    while (i < n) {
+        const size_t in = i + step;  // the next element's loads go before this one's store
+        const double yn = in < n ? HBK_LD(G, y, in) : 0.0, hn = in < n ? HBK_LD(G, rh, in) : 0.0;
+        const double qn = in < n ? HBK_LD(G, q, in) : 0.0;
+        const double r = fma(-w, yi, qi);
+        rn[i] = r;
+        acc.x = fma(r, r, acc.x);
+        acc.y = fma(hi, r, acc.y);
+        const unsigned long long b = abs_bits(r);
+        mx = b > mx ? b : mx;
+        yi = yn, hi = hn, qi = qn, i = in;
+    }
+    if (c.v.slot_max) block_max_to(mx, smx, c.v.slot_max + (size_t)(u.slots + 1) * HBK_SLOT_SPREAD);  // r_k
+    store_part2(acc, sh, parts(c, P_RR) + g.b(), parts(c, P_RRH) + g.b());
+}
+__global__ void __launch_bounds__(1024) k_seed_update(Ctx c) { seed_update_body(c, HwGridX{1}); }
 
-    // (3) convergence test on the recursive residual; argmax of |1/(zeta pi)|
-    //     over the systems still running, strict '>' from 1.0 (lowest index
-    //     wins an exact tie)
-    const double thr = mul(mul(sc->tol, sc->tol), sc->bb);
+// ---------------------------------------------------------------------------
+// Argmax of |1/(zeta_j pi_j)| over the systems still running after this
+// iteration's test, strict '>' from 1.0, lowest index on an exact tie (the
+// reference's order, src/solver_dynamic.c:278-303); run by warp 0, result in
+// every lane; -1: none.
+__device__ int running_argmax(const hbk_shifts &S, int seed, double bk, double rr, double thr) {
     double best = 1.0;
-    int bidx = -1, nconv = 0;
-    for (int j = threadIdx.x; j < m; j += NT) {
-        if (S.done[j]) continue;
-        const double a = (j == seed) ? 1.0 : fabs(dvd(1.0, mul(S.zeta[j], S.pi[(size_t)j * kcap + k])));
-        if (mul(mul(a, a), rr) <= thr) {
-            S.done[j] = 1;
-            S.conv_k[j] = k;
-            nconv++;
-        } else if (a > best) {
+    int bidx = -1;
+    for (int j = threadIdx.x; j < S.m; j += 32) {
+        if (j == seed || __ldcg(S.live + j) != 1) continue;
+        const double *co = S.coef + (size_t)j * HBK_NCOEF;
+        if (!fin(mul(__ldcg(co + 4), bk))) continue;
+        const double a = fabs(__ldcg(co + 5));
+        if (mul(mul(a, a), rr) > thr && a > best) {
             best = a;
             bidx = j;
         }
     }
-    // block argmax: larger value wins, lower index on ties
 #pragma unroll
     for (int o = 16; o; o >>= 1) {
         const double ob = __shfl_xor_sync(0xffffffffu, best, o);
@@ -371,54 +562,184 @@ __device__ void seed_step_scalars(const Ctx &c, double rr, double rrh) {
             bidx = oi;
         }
     }
-    if ((threadIdx.x & 31) == 0) {
-        s_best[threadIdx.x >> 5] = best;
-        s_bidx[threadIdx.x >> 5] = bidx;
+    return bidx;
+}
+
+// What an iteration's end decides, the same in every block of K5.
+struct StepEnd {
+    double bk, bw, rr, rrh, thr, rsc;  // bw = -beta omega
+    int ok;      // beta is finite
+    int n_done;  // finished systems, this iteration's included
+    int sw, t;   // seed switch to system t; rsc = 1 / (zeta_t pi_t)
+};
+
+// beta from K4's partial sums, the convergence test on the recursive residual
+// (src/solver_dynamic.c:278-303) and the decision to switch (:312-326).
+// Every thread returns the same.
+__device__ __forceinline__ StepEnd step_end(const Ctx &c, const hbk_cur &u, double wk, double *sh) {
+    __shared__ double s_bk, s_bw, s_rr, s_rrh, s_thr, s_rsc;
+    __shared__ int s_t;
+    const hbk_scalars *sc = c.sh.sc;
+    const hbk_shifts &S = c.sh;
+    const int m = S.m;
+    // loaded before the sums are known
+    int live = 0;
+    double c4 = 1.0, c5 = 1.0;
+    if ((int)threadIdx.x < m) {
+        live = __ldcg(S.live + threadIdx.x);
+        const double2 cc = __ldcg(reinterpret_cast<const double2 *>(S.coef + (size_t)threadIdx.x * HBK_NCOEF + 4));
+        c4 = cc.x;
+        c5 = cc.y;
     }
-    if (threadIdx.x == 0) s_nconv = 0;
+    const double aw = __ldcg(&sc->aw), rho = __ldcg(&sc->rr_hat_old), tol = __ldcg(&sc->tol), bb = __ldcg(&sc->bb);
+    const int switching = __ldcg(&sc->switching);
+    const double2 t = sum_parts<2>(parts(c, P_RR), parts(c, P_RRH), c.np_r, sh);
+    if (threadIdx.x < 32) {
+        const double bk = mul(aw, dvd(t.y, rho));
+        if (threadIdx.x == 0) s_bk = bk, s_bw = -mul(bk, wk), s_rr = t.x, s_rrh = t.y;
+    } else if (threadIdx.x < 64) {  // (one warp: every other would pay for the two operations too)
+        const double thr = mul(mul(tol, tol), bb);
+        if (threadIdx.x == 32) s_thr = thr;
+    }
     __syncthreads();
-    if (nconv) atomicAdd(&s_nconv, nconv);
+    StepEnd e;
+    e.bk = s_bk;
+    e.rr = s_rr;
+    e.rrh = s_rrh;
+    e.ok = fin(e.bk);
+    e.sw = 0;
+    e.t = u.max_sigma;
+    e.rsc = 1.0;
+    e.n_done = u.n_done;
+    e.thr = s_thr;
+    e.bw = s_bw;
+    if (!e.ok) return e;
+    int seed_done = 0;
+    for (int j0 = 0; j0 < m; j0 += (int)blockDim.x) {
+        const int j = j0 + (int)threadIdx.x;
+        if (j0 && j < m) {
+            live = __ldcg(S.live + j);
+            c4 = __ldcg(S.coef + (size_t)j * HBK_NCOEF + 4);
+            c5 = __ldcg(S.coef + (size_t)j * HBK_NCOEF + 5);
+        }
+        int now = 0;
+        if (j < m && live) {
+            if (j == u.seed) now = e.rr <= e.thr;
+            else now = live == 2 || !fin(mul(c4, e.bk)) || mul(mul(c5, c5), e.rr) <= e.thr;
+        }
+        seed_done |= j == u.seed && (now || !live);
+        e.n_done += __syncthreads_count(now);
+    }
+    if (!switching) return e;
+    if (!__syncthreads_or(seed_done) || e.n_done >= m) return e;
+    if (threadIdx.x < 32) {
+        const int b = running_argmax(S, u.seed, e.bk, e.rr, e.thr);
+        if (threadIdx.x == 0) {
+            s_t = b >= 0 ? b : u.max_sigma;
+            s_rsc = __ldcg(S.coef + (size_t)s_t * HBK_NCOEF + 5);  // 1 / (zeta_t pi_t)
+        }
+    }
     __syncthreads();
+    e.sw = 1;
+    e.t = s_t;
+    e.rsc = s_rsc;
+    return e;
+}
+
+// The extra block of K5: records the iteration, replays the histories after a
+// switch (src/solver_dynamic.c:312-359) and advances the iteration.
+__device__ void record_step(const Ctx &c, const hbk_cur &u, const StepEnd &e) {
+    hbk_scalars *sc = c.sh.sc;
+    const hbk_shifts &S = c.sh;
+    const int k = u.k, seed = u.seed, m = S.m, kcap = S.kcap;
+    int nfail = 0, nact = 0;
+    for (int j = threadIdx.x; j < m; j += blockDim.x) {
+        const int live = __ldcg(S.live + j);
+        if (!live) continue;
+        const double *co = S.coef + (size_t)j * HBK_NCOEF;
+        const double a = j == seed ? 1.0 : __ldcg(co + 5);
+        if (j != seed && (live == 2 || !fin(mul(__ldcg(co + 4), e.bk)))) {
+            S.done[j] = 1;
+            S.conv_k[j] = -k;
+            nfail = 1;
+            continue;
+        }
+        if (j != seed) nact++;
+        if (mul(mul(a, a), e.rr) <= e.thr) {
+            S.done[j] = 1;
+            S.conv_k[j] = k;
+        }
+    }
+    __shared__ int s_nact;
+    if (threadIdx.x == 0) s_nact = 0;
+    nfail = __syncthreads_or(nfail);
+    if (nact) atomicAdd(&s_nact, nact);
+    __syncthreads();
+    int top = -1;
+    if (threadIdx.x < 32) top = running_argmax(S, seed, e.bk, e.rr, e.thr);
     if (threadIdx.x == 0) {
-        double bb2 = 1.0;
-        int bi = -1;
-        for (int w = 0; w < NW; w++) {
-            const int oi = s_bidx[w];
-            const double ob = s_best[w];
-            if (oi >= 0 && (bi < 0 || ob > bb2 || (ob == bb2 && oi < bi))) {
-                bb2 = ob;
-                bi = oi;
+        if (k < kcap) {
+            S.rr_hist[k] = e.rr;
+            S.act_hist[k] = s_nact;
+        }
+        S.b_hist[k] = e.bk;
+        sc->beta = e.bk;
+        sc->rr = e.rr;
+        sc->rr_hat = e.rrh;
+        sc->rr_pend = e.sw;
+        sc->n_done = e.n_done;
+        if (top >= 0) sc->max_sigma = top;
+        int status = __ldcg(&sc->status);
+        if (nfail) status |= HBK_ST_SHIFT_FAIL;
+        int finished = e.n_done >= m || k + 1 >= kcap;
+        if (e.sw) {
+            const int n_sw = __ldcg(&sc->n_sw);
+            if (n_sw < m) {
+                S.sw_k[n_sw] = k;
+                S.sw_seed[n_sw] = e.t;
+            }
+            sc->n_sw = n_sw + 1;
+            sc->seed = e.t;
+        }
+        if (c.v.deferred) {
+            const int slots = u.slots + (e.sw ? 3 : 2);
+            sc->slot_r_old = slots - 1;  // r_k (after a switch the rescaled r_k)
+            sc->slots = slots;
+            if (e.sw) {
+                sc->need_ps = 1;
+                if (!__ldcg(&sc->inline_ps)) {
+                    status |= HBK_ST_NEED_PS;
+                    finished = 1;  // the host has the new seed's p formed and resumes
+                }
+            }
+            if (!(e.n_done >= m || k + 1 >= kcap) && slots + 3 > __ldcg(&sc->slot_cap)) {
+                status |= HBK_ST_BASIS_FULL;
+                finished = 1;  // the host flushes the basis and resumes
             }
         }
-        if (bi >= 0) sc->max_sigma = bi;
-        sc->n_done += s_nconv + s_nfail;
-        if (s_nfail) sc->status |= HBK_ST_SHIFT_FAIL;
-        s_sw = (sc->switching && S.done[seed] && sc->n_done < m) ? 1 : 0;
-        s_t = sc->max_sigma;
-        sc->next_seed = s_sw ? s_t : seed;
-        sc->switched = s_sw;
-        sc->r_scale = 1.0;
+        sc->status = status;
+        sc->k = k + 1;
+        sc->finished = finished;
     }
+    if (!e.sw) return;
+    // rescale the seed history, replay eta/pi/zeta of every running shift
+    // relative to sigma_t
     __syncthreads();
-    if (!s_sw) return;
-
-    // (4) seed switch to t: rescale the seed history, rescale r (K5), replay
-    //     eta/pi/zeta of every running shift relative to sigma_t
-    const int t = s_t;
+    const int t = e.t;
+    const double sig_s = S.sigma[seed], sig_t = S.sigma[t];
     const double *pit = S.pi + (size_t)t * kcap;
-    const double dst = sub(sig_s, S.sigma[t]);
-    if (threadIdx.x == 0) sc->r_scale = dvd(1.0, mul(S.zeta[t], pit[k]));
-    for (int i = 1 + threadIdx.x; i <= k; i += NT) {
-        const double rp = dvd(pit[i - 1], pit[i]);
-        S.a_hist[i] = mul(rp, S.a_hist[i]);
-        S.b_hist[i] = mul(mul(rp, rp), S.b_hist[i]);
-        S.w_hist[i] = dvd(S.w_hist[i], sub(1.0, mul(S.w_hist[i], dst)));
+    const double dst = sub(sig_s, sig_t);
+    for (int i = 1 + threadIdx.x; i <= k; i += blockDim.x) {
+        const double rp = dvd(__ldcg(pit + i - 1), __ldcg(pit + i));
+        S.a_hist[i] = mul(rp, __ldcg(S.a_hist + i));
+        S.b_hist[i] = mul(mul(rp, rp), i == k ? e.bk : __ldcg(S.b_hist + i));
+        const double wi = __ldcg(S.w_hist + i);
+        S.w_hist[i] = dvd(wi, sub(1.0, mul(wi, dst)));
     }
     __syncthreads();
-    for (int i = 1 + threadIdx.x; i <= k; i += NT) S.ratio[i] = mul(dvd(S.b_hist[i - 1], S.a_hist[i - 1]), S.a_hist[i]);
+    for (int i = 1 + threadIdx.x; i <= k; i += blockDim.x) S.ratio[i] = mul(dvd(S.b_hist[i - 1], S.a_hist[i - 1]), S.a_hist[i]);
     __syncthreads();
-    const double sig_t = S.sigma[t];
-    for (int j = threadIdx.x; j < m; j += NT) {
+    for (int j = threadIdx.x; j < m; j += blockDim.x) {
         if (S.done[j] || j == t) {
             S.eta[j] = 0.0;
             S.zeta[j] = 1.0;
@@ -426,269 +747,316 @@ __device__ void seed_step_scalars(const Ctx &c, double rr, double rrh) {
         }
         double *pij = S.pi + (size_t)j * kcap;
         const double d = sub(sig_t, S.sigma[j]);
-        double e = 0.0, z = 1.0, pprev = pij[0];
+        double eta = 0.0, z = 1.0, pprev = __ldcg(pij);
         for (int i = 1; i <= k; i++) {
-            e = sub(mul(S.ratio[i], e), mul(mul(d, S.a_hist[i]), pprev));
-            const double pc = add(e, pprev);
+            eta = sub(mul(S.ratio[i], eta), mul(mul(d, S.a_hist[i]), pprev));
+            const double pc = add(eta, pprev);
             pij[i] = pc;
             z = mul(sub(1.0, mul(S.w_hist[i], d)), z);
             pprev = pc;
         }
-        S.eta[j] = e;
+        S.eta[j] = eta;
         S.zeta[j] = z;
     }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        S.eta[t] = 0.0;
-        S.zeta[t] = 1.0;
-        if (sc->n_sw < m) {
-            S.sw_k[sc->n_sw] = k;
-            S.sw_seed[sc->n_sw] = t;
-        }
-        sc->n_sw++;
-    }
 }
 
-// K4: x_s += alpha p_s + omega q ; r_k = q - omega y ; (r,r), (r^,r)
-// (at least 4 CTAs per SM: the streaming loop needs the warps; the scalar
-// stage that runs in one CTA per iteration may spill)
+// beta not finite: the solve stops after the seed's x of this iteration
 template <class G>
-__device__ __forceinline__ void seed_update_body(const Ctx &c, const G &g) {
-    __shared__ double sh[2 * NW];
-    __shared__ unsigned long long smx[NW];
+__device__ __forceinline__ void seed_x_only(const Ctx &c, const hbk_cur &u, const G &g) {
     hbk_scalars *sc = c.sh.sc;
-    if (stopped(sc)) return;
-    const double a = sc->alpha, w = sc->omega;
-    const int seed = sc->seed;
-    const unsigned n = c.v.n;
-    const double *__restrict__ ps = seed_p(c, seed);
-    const double *__restrict__ q = vec_q(c, sc);
-    const double *__restrict__ y = c.v.y;
-    const double *__restrict__ rh = c.v.r_hat;
-    double *__restrict__ rn = vec_r_new(c, sc);
-    double2 acc = make_double2(0.0, 0.0);
-    unsigned long long mx = 0;
-    // the seed's x in both shift modes (in deferred mode its x coefficients
-    // are kept at zero, so the basis flushes leave it as it is; there x_j are
-    // panel-major)
-    const bool dm = c.v.deferred != 0;
-    double *__restrict__ xrow = dm ? c.v.Xp : c.v.X + (size_t)seed * ldn(n);
-    const int pm = c.v.pm;
-    for (size_t i = g.b() * (size_t)NT + threadIdx.x; i < n; i += (size_t)g.nb() * NT) {
-        const double qi = HBK_LD(G, q, i);
-        double *xi = dm ? xrow + panel_idx(seed, (unsigned)i, pm) : xrow + i;
-        *xi = fma(w, qi, fma(a, HBK_LD(G, ps, i), HBK_LD(G, xi, 0)));
-        const double r = fma(-w, HBK_LD(G, y, i), qi);
-        rn[i] = r;
-        acc.x = fma(r, r, acc.x);
-        acc.y = fma(HBK_LD(G, rh, i), r, acc.y);
-        const unsigned long long b = abs_bits(r);
-        mx = b > mx ? b : mx;
-    }
-    if (c.v.slot_max) block_max_to(mx, smx, c.v.slot_max + (size_t)(sc->slots + 1) * HBK_SLOT_SPREAD);  // r_k
-    acc = block_sum2(acc, sh);
-    if (threadIdx.x == 0) {
-        c.sh.partials[g.b()] = acc.x;
-        c.sh.partials[HBK_MAX_GRID + g.b()] = acc.y;
-    }
-    if (take_ticket(c.sh.counters + 2, g.nb())) {
-        const double rr = sum_partials(c.sh.partials, g.nb(), sh);
-        const double rrh = sum_partials(c.sh.partials + HBK_MAX_GRID, g.nb(), sh);
-        seed_step_scalars(c, rr, rrh);
-        if (threadIdx.x == 0) c.sh.counters[2] = 0;
-    }
-}
-__global__ void __launch_bounds__(NT, 4) k_seed_update(Ctx c) { seed_update_body(c, HwGrid()); }
-
-// End of an iteration (one thread): apply the switch, advance k, test the loop.
-__device__ void finish_iteration(const Ctx &c, hbk_scalars *sc, double rrh_scaled) {
-    if (sc->switched) {
-        sc->rr_hat = rrh_scaled;
-        sc->seed = sc->next_seed;
-        sc->switched = 0;
-        if (c.v.deferred) {
-            sc->slot_r_old = sc->slots + 2;  // the rescaled r_k
-            sc->slots += 3;
-            sc->need_ps = 1;
+    if (g.extra()) {
+        if (threadIdx.x == 0) {
+            sc->status = __ldcg(&sc->status) | HBK_ST_BREAKDOWN;
+            sc->finished = 1;
         }
-    } else if (c.v.deferred) {
-        sc->slot_r_old = sc->slots + 1;
-        sc->slots += 2;
+        return;
     }
-    sc->k += 1;
-    if (sc->n_done >= sc->m || sc->k >= sc->kcap) sc->finished = 1;
-    if (c.v.deferred && !sc->finished && sc->slots + 3 > sc->slot_cap) {
-        sc->status |= HBK_ST_BASIS_FULL;
-        sc->finished = 1;  // the host flushes the basis and resumes
+    const double a = __ldcg(&sc->alpha), w = __ldcg(&sc->omega);
+    const unsigned n = c.v.n;
+    const double *ps = seed_p(c, u.seed), *q = vec_q(c, u);
+    for (size_t i = g.b() * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)g.nb() * blockDim.x) {
+        double *xi = c.v.deferred ? c.v.Xp + panel_idx(u.seed, (unsigned)i, c.v.pm)
+                                  : c.v.X + (size_t)u.seed * ldn(n) + i;
+        *xi = fma(w, HBK_LD(G, q, i), fma(a, HBK_LD(G, ps, i), HBK_LD(G, xi, 0)));
     }
 }
 
-// K5 (incremental): p_s, then every running shift's x_j and p_j in one pass
-// over q, r_{k-1}, r_k (src/solver_dynamic.c:208-210, :248-255)
+// K5 (incremental): the seed's x_s and p_s, then every running shift's x_j and
+// p_j in one pass over q, r_{k-1}, r_k (src/solver_dynamic.c:200-210, :248-255);
+// r_k rescaled on a switch.  The first element's vectors and, up to MAXS
+// shifts, the coefficients are loaded before the iteration's end is decided,
+// and each shift's x_j, p_j before the shift ahead of it is stored.
 template <int MAXS, class G>
 __device__ __forceinline__ void shift_update_body(const Ctx &c, const G &g) {
     __shared__ double s_co[MAXS * 6];
-    __shared__ int s_j[MAXS];
-    __shared__ double sh[NW];
+    __shared__ int s_j[MAXS], s_cnt, s_next;
+    __shared__ unsigned s_act[MAXS / 32];
+    __shared__ double sh[2 * MAXW];
     hbk_scalars *sc = c.sh.sc;
-    if (stopped(sc)) return;
-    const int seed = sc->seed, na = sc->n_active, k = sc->k;
-    const double bk = sc->beta, wk = sc->omega, bw = -mul(bk, wk);
-    const int sw = sc->switched;
-    const double rsc = sc->r_scale;
+    body_begin<G>();
+    body_ready<G>();
+    const hbk_cur u = load_cur(sc);
+    const double ak = __ldcg(&sc->alpha), wk = __ldcg(&sc->omega);
+    const int m = c.sh.m;
+    const unsigned t = threadIdx.x;
+    const bool once = m <= MAXS;
+    int live = 0;
+    double co[6];
+    if (once && t < MAXS) {
+        const double2 *p = reinterpret_cast<const double2 *>(c.sh.coef + (size_t)t * HBK_NCOEF);
+        if ((int)t < m) {
+            live = __ldcg(c.sh.live + t);
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                const double2 v = __ldcg(p + k);
+                co[2 * k] = v.x, co[2 * k + 1] = v.y;
+            }
+        }
+    }
+    if (!u.active || !fin(ak) || !fin(wk) || is_zero(wk)) return;
+    const int seed = u.seed, k = u.k;
     const unsigned n = c.v.n;
-    const size_t ld = ldn(n);
+    const size_t ld = ldn(n), step = (size_t)g.nb() * blockDim.x;
+    double *__restrict__ xs = c.v.X + (size_t)seed * ld;
     double *__restrict__ ps = c.v.P + (size_t)seed * ld;
     const double *__restrict__ q = c.v.q;
     const double *__restrict__ s = c.v.s;
     const double *__restrict__ ro = c.v.rbuf[(k - 1) & 1];
     double *__restrict__ rn = c.v.rbuf[k & 1];
     const double *__restrict__ rh = c.v.r_hat;
+    size_t i = g.extra() ? (size_t)n : g.b() * (size_t)blockDim.x + t;
+    double qi = 0.0, oi = 0.0, ri = 0.0, pi = 0.0, xi = 0.0, si = 0.0;
+    if (i < n) {
+        qi = HBK_LD(G, q, i), oi = HBK_LD(G, ro, i), ri = HBK_LD(G, rn, i);
+        pi = HBK_LD(G, ps, i), xi = HBK_LD(G, xs, i), si = HBK_LD(G, s, i);
+    }
+    const StepEnd e = step_end(c, u, wk, sh);
+    if (!e.ok) {
+        seed_x_only(c, u, g);
+        return;
+    }
+    if (g.extra()) {
+        record_step(c, u, e);
+        return;
+    }
+    const double bk = e.bk, bw = e.bw;
     double acc = 0.0;
-    for (int base = 0; base < na || base == 0; base += MAXS) {
-        const int cnt = min(MAXS, na - base);
-        for (int a = threadIdx.x; a < cnt; a += NT) {
-            const int j = c.sh.act_list[base + a];
-            s_j[a] = j;
-            const double *co = c.sh.coef + (size_t)j * HBK_NCOEF;
+    for (int next = 0, first = 1;; first = 0) {
+        // up to MAXS running shifts in index order
+        int cnt;
+        if (once) {
+            bool act = false;
+            if (t < MAXS) {
+                if ((int)t < m && live == 1 && (int)t != seed) {
+                    co[4] = mul(co[4], bk);
+                    act = fin(co[4]);
+                }
+                const unsigned b = __ballot_sync(0xffffffffu, act);
+                if ((t & 31) == 0) s_act[t / 32] = b;
+            }
+            __syncthreads();
+            cnt = 0;
+            unsigned at = 0;
 #pragma unroll
-            for (int t = 0; t < 6; t++) s_co[a * 6 + t] = co[t];
+            for (int w = 0; w < MAXS / 32; ++w) {
+                if ((unsigned)w == t / 32) at = cnt + __popc(s_act[w] & ((1u << (t & 31)) - 1u));
+                cnt += __popc(s_act[w]);
+            }
+            if (act) {
+                s_j[at] = (int)t;
+#pragma unroll
+                for (int v = 0; v < 6; ++v) s_co[at * 6 + v] = co[v];
+            }
+            next = m;
+        } else {
+            if (t < 32) {
+                int found = 0, j0 = next;
+                for (; j0 < m && found + 32 <= MAXS; j0 += 32) {
+                    const int j = j0 + (int)t;
+                    const bool act = j < m && j != seed && __ldcg(c.sh.live + j) == 1 &&
+                                     fin(mul(__ldcg(c.sh.coef + (size_t)j * HBK_NCOEF + 4), bk));
+                    const unsigned b = __ballot_sync(0xffffffffu, act);
+                    if (act) s_j[found + __popc(b & ((1u << t) - 1u))] = j;
+                    found += __popc(b);
+                }
+                if (t == 0) s_cnt = found, s_next = j0;
+            }
+            __syncthreads();
+            cnt = s_cnt;
+            next = s_next;
+            for (int a = (int)t; a < cnt * 6; a += (int)blockDim.x) {
+                const double v = __ldcg(c.sh.coef + (size_t)s_j[a / 6] * HBK_NCOEF + a % 6);
+                s_co[a] = a % 6 == 4 ? mul(v, bk) : v;
+            }
+            if (!first) {
+                i = g.b() * (size_t)blockDim.x + t;
+                if (i < n) qi = HBK_LD(G, q, i), oi = HBK_LD(G, ro, i), ri = HBK_LD(G, rn, i);
+            }
         }
         __syncthreads();
-        for (size_t i = g.b() * (size_t)NT + threadIdx.x; i < n; i += (size_t)g.nb() * NT) {
-            const double qi = HBK_LD(G, q, i), oi = HBK_LD(G, ro, i), ri = HBK_LD(G, rn, i);
-            if (base == 0) ps[i] = fma(bw, HBK_LD(G, s, i), fma(bk, HBK_LD(G, ps, i), ri));
-            for (int a = 0; a < cnt; a++) {
-                const double *co = s_co + a * 6;
-                double *xj = c.v.X + (size_t)s_j[a] * ld;
-                double *pj = c.v.P + (size_t)s_j[a] * ld;
-                double x = HBK_LD(G, xj, i), p = HBK_LD(G, pj, i);
-                x = fma(co[0], qi, x);
-                x = fma(co[1], p, x);
-                p = fma(co[2], qi, p);
-                p = fma(co[3], oi, p);
-                p = co[4] * p;
-                p = fma(co[5], ri, p);
-                xj[i] = x;
-                pj[i] = p;
+        while (i < n) {
+            double xn = 0.0, pn = 0.0;
+            if (cnt) {
+                xn = HBK_LD(G, c.v.X + (size_t)s_j[0] * ld, i);
+                pn = HBK_LD(G, c.v.P + (size_t)s_j[0] * ld, i);
             }
-            if (sw && base + MAXS >= na) {
-                const double rs = ri * rsc;
+            if (first) {
+                xs[i] = fma(wk, qi, fma(ak, pi, xi));
+                ps[i] = fma(bw, si, fma(bk, pi, ri));
+            }
+            for (int a = 0; a < cnt; a++) {
+                const double *cf = s_co + a * 6;
+                double x = xn, p = pn;
+                if (a + 1 < cnt) {
+                    xn = HBK_LD(G, c.v.X + (size_t)s_j[a + 1] * ld, i);
+                    pn = HBK_LD(G, c.v.P + (size_t)s_j[a + 1] * ld, i);
+                }
+                x = fma(cf[0], qi, x);
+                x = fma(cf[1], p, x);
+                p = fma(cf[2], qi, p);
+                p = fma(cf[3], oi, p);
+                p = cf[4] * p;
+                p = fma(cf[5], ri, p);
+                c.v.X[(size_t)s_j[a] * ld + i] = x;
+                c.v.P[(size_t)s_j[a] * ld + i] = p;
+            }
+            if (e.sw && next >= m) {
+                const double rs = ri * e.rsc;
                 rn[i] = rs;
                 acc = fma(HBK_LD(G, rh, i), rs, acc);
             }
+            i += step;
+            if (i < n) {
+                qi = HBK_LD(G, q, i), oi = HBK_LD(G, ro, i), ri = HBK_LD(G, rn, i);
+                if (first) pi = HBK_LD(G, ps, i), xi = HBK_LD(G, xs, i), si = HBK_LD(G, s, i);
+            }
         }
+        if (next >= m) break;
         __syncthreads();
-        if (na <= MAXS) break;
     }
-    acc = block_sum(acc, sh);
-    if (threadIdx.x == 0) c.sh.partials[g.b()] = acc;
-    if (take_ticket(c.sh.counters + 3, g.nb())) {
-        const double rrh = sum_partials(c.sh.partials, g.nb(), sh);
-        if (threadIdx.x == 0) {
-            finish_iteration(c, sc, rrh);
-            c.sh.counters[3] = 0;
-        }
+    if (e.sw) {
+        __syncthreads();
+        store_part(acc, sh, parts(c, P_RRS) + g.b());
     }
 }
 template <int MAXS>
-__global__ void __launch_bounds__(NT) k_shift_update(Ctx c) { shift_update_body<MAXS>(c, HwGrid()); }
+__global__ void __launch_bounds__(1024) k_shift_update(Ctx c) { shift_update_body<MAXS>(c, HwGridX{1}); }
 
-// K5 (deferred): p_s update; on a switch the rescaled r_k goes to a new slot
+// Deferred mode: coefficient update of every running system over the basis
+// slots in use, items it0, it0 + step, ... of m x L.  Per coefficient the
+// operations follow the vector update's order (x += c0 q; x += c1 p;
+// p += c2 q; p += c3 r_{k-1}; p *= beta_j; p += c5 r_k).
+template <class G>
+__device__ __forceinline__ void coef_update(const Ctx &c, const hbk_cur &u, double bk, unsigned it0, unsigned step) {
+    const int sq = u.slots, sr = u.slots + 1, so = u.slot_r_old;
+    const unsigned L = (unsigned)u.slots + 2;
+    const int cap = c.v.slot_cap;
+    const unsigned tot = (unsigned)c.sh.m * L;
+    for (unsigned it = it0; it < tot; it += step) {
+        const int j = (int)(it / L), i = (int)(it - (unsigned)j * L);
+        const double *co = c.sh.coef + (size_t)j * HBK_NCOEF;
+        double *xc = c.v.Xc + (size_t)j * cap + i;
+        double *pc = c.v.Pc + (size_t)j * cap + i;
+        const int live = __ldcg(c.sh.live + j);
+        const double c1 = __ldcg(co + 1), c4 = mul(__ldcg(co + 4), bk);
+        double x = HBK_LD(G, xc, 0), p = HBK_LD(G, pc, 0);
+        if (j != u.seed && (live != 1 || !fin(c4))) continue;
+        if (i == sq) x = x + __ldcg(co);
+        x = fma(c1, p, x);
+        if (i == sq) p = p + __ldcg(co + 2);
+        if (i == so) p = p + __ldcg(co + 3);
+        p = c4 * p;
+        if (i == sr) p = p + __ldcg(co + 5);
+        *xc = x;
+        *pc = p;
+        if (i == 0) {
+            double *ow = c.v.own + 2 * (size_t)j;
+            const double o1 = HBK_LD(G, ow, 1);
+            ow[0] = fma(c1, o1, HBK_LD(G, ow, 0));
+            ow[1] = c4 * o1;
+            c.sh.lslot[j] = (int)L;
+        }
+    }
+}
+
+// K5 (deferred): x_s and p_s, the coefficient update (in a one-family launch
+// by g.ncoef() extra blocks, else by every block), on a switch the rescaled
+// r_k in a new slot
 template <class G>
 __device__ __forceinline__ void seed_p_deferred_body(const Ctx &c, const G &g) {
-    __shared__ double sh[NW];
-    __shared__ unsigned long long smx[NW];
+    __shared__ double sh[2 * MAXW];
+    __shared__ unsigned long long smx[MAXW];
     hbk_scalars *sc = c.sh.sc;
-    if (stopped(sc)) return;
-    const double bk = sc->beta, bw = -mul(bk, sc->omega);
-    const int sw = sc->switched;
-    const double rsc = sc->r_scale;
+    body_begin<G>();
+    body_ready<G>();
+    const hbk_cur u = load_cur(sc);
+    const double ak = __ldcg(&sc->alpha), wk = __ldcg(&sc->omega);
+    if (!u.active || !fin(ak) || !fin(wk) || is_zero(wk)) return;
     const unsigned n = c.v.n;
-    const size_t ld = ldn(n);
+    const size_t ld = ldn(n), step = (size_t)g.nb() * blockDim.x;
     double *__restrict__ ps = c.v.ps;
     const double *__restrict__ s = c.v.s;
-    const double *__restrict__ rn = c.v.V + (size_t)(sc->slots + 1) * ld;
-    double *__restrict__ rsl = c.v.V + (size_t)(sc->slots + 2) * ld;
+    const double *__restrict__ q = vec_q(c, u);
+    const double *__restrict__ rn = c.v.V + (size_t)(u.slots + 1) * ld;
+    double *__restrict__ rsl = c.v.V + (size_t)(u.slots + 2) * ld;
+    double *__restrict__ xp = c.v.Xp;
     const double *__restrict__ rh = c.v.r_hat;
+    const int pm = c.v.pm, seed = u.seed;
+    size_t i = g.extra() || g.coef_only() ? (size_t)n : g.b() * (size_t)blockDim.x + threadIdx.x;
+    double ri = 0.0, pi = 0.0, si = 0.0, qi = 0.0, xi = 0.0;
+    if (i < n) {
+        ri = HBK_LD(G, rn, i), pi = HBK_LD(G, ps, i), si = HBK_LD(G, s, i), qi = HBK_LD(G, q, i);
+        xi = HBK_LD(G, xp, panel_idx(seed, (unsigned)i, pm));
+    }
+    const StepEnd e = step_end(c, u, wk, sh);
+    if (!e.ok) {
+        if (!g.coef_only()) seed_x_only(c, u, g);
+        return;
+    }
+    if (g.extra()) {
+        record_step(c, u, e);
+        return;
+    }
+    if (g.does_coef()) coef_update<G>(c, u, e.bk, g.cb() * blockDim.x + threadIdx.x, g.ncb() * blockDim.x);
+    if (g.coef_only()) return;
+    const double bk = e.bk, bw = e.bw;
     double acc = 0.0;
     unsigned long long mx = 0;
-    for (size_t i = g.b() * (size_t)NT + threadIdx.x; i < n; i += (size_t)g.nb() * NT) {
-        const double ri = HBK_LD(G, rn, i);
-        ps[i] = fma(bw, HBK_LD(G, s, i), fma(bk, HBK_LD(G, ps, i), ri));
-        if (sw) {
-            const double rs = ri * rsc;
+    while (i < n) {
+        const size_t in = i + step;  // the next element's loads go before this one's stores
+        double r2 = 0.0, p2 = 0.0, s2 = 0.0, q2 = 0.0, x2 = 0.0;
+        if (in < n) {
+            r2 = HBK_LD(G, rn, in), p2 = HBK_LD(G, ps, in), s2 = HBK_LD(G, s, in), q2 = HBK_LD(G, q, in);
+            x2 = HBK_LD(G, xp, panel_idx(seed, (unsigned)in, pm));
+        }
+        xp[panel_idx(seed, (unsigned)i, pm)] = fma(wk, qi, fma(ak, pi, xi));
+        ps[i] = fma(bw, si, fma(bk, pi, ri));
+        if (e.sw) {
+            const double rs = ri * e.rsc;
             rsl[i] = rs;
             acc = fma(HBK_LD(G, rh, i), rs, acc);
             const unsigned long long b = abs_bits(rs);
             mx = b > mx ? b : mx;
         }
+        ri = r2, pi = p2, si = s2, qi = q2, xi = x2, i = in;
     }
-    if (!sw) return;  // uniform: the reduction is needed only after a switch
-    if (c.v.slot_max) block_max_to(mx, smx, c.v.slot_max + (size_t)(sc->slots + 2) * HBK_SLOT_SPREAD);  // rescaled r_k
-    acc = block_sum(acc, sh);
-    if (threadIdx.x == 0) c.sh.partials[g.b()] = acc;
-    if (take_ticket(c.sh.counters + 3, g.nb())) {
-        const double rrh = sum_partials(c.sh.partials, g.nb(), sh);
-        if (threadIdx.x == 0) {
-            sc->rs_switch = rrh;
-            c.sh.counters[3] = 0;
-        }
-    }
+    if (!e.sw) return;  // uniform: the reduction is needed only after a switch
+    if (c.v.slot_max) block_max_to(mx, smx, c.v.slot_max + (size_t)(u.slots + 2) * HBK_SLOT_SPREAD);  // rescaled r_k
+    __syncthreads();
+    store_part(acc, sh, parts(c, P_RRS) + g.b());
 }
-__global__ void __launch_bounds__(NT) k_seed_p_deferred(Ctx c) { seed_p_deferred_body(c, HwGrid()); }
-
-// K6 (deferred): coefficient update of every running system over the basis
-// slots in use, then the end-of-iteration bookkeeping.  Per coefficient the
-// operations follow the vector update's order (x += c0 q; x += c1 p;
-// p += c2 q; p += c3 r_{k-1}; p *= beta_j; p += c5 r_k).
-template <class G>
-__device__ __forceinline__ void coef_update_body(const Ctx &c, const G &g) {
-    hbk_scalars *sc = c.sh.sc;
-    if (stopped(sc)) return;
-    const int na = sc->n_active;
-    const int sq = sc->slots, sr = sc->slots + 1, so = sc->slot_r_old;
-    const int L = sc->slots + 2;
-    const int cap = c.v.slot_cap;
-    const size_t tot = (size_t)na * L;
-    for (size_t it = g.b() * (size_t)NT + threadIdx.x; it < tot; it += (size_t)g.nb() * NT) {
-        const int a = (int)(it / L), i = (int)(it % L);
-        const int j = HBK_LD(G, c.sh.act_list, a);
-        const double *co = c.sh.coef + (size_t)j * HBK_NCOEF;
-        double *xc = c.v.Xc + (size_t)j * cap + i;
-        double *pc = c.v.Pc + (size_t)j * cap + i;
-        double x = HBK_LD(G, xc, 0), p = HBK_LD(G, pc, 0);
-        if (i == sq) x = x + co[0];
-        x = fma(co[1], p, x);
-        if (i == sq) p = p + co[2];
-        if (i == so) p = p + co[3];
-        p = co[4] * p;
-        if (i == sr) p = p + co[5];
-        *xc = x;
-        *pc = p;
-        if (i == 0) {
-            double *ow = c.v.own + 2 * (size_t)j;
-            ow[0] = fma(co[1], HBK_LD(G, ow, 1), HBK_LD(G, ow, 0));
-            ow[1] = co[4] * HBK_LD(G, ow, 1);
-            c.sh.lslot[j] = L;
-        }
-    }
-    if (take_ticket(c.sh.counters + 4, g.nb())) {
-        if (threadIdx.x == 0) {
-            finish_iteration(c, sc, sc->rs_switch);
-            c.sh.counters[4] = 0;
-        }
-    }
+__global__ void __launch_bounds__(1024) k_seed_p_deferred(Ctx c, unsigned ncoef) {
+    seed_p_deferred_body(c, HwGridX{1 + ncoef});
 }
-__global__ void __launch_bounds__(NT) k_coef_update(Ctx c) { coef_update_body(c, HwGrid()); }
 
-// K7 (deferred): after a switch, the new seed's p = own term + Pc[t] . V
+// Deferred mode, after a switch: the new seed's p = own term + Pc[t] . V, and
+// its shift on the diagonal of the seed kernels' products
 template <class G>
 __device__ __forceinline__ void materialize_ps_body(const Ctx &c, const G &g) {
     __shared__ double s_c[1024];
     hbk_scalars *sc = c.sh.sc;
     if (!__ldcg(&sc->need_ps)) return;
-    const int t = sc->seed;
+    const int t = __ldcg(&sc->seed);
     const int L = HBK_LD(G, c.sh.lslot, t);
     const unsigned n = c.v.n;
     const size_t ld = ldn(n);
@@ -708,7 +1076,7 @@ __device__ __forceinline__ void materialize_ps_body(const Ctx &c, const G &g) {
         }
         if (i < n) c.v.ps[i] = acc;
     }
-    if (c.v.sval_shift) {  // the new seed's shift on the diagonal of the seed kernels' products
+    if (c.v.sval_shift) {
         const double sg = c.sh.sigma[t];
         for (size_t r = g.b() * (size_t)NT + threadIdx.x; r < n; r += (size_t)g.nb() * NT) {
             const unsigned long long d = c.v.sdiag[r];
@@ -719,6 +1087,12 @@ __device__ __forceinline__ void materialize_ps_body(const Ctx &c, const G &g) {
         if (threadIdx.x == 0) {
             sc->need_ps = 0;
             c.sh.counters[5] = 0;
+            const int status = __ldcg(&sc->status);
+            if (status & HBK_ST_NEED_PS) {  // paused for this: run on, unless the basis is full or the solve over
+                sc->status = status & ~HBK_ST_NEED_PS;
+                if (!(status & (HBK_ST_BASIS_FULL | HBK_ST_BREAKDOWN)) && sc->n_done < sc->m && sc->k < sc->kcap)
+                    sc->finished = 0;
+            }
         }
     }
 }
@@ -881,14 +1255,14 @@ __global__ void __launch_bounds__(NT) k_panel_to_rows(const double *__restrict__
 // the same CTAs from step to step) and run, for every family at once, the
 // same steps as the one-family kernels (K1..K5, and K6, K7 for the families
 // in the deferred mode, with a virtual block in place of the launch's block:
-// same partial sums, same last-block tickets and scalar stage per family).  A
-// grid-wide barrier separates the steps.  Families stop one by one
+// same partial sums and, per family, one more entry for the extra block of K4
+// and K5).  A grid-wide barrier separates the steps.  Families stop one by one
 // (converged, max_iter, breakdown) or pause with a full basis; their virtual
 // blocks then return at once, and the launch ends when every family has
 // stopped or paused (the host flushes the paused ones and launches again).
 struct GroupFam {
     Ctx c;
-    unsigned vb0, nvb;  // the family's virtual blocks [vb0, vb0 + nvb)
+    unsigned vb0, nvb;  // entry vb0: the extra block of K4 and K5; then its nvb virtual blocks
 };
 
 __device__ __forceinline__ unsigned ld_acquire_u32(const unsigned *p) {
@@ -956,9 +1330,6 @@ __device__ __forceinline__ void step5_body(const Ctx &c, const VGrid &g) {
     if (c.v.deferred) seed_p_deferred_body(c, g);
     else shift_update_body<MAXS>(c, g);
 }
-__device__ __forceinline__ void coef_update_if_deferred(const Ctx &c, const VGrid &g) {
-    if (c.v.deferred) coef_update_body(c, g);
-}
 __device__ __forceinline__ void materialize_if_deferred(const Ctx &c, const VGrid &g) {
     if (c.v.deferred) materialize_ps_body(c, g);
 }
@@ -968,10 +1339,12 @@ template <int MAXS>
 __global__ void __launch_bounds__(NT, 3) k_group(const GroupFam *__restrict__ fams, int nf,
                                                  const unsigned *__restrict__ vb_fam, unsigned nvb, unsigned *bar,
                                                  int *err, int iter_cap, int any_deferred, int withhold) {
-#define HBK_GROUP_STEP(body)                                                       \
+#define HBK_GROUP_STEP(body, with_extra)                                           \
     for (unsigned vb = blockIdx.x; vb < nvb; vb += gridDim.x) {                    \
         const GroupFam &F = fams[vb_fam[vb]];                                      \
-        body(F.c, VGrid{vb - F.vb0, F.nvb});                                       \
+        const bool extra = vb == F.vb0; /* a family's first entry */               \
+        if (extra && !(with_extra)) continue;                                      \
+        body(F.c, VGrid{vb - F.vb0 - 1u, F.nvb, extra});                           \
     }                                                                              \
     if (!grid_barrier(bar, err)) return;
     for (int it = 0; it <= iter_cap; ++it) {
@@ -981,14 +1354,13 @@ __global__ void __launch_bounds__(NT, 3) k_group(const GroupFam *__restrict__ fa
         for (int f = threadIdx.x; f < nf; f += NT) alive |= __ldcg(&fams[f].c.sh.sc->finished) == 0;
         alive = __syncthreads_or(alive);
         if (!grid_barrier(bar, err, withhold && it == 0 && blockIdx.x == 0) || !alive) return;
-        HBK_GROUP_STEP(seed_s_body<HBK_FMT_SELL>)
-        HBK_GROUP_STEP(seed_q_body)
-        HBK_GROUP_STEP(seed_y_body<HBK_FMT_SELL>)
-        HBK_GROUP_STEP(seed_update_body)
-        HBK_GROUP_STEP(step5_body<MAXS>)
+        HBK_GROUP_STEP(seed_s_body<HBK_FMT_SELL>, false)
+        HBK_GROUP_STEP(seed_q_body, false)
+        HBK_GROUP_STEP(seed_y_body<HBK_FMT_SELL>, false)
+        HBK_GROUP_STEP(seed_update_body, true)
+        HBK_GROUP_STEP(step5_body<MAXS>, true)
         if (any_deferred) {
-            HBK_GROUP_STEP(coef_update_if_deferred)
-            HBK_GROUP_STEP(materialize_if_deferred)
+            HBK_GROUP_STEP(materialize_if_deferred, false)
         }
     }
 #undef HBK_GROUP_STEP
@@ -1014,6 +1386,7 @@ int hbk_panel_to_rows(const double *Xp, int m, unsigned n, double *X, size_t ld,
 
 static Ctx make_ctx(const hbk_matrix *A, const hbk_vectors *v, const hbk_shifts *sh) {
     Ctx c;
+    c.np_s = c.np_y = c.np_r = c.np_p = 0;
     c.A = *A;
     c.v = *v;
     c.sh = *sh;
@@ -1027,7 +1400,7 @@ static Ctx make_ctx(const hbk_matrix *A, const hbk_vectors *v, const hbk_shifts 
 }
 
 int hbk_fused_init(const hbk_matrix *A, const hbk_vectors *v, const hbk_shifts *sh, const double *b, int seed,
-                   double tol, cudaStream_t st) {
+                   double tol, int switching, int inline_ps, cudaStream_t st) {
     Ctx c = make_ctx(A, v, sh);
     const unsigned n = v->n;
     const size_t ld = ((size_t)n + 31) / 32 * 32;
@@ -1060,7 +1433,7 @@ int hbk_fused_init(const hbk_matrix *A, const hbk_vectors *v, const hbk_shifts *
     } else if ((e = (int)cudaMemsetAsync(v->X, 0, sizeof(double) * ld * (size_t)sh->m, st))) {
         return e;
     }
-    k_init<<<1, NT, 0, st>>>(c, seed, tol);
+    k_init<<<1, NT, 0, st>>>(c, seed, tol, switching, inline_ps);
     return (int)cudaGetLastError();
 }
 
@@ -1069,38 +1442,80 @@ int hbk_hyb_wave_fused(void) {
     return a < b ? a : b;
 }
 
-int hbk_fused_iteration(const hbk_matrix *A, const hbk_vectors *v, const hbk_shifts *sh, cudaStream_t st) {
+}  // extern "C"
+
+// Blocks of a vector kernel beside `extra` others: one per SM at most, of
+// n / SMs rows rounded up to two warps (128..1024 threads; longer vectors in a
+// grid-stride loop).  Above 512 threads an SM holds one block, so the extra
+// ones take SMs of their own.
+struct VecGrid {
+    int blocks, threads;
+};
+static VecGrid vec_grid(unsigned n, int extra) {
+    const int sms = sm_count();
+    const unsigned per = (n / (unsigned)sms + 64) / 64 * 64;
+    const unsigned t = per < 128 ? 128 : (per > 1024 ? 1024 : per);
+    const int most = t <= 512 ? sms : (sms > 2 * extra ? sms - extra : 1);
+    const unsigned need = n ? (n + t - 1) / t : 1;
+    return {need < (unsigned)most ? (int)need : most, (int)t};
+}
+
+// kernel<<<...>>>, allowed to start before the stream's previous kernel ends
+// (the kernel waits for it before it reads anything the iteration writes)
+template <class... P, class... Arg>
+static void launch(void (*kernel)(P...), int blocks, int threads, bool early, cudaStream_t st, Arg... arg) {
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)blocks);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.stream = st;
+    cfg.attrs = at;
+    cfg.numAttrs = early ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, kernel, P(arg)...);
+}
+
+template <int FMT>
+static void launch_iteration(Ctx &c, const hbk_matrix *A, int early, cudaStream_t st) {
+    // the products are grid-stride loops: at most one wave of them
+    const int gs = wave_grid<k_seed_s<FMT>>(A->grid), gy = wave_grid<k_seed_y<FMT>>(A->grid);
+    // (K4 leaves two SMs: the grid also fixes the order of its dot products' sums,
+    // and with the order, all being equally accurate, the 256^3 family's solve
+    // takes 413..457 iterations; with 150 blocks it takes 415, as the
+    // reference's own 414 does to within 2 %)
+    const VecGrid q = vec_grid(c.v.n, 0), r = vec_grid(c.v.n, 2);
+    const unsigned ncoef = !c.v.deferred ? 0 : ((unsigned)(c.sh.m < 256 ? c.sh.m : 256) * 64u + q.threads - 1) / q.threads;
+    const VecGrid p = vec_grid(c.v.n, 1 + (int)ncoef);
+    c.np_s = (unsigned)gs, c.np_y = (unsigned)gy, c.np_r = (unsigned)r.blocks, c.np_p = (unsigned)p.blocks;
+    // Early starts: measured on whole solves, SELL-32, n = 512: 1163 -> 1061 us;
+    // 97 k rows: 20.1 -> 18.5 ms; 128^3: 64.2 -> 63.0 ms.  Not where blocks
+    // that start early would crowd onto the SMs the kernel before leaves free
+    // and then run long: the incremental update (FP64-bound; 32^3: 3.4 -> 4.7
+    // ms) and the products of the other forms (HYB: 68 -> 75 ms).
+    const bool e = early > 0, es = e && FMT == HBK_FMT_SELL;
+    launch(k_seed_s<FMT>, gs, NT, es && early > 1, st, c);
+    launch(k_seed_q, q.blocks, q.threads, e, st, c);
+    launch(k_seed_y<FMT>, gy, NT, es, st, c);
+    launch(k_seed_update, r.blocks + 1, r.threads, e, st, c);
+    if (!c.v.deferred) launch(k_shift_update<64>, p.blocks + 1, p.threads, false, st, c);
+    else launch(k_seed_p_deferred, p.blocks + 1 + (int)ncoef, p.threads, e, st, c, ncoef);
+}
+
+extern "C" {
+
+int hbk_fused_iteration(const hbk_matrix *A, const hbk_vectors *v, const hbk_shifts *sh, int early, cudaStream_t st) {
     Ctx c = make_ctx(A, v, sh);
-    const int gv = grid_for(v->n, 2);
-    // every kernel here is a grid-stride loop: launch at most one wave of it
-    if (A->fmt == HBK_FMT_SELL) {
-        k_seed_s<HBK_FMT_SELL><<<wave_grid<k_seed_s<HBK_FMT_SELL>>(A->grid), NT, 0, st>>>(c);
-        k_seed_q<<<wave_grid<k_seed_q>(gv), NT, 0, st>>>(c);
-        k_seed_y<HBK_FMT_SELL><<<wave_grid<k_seed_y<HBK_FMT_SELL>>(A->grid), NT, 0, st>>>(c);
-    } else if (A->fmt == HBK_FMT_MERGE) {
-        k_seed_s<HBK_FMT_MERGE><<<wave_grid<k_seed_s<HBK_FMT_MERGE>>(A->grid), NT, 0, st>>>(c);
-        k_seed_q<<<wave_grid<k_seed_q>(gv), NT, 0, st>>>(c);
-        k_seed_y<HBK_FMT_MERGE><<<wave_grid<k_seed_y<HBK_FMT_MERGE>>(A->grid), NT, 0, st>>>(c);
-    } else if (A->fmt == HBK_FMT_HYB) {
-        k_seed_s<HBK_FMT_HYB><<<wave_grid<k_seed_s<HBK_FMT_HYB>>(A->grid), NT, 0, st>>>(c);
-        k_seed_q<<<wave_grid<k_seed_q>(gv), NT, 0, st>>>(c);
-        k_seed_y<HBK_FMT_HYB><<<wave_grid<k_seed_y<HBK_FMT_HYB>>(A->grid), NT, 0, st>>>(c);
-    } else {
-        k_seed_s<HBK_FMT_TILE><<<wave_grid<k_seed_s<HBK_FMT_TILE>>(A->grid), NT, 0, st>>>(c);
-        k_seed_q<<<wave_grid<k_seed_q>(gv), NT, 0, st>>>(c);
-        k_seed_y<HBK_FMT_TILE><<<wave_grid<k_seed_y<HBK_FMT_TILE>>(A->grid), NT, 0, st>>>(c);
-    }
-    k_seed_update<<<wave_grid<k_seed_update>(gv), NT, 0, st>>>(c);
-    if (!v->deferred) {
-        // one element per thread: the update is FP64-bound (6 operations per
-        // element and running shift), so on small systems it wants every SM's
-        // FP64 pipe, not the two elements per thread of the streaming kernels
-        k_shift_update<64><<<wave_grid<k_shift_update<64>>(grid_for(v->n, 1)), NT, 0, st>>>(c);
-    } else {
-        k_seed_p_deferred<<<wave_grid<k_seed_p_deferred>(gv), NT, 0, st>>>(c);
-        k_coef_update<<<grid_for((unsigned)((size_t)sh->m * v->slot_cap), 1), NT, 0, st>>>(c);
-        k_materialize_ps<<<wave_grid<k_materialize_ps>(gv), NT, 0, st>>>(c);
-    }
+    if (A->fmt == HBK_FMT_SELL) launch_iteration<HBK_FMT_SELL>(c, A, early, st);
+    else if (A->fmt == HBK_FMT_MERGE) launch_iteration<HBK_FMT_MERGE>(c, A, early, st);
+    else if (A->fmt == HBK_FMT_HYB) launch_iteration<HBK_FMT_HYB>(c, A, early, st);
+    else launch_iteration<HBK_FMT_TILE>(c, A, early, st);
+    return (int)cudaGetLastError();
+}
+
+int hbk_materialize_ps(const hbk_matrix *A, const hbk_vectors *v, const hbk_shifts *sh, cudaStream_t st) {
+    Ctx c = make_ctx(A, v, sh);
+    k_materialize_ps<<<wave_grid<k_materialize_ps>(grid_for(v->n, 2)), NT, 0, st>>>(c);
     return (int)cudaGetLastError();
 }
 
@@ -1123,7 +1538,7 @@ static size_t group_bytes(int nf, size_t nvb) {
 
 size_t hbk_group_ws_bytes(int nf, const hbk_vectors *v, unsigned rows_per_vb) {
     size_t nvb = 0;
-    for (int f = 0; f < nf; ++f) nvb += group_vblocks(v[f].n, rows_per_vb);
+    for (int f = 0; f < nf; ++f) nvb += 1 + group_vblocks(v[f].n, rows_per_vb);
     return group_bytes(nf, nvb);
 }
 
@@ -1152,7 +1567,8 @@ int hbk_group_run(int nf, const hbk_matrix *A, const hbk_vectors *v, const hbk_s
         tab[f].c = make_ctx(&A[f], &v[f], &sh[f]);
         tab[f].vb0 = (unsigned)map.size();
         tab[f].nvb = group_vblocks(v[f].n, rows_per_vb);
-        map.insert(map.end(), tab[f].nvb, (unsigned)f);
+        tab[f].c.np_s = tab[f].c.np_y = tab[f].c.np_r = tab[f].c.np_p = tab[f].nvb;
+        map.insert(map.end(), 1 + tab[f].nvb, (unsigned)f);
     }
     const unsigned nvb = (unsigned)map.size();
     if (ws_bytes < group_bytes(nf, nvb)) return (int)cudaErrorInvalidValue;

@@ -10,7 +10,7 @@
  *          back to the host, which keeps the scalars, runs the shift
  *          recurrences, the convergence test and the seed switch exactly as
  *          src/solver_dynamic.c:147-381 does (the per-kernel form);
- *   fused  five to seven kernels per iteration with every scalar on the device
+ *   fused  five kernels per iteration with every scalar on the device
  *          (hbk_fused_iteration); iterations are captured in CUDA graphs and
  *          the host only polls a finished flag between graph launches.
  * In the fused form the shifts are either updated every iteration by one
@@ -409,14 +409,14 @@ int hbicg_solver_create(hbicg_context *ctx, hbicg_matrix *A, int m, const hbicg_
     DALLOC(sh->zeta, sizeof(double) * mm);
     DALLOC(sh->done, sizeof(int) * mm);
     DALLOC(sh->conv_k, sizeof(int) * mm);
-    DALLOC(sh->act_list, sizeof(int) * mm);
+    DALLOC(sh->live, sizeof(int) * mm);
     DALLOC(sh->lslot, sizeof(int) * mm);
     DALLOC(sh->coef, sizeof(double) * HBK_NCOEF * (size_t)mm);
     DALLOC(sh->sw_k, sizeof(int) * mm);
     DALLOC(sh->sw_seed, sizeof(int) * mm);
     DALLOC(sh->act_hist, sizeof(int) * ((size_t)s->kcap + 1));
     CUDA_TRY(cudaMemset(sh->act_hist, 0, sizeof(int) * ((size_t)s->kcap + 1)));
-    size_t nparts = (size_t)(mm > 4 ? mm : 4) * HBK_MAX_GRID;
+    size_t nparts = (size_t)(mm > HBK_NPART ? mm : HBK_NPART) * HBK_MAX_GRID;
     DALLOC(sh->partials, sizeof(double) * nparts);
     DALLOC(sh->counters, sizeof(unsigned) * (16 + (size_t)mm));
     CUDA_TRY(cudaMemset(sh->counters, 0, sizeof(unsigned) * (16 + (size_t)mm)));
@@ -429,7 +429,7 @@ int hbicg_solver_create(hbicg_context *ctx, hbicg_matrix *A, int m, const hbicg_
         s->d_r = v->rbuf[0];
     }
     s->chunk = p.graph_chunk > 0 ? p.graph_chunk : (n >= (1u << 22) ? 2 : (n >= (1u << 18) ? 4 : 16));
-    s->launches_per_iter = s->mode == HBICG_SHIFTS_DEFERRED ? 7 : 5;
+    s->launches_per_iter = 5;
     hbicg__ctx_retain(ctx);
     *out = s;
     return HBICG_OK;
@@ -443,7 +443,7 @@ void hbicg_solver_destroy(hbicg_solver *s) {
     hbk_shifts *sh = &s->sh;
     void *ptrs[] = {v->r_hat, v->rbuf[0], v->rbuf[1], v->s, v->q, v->y, v->X, v->P, v->V, v->ps, v->Xc, v->Pc,
                     v->own, v->Pmat, v->Xp, v->slot_max, v->sval_shift, s->d_sc, s->d_sigma, sh->a_hist, sh->b_hist, sh->w_hist, sh->ratio, sh->pi,
-                    sh->eta, sh->zeta, sh->done, sh->conv_k, sh->act_list, sh->lslot, sh->coef, sh->sw_k,
+                    sh->eta, sh->zeta, sh->done, sh->conv_k, sh->live, sh->lslot, sh->coef, sh->sw_k,
                     sh->rr_hist, sh->sw_seed, sh->act_hist, sh->partials, sh->counters, s->d_b, s->d_res, s->d_dot, s->d_rold,
                     s->d_qcopy, s->tc_ws, s->d_tc_err};
     for (size_t i = 0; i < sizeof ptrs / sizeof ptrs[0]; i++)
@@ -695,7 +695,7 @@ static int capture_loop_graph(hbicg_solver *s) {
         goto out;
     capturing = 1;
     for (int i = 0; i < s->chunk; i++)
-        if (hbk_fused_iteration(&s->A->k, &s->v, &s->sh, st)) goto out;
+        if (hbk_fused_iteration(&s->A->k, &s->v, &s->sh, 0, st)) goto out;
     if (hbk_loop_condition(&s->sh, cond, 2 * s->kcap + 64, st)) goto out;
     capturing = 0;
     if (cudaStreamEndCapture(st, &body_out) != cudaSuccess) goto out;
@@ -718,7 +718,7 @@ static int capture_graph(hbicg_solver *s) {
     s->graph_loop = 0;
     CUDA_TRY(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
     for (int i = 0; i < s->chunk; i++) {
-        int e = hbk_fused_iteration(&s->A->k, &s->v, &s->sh, st);
+        int e = hbk_fused_iteration(&s->A->k, &s->v, &s->sh, i ? 2 : 1, st);
         if (e) {
             cudaStreamEndCapture(st, &g);
             set_msg("capture: %s", hbk_error_string(e));
@@ -774,14 +774,12 @@ static int do_flush(hbicg_solver *s, int keep_p, int L, int k_last, int *launche
     return HBICG_OK;
 }
 
-/* first step of a fused solve: the device scalars, r and p_j (or the basis) from b */
-static int fused_init(hbicg_solver *s, int seed, int *launches) {
+/* first step of a fused solve: the device scalars, r and p_j (or the basis)
+ * from b.  inline_ps: the launch that runs the iterations forms a new seed's
+ * p itself (hbk_group_run); else the solve pauses for it (HBK_ST_NEED_PS). */
+static int fused_init(hbicg_solver *s, int seed, int inline_ps, int *launches) {
     cudaStream_t st = s->ctx->stream;
-    HBK_TRY(hbk_fused_init(&s->A->k, &s->v, &s->sh, s->d_b, seed, s->p.tol, st));
-    /* switching flag lives in the device scalars */
-    int sw = s->p.switching ? 1 : 0;
-    CUDA_TRY(cudaMemcpyAsync(&s->d_sc->switching, &sw, sizeof(int), cudaMemcpyHostToDevice, st));
-    CUDA_TRY(cudaStreamSynchronize(st));
+    HBK_TRY(hbk_fused_init(&s->A->k, &s->v, &s->sh, s->d_b, seed, s->p.tol, s->p.switching ? 1 : 0, inline_ps, st));
     *launches += 6 + (s->v.deferred ? 1 : s->m);
     return HBICG_OK;
 }
@@ -902,14 +900,15 @@ static int run_persistent(hbicg_solver *s, int *launches, int *flushes, double *
 static int run_fused(hbicg_solver *s, int seed, int *launches, int *flushes, double *flush_ms) {
     cudaStream_t st = s->ctx->stream;
     hbk_scalars *h = s->ctx->h_sc;
-    int rc0 = fused_init(s, seed, launches);
+    const int persistent = s->p.use_graph == 3 && s->A->k.fmt == HBK_FMT_SELL && s->m > 0;
+    int rc0 = fused_init(s, seed, persistent, launches);
     if (rc0) return rc0;
-    if (s->p.use_graph == 3 && s->A->k.fmt == HBK_FMT_SELL && s->m > 0) return run_persistent(s, launches, flushes, flush_ms);
+    if (persistent) return run_persistent(s, launches, flushes, flush_ms);
     const int use_graph = s->p.use_graph;
     /* every launch of a chunk advances k by chunk unless the solve ends or
      * the basis pauses it; bound the host loop all the same */
     long guard = 0;
-    const long guard_max = 4L * s->kcap / s->chunk + 64;
+    const long guard_max = 4L * s->kcap / s->chunk + 64 + s->m; /* (a pause per seed switch) */
     int k_flushed = 0; /* last iteration covered by a flush */
     int loops_seen = 0; /* loop-graph bodies counted so far (k_init zeroes the device count) */
     for (;;) {
@@ -926,7 +925,7 @@ static int run_fused(hbicg_solver *s, int seed, int *launches, int *flushes, dou
             CUDA_TRY(cudaGraphLaunch(s->graph, st));
             looped = s->graph_loop;
         } else {
-            for (int i = 0; i < s->chunk; i++) HBK_TRY(hbk_fused_iteration(&s->A->k, &s->v, &s->sh, st));
+            for (int i = 0; i < s->chunk; i++) HBK_TRY(hbk_fused_iteration(&s->A->k, &s->v, &s->sh, 0, st));
         }
         CUDA_TRY(cudaMemcpyAsync(h, s->d_sc, sizeof(hbk_scalars), cudaMemcpyDeviceToHost, st));
         CUDA_TRY(cudaStreamSynchronize(st));
@@ -937,12 +936,16 @@ static int run_fused(hbicg_solver *s, int seed, int *launches, int *flushes, dou
             *launches += s->chunk * s->launches_per_iter;
         }
         if (!h->finished) continue;
-        if ((h->status & HBK_ST_BASIS_FULL) && !(h->status & HBK_ST_BREAKDOWN)) {
+        const int over = (h->status & HBK_ST_BREAKDOWN) || h->n_done >= h->m || h->k >= h->kcap;
+        if (!over && (h->status & HBK_ST_NEED_PS)) { /* before a flush: it restarts the basis */
+            HBK_TRY(hbk_materialize_ps(&s->A->k, &s->v, &s->sh, st));
+            ++*launches;
+        }
+        if (!over && (h->status & HBK_ST_BASIS_FULL)) {
             int rc = fused_pause_flush(s, &k_flushed, launches, flushes, flush_ms);
             if (rc) return rc;
-            continue;
         }
-        break;
+        if (over) break;
     }
     return fused_tail(s, k_flushed, launches, flush_ms);
 }
@@ -1445,7 +1448,11 @@ int hbicg__group_add(hbicg__group *g, hbicg_solver *s, const double *b, const do
     int rc = hbicg__group_eligible(s) ? HBICG_OK : HBICG_E_ARG;
     if (rc) set_msg("a solver that is not fused and SELL-32 cannot join the shared launch");
     if (rc == HBICG_OK) rc = run_begin(s, b, sigma, r);
-    if (rc == HBICG_OK) rc = fused_init(s, seed, &r->launches);
+    if (rc == HBICG_OK) rc = fused_init(s, seed, 1, &r->launches);
+    if (rc == HBICG_OK && cudaStreamSynchronize(s->ctx->stream) != cudaSuccess) { /* the launch has a stream of its own */
+        set_msg("shared launch: a family's first step failed");
+        rc = HBICG_E_CUDA;
+    }
     g->rc[slot] = rc;
     g->in[slot] = rc == HBICG_OK;
     if (rc) group_keep(g->msg[slot]);
