@@ -46,6 +46,7 @@ extern "C" {
 #define HBK_HYB_WINDOW 1024  /* rows are sorted by length only inside windows of this many consecutive rows */
 #define HBK_HYB_L4 128       /* long rows up to this length: 4 lanes each, 8 rows per warp */
 #define HBK_HYB_L16 512      /* longer rows up to this length: 16 lanes each, 2 rows per warp; longer: a warp */
+#define HBK_FMT_HYBW 4       /* kernels of a HYB matrix with nwide > 0 (hbk_matrix.fmt stays HBK_FMT_HYB) */
 #define HBK_FMT_MERGE 3      /* CSR; rows up to HBK_MERGE_LONG entries in merge-path blocks, longer rows one warp each */
 #define HBK_MERGE_IPT 8      /* merge items (row ends + nonzeros) per lane of a block */
 #define HBK_MERGE_ITEMS (32 * HBK_MERGE_IPT) /* items per block (one warp) */
@@ -73,6 +74,8 @@ typedef struct {
     const unsigned *hwbeg;     /* HYB: work list of warp w = items hitem[hwbeg[w] .. hwbeg[w + 1]) */
     const unsigned *hitem;     /* HYB: work items (hbk_hyb_classes), then slice i - hitl */
     unsigned hnw;              /* HYB: warps the lists were balanced for */
+    unsigned nwide;            /* HYB: the first nwide long rows take a whole block each, and the warps batch their
+                                  loads (k<HBK_FMT_HYBW>); 0: warps only */
     unsigned hrow32, hrow16;   /* HYB: long rows [0, hrow32) have 32 lanes each, [hrow32, hrow16) 16, the rest 4 */
     unsigned hit16, hit4, hitl; /* HYB: first item of 16-lane rows, of 4-lane rows, of the slices */
     const unsigned *mblk;      /* MERGE: [2 nmblk] first and end row of each block of short rows */
@@ -205,8 +208,8 @@ int hbk_merge_grid(unsigned units);
 int hbk_sell_widths(unsigned n, const unsigned *ptr, unsigned *w, cudaStream_t st);
 /* ... then, with sptr = exclusive prefix sum of 32*w (host), fill the arrays */
 /* one-wave grid (blocks) of the kernels that take the HYB form */
-int hbk_hyb_wave_fused(void);
-int hbk_hyb_wave_blas(void);
+int hbk_hyb_wave_fused(int wide);
+int hbk_hyb_wave_blas(int wide);
 /* HYB slices: slice s, lane l holds row srow[32 s + l] (entry e at sptr[s] + 32 e + l) */
 int hbk_hyb_fill(unsigned nslice, const unsigned *srow, unsigned n, const unsigned *ptr, const unsigned *col,
                  const double *val, const unsigned long long *sptr, double *sval, unsigned *scol, cudaStream_t st);

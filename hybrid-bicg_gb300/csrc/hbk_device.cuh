@@ -24,6 +24,8 @@ constexpr int NT = HBK_THREADS;
 #endif
 // blocks per SM of the SELL-32 kernels: their slice pipeline holds 80 registers
 #define HBK_SELL_MINB 3
+// and of the kernels of HYB matrices whose longest rows take a block each
+#define HBK_HYBW_MINB 4
 constexpr int NW = NT / 32;
 
 __device__ __forceinline__ double warp_sum(double v) {
@@ -385,11 +387,56 @@ __device__ __forceinline__ void spmv_rows_tile(const hbk_matrix &A, const double
 // a slice, and the tree), so no warp is left with several of the longest
 // rows; warp w of the grid runs lists w, w + (warps of the grid), ...  A row's
 // arithmetic does not depend on the list it is in.
-template <class Pre, class Epi>
+//
+// WIDE: where the longest rows would outlast the other lists (small matrices:
+// a 4000-entry row is 125 dependent steps of a warp, about 40 us, whatever the
+// matrix's size), rows above HBK_HYB_L16 take a whole block each, block b the
+// rows b, b + (blocks), ... before its warps' lists, and every lane has
+// HYB_BATCH entries' loads in flight at once.  Twice the registers, so half
+// the warps per SM: the plan takes it only where the longest row outlasts the
+// mean list (both sides measured there, build_hyb).
+constexpr unsigned HYB_BATCH = 4;
+
+// sum of val[e] x[col[e]] over e = e0, e0 + step, ... < e1, in stored order
+// from 0: HYB_BATCH entries' loads at once
+__device__ __forceinline__ double hyb_batched(const double *__restrict__ val, const unsigned *__restrict__ col,
+                                              const double *__restrict__ x, unsigned e0, unsigned e1, unsigned step) {
+    double acc = 0.0;
+    for (unsigned e = e0; e < e1;) {
+        double v[HYB_BATCH], w[HYB_BATCH];
+        unsigned c[HYB_BATCH];
+        const unsigned left = (e1 - e + step - 1) / step;
+#pragma unroll
+        for (unsigned k = 0; k < HYB_BATCH; ++k) {
+            c[k] = k < left ? __ldg(col + e + k * step) : 0u;
+            v[k] = k < left ? __ldg(val + e + k * step) : 0.0;
+        }
+#pragma unroll
+        for (unsigned k = 0; k < HYB_BATCH; ++k) w[k] = k < left ? __ldg(x + c[k]) : 0.0;
+#pragma unroll
+        for (unsigned k = 0; k < HYB_BATCH; ++k)
+            if (k < left) acc = fma(v[k], w[k], acc);
+        e += left < HYB_BATCH ? left * step : HYB_BATCH * step;
+    }
+    return acc;
+}
+
+template <bool WIDE, class Pre, class Epi>
 __device__ __forceinline__ void spmv_rows_hyb(const hbk_matrix &A, const double *__restrict__ x, const Pre &pre,
                                               Epi &epi) {
     const unsigned lane = threadIdx.x & 31;
     const unsigned nw = (gridDim.x * NT) >> 5;
+    if constexpr (WIDE) {
+        __shared__ double red[NW];
+        for (unsigned i = blockIdx.x; i < A.nwide; i += gridDim.x) {
+            const uint2 rg = __ldg(reinterpret_cast<const uint2 *>(A.wrng) + i);
+            const double acc = block_sum(hyb_batched(A.val, A.col, x, rg.x + threadIdx.x, rg.y, NT), red);
+            if (threadIdx.x == 0) {
+                const unsigned r = __ldg(A.wrow + i);
+                epi(r, acc, pre(r));
+            }
+        }
+    }
     for (unsigned w = (blockIdx.x * NT + threadIdx.x) >> 5; w < A.hnw; w += nw) {
         const unsigned k1 = __ldg(A.hwbeg + w + 1);
         for (unsigned k = __ldg(A.hwbeg + w); k < k1; ++k) {
@@ -417,8 +464,12 @@ __device__ __forceinline__ void spmv_rows_hyb(const hbk_matrix &A, const double 
                     r = __ldg(A.wrow + i);
                 }
                 double acc = 0.0;
-                for (unsigned e = rg.x + (lane & (g - 1)); e < rg.y; e += g)
-                    acc = fma(__ldg(A.val + e), __ldg(x + __ldg(A.col + e)), acc);
+                if constexpr (WIDE) {
+                    acc = hyb_batched(A.val, A.col, x, rg.x + (lane & (g - 1)), rg.y, g);
+                } else {
+                    for (unsigned e = rg.x + (lane & (g - 1)); e < rg.y; e += g)
+                        acc = fma(__ldg(A.val + e), __ldg(x + __ldg(A.col + e)), acc);
+                }
                 for (unsigned o = g >> 1; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
                 if (valid && (lane & (g - 1)) == 0) epi(r, acc, pre(r));
             } else {
@@ -430,9 +481,13 @@ __device__ __forceinline__ void spmv_rows_hyb(const hbk_matrix &A, const double 
                 const double *__restrict__ vv = A.sval + base + lane;
                 const unsigned *__restrict__ cc = A.scol + base + lane;
                 double acc = 0.0;
+                if constexpr (WIDE) {
+                    acc = hyb_batched(vv, cc, x, 0u, 32u * len, 32u);
+                } else {
 #pragma unroll 4
-                for (unsigned e = 0; e < wd; ++e)
-                    if (e < len) acc = fma(__ldg(vv + 32 * (size_t)e), __ldg(x + __ldg(cc + 32 * (size_t)e)), acc);
+                    for (unsigned e = 0; e < wd; ++e)
+                        if (e < len) acc = fma(__ldg(vv + 32 * (size_t)e), __ldg(x + __ldg(cc + 32 * (size_t)e)), acc);
+                }
                 if (r < A.n) epi(r, acc, pre(r));
             }
         }
@@ -614,8 +669,8 @@ struct SpmvRows {
     __device__ __forceinline__ void start() {}
     template <class Pre, class Epi>
     __device__ __forceinline__ void run(const double *__restrict__ x, const Pre &pre, Epi &epi) {
-        if constexpr (FMT == HBK_FMT_HYB) {
-            spmv_rows_hyb(A, x, pre, epi);
+        if constexpr (FMT == HBK_FMT_HYB || FMT == HBK_FMT_HYBW) {
+            spmv_rows_hyb<FMT == HBK_FMT_HYBW>(A, x, pre, epi);
         } else if constexpr (FMT == HBK_FMT_MERGE) {
             __shared__ MergeSmem sm;
             spmv_rows_merge(A, x, pre, epi, sm);
@@ -674,6 +729,7 @@ inline int wave_grid(int want) {
 #define HBK_LAUNCH_FMT(A, kern, grid, block, stream, ...)                                   \
     do {                                                                                    \
         if ((A).fmt == HBK_FMT_SELL) kern<HBK_FMT_SELL><<<grid, block, 0, stream>>>(__VA_ARGS__); \
+        else if ((A).fmt == HBK_FMT_HYB && (A).nwide) kern<HBK_FMT_HYBW><<<grid, block, 0, stream>>>(__VA_ARGS__); \
         else if ((A).fmt == HBK_FMT_HYB) kern<HBK_FMT_HYB><<<grid, block, 0, stream>>>(__VA_ARGS__); \
         else if ((A).fmt == HBK_FMT_MERGE) kern<HBK_FMT_MERGE><<<grid, block, 0, stream>>>(__VA_ARGS__); \
         else kern<HBK_FMT_TILE><<<grid, block, 0, stream>>>(__VA_ARGS__);                  \

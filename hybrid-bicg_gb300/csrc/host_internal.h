@@ -41,6 +41,7 @@ struct hbicg_matrix {
     size_t slen_off;                    /* entries of the map before the lengths */
     unsigned long long *d_hsptr;
     unsigned nslice, nwrow;
+    unsigned nwide; /* long rows that take a block each */
     unsigned hnw;  /* warp work lists in d_wrow (after the long rows' entry ranges and the long rows) */
     int hyb_grid;  /* blocks of the HYB kernels: one list per warp */
     unsigned hrow32, hrow16, hit16, hit4, hitl; /* HYB lane classes of the long rows (hbk.h) */

@@ -127,6 +127,12 @@ __global__ void __launch_bounds__(NT, HBK_SELL_MINB) k_true_res<HBK_FMT_SELL>(
     true_res_body<HBK_FMT_SELL>(A, X, ld, b, sigma, partials, counters, out);
 }
 template <>
+__global__ void __launch_bounds__(NT, HBK_HYBW_MINB) k_true_res<HBK_FMT_HYBW>(
+    hbk_matrix A, const double *__restrict__ X, size_t ld, const double *__restrict__ b,
+    const double *__restrict__ sigma, double *partials, unsigned *counters, double *out) {
+    true_res_body<HBK_FMT_HYBW>(A, X, ld, b, sigma, partials, counters, out);
+}
+template <>
 __global__ void __launch_bounds__(NT, HBK_HYB_MINB) k_true_res<HBK_FMT_HYB>(
     hbk_matrix A, const double *__restrict__ X, size_t ld, const double *__restrict__ b,
     const double *__restrict__ sigma, double *partials, unsigned *counters, double *out) {
@@ -312,12 +318,18 @@ int hbk_spmv_grid(unsigned nblk) {
     return g < 1 ? 1 : g;
 }
 
-int hbk_hyb_wave_blas(void) {
-    int g = wave_grid<k_spmv<HBK_FMT_HYB>>(HBK_MAX_GRID);
-    const int a = wave_grid<k_spmv_acc<HBK_FMT_HYB>>(HBK_MAX_GRID), t = wave_grid<k_true_res<HBK_FMT_HYB>>(HBK_MAX_GRID);
+}  // extern "C"
+
+template <int FMT>
+static int hyb_wave(void) {
+    int g = wave_grid<k_spmv<FMT>>(HBK_MAX_GRID);
+    const int a = wave_grid<k_spmv_acc<FMT>>(HBK_MAX_GRID), t = wave_grid<k_true_res<FMT>>(HBK_MAX_GRID);
     if (a < g) g = a;
     return t < g ? t : g;
 }
+extern "C" int hbk_hyb_wave_blas(int wide) { return wide ? hyb_wave<HBK_FMT_HYBW>() : hyb_wave<HBK_FMT_HYB>(); }
+
+extern "C" {
 
 // MERGE form: one wave of the product kernel (its units are dealt round-robin,
 // so a second wave would wait for whole CTAs of the first)

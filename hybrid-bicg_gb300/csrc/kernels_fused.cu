@@ -275,6 +275,10 @@ __global__ void __launch_bounds__(NT, HBK_SELL_MINB) k_seed_s<HBK_FMT_SELL>(Ctx 
     seed_s_body<HBK_FMT_SELL>(c, HwGrid());
 }
 template <>
+__global__ void __launch_bounds__(NT, HBK_HYBW_MINB) k_seed_s<HBK_FMT_HYBW>(Ctx c) {
+    seed_s_body<HBK_FMT_HYBW>(c, HwGrid());
+}
+template <>
 __global__ void __launch_bounds__(NT, HBK_HYB_MINB) k_seed_s<HBK_FMT_HYB>(Ctx c) {
     seed_s_body<HBK_FMT_HYB>(c, HwGrid());
 }
@@ -373,6 +377,10 @@ __global__ void __launch_bounds__(NT) k_seed_y(Ctx c) { seed_y_body<FMT>(c, HwGr
 template <>
 __global__ void __launch_bounds__(NT, HBK_SELL_MINB) k_seed_y<HBK_FMT_SELL>(Ctx c) {
     seed_y_body<HBK_FMT_SELL>(c, HwGrid());
+}
+template <>
+__global__ void __launch_bounds__(NT, HBK_HYBW_MINB) k_seed_y<HBK_FMT_HYBW>(Ctx c) {
+    seed_y_body<HBK_FMT_HYBW>(c, HwGrid());
 }
 template <>
 __global__ void __launch_bounds__(NT, HBK_HYB_MINB) k_seed_y<HBK_FMT_HYB>(Ctx c) {
@@ -1437,8 +1445,9 @@ int hbk_fused_init(const hbk_matrix *A, const hbk_vectors *v, const hbk_shifts *
     return (int)cudaGetLastError();
 }
 
-int hbk_hyb_wave_fused(void) {
-    const int a = wave_grid<k_seed_s<HBK_FMT_HYB>>(HBK_MAX_GRID), b = wave_grid<k_seed_y<HBK_FMT_HYB>>(HBK_MAX_GRID);
+int hbk_hyb_wave_fused(int wide) {
+    const int a = wide ? wave_grid<k_seed_s<HBK_FMT_HYBW>>(HBK_MAX_GRID) : wave_grid<k_seed_s<HBK_FMT_HYB>>(HBK_MAX_GRID);
+    const int b = wide ? wave_grid<k_seed_y<HBK_FMT_HYBW>>(HBK_MAX_GRID) : wave_grid<k_seed_y<HBK_FMT_HYB>>(HBK_MAX_GRID);
     return a < b ? a : b;
 }
 
@@ -1508,6 +1517,7 @@ int hbk_fused_iteration(const hbk_matrix *A, const hbk_vectors *v, const hbk_shi
     Ctx c = make_ctx(A, v, sh);
     if (A->fmt == HBK_FMT_SELL) launch_iteration<HBK_FMT_SELL>(c, A, early, st);
     else if (A->fmt == HBK_FMT_MERGE) launch_iteration<HBK_FMT_MERGE>(c, A, early, st);
+    else if (A->fmt == HBK_FMT_HYB && A->nwide) launch_iteration<HBK_FMT_HYBW>(c, A, early, st);
     else if (A->fmt == HBK_FMT_HYB) launch_iteration<HBK_FMT_HYB>(c, A, early, st);
     else launch_iteration<HBK_FMT_TILE>(c, A, early, st);
     return (int)cudaGetLastError();

@@ -91,6 +91,18 @@ int hbicg__hyb_plan(size_t ni, const unsigned *cost, unsigned hnw, unsigned *hwb
  * its 32 lengths in one line instead of 64 scattered row pointers.  One
  * allocation holds each long row's entry range, the long rows, and the warp
  * work lists (hbicg__hyb_plan) for one wave of the kernels that take this form. */
+/* grid of the HYB kernels: one wave of the heaviest, so every warp of a
+ * launch runs exactly one list; fewer where rows (with block rows: where
+ * nonzeros, 4 per thread) leave blocks without work */
+static int hyb_grid_for(const unsigned *h_ptr, unsigned n, int wide) {
+    const unsigned by_rows = (n + HBK_THREADS - 1) / HBK_THREADS, by_nnz = h_ptr[n] / (4u * HBK_THREADS) + 1u;
+    int g = hbk_spmv_grid(wide && by_nnz > by_rows ? by_nnz : by_rows);
+    const int wf = hbk_hyb_wave_fused(wide), wb = hbk_hyb_wave_blas(wide);
+    if (wf < g) g = wf;
+    if (wb < g) g = wb;
+    return g < 1 ? 1 : g;
+}
+
 static int build_hyb(hbicg_matrix *A, const unsigned *h_ptr, unsigned n) {
     cudaStream_t st = A->ctx->stream;
     if (!n || A->d_hval) return HBICG_OK;
@@ -111,24 +123,31 @@ static int build_hyb(hbicg_matrix *A, const unsigned *h_ptr, unsigned n) {
     const size_t srow_bytes = sizeof(unsigned) * (cap + 1) + cap + 1;
     unsigned *srow = malloc(srow_bytes);
     unsigned long long *wkey = malloc(sizeof(unsigned long long) * (nw + 1));
-    /* grid of the HYB kernels: one wave of the heaviest, so every warp of a
-     * launch runs exactly one list */
-    int hgrid = hbk_spmv_grid((n + HBK_THREADS - 1) / HBK_THREADS);
-    {
-        const int wf = hbk_hyb_wave_fused(), wb = hbk_hyb_wave_blas();
-        if (wf < hgrid) hgrid = wf;
-        if (wb < hgrid) hgrid = wb;
-        if (hgrid < 1) hgrid = 1;
-    }
-    const unsigned hnw = (unsigned)hgrid * (HBK_THREADS / 32);
     /* long rows by lanes per row (longest first, so each class is a range) */
     size_t r32 = 0, r16 = 0;
+    unsigned maxlen = 0;
     for (unsigned r = 0; r < n; ++r) {
         const unsigned len = h_ptr[r + 1] - h_ptr[r];
         r32 += len > HBK_HYB_L16;
         r16 += len > HBK_HYB_L4;
+        if (len > maxlen) maxlen = len;
     }
-    const size_t it16 = r32, it4 = it16 + (r16 - r32 + 1) / 2, itl = it4 + (nw - r16 + 7) / 8;
+    int hgrid = hyb_grid_for(h_ptr, n, 0);
+    /* Does the longest row outlast the lists?  Its steps against the mean
+     * list's (a slice costs about a step per entry of its rows, a long row one
+     * per 32 entries): if so, the rows above HBK_HYB_L16 take a block each
+     * (spmv_rows_hyb).  Measured, one product of power-law rows, warps only
+     * against block rows: n = 20 k 32.8 / 12.3 us, 60 k 36.9 / 14.4, 300 k
+     * 51.2 / 30.4, 600 k (longest row 1.4 mean lists) 85.7 / 62.5, 1 M (0.8)
+     * 91.8 / 94.5, 2 M (0.4) 152.9 / 175.9. */
+    const double mean = ((double)h_ptr[n] / 32.0 + 6.0 * (double)ns + 7.0 * (double)nw) /
+                        ((double)hgrid * (HBK_THREADS / 32));
+    size_t nwide = 0;
+    if (maxlen > HBK_HYB_L16 && (double)maxlen / 32.0 > mean) nwide = r32;
+    if (nwide) hgrid = hyb_grid_for(h_ptr, n, 1);
+    const unsigned hnw = (unsigned)hgrid * (HBK_THREADS / 32);
+    /* items: none for the rows that take a block */
+    const size_t it16 = r32 - nwide, it4 = it16 + (r16 - r32 + 1) / 2, itl = it4 + (nw - r16 + 7) / 8;
     const size_t ni = itl + ns;
     /* [2 nw] entry ranges, [nw] rows, [hnw + 1] list starts, [ni] items */
     const size_t plan_words = 3 * nw + hnw + 1 + ni;
@@ -187,6 +206,7 @@ static int build_hyb(hbicg_matrix *A, const unsigned *h_ptr, unsigned n) {
         /* item costs: a header (2 for rows, 3 for a slice), one step per g
          * entries of the group's longest row (the first: rows are longest
          * first) or per entry of the slice, and log2 g steps of the tree */
+        const unsigned batch = nwide ? 4u : 1u; /* entries whose loads a lane has in flight at once */
         for (size_t k = 0; k < ni; ++k) {
             unsigned first, g, tree;
             if (k < it16) {
@@ -196,10 +216,10 @@ static int build_hyb(hbicg_matrix *A, const unsigned *h_ptr, unsigned n) {
             } else if (k < itl) {
                 first = (unsigned)(r16 + 8 * (k - it4)), g = 4, tree = 2;
             } else {
-                cost[k] = 3u + (unsigned)((sp[k - itl + 1] - sp[k - itl]) / 32);
+                cost[k] = 3u + (unsigned)((sp[k - itl + 1] - sp[k - itl]) / 32 + batch - 1) / batch;
                 continue;
             }
-            cost[k] = 2u + (wrng[2 * first + 1] - wrng[2 * first] + g - 1) / g + tree;
+            cost[k] = 2u + (wrng[2 * first + 1] - wrng[2 * first] + g * batch - 1) / (g * batch) + tree;
         }
         rc = hbicg__hyb_plan(ni, cost, hnw, wrow + nw, wrow + nw + hnw + 1);
         if (rc) goto done;
@@ -232,6 +252,7 @@ static int build_hyb(hbicg_matrix *A, const unsigned *h_ptr, unsigned n) {
     A->nwrow = (unsigned)nw;
     A->slen_off = cap + 1;
     A->hnw = hnw;
+    A->nwide = (unsigned)nwide;
     A->hyb_grid = hgrid;
     A->hrow32 = (unsigned)r32;
     A->hrow16 = (unsigned)r16;
@@ -276,6 +297,7 @@ static void use_hyb(hbicg_matrix *A) {
     A->k.hwbeg = A->k.wrow ? A->k.wrow + A->nwrow : NULL;
     A->k.hitem = A->k.hwbeg ? A->k.hwbeg + A->hnw + 1 : NULL;
     A->k.hnw = A->hnw;
+    A->k.nwide = A->nwide;
     A->k.hrow32 = A->hrow32;
     A->k.hrow16 = A->hrow16;
     A->k.hit16 = A->hit16;
