@@ -35,6 +35,18 @@
 // and p.  Every wait is bounded: a timeout sets an error flag, the CTA skips
 // its remaining work and still frees its TMEM.
 //
+// What bounds it (clock stamps, n = 2 M, 64 shifts, 59 slots; about 15 k clocks
+// per tile): the epilogue warps are busy for all but 1.5 k of them (rounding,
+// own terms and stores 9.5 k, of which the FP64 pipe 6.1 k, draining 2.1 k,
+// loads 1.8 k) and the builders for nearly all (digits 6.1 k, waiting for
+// their loads 3.5 k); both share the SM quarters' integer pipes, and the tensor
+// core waits 8.5 k.  So instructions count: digits as packed BF16 pairs,
+// unconditional basis loads and a rounding whose rare cases are out of line
+// took a flush from 2.62 to 2.49 ms.  Tried and not kept: x + y of two columns
+// in one FP64 add through shuffles (2.68), rounding the next columns before
+// each store (3.08), a fourth builder warp (2.71), prefetching the basis to
+// L2 (no change).
+//
 // Only the live shifts are formed: a shift that had converged by the previous
 // flush has zero coefficients and own terms (0, 1) since that flush's reset,
 // so its rows would come out unchanged.  The rows of a group are the live
@@ -165,16 +177,17 @@ __device__ __forceinline__ int exp_of_bits(uint64_t bits) {
 // (|v| < 2^scale, so the result is below 2^62), plus DIGIT_BIAS.  The
 // significand M < 2^53 is placed at M 2^10 and shifted right by
 // r = 1023 + scale - max(eb, 1) >= 0 (|v| < 2^scale bounds the left shift
-// M 2^(62 - scale + eb - 1075) by 2^10).
+// M 2^(62 - scale + eb - 1075) by 2^10); M 2^10 < 2^63, so a shift by 63
+// stands for every longer one.
 __device__ __forceinline__ uint64_t biased62(uint64_t bits, int scale) {
-    const int eb = (int)((bits >> 52) & 0x7ff);
-    const uint64_t frac = bits & ((1ull << 52) - 1);
-    const uint64_t M = eb ? (frac | (1ull << 52)) : frac;
-    const int r = 1023 + scale - (eb ? eb : 1);
-    uint64_t q = r < 64 ? (M << 10) >> r : 0;
+    const uint32_t hi = (uint32_t)(bits >> 32);
+    const int eb = (int)((hi >> 20) & 0x7ffu);
+    const uint32_t mh = (hi & 0xfffffu) | (eb ? 1u << 20 : 0u);
+    const uint64_t M = ((uint64_t)mh << 32) | (uint32_t)bits;
+    const int r = 1023 + scale - max(eb, 1);
+    const uint64_t q = (M << 10) >> min(r, 63);
     const uint64_t sg = (uint64_t)((int64_t)bits >> 63);  // 0 or all ones
-    q = (q ^ sg) - sg;
-    return q + DIGIT_BIAS;
+    return (q ^ sg) + DIGIT_BIAS + (hi >> 31);            // -q = ~q + 1
 }
 
 // balanced digit s (weight 2^(56 - 7 s)) of a biased value, as an exact float
@@ -184,9 +197,17 @@ __device__ __forceinline__ float digit(uint64_t U) {
     return __uint_as_float(0x4B000000u | e) - 8388672.0f;  // (2^23 + e) - (2^23 + 64)
 }
 
+// the same digits of two values as a BF16 pair: digit + 64 is at most 128, and
+// BF16 0x4300 + e is 128 + e for e = 0..128 (seven fraction bits), so one packed
+// subtraction of 192 leaves the digits, exact
 template <int S>
 __device__ __forceinline__ uint32_t digit_pair(uint64_t U0, uint64_t U1) {
-    const __nv_bfloat162 h = __floats2bfloat162_rn(digit<S>(U0), digit<S>(U1));
+    constexpr int sh = 56 - 7 * S;
+    constexpr uint32_t mask = S == 0 ? 0x00ff00ffu : 0x007f007fu;
+    const uint32_t x0 = (uint32_t)(U0 >> sh);
+    const uint32_t x1 = sh >= 16 ? (uint32_t)(U1 >> (sh >= 16 ? sh - 16 : 0)) : (uint32_t)U1 << (sh >= 16 ? 0 : 16 - sh);
+    const uint32_t e = (__byte_perm(x0, x1, 0x7610) & mask) | 0x43004300u;
+    const __nv_bfloat162 h = __hsub2(*reinterpret_cast<const __nv_bfloat162 *>(&e), __nv_bfloat162{192.0f, 192.0f});
     return *reinterpret_cast<const uint32_t *>(&h);
 }
 
@@ -223,10 +244,12 @@ __device__ __forceinline__ long long diag_sum(const uint32_t (&B)[NDIAG]) {
 }
 
 // T 2^k rounded to FP64: round half up on the 64-bit magnitude, whose leading
-// bit is normalised to bit 63 (error <= 0.5 ulp of the result)
-__device__ __forceinline__ double join_t(long long T, int k) {
-    const long long sg = T >> 63;
-    const unsigned long long a = (unsigned long long)((T ^ sg) - sg);
+// bit is normalised to bit 63 (error <= 0.5 ulp of the result).  The common
+// case has a bit set in T's upper word and a normal result; the rest (zero
+// rows, results near the ends of the range) is out of line.
+__device__ __noinline__ double join_rest(long long T, int k) {
+    const unsigned long long sg = (unsigned long long)(T >> 63);
+    const unsigned long long a = ((unsigned long long)T ^ sg) - sg;
     if (a == 0) return 0.0;
     const int z = __clzll((long long)a);
     const unsigned long long W = a << z;
@@ -237,7 +260,19 @@ __device__ __forceinline__ double join_t(long long T, int k) {
         return sg ? -INFINITY : INFINITY;
     }
     const unsigned long long bits = ((unsigned long long)ebm1 << 52) + mant;
-    return __longlong_as_double((long long)(bits | ((unsigned long long)sg << 63)));
+    return __longlong_as_double((long long)(bits | (sg << 63)));
+}
+__device__ __forceinline__ double join_t(long long T, int k) {
+    const unsigned long long sg = (unsigned long long)(T >> 63);
+    const unsigned long long a = ((unsigned long long)T ^ sg) - sg;
+    const unsigned ah = (unsigned)(a >> 32);
+    const int z = __clz((int)ah);
+    const int ebm1 = 1085 - z + k;
+    if (ah == 0 || (unsigned)ebm1 > 2044u) return join_rest(T, k);
+    const unsigned long long W = a << z;
+    const unsigned long long mant = (W >> 11) + (((unsigned)W >> 10) & 1u);
+    const unsigned hi = (unsigned)(mant >> 32) + ((unsigned)ebm1 << 20);
+    return __hiloint2double((int)(hi | ((unsigned)sg & 0x80000000u)), (int)(unsigned)mant);
 }
 
 // one 32-byte sector per lane and instruction (x and p rows are read and
@@ -413,7 +448,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_flush_tc(TcArgs a) {
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
     if (tid < TC_K) {
-        const unsigned long long sm = tid < a.L ? a.slot_max[tid] : 0ull;
+        const unsigned long long sm = a.slot_max[tid < a.L ? tid : a.L - 1];  // (past L: slot L - 1 again)
         s_slotexp[tid] = sm ? exp_of_bits(sm) : 0;
     }
     if (tid < TC_M) {
@@ -474,16 +509,26 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_flush_tc(TcArgs a) {
             io[u] = it / TC_N;
             ii[u] = it % TC_N;
         }
+        // Every load is unconditional: slots past L read slot L - 1 again (their
+        // coefficient digits are zero, and with slot L - 1's exponent they do
+        // not move the element's), elements past n read element n - 1.
         double v[ITEMS_PER][8];
+        const double *vcol[ITEMS_PER];
+        uint32_t wmax[ITEMS_PER];
+#pragma unroll
+        for (int u = 0; u < ITEMS_PER; ++u) {
+            const int l0 = min(8 * io[u], a.L - 1);
+            vcol[u] = a.V + (size_t)l0 * ld;
+            wmax[u] = (uint32_t)min(7, a.L - 1 - l0);
+        }
+        const uint32_t ld32 = (uint32_t)ld;
         auto load_tile = [&](unsigned t) {
-            const unsigned i0 = t * TC_N;
 #pragma unroll
-            for (int u = 0; u < ITEMS_PER; ++u)
+            for (int u = 0; u < ITEMS_PER; ++u) {
+                const double *p = vcol[u] + min(t * TC_N + ii[u], n - 1);
 #pragma unroll
-                for (int w = 0; w < 8; ++w) {
-                    const int l = 8 * io[u] + w;
-                    v[u][w] = (l < a.L && i0 + ii[u] < n) ? __ldcs(a.V + (size_t)l * ld + i0 + ii[u]) : 0.0;
-                }
+                for (uint32_t w = 0; w < 8; ++w) v[u][w] = __ldcs(p + (uint64_t)min(w, wmax[u]) * ld32);
+            }
         };
         int it = 0;
         if (blockIdx.x < ntiles) load_tile(blockIdx.x);
@@ -495,13 +540,17 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_flush_tc(TcArgs a) {
             int em[ITEMS_PER];
 #pragma unroll
             for (int u = 0; u < ITEMS_PER; ++u) {
+                const int4 *sx = reinterpret_cast<const int4 *>(s_slotexp + 8 * io[u]);
+                const int4 sa = sx[0], sb = sx[1];
+                const int se[8] = {sa.x, sa.y, sa.z, sa.w, sb.x, sb.y, sb.z, sb.w};
                 int e = EXP_NONE;
 #pragma unroll
                 for (int w = 0; w < 8; ++w) {
                     // |v| < 2^(eb - 1022) for every v, zero and subnormals included
-                    const int eb = (int)((uint64_t)__double_as_longlong(v[u][w]) >> 52) & 0x7ff;
-                    e = max(e, eb - 1022 - s_slotexp[8 * io[u] + w]);
+                    const int eb = (__double2hiint(v[u][w]) >> 20) & 0x7ff;
+                    e = max(e, eb - se[w]);
                 }
+                e -= 1022;
                 em[u] = e;
                 cexp[io[u] * TC_N + ii[u]] = e;
             }
@@ -528,10 +577,13 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_flush_tc(TcArgs a) {
             unsigned char *sBt = sB + (it & 1) * B_BYTES;
 #pragma unroll
             for (int u = 0; u < ITEMS_PER; ++u) {
+                const int4 *sx = reinterpret_cast<const int4 *>(s_slotexp + 8 * io[u]);
+                const int4 sa = sx[0], sb = sx[1];
+                const int se[8] = {sa.x, sa.y, sa.z, sa.w, sb.x, sb.y, sb.z, sb.w};
                 uint64_t U[8];
 #pragma unroll
                 for (int w = 0; w < 8; ++w)
-                    U[w] = biased62((uint64_t)__double_as_longlong(v[u][w]), Fv[u] + s_slotexp[8 * io[u] + w]);
+                    U[w] = biased62((uint64_t)__double_as_longlong(v[u][w]), Fv[u] + se[w]);
                 if (io[u] == 0) s_F[(it & 3) * TC_N + ii[u]] = Fv[u];
                 store_digits<0>(sBt, umma_off(ii[u], 8 * io[u]), U);
             }
@@ -639,7 +691,6 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_flush_tc(TcArgs a) {
         double *const pbase =
             live && (which == 0 || a.Pmat) ? (which ? a.Pmat : a.X) + (size_t)j * TC_N + cg * EPI_COLS : nullptr;
         const size_t pstride = (size_t)a.m * TC_N;
-        const bool have_p = a.Pmat != nullptr;
         // x and p values of a tile, loaded one tile ahead: the loads are in
         // flight while the warp waits for that tile's MMAs and drains them.
         // 32-byte sector accesses (pieces are 16 values from a 32-byte aligned base)
@@ -701,9 +752,10 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_flush_tc(TcArgs a) {
                 double o4[4];
 #pragma unroll
                 for (int h = 0; h < 4; ++h) {
-                    const double G = E != EXP_NONE ? join_t(T[u + h], E + Fc[u + h] - 56) : 0.0;
+                    // (a row of zero coefficients has T = 0)
+                    const double G = join_t(T[u + h], E + Fc[u + h] - 56);
                     const double po = __shfl_xor_sync(0xffffffffu, pv[u + h], 16);
-                    const double pold = which ? pv[u + h] : (have_p ? po : 0.0);
+                    const double pold = which ? pv[u + h] : po;  // (0 without a Pmat: pv is then)
                     const double y = fma(own, pold, G);
                     o4[h] = which ? y : pv[u + h] + y;
                 }
