@@ -183,6 +183,8 @@ typedef struct {
 
 /* ---- plain BLAS-1 and SpMV kernels (one launch per reference step) ---- */
 int hbk_copy(unsigned n, const double *x, double *y, cudaStream_t st);
+/* m rows of n values, leading dimensions ldx and ldy */
+int hbk_copy_rows(int m, unsigned n, const double *x, size_t ldx, double *y, size_t ldy, cudaStream_t st);
 int hbk_zero(unsigned n, double *x, cudaStream_t st);
 int hbk_axpy(unsigned n, double a, const double *x, double *y, cudaStream_t st);
 int hbk_scal(unsigned n, double a, double *x, cudaStream_t st);
@@ -262,10 +264,6 @@ int hbk_group_run(int nf, const hbk_matrix *A, const hbk_vectors *v, const hbk_s
 void hbk_group_test_withhold(int on);
 /* deferred mode: x_j (and p_j when keep_p) = coefficients x basis, then reset the basis */
 int hbk_deferred_flush(const hbk_vectors *v, const hbk_shifts *sh, int keep_p, cudaStream_t st);
-/* ||b - (A + sigma_j I) x_j||^2 for every shift into out[m] (device) */
-int hbk_true_residuals(const hbk_matrix *A, const double *X, const double *b, const double *sigma, int m,
-                       double *partials, unsigned *counter, double *out, cudaStream_t st);
-
 /* basis flush on the tensor cores (flush_tc.cu): x_j += xi_j Pmat_j + Xc_j . V,
  * p_j = rho_j Pmat_j + Pc_j . V over the first L <= hbk_flush_tc_max_slots()
  * slots, FP64-accurate; X and Pmat panel-major (HBK_PANEL) with m systems;
@@ -306,7 +304,8 @@ int hbk_panel_to_rows(const double *Xp, int m, unsigned n, double *X, size_t ld,
 /* after a flush: zero the coefficients, own = (0, keep_p), basis slot 0 = r_{k-1} */
 int hbk_deferred_reset(const hbk_vectors *v, const hbk_shifts *sh, int keep_p, cudaStream_t st);
 
-/* the same with an explicit leading dimension of X and at most grid_cap blocks */
+/* ||b - (A + sigma_j I) x_j||^2 for every shift into out[m] (device): leading
+ * dimension ldx of X, at most grid_cap blocks per shift */
 int hbk_true_residuals_ld(const hbk_matrix *A, const double *X, size_t ldx, const double *b, const double *sigma,
                           int m, int grid_cap, double *partials, unsigned *counters, double *out, cudaStream_t st);
 

@@ -13,6 +13,14 @@ __global__ void __launch_bounds__(NT) k_copy(unsigned n, const double *__restric
     for (size_t i = blockIdx.x * (size_t)NT + threadIdx.x; i < n; i += (size_t)gridDim.x * NT) y[i] = x[i];
 }
 
+// m rows of n values between leading dimensions
+__global__ void __launch_bounds__(NT) k_copy_rows(unsigned n, const double *__restrict__ x, size_t ldx,
+                                                  double *__restrict__ y, size_t ldy) {
+    x += blockIdx.y * ldx;
+    y += blockIdx.y * ldy;
+    for (size_t i = blockIdx.x * (size_t)NT + threadIdx.x; i < n; i += (size_t)gridDim.x * NT) y[i] = x[i];
+}
+
 __global__ void __launch_bounds__(NT) k_fill(unsigned n, double v, double *__restrict__ x) {
     for (size_t i = blockIdx.x * (size_t)NT + threadIdx.x; i < n; i += (size_t)gridDim.x * NT) x[i] = v;
 }
@@ -279,6 +287,15 @@ int hbk_copy(unsigned n, const double *x, double *y, cudaStream_t st) {
     return (int)cudaGetLastError();
 }
 
+int hbk_copy_rows(int m, unsigned n, const double *x, size_t ldx, double *y, size_t ldy, cudaStream_t st) {
+    for (int j = 0; n && j < m; j += 32768) {
+        const int rows = m - j < 32768 ? m - j : 32768;
+        k_copy_rows<<<dim3((unsigned)grid_for(n, 4), (unsigned)rows), NT, 0, st>>>(n, x + (size_t)j * ldx, ldx,
+                                                                                   y + (size_t)j * ldy, ldy);
+    }
+    return (int)cudaGetLastError();
+}
+
 int hbk_fill(unsigned n, double v, double *x, cudaStream_t st) {
     if (!n) return 0;
     k_fill<<<grid_for(n, 4), NT, 0, st>>>(n, v, x);
@@ -355,15 +372,6 @@ int hbk_spmv(const hbk_matrix *A, const double *x, double *y, double sigma, int 
 int hbk_spmv_accumulate(const hbk_matrix *A, const double *x, double *y, cudaStream_t st) {
     if (!A->n) return 0;
     HBK_LAUNCH_FMT(*A, k_spmv_acc, product_grid(A), NT, st, *A, x, y);
-    return (int)cudaGetLastError();
-}
-
-int hbk_true_residuals(const hbk_matrix *A, const double *X, const double *b, const double *sigma, int m,
-                       double *partials, unsigned *counters, double *out, cudaStream_t st) {
-    if (!A->n || m <= 0) return 0;
-    size_t ld = ((size_t)A->n + 31) / 32 * 32;
-    dim3 grid(product_grid(A), m);
-    HBK_LAUNCH_FMT(*A, k_true_res, grid, NT, st, *A, X, ld, b, sigma, partials, counters, out);
     return (int)cudaGetLastError();
 }
 

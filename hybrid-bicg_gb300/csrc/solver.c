@@ -171,6 +171,10 @@ struct hbicg_solver {
     int *d_tc_err;    /* set by the tensor-core flush on a bounded-wait timeout */
     int launches_per_iter;
     double flush_bytes; /* compulsory HBM bytes of this solve's basis flushes */
+    /* where this solve's x_j end up, rows xld apart: the workspace's X, or the
+     * caller's device array (the deferred mode writes rows straight into it) */
+    double *xrows;
+    size_t xld;
     /* deferred mode, pinned host x: solutions that became final at a flush
      * are copied out while the solve goes on */
     double *early_x;        /* the caller's x (host, pinned), or NULL */
@@ -824,7 +828,7 @@ static int fused_tail(hbicg_solver *s, int k_flushed, int *launches, double *flu
             CUDA_TRY(cudaEventRecord(s->ctx->cev, s->ctx->cstream));
             CUDA_TRY(cudaStreamWaitEvent(st, s->ctx->cev, 0));
         }
-        HBK_TRY(hbk_panel_to_rows(s->v.Xp, s->v.pm, s->A->k.n, s->v.X, s->ld, st));
+        HBK_TRY(hbk_panel_to_rows(s->v.Xp, s->v.pm, s->A->k.n, s->xrows, s->xld, st));
         ++*launches;
         CUDA_TRY(cudaMemcpyAsync(h, s->d_sc, sizeof(hbk_scalars), cudaMemcpyDeviceToHost, st));
         int tc_err = 0;
@@ -1042,7 +1046,6 @@ static int refine_shifts(hbicg_solver *s, const double *h_sigma, int *refined, u
     cudaStream_t st = s->ctx->stream;
     const unsigned n = s->A->k.n;
     const int m = s->m;
-    const size_t ld = s->ld;
     double *h = malloc(sizeof(double) * (size_t)m), *r = NULL, *e = NULL;
     hbicg_solver *sub = NULL;
     int rc = HBICG_OK;
@@ -1052,8 +1055,8 @@ static int refine_shifts(hbicg_solver *s, const double *h_sigma, int *refined, u
     CUDA_GOTO(cudaStreamSynchronize(st));
     const double bn = sqrt(s->ctx->h_dbl[0]);
     for (int round = 0; round < 3 && rc == HBICG_OK && bn > 0.0; ++round) {
-        HBK_GOTO(hbk_true_residuals(&s->A->k, s->v.X, s->d_b, s->d_sigma, m, s->sh.partials, s->sh.counters + 16,
-                                   s->d_res, st));
+        HBK_GOTO(hbk_true_residuals_ld(&s->A->k, s->xrows, s->xld, s->d_b, s->d_sigma, m, HBK_MAX_GRID, s->sh.partials,
+                                       s->sh.counters + 16, s->d_res, st));
         CUDA_GOTO(cudaMemcpyAsync(h, s->d_res, sizeof(double) * (size_t)m, cudaMemcpyDeviceToHost, st));
         CUDA_GOTO(cudaStreamSynchronize(st));
         int any = 0;
@@ -1072,7 +1075,7 @@ static int refine_shifts(hbicg_solver *s, const double *h_sigma, int *refined, u
                 p1.shift_mode = HBICG_SHIFTS_INCREMENTAL;
                 if ((rc = hbicg_solver_create(s->ctx, s->A, 1, &p1, &sub)) != HBICG_OK) break;
             }
-            double *xj = s->v.X + (size_t)j * ld;
+            double *xj = s->xrows + (size_t)j * s->xld;
             HBK_GOTO(hbk_spmv(&s->A->k, xj, e, h_sigma[j], 1, st)); /* e = (A + sigma_j I) x_j */
             HBK_GOTO(hbk_copy(n, s->d_b, r, st));
             HBK_GOTO(hbk_axpy(n, -1.0, e, r, st));                   /* r = b - e */
@@ -1187,6 +1190,12 @@ static int run_begin(hbicg_solver *s, const double *b, const double *sigma, run_
     s->early = NULL;
     if (s->p.form != HBICG_FORM_PLAIN && s->v.deferred && x_pinned && (s->early = calloc((size_t)m, 1)) != NULL)
         s->early_x = x;
+    s->xrows = s->v.X;
+    s->xld = s->ld;
+    if (s->p.form != HBICG_FORM_PLAIN && s->v.deferred && out_where == HBICG_DEVICE && x) {
+        s->xrows = x;
+        s->xld = n;
+    }
     CUDA_TRY(cudaEventRecord(ctx->ev0, st));
     s->flush_bytes = 0.0;
     r->k = 1;
@@ -1281,8 +1290,14 @@ static int run_end(hbicg_solver *s, run_t *r, int rc) {
                 if (!s->early[j] || fixed[j])
                     CUDA_TRY(cudaMemcpyAsync(x + (size_t)j * n, s->v.X + (size_t)j * s->ld, sizeof(double) * n,
                                              kout, st));
+        } else if (s->xrows == x) {
+            /* already there */
+        } else if (s->xld == n) { /* (a two-dimensional copy on the device runs at 0.6 TB/s) */
+            CUDA_TRY(cudaMemcpyAsync(x, s->xrows, sizeof(double) * (size_t)n * (size_t)m, kout, st));
+        } else if (out_where == HBICG_DEVICE) {
+            HBK_TRY(hbk_copy_rows(m, n, s->xrows, s->xld, x, n, st));
         } else {
-            CUDA_TRY(cudaMemcpy2DAsync(x, sizeof(double) * n, s->v.X, sizeof(double) * s->ld, sizeof(double) * n, m,
+            CUDA_TRY(cudaMemcpy2DAsync(x, sizeof(double) * n, s->xrows, sizeof(double) * s->xld, sizeof(double) * n, m,
                                        kout, st));
         }
     }
@@ -1290,8 +1305,8 @@ static int run_end(hbicg_solver *s, run_t *r, int rc) {
     double maxres = 0.0;
     double *h_res = NULL;
     if (rc == HBICG_OK && s->p.true_residuals && m > 0) {
-        HBK_TRY(hbk_true_residuals(&s->A->k, s->v.X, s->d_b, s->d_sigma, m, s->sh.partials, s->sh.counters + 16,
-                                   s->d_res, st));
+        HBK_TRY(hbk_true_residuals_ld(&s->A->k, s->xrows, s->xld, s->d_b, s->d_sigma, m, HBK_MAX_GRID, s->sh.partials,
+                                      s->sh.counters + 16, s->d_res, st));
         HBK_TRY(hbk_dot(n, s->d_b, s->d_b, s->sh.partials, s->sh.counters + 7, s->d_dot, st));
         if (!(h_res = hb->h_res = malloc(sizeof(double) * m))) {
             set_msg("host scratch of %d residuals", m);
