@@ -40,11 +40,11 @@
 // own terms and stores 9.5 k, of which the FP64 pipe 6.1 k, draining 2.1 k,
 // loads 1.8 k) and the builders for nearly all (digits 6.1 k, waiting for
 // their loads 3.5 k); both share the SM quarters' integer pipes, and the tensor
-// core waits 8.5 k.  So instructions count: digits as packed BF16 pairs,
-// unconditional basis loads and a rounding whose rare cases are out of line
-// took a flush from 2.62 to 2.49 ms.  Tried and not kept: x + y of two columns
-// in one FP64 add through shuffles (2.68), rounding the next columns before
-// each store (3.08), a fourth builder warp (2.71), prefetching the basis to
+// core waits 8.5 k.  So instructions count: digits as packed BF16 pairs, basis
+// loads with fewer conditions and a rounding whose rare cases are out of line
+// took a flush from 2.49 to 2.20 ms (256^3, all shifts live: 19.5 to 17.2).  Tried and not kept: x + y of two columns
+// in one FP64 add through shuffles (+3 %), rounding the next columns before
+// each store (+20 %), a fourth builder warp (+7 %), prefetching the basis to
 // L2 (no change).
 //
 // Only the live shifts are formed: a shift that had converged by the previous
@@ -245,8 +245,9 @@ __device__ __forceinline__ long long diag_sum(const uint32_t (&B)[NDIAG]) {
 
 // T 2^k rounded to FP64: round half up on the 64-bit magnitude, whose leading
 // bit is normalised to bit 63 (error <= 0.5 ulp of the result).  The common
-// case has a bit set in T's upper word and a normal result; the rest (zero
-// rows, results near the ends of the range) is out of line.
+// cases are T = 0 (every column of a row without coefficients) and a bit set in
+// T's upper word with a normal result; the rest (results near the ends of the
+// range) is out of line.
 __device__ __noinline__ double join_rest(long long T, int k) {
     const unsigned long long sg = (unsigned long long)(T >> 63);
     const unsigned long long a = ((unsigned long long)T ^ sg) - sg;
@@ -268,10 +269,10 @@ __device__ __forceinline__ double join_t(long long T, int k) {
     const unsigned ah = (unsigned)(a >> 32);
     const int z = __clz((int)ah);
     const int ebm1 = 1085 - z + k;
-    if (ah == 0 || (unsigned)ebm1 > 2044u) return join_rest(T, k);
+    if (ah == 0 ? (unsigned)a != 0u : (unsigned)ebm1 > 2044u) return join_rest(T, k);
     const unsigned long long W = a << z;
     const unsigned long long mant = (W >> 11) + (((unsigned)W >> 10) & 1u);
-    const unsigned hi = (unsigned)(mant >> 32) + ((unsigned)ebm1 << 20);
+    const unsigned hi = ah ? (unsigned)(mant >> 32) + ((unsigned)ebm1 << 20) : 0u;
     return __hiloint2double((int)(hi | ((unsigned)sg & 0x80000000u)), (int)(unsigned)mant);
 }
 
@@ -509,9 +510,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_flush_tc(TcArgs a) {
             io[u] = it / TC_N;
             ii[u] = it % TC_N;
         }
-        // Every load is unconditional: slots past L read slot L - 1 again (their
-        // coefficient digits are zero, and with slot L - 1's exponent they do
-        // not move the element's), elements past n read element n - 1.
+        // slots past L read as zero (with slot L - 1's exponent they do not move
+        // the element's), elements past n as element n - 1 (never stored)
         double v[ITEMS_PER][8];
         const double *vcol[ITEMS_PER];
         uint32_t wmax[ITEMS_PER];
@@ -519,7 +519,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_flush_tc(TcArgs a) {
         for (int u = 0; u < ITEMS_PER; ++u) {
             const int l0 = min(8 * io[u], a.L - 1);
             vcol[u] = a.V + (size_t)l0 * ld;
-            wmax[u] = (uint32_t)min(7, a.L - 1 - l0);
+            wmax[u] = (uint32_t)min(7, a.L - 1 - l0);  // (an octet past L: slot L - 1 again, against zero digits)
         }
         const uint32_t ld32 = (uint32_t)ld;
         auto load_tile = [&](unsigned t) {
@@ -527,7 +527,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_flush_tc(TcArgs a) {
             for (int u = 0; u < ITEMS_PER; ++u) {
                 const double *p = vcol[u] + min(t * TC_N + ii[u], n - 1);
 #pragma unroll
-                for (uint32_t w = 0; w < 8; ++w) v[u][w] = __ldcs(p + (uint64_t)min(w, wmax[u]) * ld32);
+                for (uint32_t w = 0; w < 8; ++w) v[u][w] = w <= wmax[u] ? __ldcs(p + (uint64_t)w * ld32) : 0.0;
             }
         };
         int it = 0;

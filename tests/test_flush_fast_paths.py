@@ -60,18 +60,18 @@ def _join_short(T, k):
     a, ah = abs(T), abs(T) >> 32
     z = 32 - ah.bit_length()
     e = 1085 - z + k
-    if ah == 0 or not 0 <= e <= 2044:
+    if a != 0 if ah == 0 else not 0 <= e <= 2044:
         return None  # the out-of-line form
     w = (a << z) & M64
     mant = (w >> 11) + (((w & 0xFFFFFFFF) >> 10) & 1)
-    hi = (mant >> 32) + (e << 20)
+    hi = (mant >> 32) + (e << 20) if ah else 0
     return ((hi | (1 << 31 if T < 0 else 0)) << 32) | (mant & 0xFFFFFFFF)
 
 
 @pytest.mark.parametrize("k", [-1090, -700, -56, 0, 11, 900, 960])
 def test_rounding(k):
     rng = random.Random(k)
-    cases = [1 << 32, (1 << 63) - 1, (1 << 62) + (1 << 8), (1 << 53) - 1, (1 << 54) - 1, (1 << 33) + 1]
+    cases = [0, 1 << 32, (1 << 63) - 1, (1 << 62) + (1 << 8), (1 << 53) - 1, (1 << 54) - 1, (1 << 33) + 1]
     cases += [rng.getrandbits(rng.randrange(1, 64)) for _ in range(3000)]
     short = 0
     for a in cases:
@@ -81,5 +81,5 @@ def test_rounding(k):
                 short += 1
                 assert got == _join(T, k)
             else:
-                assert abs(T) < 1 << 32 or not 0 <= abs(T).bit_length() + k + 1021 <= 2044
+                assert 0 < abs(T) < 1 << 32 or not 0 <= abs(T).bit_length() + k + 1021 <= 2044
     assert short > 1000 or k < -1000
