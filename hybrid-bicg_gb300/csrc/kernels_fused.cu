@@ -98,34 +98,45 @@ constexpr int MAXW = 32;  // warps of the largest block
 // Sum of np partials per set over the block, in a fixed order: the totals are
 // valid in warp 0 (every lane).  NA = 2: both sets at once.  FP64 adds cost 64
 // clocks per warp and SM quarter whatever the active lanes, so warps without
-// partials take no part.  `sh` needs 2 MAXW doubles.  One barrier.
+// partials take no part.  load() issues the loads with the kernel's others;
+// total() needs 2 MAXW doubles and has one barrier.
 template <int NA>
-__device__ __forceinline__ double2 sum_parts(const double *p0, const double *p1, unsigned np, double *sh) {
-    const unsigned t = threadIdx.x, w = t >> 5, l = t & 31;
-    const unsigned nw = min(min(blockDim.x >> 5, 16u), (np + 31) >> 5);
-    double x = 0.0, y = 0.0;
-    if (w < nw) {
-        for (unsigned i = t; i < np; i += nw * 32) {
-            x += __ldcg(p0 + i);
-            if (NA == 2) y += __ldcg(p1 + i);
+struct PartSum {
+    double x, y;
+    unsigned nw;
+    __device__ __forceinline__ void load(const double *p0, const double *p1, unsigned np) {
+        const unsigned t = threadIdx.x;
+        nw = min(min(blockDim.x >> 5, 16u), (np + 31) >> 5);
+        x = y = 0.0;
+        if (t < nw * 32 && t < np) {
+            x = __ldcg(p0 + t);
+            if (NA == 2) y = __ldcg(p1 + t);
+            for (unsigned i = t + nw * 32; i < np; i += nw * 32) {
+                x += __ldcg(p0 + i);
+                if (NA == 2) y += __ldcg(p1 + i);
+            }
         }
-        if (NA == 2) x = warp_sum_pair(x, y);
-        else x = warp_sum(x);
-        if (NA == 2 ? (l & 15) == 0 : l == 0) sh[(l >> 4) * MAXW + w] = x;
     }
-    __syncthreads();
-    double2 r = make_double2(0.0, 0.0);
-    if (w == 0) {
-        double v = 0.0;
-        if ((l & 15) < nw && (NA == 2 || l < 16)) v = sh[(l >> 4) * MAXW + (l & 15)];
+    __device__ __forceinline__ double2 total(double *sh) {
+        const unsigned w = threadIdx.x >> 5, l = threadIdx.x & 31;
+        if (w < nw) {
+            x = NA == 2 ? warp_sum_pair(x, y) : warp_sum(x);
+            if (NA == 2 ? (l & 15) == 0 : l == 0) sh[(l >> 4) * MAXW + w] = x;
+        }
+        __syncthreads();
+        double2 r = make_double2(0.0, 0.0);
+        if (w == 0) {
+            double v = 0.0;
+            if ((l & 15) < nw && (NA == 2 || l < 16)) v = sh[(l >> 4) * MAXW + (l & 15)];
 #pragma unroll
-        for (unsigned k = 8; k; k >>= 1)
-            if (k < nw) v += __shfl_xor_sync(0xffffffffu, v, k);
-        r.x = __shfl_sync(0xffffffffu, v, 0);
-        if (NA == 2) r.y = __shfl_sync(0xffffffffu, v, 16);
+            for (unsigned k = 8; k; k >>= 1)
+                if (k < nw) v += __shfl_xor_sync(0xffffffffu, v, k);
+            r.x = __shfl_sync(0xffffffffu, v, 0);
+            if (NA == 2) r.y = __shfl_sync(0xffffffffu, v, 16);
+        }
+        return r;
     }
-    return r;
-}
+};
 
 // This block's share of one or two dot products into its partial-sum slot.
 __device__ __forceinline__ void store_part(double v, double *sh, double *out) {
@@ -296,20 +307,21 @@ __device__ __forceinline__ void seed_q_body(const Ctx &c, const G &g) {
     size_t i = g.b() * (size_t)blockDim.x + threadIdx.x;
     body_ready<G>();
     const hbk_cur u = load_cur(sc);
+    PartSum<1> rs;
+    rs.load(parts(c, P_RS), nullptr, c.np_s);
+    const double rr_hat = __ldcg(&sc->rr_hat);
     double si = i < n ? HBK_LD(G, s, i) : 0.0;
     if (!u.active) return;
     const double *__restrict__ ro = vec_r_old(c, u);
     double *__restrict__ q = vec_q(c, u);
     double ri = i < n ? HBK_LD(G, ro, i) : 0.0;
-    double2 t;
-    if (u.rr_pend) {  // (np_p sums, not np_s: two passes)
-        const double rr = sum_parts<1>(parts(c, P_RRS), nullptr, c.np_p, red).x;
+    double2 t = rs.total(red);
+    t.y = rr_hat;
+    if (u.rr_pend) {
         __syncthreads();
-        t = sum_parts<1>(parts(c, P_RS), nullptr, c.np_s, red);
-        t.y = rr;
-    } else {
-        t = sum_parts<1>(parts(c, P_RS), nullptr, c.np_s, red);
-        t.y = __ldcg(&sc->rr_hat);
+        PartSum<1> rr;
+        rr.load(parts(c, P_RRS), nullptr, c.np_p);
+        t.y = rr.total(red).x;
     }
     if (threadIdx.x < 32) {
         const double a = dvd(t.y, t.x);
@@ -392,27 +404,41 @@ __global__ void __launch_bounds__(NT, HBK_HYB_MINB) k_seed_y<HBK_FMT_HYB>(Ctx c)
 // and this iteration's vector coefficients but for the factor beta, which K5
 // multiplies in.  Four lanes per shift: FP64 division takes 573 clocks of a
 // warp, so a shift's independent quotients go side by side, in two rounds.
-__device__ void shift_recurrences(const Ctx &c, const hbk_cur &u, double wk) {
+struct ShiftState {  // of this thread's shift: read before omega is known
+    double pik1, z, e0, sj;
+    bool run;
+    __device__ __forceinline__ void load(const Ctx &c, const hbk_cur &u, int j0) {
+        const hbk_shifts &S = c.sh;
+        const int j = j0 + (int)(threadIdx.x / 4);
+        pik1 = z = 1.0;
+        e0 = sj = 0.0;
+        run = false;
+        if (j < S.m) {
+            run = j == u.seed || !__ldcg(S.done + j);
+            sj = S.sigma[j];
+            if (j != u.seed) {
+                pik1 = __ldcg(S.pi + (size_t)j * S.kcap + u.k - 1);
+                z = __ldcg(S.zeta + j);
+                e0 = __ldcg(S.eta + j);
+            }
+        }
+    }
+};
+__device__ void shift_recurrences(const Ctx &c, const hbk_cur &u, double ak, double wk, ShiftState &st) {
     hbk_scalars *sc = c.sh.sc;
     const hbk_shifts &S = c.sh;
     const int k = u.k, seed = u.seed, m = S.m, kcap = S.kcap;
-    const double ak = __ldcg(&sc->alpha);
     const double c_prev = mul(__ldcg(&sc->ba), ak);
     const double sig_s = S.sigma[seed];
     const unsigned l = threadIdx.x & 31, quad = l & ~3u, part = threadIdx.x & 3;
     // (whole warps leave together: the shuffles below need all lanes)
     for (int j0 = 0; j0 + (int)(threadIdx.x & ~31u) / 4 < m; j0 += (int)blockDim.x / 4) {
         const int j = j0 + (int)(threadIdx.x / 4);
+        if (j0) st.load(c, u, j0);
         const bool here = j < m;
         const bool is_seed = j == seed;
-        const bool run = here && (is_seed || !__ldcg(S.done + j));
-        double pik1 = 1.0, z = 1.0, e0 = 0.0, sj = sig_s;
-        if (run && !is_seed) {
-            pik1 = __ldcg(S.pi + (size_t)j * kcap + k - 1);
-            z = __ldcg(S.zeta + j);
-            e0 = __ldcg(S.eta + j);
-            sj = S.sigma[j];
-        }
+        const bool run = st.run;
+        const double pik1 = st.pik1, z = st.z, e0 = st.e0, sj = here ? st.sj : sig_s;
         const double d = sub(sig_s, sj);
         const double eta = sub(mul(c_prev, e0), mul(mul(d, ak), pik1));
         const double pik = add(eta, pik1);
@@ -494,12 +520,17 @@ __device__ __forceinline__ void seed_update_body(const Ctx &c, const G &g) {
     double hi = i < n ? HBK_LD(G, rh, i) : 0.0;
     body_ready<G>();
     const hbk_cur u = load_cur(sc);
+    const double ak = __ldcg(&sc->alpha);
+    PartSum<2> qs;
+    qs.load(parts(c, P_QQ), parts(c, P_QY), c.np_y);
     double yi = i < n ? HBK_LD(G, y, i) : 0.0;
-    if (!u.active || !fin(__ldcg(&sc->alpha))) return;
+    if (!u.active || !fin(ak)) return;
     const double *__restrict__ q = vec_q(c, u);
     double *__restrict__ rn = vec_r_new(c, u);
     double qi = i < n ? HBK_LD(G, q, i) : 0.0;
-    const double2 t = sum_parts<2>(parts(c, P_QQ), parts(c, P_QY), c.np_y, sh);
+    ShiftState st;
+    if (extra) st.load(c, u, 0);
+    const double2 t = qs.total(sh);
     if (threadIdx.x < 32) {
         const double w = dvd(t.x, t.y);
         if (threadIdx.x == 0) {
@@ -520,7 +551,7 @@ __device__ __forceinline__ void seed_update_body(const Ctx &c, const G &g) {
     const double w = s_w;
     if (!fin(w) || is_zero(w)) return;
     if (extra) {
-        shift_recurrences(c, u, w);
+        shift_recurrences(c, u, ak, w, st);
         return;
     }
     double2 acc = make_double2(0.0, 0.0);
@@ -581,27 +612,42 @@ struct StepEnd {
     int sw, t;   // seed switch to system t; rsc = 1 / (zeta_t pi_t)
 };
 
+// What step_end reads, loaded with the kernel's other first loads.
+struct StepLoads {
+    PartSum<2> rs;
+    double aw, rho, tol, bb, c4, c5;
+    int live, switching;
+    __device__ __forceinline__ void load(const Ctx &c) {
+        const hbk_scalars *sc = c.sh.sc;
+        rs.load(parts(c, P_RR), parts(c, P_RRH), c.np_r);
+        aw = __ldcg(&sc->aw), rho = __ldcg(&sc->rr_hat_old), tol = __ldcg(&sc->tol), bb = __ldcg(&sc->bb);
+        switching = __ldcg(&sc->switching);
+        live = 0;
+        c4 = c5 = 1.0;
+        if ((int)threadIdx.x < c.sh.m) {
+            live = __ldcg(c.sh.live + threadIdx.x);
+            const double2 cc =
+                __ldcg(reinterpret_cast<const double2 *>(c.sh.coef + (size_t)threadIdx.x * HBK_NCOEF + 4));
+            c4 = cc.x;
+            c5 = cc.y;
+        }
+    }
+};
+
 // beta from K4's partial sums, the convergence test on the recursive residual
 // (src/solver_dynamic.c:278-303) and the decision to switch (:312-326).
 // Every thread returns the same.
-__device__ __forceinline__ StepEnd step_end(const Ctx &c, const hbk_cur &u, double wk, double *sh) {
+__device__ __forceinline__ StepEnd step_end(const Ctx &c, const hbk_cur &u, double wk, StepLoads &ld, double *sh) {
     __shared__ double s_bk, s_bw, s_rr, s_rrh, s_thr, s_rsc;
     __shared__ int s_t;
-    const hbk_scalars *sc = c.sh.sc;
     const hbk_shifts &S = c.sh;
     const int m = S.m;
-    // loaded before the sums are known
-    int live = 0;
-    double c4 = 1.0, c5 = 1.0;
-    if ((int)threadIdx.x < m) {
-        live = __ldcg(S.live + threadIdx.x);
-        const double2 cc = __ldcg(reinterpret_cast<const double2 *>(S.coef + (size_t)threadIdx.x * HBK_NCOEF + 4));
-        c4 = cc.x;
-        c5 = cc.y;
-    }
-    const double aw = __ldcg(&sc->aw), rho = __ldcg(&sc->rr_hat_old), tol = __ldcg(&sc->tol), bb = __ldcg(&sc->bb);
-    const int switching = __ldcg(&sc->switching);
-    const double2 t = sum_parts<2>(parts(c, P_RR), parts(c, P_RRH), c.np_r, sh);
+    int live = ld.live;
+    double c4 = ld.c4, c5 = ld.c5;
+    const double aw = ld.aw, rho = ld.rho, tol = ld.tol, bb = ld.bb;
+    const int switching = ld.switching;
+    PartSum<2> &rs = ld.rs;
+    const double2 t = rs.total(sh);
     if (threadIdx.x < 32) {
         const double bk = mul(aw, dvd(t.y, rho));
         if (threadIdx.x == 0) s_bk = bk, s_bw = -mul(bk, wk), s_rr = t.x, s_rrh = t.y;
@@ -805,6 +851,8 @@ __device__ __forceinline__ void shift_update_body(const Ctx &c, const G &g) {
     body_ready<G>();
     const hbk_cur u = load_cur(sc);
     const double ak = __ldcg(&sc->alpha), wk = __ldcg(&sc->omega);
+    StepLoads sl;
+    sl.load(c);
     const int m = c.sh.m;
     const unsigned t = threadIdx.x;
     const bool once = m <= MAXS;
@@ -838,7 +886,7 @@ __device__ __forceinline__ void shift_update_body(const Ctx &c, const G &g) {
         qi = HBK_LD(G, q, i), oi = HBK_LD(G, ro, i), ri = HBK_LD(G, rn, i);
         pi = HBK_LD(G, ps, i), xi = HBK_LD(G, xs, i), si = HBK_LD(G, s, i);
     }
-    const StepEnd e = step_end(c, u, wk, sh);
+    const StepEnd e = step_end(c, u, wk, sl, sh);
     if (!e.ok) {
         seed_x_only(c, u, g);
         return;
@@ -999,6 +1047,8 @@ __device__ __forceinline__ void seed_p_deferred_body(const Ctx &c, const G &g) {
     body_ready<G>();
     const hbk_cur u = load_cur(sc);
     const double ak = __ldcg(&sc->alpha), wk = __ldcg(&sc->omega);
+    StepLoads sl;
+    sl.load(c);
     if (!u.active || !fin(ak) || !fin(wk) || is_zero(wk)) return;
     const unsigned n = c.v.n;
     const size_t ld = ldn(n), step = (size_t)g.nb() * blockDim.x;
@@ -1016,7 +1066,7 @@ __device__ __forceinline__ void seed_p_deferred_body(const Ctx &c, const G &g) {
         ri = HBK_LD(G, rn, i), pi = HBK_LD(G, ps, i), si = HBK_LD(G, s, i), qi = HBK_LD(G, q, i);
         xi = HBK_LD(G, xp, panel_idx(seed, (unsigned)i, pm));
     }
-    const StepEnd e = step_end(c, u, wk, sh);
+    const StepEnd e = step_end(c, u, wk, sl, sh);
     if (!e.ok) {
         if (!g.coef_only()) seed_x_only(c, u, g);
         return;
