@@ -64,10 +64,10 @@ int hbicg_adjoint_gradients(hbicg_matrix *A, int m, const double *X, unsigned lo
     /* the gradients of b and the shifts read X and Lam once and wait for
      * memory, that of the values waits for the FP64 pipe: side by side
      * (128^3, 32 shifts: 1487 -> 1437 us) */
+    if (dJ_dsigma && m > 0) CK(hbicg__dev_alloc(&tmp, hbk_adjoint_tmp_bytes(m), st));
     CK(cudaEventRecord(ctx->cev, st));
     CK(cudaStreamWaitEvent(sb, ctx->cev, 0));
-    if (dJ_dsigma && m > 0) {
-        CK(hbicg__dev_alloc(&tmp, hbk_adjoint_tmp_bytes(m), st));
+    if (tmp) {
         CK((cudaError_t)hbk_shift_dots(k->n, m, X, ldx, Lam, ldl, 0, w, -1.0, dJ_dsigma, tmp, sb));
     }
     if (dJ_db) CK((cudaError_t)hbk_grad_b(k->n, m, Lam, ldl, w, dJ_db, sb));

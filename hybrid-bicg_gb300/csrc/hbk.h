@@ -119,6 +119,7 @@ typedef struct {
     int need_ps;        /* deferred mode: the new seed's p must be formed from the basis */
     int rr_pend;        /* the iteration ended with a switch: (r^, r) of the rescaled r is in K5's partial sums */
     int inline_ps;      /* 1: the launch that runs the iterations forms the new seed's p itself (shared launches) */
+    double flush_rows;  /* deferred mode: rows of n values that the basis flushes read and wrote */
     double aw;          /* alpha_k / omega_k */
     double ba;          /* beta_{k-1} / alpha_{k-1} */
     int loops;          /* bodies of the device-side iteration loop run in this solve (bound on the loop) */
@@ -301,13 +302,20 @@ const int *hbk_flush_tc_live_count(const void *ws, int m); /* device int: live s
 int hbk_panel_row(const double *Xp, int m, unsigned n, int j, double *x, cudaStream_t st);
 /* X[j][i] (leading dimension ld) = Xp in panel layout with m systems, i < n */
 int hbk_panel_to_rows(const double *Xp, int m, unsigned n, double *X, size_t ld, cudaStream_t st);
-/* after a flush: zero the coefficients, own = (0, keep_p), basis slot 0 = r_{k-1} */
-int hbk_deferred_reset(const hbk_vectors *v, const hbk_shifts *sh, int keep_p, cudaStream_t st);
+/* after a flush: zero the coefficients, own = (0, keep_p), basis slot 0 = r_{k-1};
+ * live: device count of the shifts it formed (added to the scalars' flush_rows), or NULL */
+int hbk_deferred_reset(const hbk_vectors *v, const hbk_shifts *sh, int keep_p, const int *live, cudaStream_t st);
 
 /* ||b - (A + sigma_j I) x_j||^2 for every shift into out[m] (device): leading
  * dimension ldx of X, at most grid_cap blocks per shift */
 int hbk_true_residuals_ld(const hbk_matrix *A, const double *X, size_t ldx, const double *b, const double *sigma,
                           int m, int grid_cap, double *partials, unsigned *counters, double *out, cudaStream_t st);
+
+/* What the host needs at the end of a fused solve, in one block: flush_rows,
+ * res[m], alpha, beta, omega and (r,r) of iterations [0, nk), as doubles, then
+ * conv_k[m], sw_k[m], sw_seed[m], *err (0 when NULL) and act_hist[nk], as ints */
+size_t hbk_pack_bytes(int m, int nk);
+int hbk_pack(const hbk_shifts *sh, int nk, const double *res, const int *err, void *out, cudaStream_t st);
 
 int hbk_last_error(void);
 const char *hbk_error_string(int code);

@@ -16,6 +16,7 @@ struct hbicg_context {
     hbk_scalars *h_sc; /* pinned */
     double *h_dbl;     /* pinned scratch */
     int refs;          /* the caller's handle + one per live matrix or solver */
+    int device, high;  /* what an idle context can serve again */
 };
 
 struct hbicg_matrix {

@@ -210,6 +210,7 @@ __global__ void __launch_bounds__(NT) k_init(Ctx c, int seed, double tol, int sw
         sc->status = 0;
         sc->n_sw = 0;
         sc->loops = 0;
+        sc->flush_rows = 0.0;
         sc->max_sigma = seed;
         sc->m = m;
         sc->kcap = kcap;
@@ -1218,7 +1219,7 @@ __global__ void __launch_bounds__(NT) k_flush(Ctx c, int keep_p, int which) {
 }
 
 // after a flush: reset the coefficients, own = (0, 1), slot 0 = r_{k-1}
-__global__ void __launch_bounds__(NT) k_flush_reset(Ctx c, int keep_p) {
+__global__ void __launch_bounds__(NT) k_flush_reset(Ctx c, int keep_p, const int *__restrict__ live) {
     hbk_scalars *sc = c.sh.sc;
     const int m = c.sh.m, cap = c.v.slot_cap;
     const unsigned n = c.v.n;
@@ -1253,6 +1254,7 @@ __global__ void __launch_bounds__(NT) k_flush_reset(Ctx c, int keep_p) {
     }
     if (take_ticket(c.sh.counters + 6)) {
         if (threadIdx.x == 0) {
+            if (live) sc->flush_rows += (keep_p ? 4.0 : 3.0) * *live;
             sc->slots = 1;
             sc->slot_r_old = 0;
             sc->status &= ~HBK_ST_BASIS_FULL;
@@ -1262,15 +1264,55 @@ __global__ void __launch_bounds__(NT) k_flush_reset(Ctx c, int keep_p) {
     }
 }
 
-// out[0 .. HBK_SLOT_SPREAD) take the bits of max |x| (zeroed by the caller)
-__global__ void __launch_bounds__(NT) k_absmax(const double *__restrict__ x, unsigned n, unsigned long long *out) {
+// first vectors of a solve, all equal to b: incremental mode r_0 and every
+// p_j; deferred mode basis slot 0 (with its maximum) and the seed's p.  The
+// shadow residual is the caller's copy of b itself when the two are one array.
+__global__ void __launch_bounds__(NT) k_init_vectors(Ctx c, const double *b) {
     __shared__ unsigned long long smx[NW];
+    const unsigned n = c.v.n;
+    const size_t ld = ldn(n);
     unsigned long long mx = 0;
     for (size_t i = blockIdx.x * (size_t)NT + threadIdx.x; i < n; i += (size_t)gridDim.x * NT) {
-        const unsigned long long b = abs_bits(x[i]);
-        mx = b > mx ? b : mx;
+        const double bi = b[i];
+        if (c.v.r_hat != b) c.v.r_hat[i] = bi;
+        if (c.v.deferred) {
+            c.v.V[i] = bi;
+            c.v.ps[i] = bi;
+            const unsigned long long a = abs_bits(bi);
+            mx = a > mx ? a : mx;
+        } else {
+            c.v.rbuf[0][i] = bi;
+            for (int j = 0; j < c.sh.m; ++j) c.v.P[(size_t)j * ld + i] = bi;
+        }
     }
-    block_max_to(mx, smx, out);
+    if (c.v.deferred && c.v.slot_max) block_max_to(mx, smx, c.v.slot_max);
+}
+
+// hbk_pack's block (hbk.h)
+__global__ void __launch_bounds__(NT) k_pack(hbk_shifts S, int nk, const double *__restrict__ res,
+                                             const int *__restrict__ err, double *__restrict__ out) {
+    const int m = S.m;
+    int *w = reinterpret_cast<int *>(out + 1 + m + 4 * (size_t)nk);
+    for (int i = blockIdx.x * NT + threadIdx.x; i < nk || i < m; i += gridDim.x * NT) {
+        if (i < m) {
+            out[1 + i] = res[i];
+            w[i] = S.conv_k[i];
+            w[m + i] = S.sw_k[i];
+            w[2 * m + i] = S.sw_seed[i];
+        }
+        if (i < nk) {
+            double *h = out + 1 + m;
+            h[i] = S.a_hist[i];
+            h[(size_t)nk + i] = S.b_hist[i];
+            h[2 * (size_t)nk + i] = S.w_hist[i];
+            h[3 * (size_t)nk + i] = S.rr_hist[i];
+            w[3 * m + 1 + i] = S.act_hist[i];
+        }
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        out[0] = S.sc->flush_rows;
+        w[3 * m] = err ? *err : 0;
+    }
 }
 
 // End of a while-loop body in a CUDA graph: run again while the solve goes on
@@ -1463,29 +1505,19 @@ int hbk_fused_init(const hbk_matrix *A, const hbk_vectors *v, const hbk_shifts *
     const unsigned n = v->n;
     const size_t ld = ((size_t)n + 31) / 32 * 32;
     int e;
-    if ((e = hbk_copy(n, b, v->r_hat, st))) return e;
     if ((e = hbk_dot(n, b, b, sh->partials, sh->counters + 7, &sh->sc->bb, st))) return e;
-    if (!v->deferred) {
-        if ((e = hbk_copy(n, b, v->rbuf[0], st))) return e;
-        for (int j = 0; j < sh->m; j++) {
-            if ((e = hbk_copy(n, b, v->P + (size_t)j * ld, st))) return e;
-        }
-    } else {
-        if ((e = hbk_copy(n, b, v->V, st))) return e;
-        if ((e = hbk_copy(n, b, v->ps, st))) return e;
+    if (v->deferred) {
         if (v->sval_shift && A->fmt == HBK_FMT_SELL && A->sval == v->sval_orig &&
             (e = hbk_fold_diag(n, A->sval, A->sell_len, v->sdiag, sh->sigma + seed, v->sval_shift, st)))
             return e;
-        if (v->slot_max) {
-            if ((e = (int)cudaMemsetAsync(v->slot_max, 0,
-                                          sizeof(unsigned long long) * (size_t)v->slot_cap * HBK_SLOT_SPREAD, st)))
-                return e;
-            k_absmax<<<grid_for(n ? n : 1, 4), NT, 0, st>>>(b, n, v->slot_max);  // slot 0 = b
-            if ((e = (int)cudaGetLastError())) return e;
-        }
+        if (v->slot_max && (e = (int)cudaMemsetAsync(v->slot_max, 0,
+                                                     sizeof(unsigned long long) * (size_t)v->slot_cap * HBK_SLOT_SPREAD,
+                                                     st)))
+            return e;
         k_init_coef<<<grid_for((unsigned)((size_t)sh->m * v->slot_cap), 1), NT, 0, st>>>(c);
-        if ((e = (int)cudaGetLastError())) return e;
     }
+    k_init_vectors<<<grid_for(n ? n : 1, 2), NT, 0, st>>>(c, b);
+    if ((e = (int)cudaGetLastError())) return e;
     if (v->deferred) {
         if ((e = (int)cudaMemsetAsync(v->Xp, 0, sizeof(double) * hbk_panel_elems(n, v->pm), st))) return e;
     } else if ((e = (int)cudaMemsetAsync(v->X, 0, sizeof(double) * ld * (size_t)sh->m, st))) {
@@ -1570,6 +1602,18 @@ int hbk_fused_iteration(const hbk_matrix *A, const hbk_vectors *v, const hbk_shi
     else if (A->fmt == HBK_FMT_HYB && A->nwide) launch_iteration<HBK_FMT_HYBW>(c, A, early, st);
     else if (A->fmt == HBK_FMT_HYB) launch_iteration<HBK_FMT_HYB>(c, A, early, st);
     else launch_iteration<HBK_FMT_TILE>(c, A, early, st);
+    return (int)cudaGetLastError();
+}
+
+size_t hbk_pack_bytes(int m, int nk) {
+    return sizeof(double) * (1 + (size_t)(m > 0 ? m : 0) + 4 * (size_t)nk) +
+           sizeof(int) * (3 * (size_t)(m > 0 ? m : 0) + 2 + (size_t)nk);
+}
+
+int hbk_pack(const hbk_shifts *sh, int nk, const double *res, const int *err, void *out, cudaStream_t st) {
+    const int most = nk > sh->m ? nk : sh->m;
+    const int blocks = most / NT + 1;
+    k_pack<<<blocks < 32 ? blocks : 32, NT, 0, st>>>(*sh, nk, res, err, (double *)out);
     return (int)cudaGetLastError();
 }
 
@@ -1669,14 +1713,14 @@ int hbk_deferred_flush(const hbk_vectors *v, const hbk_shifts *sh, int keep_p, c
     // x first: it reads the old Pmat, which the p pass then overwrites
     k_flush<<<grid, NT, 0, st>>>(c, keep_p, 0);
     if (keep_p) k_flush<<<grid, NT, 0, st>>>(c, keep_p, 1);
-    k_flush_reset<<<grid_for(v->n, 2), NT, 0, st>>>(c, keep_p);
+    k_flush_reset<<<grid_for(v->n, 2), NT, 0, st>>>(c, keep_p, nullptr);
     return (int)cudaGetLastError();
 }
 
-int hbk_deferred_reset(const hbk_vectors *v, const hbk_shifts *sh, int keep_p, cudaStream_t st) {
+int hbk_deferred_reset(const hbk_vectors *v, const hbk_shifts *sh, int keep_p, const int *live, cudaStream_t st) {
     hbk_matrix A0 = {};
     Ctx c = make_ctx(&A0, v, sh);
-    k_flush_reset<<<grid_for(v->n, 2), NT, 0, st>>>(c, keep_p);
+    k_flush_reset<<<grid_for(v->n, 2), NT, 0, st>>>(c, keep_p, live);
     return (int)cudaGetLastError();
 }
 

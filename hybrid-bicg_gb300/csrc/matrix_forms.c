@@ -421,7 +421,7 @@ static int build_sell(hbicg_matrix *A, const unsigned *h_ptr, unsigned n, unsign
         rc = HBICG_E_NOMEM;
         goto out;
     }
-    CUDA_GOTO(cudaMalloc((void **)&d_w, sizeof(unsigned) * ns));
+    CUDA_GOTO(hbicg__dev_alloc((void **)&d_w, sizeof(unsigned) * ns, st));
     HBK_GOTO(hbk_sell_widths(n, A->d_ptr, d_w, st));
     CUDA_GOTO(cudaMemcpyAsync(h_w, d_w, sizeof(unsigned) * ns, cudaMemcpyDeviceToHost, st));
     CUDA_GOTO(cudaStreamSynchronize(st));
@@ -443,7 +443,7 @@ static int build_sell(hbicg_matrix *A, const unsigned *h_ptr, unsigned n, unsign
     A->k.sell_len = padded;
     A->diag_state = 0; /* a new SELL-32 layout */
 out:
-    cudaFree(d_w);
+    hbicg__dev_free(d_w, st);
     free(h_w);
     free(h_sp);
     return rc;
@@ -457,14 +457,14 @@ int hbicg__sell_diag(hbicg_matrix *A) {
     int *d_missing = NULL, missing = 0;
     int rc = HBICG_OK;
     if (!A->d_sdiag) CUDA_GOTO(hbicg__dev_alloc((void **)&A->d_sdiag, sizeof(unsigned long long) * ((size_t)n + 1), st));
-    CUDA_GOTO(cudaMalloc((void **)&d_missing, sizeof(int)));
+    CUDA_GOTO(hbicg__dev_alloc((void **)&d_missing, sizeof(int), st));
     CUDA_GOTO(cudaMemsetAsync(d_missing, 0, sizeof(int), st));
     HBK_GOTO(hbk_sell_diag(n, A->d_ptr, A->d_sptr, A->d_scol, A->d_sdiag, d_missing, st));
     CUDA_GOTO(cudaMemcpyAsync(&missing, d_missing, sizeof(int), cudaMemcpyDeviceToHost, st));
     CUDA_GOTO(cudaStreamSynchronize(st));
     A->diag_state = missing ? 2 : 1;
 out: /* d_missing is freed on every path; d_sdiag belongs to the matrix */
-    cudaFree(d_missing);
+    hbicg__dev_free(d_missing, st);
     return rc;
 }
 
@@ -562,6 +562,7 @@ out: /* on failure the partial matrix goes, its device arrays with it */
         return rc;
     }
     if (A->k.fmt == HBK_FMT_SELL) A->k.grid = hbk_spmv_grid((n + HBK_THREADS - 1) / HBK_THREADS);
+    CUDA_TRY(cudaStreamSynchronize(st)); /* usable from any stream */
     hbicg__ctx_retain(ctx);
     *out = A;
     return HBICG_OK;
@@ -590,20 +591,20 @@ int hbicg_matrix_from_coo(hbicg_context *ctx, unsigned n, unsigned nnz, const un
         d_row = NULL;
         d_col = NULL;
         d_val = NULL;
-        FC(cudaMalloc((void **)&d_row, sizeof(unsigned) * ((size_t)nnz + 1)));
-        FC(cudaMalloc((void **)&d_col, sizeof(unsigned) * ((size_t)nnz + 1)));
-        FC(cudaMalloc((void **)&d_val, sizeof(double) * ((size_t)nnz + 1)));
+        FC(hbicg__dev_alloc((void **)&d_row, sizeof(unsigned) * ((size_t)nnz + 1), st));
+        FC(hbicg__dev_alloc((void **)&d_col, sizeof(unsigned) * ((size_t)nnz + 1), st));
+        FC(hbicg__dev_alloc((void **)&d_val, sizeof(double) * ((size_t)nnz + 1), st));
         if (nnz) {
             FC(cudaMemcpyAsync(d_row, row, sizeof(unsigned) * (size_t)nnz, cudaMemcpyHostToDevice, st));
             FC(cudaMemcpyAsync(d_col, col, sizeof(unsigned) * (size_t)nnz, cudaMemcpyHostToDevice, st));
             FC(cudaMemcpyAsync(d_val, val, sizeof(double) * (size_t)nnz, cudaMemcpyHostToDevice, st));
         }
     }
-    FC(cudaMalloc((void **)&ptr, sizeof(unsigned) * ((size_t)n + 1)));
-    FC(cudaMalloc((void **)&colo, sizeof(unsigned) * ((size_t)nnz + 1)));
-    FC(cudaMalloc((void **)&valo, sizeof(double) * ((size_t)nnz + 1)));
-    FC(cudaMalloc(&tmp, hbk_coo_to_csr_tmp_bytes(nnz)));
-    FC(cudaMalloc((void **)&d_err, sizeof(int)));
+    FC(hbicg__dev_alloc((void **)&ptr, sizeof(unsigned) * ((size_t)n + 1), st));
+    FC(hbicg__dev_alloc((void **)&colo, sizeof(unsigned) * ((size_t)nnz + 1), st));
+    FC(hbicg__dev_alloc((void **)&valo, sizeof(double) * ((size_t)nnz + 1), st));
+    FC(hbicg__dev_alloc(&tmp, hbk_coo_to_csr_tmp_bytes(nnz), st));
+    FC(hbicg__dev_alloc((void **)&d_err, sizeof(int), st));
     FC(cudaMemsetAsync(d_err, 0, sizeof(int), st));
     FC((cudaError_t)hbk_coo_to_csr(n, nnz, d_row, d_col, d_val, ptr, colo, valo, tmp, d_err, st));
     FC(cudaMemcpyAsync(&h_err, d_err, sizeof(int), cudaMemcpyDeviceToHost, st));
@@ -613,39 +614,40 @@ int hbicg_matrix_from_coo(hbicg_context *ctx, unsigned n, unsigned nnz, const un
         rc = HBICG_E_ARG;
         goto fail;
     }
-    cudaFree(tmp);
-    cudaFree(d_err);
+    hbicg__dev_free(tmp, st);
+    hbicg__dev_free(d_err, st);
     tmp = NULL;
     d_err = NULL;
     if (where != HBICG_DEVICE) {
-        cudaFree(d_row);
-        cudaFree(d_col);
-        cudaFree(d_val);
+        hbicg__dev_free(d_row, st);
+        hbicg__dev_free(d_col, st);
+        hbicg__dev_free(d_val, st);
     }
     {
         hbicg_matrix *A = NULL;
         rc = hbicg_matrix_create(ctx, n, nnz, ptr, colo, valo, HBICG_DEVICE, &A);
         if (rc != HBICG_OK) {
-            cudaFree(ptr);
-            cudaFree(colo);
-            cudaFree(valo);
+            hbicg__dev_free(ptr, st);
+            hbicg__dev_free(colo, st);
+            hbicg__dev_free(valo, st);
             return rc;
         }
         A->owns = 1;
+        A->pooled = 1;
         *out = A;
     }
     return HBICG_OK;
 fail:
     if (where != HBICG_DEVICE) {
-        cudaFree(d_row);
-        cudaFree(d_col);
-        cudaFree(d_val);
+        hbicg__dev_free(d_row, st);
+        hbicg__dev_free(d_col, st);
+        hbicg__dev_free(d_val, st);
     }
-    cudaFree(ptr);
-    cudaFree(colo);
-    cudaFree(valo);
-    cudaFree(tmp);
-    cudaFree(d_err);
+    hbicg__dev_free(ptr, st);
+    hbicg__dev_free(colo, st);
+    hbicg__dev_free(valo, st);
+    hbicg__dev_free(tmp, st);
+    hbicg__dev_free(d_err, st);
     return rc;
 #undef FC
 }

@@ -85,21 +85,49 @@ void hbicg_params_default(hbicg_params *p) {
 /* ------------------------------------------------------------------------ */
 
 void hbicg__ctx_retain(hbicg_context *c) { __atomic_add_fetch(&c->refs, 1, __ATOMIC_RELAXED); }
-static void ctx_free(hbicg_context *c);
-/* the context is freed when its handle and every matrix and solver made on it
+static void ctx_retire(hbicg_context *c);
+/* the context is given up when its handle and every matrix and solver made on it
  * are gone, in whatever order a caller (or a garbage collector) destroys them */
 void hbicg__ctx_release(hbicg_context *c) {
-    if (__atomic_sub_fetch(&c->refs, 1, __ATOMIC_ACQ_REL) == 0) ctx_free(c);
+    if (__atomic_sub_fetch(&c->refs, 1, __ATOMIC_ACQ_REL) == 0) ctx_retire(c);
 }
 
 int hbicg_context_create(hbicg_context **out) { return hbicg__context_create_prio(out, 0); }
 
+/* Streams, events and pinned words of destroyed contexts wait here for the next
+ * context of the same device and priority (a one-shot call makes and destroys
+ * one: 0.2 ms), at most HBICG_CTX_KEEP of them; hbicg_release gives them back. */
+#define HBICG_CTX_KEEP 16
+static hbicg_context *g_ctx_idle[HBICG_CTX_KEEP];
+static int g_ctx_nidle;
+static pthread_mutex_t g_ctx_lock = PTHREAD_MUTEX_INITIALIZER;
+
+static void ctx_free(hbicg_context *c);
+
 /* high = 1: the context's stream at the device's greatest priority, so that
  * its short steps are scheduled ahead of other streams' pending blocks */
 int hbicg__context_create_prio(hbicg_context **out, int high) {
-    hbicg_context *c = calloc(1, sizeof *c);
+    int dev = -1;
+    hbicg_context *c = NULL;
+    if (cudaGetDevice(&dev) == cudaSuccess) {
+        pthread_mutex_lock(&g_ctx_lock);
+        for (int i = g_ctx_nidle - 1; i >= 0 && !c; --i)
+            if (g_ctx_idle[i]->device == dev && g_ctx_idle[i]->high == (high != 0)) {
+                c = g_ctx_idle[i];
+                g_ctx_idle[i] = g_ctx_idle[--g_ctx_nidle];
+            }
+        pthread_mutex_unlock(&g_ctx_lock);
+        if (c) {
+            c->refs = 1;
+            *out = c;
+            return HBICG_OK;
+        }
+    }
+    c = calloc(1, sizeof *c);
     if (!c) return HBICG_E_NOMEM;
     c->refs = 1;
+    c->device = dev;
+    c->high = high != 0;
     int rc = HBICG_OK, lo = 0, hi = 0;
     if (high && cudaDeviceGetStreamPriorityRange(&lo, &hi) == cudaSuccess)
         CUDA_GOTO(cudaStreamCreateWithPriority(&c->stream, cudaStreamNonBlocking, hi));
@@ -133,8 +161,6 @@ void hbicg_context_destroy(hbicg_context *c) {
 }
 
 static void ctx_free(hbicg_context *c) {
-    cudaStreamSynchronize(c->stream);
-    cudaStreamSynchronize(c->cstream);
     cudaStreamDestroy(c->cstream);
     cudaEventDestroy(c->cev);
     cudaFreeHost(c->h_sc);
@@ -145,6 +171,21 @@ static void ctx_free(hbicg_context *c) {
     cudaEventDestroy(c->evf1);
     cudaStreamDestroy(c->stream);
     free(c);
+}
+
+/* to the idle contexts when both streams are idle and sound, else freed */
+static void ctx_retire(hbicg_context *c) {
+    const cudaError_t e0 = cudaStreamSynchronize(c->stream), e1 = cudaStreamSynchronize(c->cstream);
+    int kept = 0;
+    if (!e0 && !e1 && c->device >= 0) {
+        pthread_mutex_lock(&g_ctx_lock);
+        if (g_ctx_nidle < HBICG_CTX_KEEP) {
+            g_ctx_idle[g_ctx_nidle++] = c;
+            kept = 1;
+        }
+        pthread_mutex_unlock(&g_ctx_lock);
+    }
+    if (!kept) ctx_free(c);
 }
 
 void *hbicg_context_stream(hbicg_context *c) { return (void *)c->stream; }
@@ -167,10 +208,14 @@ struct hbicg_solver {
     int graph_loop;    /* graph is one conditional while loop over iterations */
     int no_loop_graph; /* the runtime refused the loop graph: chunks of iterations */
     int chunk;
+    void *slab;       /* the small device arrays */
+    void *d_pack;     /* what one copy brings to the host at the end of a solve (hbk_pack_bytes) */
+    size_t pack_bytes;
     void *tc_ws;      /* tensor-core flush workspace (deferred mode) */
     int *d_tc_err;    /* set by the tensor-core flush on a bounded-wait timeout */
     int launches_per_iter;
     double flush_bytes; /* compulsory HBM bytes of this solve's basis flushes */
+    int flush_timed;    /* evf0, evf1 hold a flush whose time has not been read */
     /* where this solve's x_j end up, rows xld apart: the workspace's X, or the
      * caller's device array (the deferred mode writes rows straight into it) */
     double *xrows;
@@ -268,12 +313,11 @@ static cudaError_t solver_pool(cudaMemPool_t *out) {
     return e;
 }
 
-/* usable from any stream on return (the allocation's stream is synchronised) */
+/* usable on st at once, on another stream behind a synchronisation of st */
 static cudaError_t pool_alloc(void **p, size_t bytes, cudaStream_t st) {
     cudaMemPool_t pool;
     cudaError_t e = solver_pool(&pool);
     if (!e) e = cudaMallocFromPoolAsync(p, bytes > 0 ? bytes : 8, pool, st);
-    if (!e) e = cudaStreamSynchronize(st);
     return e;
 }
 
@@ -288,6 +332,13 @@ void hbicg__dev_free(void *p, cudaStream_t st) {
 }
 
 void hbicg_release(void) {
+    for (;;) {
+        pthread_mutex_lock(&g_ctx_lock);
+        hbicg_context *idle = g_ctx_nidle ? g_ctx_idle[--g_ctx_nidle] : NULL;
+        pthread_mutex_unlock(&g_ctx_lock);
+        if (!idle) break;
+        ctx_free(idle);
+    }
     pthread_mutex_lock(&g_pool_lock);
     for (int d = 0; d < HBICG_MAX_DEVICES; ++d)
         if (g_pools[d]) cudaMemPoolTrimTo(g_pools[d], 0);
@@ -295,6 +346,20 @@ void hbicg_release(void) {
 }
 
 #define DALLOC(ptr, bytes) CUDA_TRY(pool_alloc((void **)&(ptr), (size_t)(bytes), ctx->stream))
+
+/* the solver's small arrays in one allocation: noted first, placed together */
+#define SLAB_MAX 40
+typedef struct {
+    void **p[SLAB_MAX];
+    size_t off[SLAB_MAX], bytes;
+    int n;
+} slab_t;
+static void slab_add(slab_t *b, void **p, size_t bytes) {
+    b->p[b->n] = p;
+    b->off[b->n++] = b->bytes;
+    b->bytes += (bytes + 255) / 256 * 256;
+}
+#define SALLOC(ptr, size) slab_add(&slab, (void **)&(ptr), (size_t)(size))
 
 int hbicg_solver_create(hbicg_context *ctx, hbicg_matrix *A, int m, const hbicg_params *pp, hbicg_solver **out) {
     hbicg_params p;
@@ -318,10 +383,13 @@ int hbicg_solver_create(hbicg_context *ctx, hbicg_matrix *A, int m, const hbicg_
     s->mode = pick_mode(&p, n, m);
     size_t vb = sizeof(double) * ld;
 
+    slab_t slab;
+    memset(&slab, 0, sizeof slab);
     hbk_vectors *v = &s->v;
     memset(v, 0, sizeof *v);
     v->n = n;
-    DALLOC(v->r_hat, vb);
+    DALLOC(s->d_b, vb);
+    v->r_hat = s->d_b; /* the shadow residual is b, and both stay as they are */
     DALLOC(v->s, vb);
     DALLOC(v->y, vb);
     DALLOC(v->X, vb * mm);
@@ -370,10 +438,10 @@ int hbicg_solver_create(hbicg_context *ctx, hbicg_matrix *A, int m, const hbicg_
         } else {
             v->slot_cap = (int)cap;
             DALLOC(v->V, vb * (size_t)cap);
-            DALLOC(v->Xc, sizeof(double) * (size_t)mm * (size_t)cap);
-            DALLOC(v->Pc, sizeof(double) * (size_t)mm * (size_t)cap);
-            DALLOC(v->own, sizeof(double) * 2 * (size_t)mm);
-            DALLOC(v->slot_max, sizeof(unsigned long long) * (size_t)cap * HBK_SLOT_SPREAD);
+            SALLOC(v->Xc, sizeof(double) * (size_t)mm * (size_t)cap);
+            SALLOC(v->Pc, sizeof(double) * (size_t)mm * (size_t)cap);
+            SALLOC(v->own, sizeof(double) * 2 * (size_t)mm);
+            SALLOC(v->slot_max, sizeof(unsigned long long) * (size_t)cap * HBK_SLOT_SPREAD);
             /* SELL-32 matrices with a stored diagonal in every row: the seed's
              * shift goes onto the diagonal of a private copy of the values,
              * which saves the sigma p and sigma q terms of the two products */
@@ -388,8 +456,7 @@ int hbicg_solver_create(hbicg_context *ctx, hbicg_matrix *A, int m, const hbicg_
             }
             if (p.flush_mode != HBICG_FLUSH_FP64) {
                 DALLOC(s->tc_ws, hbk_flush_tc_workspace_bytes(mm));
-                DALLOC(s->d_tc_err, sizeof(int));
-                CUDA_TRY(cudaMemset(s->d_tc_err, 0, sizeof(int)));
+                SALLOC(s->d_tc_err, sizeof(int));
             }
         }
     }
@@ -398,42 +465,46 @@ int hbicg_solver_create(hbicg_context *ctx, hbicg_matrix *A, int m, const hbicg_
     memset(sh, 0, sizeof *sh);
     sh->m = m;
     sh->kcap = s->kcap;
-    DALLOC(s->d_sc, sizeof(hbk_scalars));
-    CUDA_TRY(cudaMemset(s->d_sc, 0, sizeof(hbk_scalars)));
-    sh->sc = s->d_sc;
-    DALLOC(s->d_sigma, sizeof(double) * mm);
-    sh->sigma = s->d_sigma;
-    DALLOC(sh->a_hist, sizeof(double) * ((size_t)s->kcap + 1));
-    DALLOC(sh->b_hist, sizeof(double) * ((size_t)s->kcap + 1));
-    DALLOC(sh->w_hist, sizeof(double) * ((size_t)s->kcap + 1));
-    DALLOC(sh->ratio, sizeof(double) * ((size_t)s->kcap + 1));
-    DALLOC(sh->rr_hist, sizeof(double) * ((size_t)s->kcap + 1));
-    DALLOC(sh->pi, sizeof(double) * (size_t)mm * ((size_t)s->kcap + 1));
-    DALLOC(sh->eta, sizeof(double) * mm);
-    DALLOC(sh->zeta, sizeof(double) * mm);
-    DALLOC(sh->done, sizeof(int) * mm);
-    DALLOC(sh->conv_k, sizeof(int) * mm);
-    DALLOC(sh->live, sizeof(int) * mm);
-    DALLOC(sh->lslot, sizeof(int) * mm);
-    DALLOC(sh->coef, sizeof(double) * HBK_NCOEF * (size_t)mm);
-    DALLOC(sh->sw_k, sizeof(int) * mm);
-    DALLOC(sh->sw_seed, sizeof(int) * mm);
-    DALLOC(sh->act_hist, sizeof(int) * ((size_t)s->kcap + 1));
-    CUDA_TRY(cudaMemset(sh->act_hist, 0, sizeof(int) * ((size_t)s->kcap + 1)));
+    SALLOC(s->d_sc, sizeof(hbk_scalars));
+    SALLOC(s->d_sigma, sizeof(double) * mm);
+    SALLOC(sh->a_hist, sizeof(double) * ((size_t)s->kcap + 1));
+    SALLOC(sh->b_hist, sizeof(double) * ((size_t)s->kcap + 1));
+    SALLOC(sh->w_hist, sizeof(double) * ((size_t)s->kcap + 1));
+    SALLOC(sh->ratio, sizeof(double) * ((size_t)s->kcap + 1));
+    SALLOC(sh->rr_hist, sizeof(double) * ((size_t)s->kcap + 1));
+    SALLOC(sh->pi, sizeof(double) * (size_t)mm * ((size_t)s->kcap + 1));
+    SALLOC(sh->eta, sizeof(double) * mm);
+    SALLOC(sh->zeta, sizeof(double) * mm);
+    SALLOC(sh->done, sizeof(int) * mm);
+    SALLOC(sh->conv_k, sizeof(int) * mm);
+    SALLOC(sh->live, sizeof(int) * mm);
+    SALLOC(sh->lslot, sizeof(int) * mm);
+    SALLOC(sh->coef, sizeof(double) * HBK_NCOEF * (size_t)mm);
+    SALLOC(sh->sw_k, sizeof(int) * mm);
+    SALLOC(sh->sw_seed, sizeof(int) * mm);
+    SALLOC(sh->act_hist, sizeof(int) * ((size_t)s->kcap + 1));
     size_t nparts = (size_t)(mm > HBK_NPART ? mm : HBK_NPART) * HBK_MAX_GRID;
-    DALLOC(sh->partials, sizeof(double) * nparts);
-    DALLOC(sh->counters, sizeof(unsigned) * (16 + (size_t)mm));
-    CUDA_TRY(cudaMemset(sh->counters, 0, sizeof(unsigned) * (16 + (size_t)mm)));
-    DALLOC(s->d_b, vb);
-    DALLOC(s->d_res, sizeof(double) * mm);
-    DALLOC(s->d_dot, sizeof(double) * 8);
+    SALLOC(sh->partials, sizeof(double) * nparts);
+    SALLOC(sh->counters, sizeof(unsigned) * (16 + (size_t)mm));
+    SALLOC(s->d_res, sizeof(double) * mm);
+    SALLOC(s->d_dot, sizeof(double) * 8);
+    s->pack_bytes = hbk_pack_bytes(mm, s->kcap);
+    SALLOC(s->d_pack, s->pack_bytes);
+    DALLOC(s->slab, slab.bytes);
+    CUDA_TRY(cudaMemsetAsync(s->slab, 0, slab.bytes, ctx->stream));
+    for (int i = 0; i < slab.n; i++) *slab.p[i] = (char *)s->slab + slab.off[i];
+    sh->sc = s->d_sc;
+    sh->sigma = s->d_sigma;
     if (p.form == HBICG_FORM_PLAIN) {
         DALLOC(s->d_rold, vb);
         DALLOC(s->d_qcopy, vb);
         s->d_r = v->rbuf[0];
     }
-    s->chunk = p.graph_chunk > 0 ? p.graph_chunk : (n >= (1u << 22) ? 2 : (n >= (1u << 18) ? 4 : 16));
+    /* (14 and 4 and 2 divide the deferred mode's 28 iterations per basis block) */
+    const int small = s->mode == HBICG_SHIFTS_DEFERRED ? 14 : 16;
+    s->chunk = p.graph_chunk > 0 ? p.graph_chunk : (n >= (1u << 22) ? 2 : (n >= (1u << 18) ? 4 : small));
     s->launches_per_iter = 5;
+    CUDA_TRY(cudaStreamSynchronize(ctx->stream)); /* the buffers are usable from any stream */
     hbicg__ctx_retain(ctx);
     *out = s;
     return HBICG_OK;
@@ -444,12 +515,8 @@ void hbicg_solver_destroy(hbicg_solver *s) {
     cudaStreamSynchronize(s->ctx->stream);
     if (s->graph) cudaGraphExecDestroy(s->graph);
     hbk_vectors *v = &s->v;
-    hbk_shifts *sh = &s->sh;
-    void *ptrs[] = {v->r_hat, v->rbuf[0], v->rbuf[1], v->s, v->q, v->y, v->X, v->P, v->V, v->ps, v->Xc, v->Pc,
-                    v->own, v->Pmat, v->Xp, v->slot_max, v->sval_shift, s->d_sc, s->d_sigma, sh->a_hist, sh->b_hist, sh->w_hist, sh->ratio, sh->pi,
-                    sh->eta, sh->zeta, sh->done, sh->conv_k, sh->live, sh->lslot, sh->coef, sh->sw_k,
-                    sh->rr_hist, sh->sw_seed, sh->act_hist, sh->partials, sh->counters, s->d_b, s->d_res, s->d_dot, s->d_rold,
-                    s->d_qcopy, s->tc_ws, s->d_tc_err};
+    void *ptrs[] = {v->rbuf[0], v->rbuf[1], v->s, v->q, v->y, v->X, v->P, v->V, v->ps, v->Pmat, v->Xp, v->sval_shift,
+                    s->d_b, s->d_rold, s->d_qcopy, s->tc_ws, s->slab};
     for (size_t i = 0; i < sizeof ptrs / sizeof ptrs[0]; i++)
         if (ptrs[i]) cudaFreeAsync(ptrs[i], s->ctx->stream); /* back to the pool, in stream order */
     hbicg_context *ctx = s->ctx;
@@ -740,12 +807,7 @@ static int ensure_pmat(hbicg_solver *s) {
     const int mm = s->m > 0 ? s->m : 1;
     const size_t bytes = sizeof(double) * hbk_panel_elems(s->A->k.n, mm); /* panel-major */
     CUDA_TRY(pool_alloc((void **)&s->v.Pmat, bytes, s->ctx->stream));
-    CUDA_TRY(cudaMemsetAsync(s->v.Pmat, 0, bytes, s->ctx->stream));
-    /* the graphs captured the old (null) Pmat pointer: capture again */
-    if (s->graph) {
-        cudaGraphExecDestroy(s->graph);
-        s->graph = NULL;
-    }
+    CUDA_TRY(cudaMemsetAsync(s->v.Pmat, 0, bytes, s->ctx->stream)); /* (no kernel of the graphs reads it) */
     return HBICG_OK;
 }
 
@@ -759,19 +821,16 @@ static int do_flush(hbicg_solver *s, int keep_p, int L, int k_last, int *launche
     /* basis slots read once; x_j read and written; Pmat_j read (and written),
      * for the shifts the flush forms */
     const double per_shift = keep_p ? 4.0 : 3.0;
+    s->flush_bytes += 8.0 * s->A->k.n * (double)L;
     if (s->tc_ws && L >= 1 && L <= hbk_flush_tc_max_slots()) {
         HBK_TRY(hbk_flush_tc_run_live(s->v.V, s->ld, s->A->k.n, L, s->v.Xc, s->v.Pc, s->v.slot_cap, s->v.own, s->m,
                                       s->v.Xp, s->v.Pmat, keep_p, s->sh.conv_k, k_last, s->v.slot_max, s->tc_ws,
                                       s->d_tc_err, st));
-        int n_live = 0; /* pageable destination: the copy waits for the flush */
-        CUDA_TRY(cudaMemcpyAsync(&n_live, hbk_flush_tc_live_count(s->tc_ws, s->m), sizeof(int),
-                                 cudaMemcpyDeviceToHost, st));
-        CUDA_TRY(cudaStreamSynchronize(st));
-        s->flush_bytes += 8.0 * s->A->k.n * ((double)L + per_shift * n_live);
-        HBK_TRY(hbk_deferred_reset(&s->v, &s->sh, keep_p, st));
+        /* the reset adds the live rows it formed to the device's count */
+        HBK_TRY(hbk_deferred_reset(&s->v, &s->sh, keep_p, hbk_flush_tc_live_count(s->tc_ws, s->m), st));
         *launches += 5; /* live list, slot maxima, coefficient digits, flush, reset */
     } else {
-        s->flush_bytes += 8.0 * s->A->k.n * ((double)L + per_shift * s->m);
+        s->flush_bytes += 8.0 * s->A->k.n * per_shift * s->m;
         HBK_TRY(hbk_deferred_flush(&s->v, &s->sh, keep_p, st));
         *launches += keep_p ? 3 : 2;
     }
@@ -784,66 +843,62 @@ static int do_flush(hbicg_solver *s, int keep_p, int L, int k_last, int *launche
 static int fused_init(hbicg_solver *s, int seed, int inline_ps, int *launches) {
     cudaStream_t st = s->ctx->stream;
     HBK_TRY(hbk_fused_init(&s->A->k, &s->v, &s->sh, s->d_b, seed, s->p.tol, s->p.switching ? 1 : 0, inline_ps, st));
-    *launches += 6 + (s->v.deferred ? 1 : s->m);
+    *launches += 4 + (s->v.deferred ? 1 : 0);
     return HBICG_OK;
 }
 
 /* A fused solve paused with a full basis (scalars in h_sc): form x_j and
  * p_j, restart the basis (the reset lets the solve run on) and note the last
- * iteration the flush covered. */
-static int fused_pause_flush(hbicg_solver *s, int *k_flushed, int *launches, int *flushes, double *flush_ms) {
+ * iteration the flush covered.  Nothing waits here: flush_elapsed reads the
+ * flush's time once it is over. */
+static int fused_pause_flush(hbicg_solver *s, int *k_flushed, int *launches, int *flushes) {
     cudaStream_t st = s->ctx->stream;
     hbk_scalars *h = s->ctx->h_sc;
     int rc = ensure_pmat(s);
     if (rc) return rc;
-    float t = 0.f;
     CUDA_TRY(cudaEventRecord(s->ctx->evf0, st));
     rc = do_flush(s, 1, h->slots, *k_flushed, launches);
     if (rc) return rc;
     *k_flushed = h->k - 1;
     if (s->early_x && (rc = early_copies(s, *k_flushed, launches))) return rc;
     CUDA_TRY(cudaEventRecord(s->ctx->evf1, st));
-    CUDA_TRY(cudaEventSynchronize(s->ctx->evf1));
-    CUDA_TRY(cudaEventElapsedTime(&t, s->ctx->evf0, s->ctx->evf1));
-    *flush_ms += t;
+    s->flush_timed = 1;
     (*flushes)++;
     return HBICG_OK;
 }
 
+/* adds the device time of the flush recorded last, waiting for it */
+static int flush_elapsed(hbicg_solver *s, double *flush_ms) {
+    if (!s->flush_timed) return HBICG_OK;
+    float t = 0.f;
+    s->flush_timed = 0;
+    CUDA_TRY(cudaEventSynchronize(s->ctx->evf1));
+    CUDA_TRY(cudaEventElapsedTime(&t, s->ctx->evf0, s->ctx->evf1));
+    *flush_ms += t;
+    return HBICG_OK;
+}
+
 /* The end of a fused solve whose iterations are over (h_sc holds its
- * scalars): in the deferred mode the last flush and x_j back to rows; the
- * final scalars in h_sc. */
-static int fused_tail(hbicg_solver *s, int k_flushed, int *launches, double *flush_ms) {
+ * scalars): in the deferred mode the last flush and x_j back to rows. */
+static int fused_tail(hbicg_solver *s, int k_flushed, int *launches) {
     cudaStream_t st = s->ctx->stream;
     hbk_scalars *h = s->ctx->h_sc;
-    if (s->v.deferred) {
-        float t = 0.f;
-        CUDA_TRY(cudaEventRecord(s->ctx->evf0, st));
-        int rc = do_flush(s, 0, h->slots, k_flushed, launches);
-        if (rc) return rc;
-        CUDA_TRY(cudaEventRecord(s->ctx->evf1, st));
-        /* x_j were panel-major during the solve; rows already on their way to
-         * the host are rewritten with the same values only after those copies */
-        if (s->early_pending) {
-            CUDA_TRY(cudaEventRecord(s->ctx->cev, s->ctx->cstream));
-            CUDA_TRY(cudaStreamWaitEvent(st, s->ctx->cev, 0));
-        }
-        HBK_TRY(hbk_panel_to_rows(s->v.Xp, s->v.pm, s->A->k.n, s->xrows, s->xld, st));
-        ++*launches;
-        CUDA_TRY(cudaMemcpyAsync(h, s->d_sc, sizeof(hbk_scalars), cudaMemcpyDeviceToHost, st));
-        int tc_err = 0;
-        if (s->d_tc_err) CUDA_TRY(cudaMemcpyAsync(&tc_err, s->d_tc_err, sizeof(int), cudaMemcpyDeviceToHost, st));
-        CUDA_TRY(cudaStreamSynchronize(st));
-        CUDA_TRY(cudaEventElapsedTime(&t, s->ctx->evf0, s->ctx->evf1));
-        *flush_ms += t;
-        if (tc_err) {
-            set_msg("tensor-core flush: an mbarrier wait timed out");
-            return HBICG_E_TIMEOUT;
-        }
-        return HBICG_OK;
+    if (!s->v.deferred) return HBICG_OK;
+    CUDA_TRY(cudaEventRecord(s->ctx->evf0, st));
+    int rc = do_flush(s, 0, h->slots, k_flushed, launches);
+    if (rc) return rc;
+    CUDA_TRY(cudaEventRecord(s->ctx->evf1, st));
+    s->flush_timed = 1;
+    h->slots = 1; /* as the reset leaves them */
+    h->slot_r_old = 0;
+    /* x_j were panel-major during the solve; rows already on their way to
+     * the host are rewritten with the same values only after those copies */
+    if (s->early_pending) {
+        CUDA_TRY(cudaEventRecord(s->ctx->cev, s->ctx->cstream));
+        CUDA_TRY(cudaStreamWaitEvent(st, s->ctx->cev, 0));
     }
-    CUDA_TRY(cudaMemcpyAsync(h, s->d_sc, sizeof(hbk_scalars), cudaMemcpyDeviceToHost, st));
-    CUDA_TRY(cudaStreamSynchronize(st));
+    HBK_TRY(hbk_panel_to_rows(s->v.Xp, s->v.pm, s->A->k.n, s->xrows, s->xld, st));
+    ++*launches;
     return HBICG_OK;
 }
 
@@ -894,11 +949,12 @@ static int run_persistent(hbicg_solver *s, int *launches, int *flushes, double *
             break;
         }
         if (!(h->finished && (h->status & HBK_ST_BASIS_FULL) && !(h->status & HBK_ST_BREAKDOWN))) break;
-        if ((rc = fused_pause_flush(s, &k_flushed, launches, flushes, flush_ms)) != HBICG_OK) break;
+        if ((rc = fused_pause_flush(s, &k_flushed, launches, flushes)) != HBICG_OK) break;
+        if ((rc = flush_elapsed(s, flush_ms)) != HBICG_OK) break;
     }
     hbicg__dev_free(ws, st);
     if (rc) return rc;
-    return fused_tail(s, k_flushed, launches, flush_ms);
+    return fused_tail(s, k_flushed, launches);
 }
 
 static int run_fused(hbicg_solver *s, int seed, int *launches, int *flushes, double *flush_ms) {
@@ -933,6 +989,7 @@ static int run_fused(hbicg_solver *s, int seed, int *launches, int *flushes, dou
         }
         CUDA_TRY(cudaMemcpyAsync(h, s->d_sc, sizeof(hbk_scalars), cudaMemcpyDeviceToHost, st));
         CUDA_TRY(cudaStreamSynchronize(st));
+        if ((rc0 = flush_elapsed(s, flush_ms)) != HBICG_OK) return rc0; /* of the flush before this launch */
         if (looped) { /* every body: a chunk of iterations' kernels and the condition kernel */
             *launches += (h->loops - loops_seen) * (s->chunk * s->launches_per_iter + 1);
             loops_seen = h->loops;
@@ -946,12 +1003,12 @@ static int run_fused(hbicg_solver *s, int seed, int *launches, int *flushes, dou
             ++*launches;
         }
         if (!over && (h->status & HBK_ST_BASIS_FULL)) {
-            int rc = fused_pause_flush(s, &k_flushed, launches, flushes, flush_ms);
+            int rc = fused_pause_flush(s, &k_flushed, launches, flushes);
             if (rc) return rc;
         }
         if (over) break;
     }
-    return fused_tail(s, k_flushed, launches, flush_ms);
+    return fused_tail(s, k_flushed, launches);
 }
 
 /* compulsory HBM bytes of the fused schedule for one solve */
@@ -1005,6 +1062,7 @@ typedef struct {
     double *h_sigma, *h_res;
     int *act, *sw_k, *sw_seed, *conv;
     unsigned char *fixed;
+    void *pack; /* fused form: what the device packed at the end (hbk_pack) */
 } run_host_t;
 
 static void run_host_free(run_host_t *hb) {
@@ -1015,6 +1073,7 @@ static void run_host_free(run_host_t *hb) {
     free(hb->sw_seed);
     free(hb->conv);
     free(hb->fixed);
+    free(hb->pack);
     memset(hb, 0, sizeof *hb);
 }
 
@@ -1031,6 +1090,10 @@ typedef struct {
     int k, n_sw, final_seed, status, launches, flushes;
     double flush_ms;
     const double *r_final;
+    const double *hist;    /* fused form: alpha, beta, omega, (r,r) of iterations [0, k), one after the other */
+    const double *checked; /* squared true residuals of every shift, when params.refine checks them */
+    double bb;             /* (b, b) */
+    int sigma_here;        /* hb.h_sigma is filled */
     double shared_ms; /* >= 0: the iterations ran in a launch shared with other solves, this long */
 } run_t;
 
@@ -1042,31 +1105,44 @@ static int run_end(hbicg_solver *s, run_t *r, int rc);
 /* params.refine: true residuals of every shift; a shift above tol gets
  * x_j += e with (A + sigma_j I) e = b - (A + sigma_j I) x_j solved (single
  * shift, incremental form) to 0.5 tol ||b|| / ||r_j||; at most 3 rounds. */
-static int refine_shifts(hbicg_solver *s, const double *h_sigma, int *refined, unsigned char *fixed) {
+static int refine_shifts(hbicg_solver *s, run_t *rn, int *refined, unsigned char *fixed) {
     cudaStream_t st = s->ctx->stream;
     const unsigned n = s->A->k.n;
     const int m = s->m;
+    double *h_sigma = rn->hb.h_sigma;
     double *h = malloc(sizeof(double) * (size_t)m), *r = NULL, *e = NULL;
     hbicg_solver *sub = NULL;
     int rc = HBICG_OK;
     if (!h) return HBICG_E_NOMEM;
-    HBK_GOTO(hbk_dot(n, s->d_b, s->d_b, s->sh.partials, s->sh.counters + 7, s->d_dot, st));
-    CUDA_GOTO(cudaMemcpyAsync(s->ctx->h_dbl, s->d_dot, sizeof(double), cudaMemcpyDeviceToHost, st));
-    CUDA_GOTO(cudaStreamSynchronize(st));
-    const double bn = sqrt(s->ctx->h_dbl[0]);
-    for (int round = 0; round < 3 && rc == HBICG_OK && bn > 0.0; ++round) {
-        HBK_GOTO(hbk_true_residuals_ld(&s->A->k, s->xrows, s->xld, s->d_b, s->d_sigma, m, HBK_MAX_GRID, s->sh.partials,
-                                       s->sh.counters + 16, s->d_res, st));
-        CUDA_GOTO(cudaMemcpyAsync(h, s->d_res, sizeof(double) * (size_t)m, cudaMemcpyDeviceToHost, st));
+    if (!rn->checked) { /* the plain form: (b, b) from the device */
+        HBK_GOTO(hbk_dot(n, s->d_b, s->d_b, s->sh.partials, s->sh.counters + 7, s->d_dot, st));
+        CUDA_GOTO(cudaMemcpyAsync(s->ctx->h_dbl, s->d_dot, sizeof(double), cudaMemcpyDeviceToHost, st));
         CUDA_GOTO(cudaStreamSynchronize(st));
+        rn->bb = s->ctx->h_dbl[0];
+    }
+    const double bn = sqrt(rn->bb);
+    for (int round = 0; round < 3 && rc == HBICG_OK && bn > 0.0; ++round) {
+        if (round == 0 && rn->checked) {
+            memcpy(h, rn->checked, sizeof(double) * (size_t)m);
+        } else {
+            HBK_GOTO(hbk_true_residuals_ld(&s->A->k, s->xrows, s->xld, s->d_b, s->d_sigma, m, HBK_MAX_GRID,
+                                           s->sh.partials, s->sh.counters + 16, s->d_res, st));
+            CUDA_GOTO(cudaMemcpyAsync(h, s->d_res, sizeof(double) * (size_t)m, cudaMemcpyDeviceToHost, st));
+            CUDA_GOTO(cudaStreamSynchronize(st));
+        }
         int any = 0;
         for (int j = 0; j < m && rc == HBICG_OK; ++j) {
             const double res = sqrt(h[j]) / bn;
             if (res <= s->p.tol) continue;
             any = 1;
+            if (!rn->sigma_here) {
+                CUDA_GOTO(cudaMemcpyAsync(h_sigma, s->d_sigma, sizeof(double) * (size_t)m, cudaMemcpyDeviceToHost, st));
+                CUDA_GOTO(cudaStreamSynchronize(st));
+                rn->sigma_here = 1;
+            }
             if (!r) {
-                CUDA_GOTO(cudaMalloc((void **)&r, sizeof(double) * ((size_t)n + 1)));
-                CUDA_GOTO(cudaMalloc((void **)&e, sizeof(double) * ((size_t)n + 1)));
+                CUDA_GOTO(pool_alloc((void **)&r, sizeof(double) * ((size_t)n + 1), st));
+                CUDA_GOTO(pool_alloc((void **)&e, sizeof(double) * ((size_t)n + 1), st));
             }
             if (!sub) {
                 hbicg_params p1 = s->p;
@@ -1093,8 +1169,8 @@ static int refine_shifts(hbicg_solver *s, const double *h_sigma, int *refined, u
     }
 out:
     hbicg_solver_destroy(sub);
-    cudaFree(r);
-    cudaFree(e);
+    hbicg__dev_free(r, st);
+    hbicg__dev_free(e, st);
     free(h);
     return rc;
 }
@@ -1156,8 +1232,11 @@ static int run_begin(hbicg_solver *s, const double *b, const double *sigma, run_
         return HBICG_E_NOMEM;
     }
     if (m > 0) {
-        if (in_where == HBICG_DEVICE) CUDA_TRY(cudaMemcpyAsync(h_sigma, sigma, sizeof(double) * m, cudaMemcpyDeviceToHost, st));
-        else memcpy(h_sigma, sigma, sizeof(double) * m);
+        /* (device shifts: the fused form needs them here only for a correction) */
+        if (in_where != HBICG_DEVICE) memcpy(h_sigma, sigma, sizeof(double) * m);
+        else if (s->p.form == HBICG_FORM_PLAIN)
+            CUDA_TRY(cudaMemcpyAsync(h_sigma, sigma, sizeof(double) * m, cudaMemcpyDeviceToHost, st));
+        r->sigma_here = in_where != HBICG_DEVICE || s->p.form == HBICG_FORM_PLAIN;
         CUDA_TRY(cudaMemcpyAsync(s->d_sigma, sigma, sizeof(double) * m, kin, st));
     }
     CUDA_TRY(cudaMemcpyAsync(s->d_b, b, sizeof(double) * n, kin, st));
@@ -1198,13 +1277,16 @@ static int run_begin(hbicg_solver *s, const double *b, const double *sigma, run_
     }
     CUDA_TRY(cudaEventRecord(ctx->ev0, st));
     s->flush_bytes = 0.0;
+    s->flush_timed = 0;
     r->k = 1;
     r->final_seed = seed;
     r->status = HBICG_OK;
     return HBICG_OK;
 }
 
-/* after the fused iterations: scalars in the context's host copy (h_sc) */
+/* After the fused iterations (scalars in the context's host copy, h_sc): the
+ * true residuals of a converged solve when params.refine checks them, and
+ * everything the host needs of the device in one copy (it waits). */
 static int fused_collect(hbicg_solver *s, run_t *r) {
     cudaStream_t st = s->ctx->stream;
     const int m = s->m;
@@ -1212,16 +1294,39 @@ static int fused_collect(hbicg_solver *s, run_t *r) {
     r->k = h->k;
     r->n_sw = h->n_sw;
     r->final_seed = h->seed;
+    r->bb = h->bb;
     if (h->status & (HBK_ST_BREAKDOWN | HBK_ST_SHIFT_FAIL)) r->status = HBICG_E_BREAKDOWN;
-    if (m > 0) {
-        CUDA_TRY(cudaMemcpyAsync(r->hb.conv, s->sh.conv_k, sizeof(int) * m, cudaMemcpyDeviceToHost, st));
-        int nl = r->n_sw < m ? r->n_sw : m;
-        if (nl) {
-            CUDA_TRY(cudaMemcpyAsync(r->hb.sw_k, s->sh.sw_k, sizeof(int) * nl, cudaMemcpyDeviceToHost, st));
-            CUDA_TRY(cudaMemcpyAsync(r->hb.sw_seed, s->sh.sw_seed, sizeof(int) * nl, cudaMemcpyDeviceToHost, st));
-        }
+    /* only after a converged solve: a solve stopped by max_iter or a breakdown
+     * keeps its x as the reference leaves it */
+    const int check = r->status == HBICG_OK && s->p.refine && m > 0 && r->k < s->kcap;
+    if (check)
+        HBK_TRY(hbk_true_residuals_ld(&s->A->k, s->xrows, s->xld, s->d_b, s->d_sigma, m, HBK_MAX_GRID, s->sh.partials,
+                                      s->sh.counters + 16, s->d_res, st));
+    CUDA_TRY(cudaEventRecord(s->ctx->ev1, st));
+    const int nk = r->k < s->kcap ? r->k : s->kcap;
+    const size_t bytes = hbk_pack_bytes(m, nk);
+    char *p = r->hb.pack = malloc(bytes);
+    if (!p) {
+        set_msg("host scratch of %zu bytes", bytes);
+        return HBICG_E_NOMEM;
     }
-    CUDA_TRY(cudaMemcpyAsync(r->hb.act, s->sh.act_hist, sizeof(int) * ((size_t)s->kcap + 1), cudaMemcpyDeviceToHost, st));
+    HBK_TRY(hbk_pack(&s->sh, nk, s->d_res, s->d_tc_err, s->d_pack, st));
+    CUDA_TRY(cudaMemcpyAsync(p, s->d_pack, bytes, cudaMemcpyDeviceToHost, st));
+    CUDA_TRY(cudaStreamSynchronize(st));
+    const double *d = (const double *)p;
+    s->flush_bytes += 8.0 * s->A->k.n * d[0];
+    if (check) r->checked = d + 1;
+    r->hist = d + 1 + m;
+    const int *w = (const int *)(r->hist + 4 * (size_t)nk);
+    const int nl = r->n_sw < m ? r->n_sw : m;
+    memcpy(r->hb.conv, w, sizeof(int) * (size_t)m);
+    memcpy(r->hb.sw_k, w + m, sizeof(int) * (size_t)nl);
+    memcpy(r->hb.sw_seed, w + 2 * m, sizeof(int) * (size_t)nl);
+    memcpy(r->hb.act, w + 3 * m + 1, sizeof(int) * (size_t)nk);
+    if (w[3 * m]) {
+        set_msg("tensor-core flush: an mbarrier wait timed out");
+        return HBICG_E_TIMEOUT;
+    }
     r->r_final = s->v.deferred ? s->v.V + (size_t)h->slot_r_old * s->ld : s->v.rbuf[(h->k - 1) & 1];
     return HBICG_OK;
 }
@@ -1266,21 +1371,19 @@ static int run_end(hbicg_solver *s, run_t *r, int rc) {
     touch_t *touch = &r->touch;
     run_host_t *hb = &r->hb;
     int *act = hb->act, *sw_k = hb->sw_k, *sw_seed = hb->sw_seed, *conv = hb->conv;
-    const double *h_sigma = hb->h_sigma;
     const enum cudaMemcpyKind kout = out_where == HBICG_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
     const int k = r->k, n_sw = r->n_sw, final_seed = r->final_seed;
     int status = r->status;
     const double *r_final = r->r_final;
-    CUDA_TRY(cudaEventRecord(ctx->ev1, st));
+    if (s->p.form == HBICG_FORM_PLAIN) CUDA_TRY(cudaEventRecord(ctx->ev1, st));
     /* copies issued during the solve finish before anything rewrites X */
     if (s->early_pending) CUDA_TRY(cudaStreamSynchronize(ctx->cstream));
     int refined = 0;
     unsigned char *fixed = hb->fixed = s->early_x ? calloc((size_t)m, 1) : NULL;
-    /* only after a converged solve: a solve stopped by max_iter or a breakdown
-     * keeps its x as the reference leaves it */
+    /* only after a converged solve (as fused_collect's check) */
     if (rc == HBICG_OK && status == HBICG_OK && s->p.refine && m > 0 && k < s->kcap) {
-        rc = refine_shifts(s, h_sigma, &refined, fixed);
-        CUDA_TRY(cudaEventRecord(ctx->ev1, st)); /* solve_ms includes the corrections */
+        rc = refine_shifts(s, r, &refined, fixed);
+        if (refined) CUDA_TRY(cudaEventRecord(ctx->ev1, st)); /* solve_ms includes the corrections */
     }
     touch_join(touch);
     if (rc == HBICG_OK && x && m > 0) {
@@ -1316,6 +1419,7 @@ static int run_end(hbicg_solver *s, run_t *r, int rc) {
         CUDA_TRY(cudaMemcpyAsync(ctx->h_dbl, s->d_dot, sizeof(double), cudaMemcpyDeviceToHost, st));
     }
     CUDA_TRY(cudaStreamSynchronize(st));
+    if (rc == HBICG_OK) rc = flush_elapsed(s, &r->flush_ms);
     if (h_res) {
         const double bn = sqrt(ctx->h_dbl[0]);
         for (int j = 0; j < m; j++) {
@@ -1354,10 +1458,9 @@ static int run_end(hbicg_solver *s, run_t *r, int rc) {
         if (stats->true_residual && h_res) memcpy(stats->true_residual, h_res, sizeof(double) * m);
         if (s->p.form == HBICG_FORM_FUSED && k > 0) {
             const size_t nk = (size_t)(k < s->kcap ? k : s->kcap);
-            if (stats->seed_alpha) cudaMemcpy(stats->seed_alpha, s->sh.a_hist, sizeof(double) * nk, cudaMemcpyDeviceToHost);
-            if (stats->seed_beta) cudaMemcpy(stats->seed_beta, s->sh.b_hist, sizeof(double) * nk, cudaMemcpyDeviceToHost);
-            if (stats->seed_omega) cudaMemcpy(stats->seed_omega, s->sh.w_hist, sizeof(double) * nk, cudaMemcpyDeviceToHost);
-            if (stats->seed_rr) cudaMemcpy(stats->seed_rr, s->sh.rr_hist, sizeof(double) * nk, cudaMemcpyDeviceToHost);
+            double *const out[4] = {stats->seed_alpha, stats->seed_beta, stats->seed_omega, stats->seed_rr};
+            for (int i = 0; i < 4; i++)
+                if (out[i] && r->hist) memcpy(out[i], r->hist + i * nk, sizeof(double) * nk);
         }
     }
     if (rc) return rc;
@@ -1557,7 +1660,13 @@ int hbicg__group_launch(hbicg__group *g) {
                 group_keep(g->msg[f]);
                 run[f] = 0;
             } else if (h->finished && (h->status & HBK_ST_BASIS_FULL) && !(h->status & HBK_ST_BREAKDOWN)) {
-                g->itrc[f] = fused_pause_flush(s, &g->k_flushed[f], &r->launches, &r->flushes, &r->flush_ms);
+                g->itrc[f] = fused_pause_flush(s, &g->k_flushed[f], &r->launches, &r->flushes);
+                /* (the next round's launch has a stream of its own: the flush is over before it) */
+                if (!g->itrc[f]) g->itrc[f] = flush_elapsed(s, &r->flush_ms);
+                if (!g->itrc[f] && cudaStreamSynchronize(s->ctx->stream) != cudaSuccess) {
+                    set_msg("shared launch: a flush failed");
+                    g->itrc[f] = HBICG_E_CUDA;
+                }
                 if (g->itrc[f]) group_keep(g->msg[f]);
                 run[f] = g->itrc[f] == HBICG_OK;
                 resumed += run[f];
@@ -1605,7 +1714,7 @@ int hbicg__group_finish(hbicg__group *g, int slot) {
                 it = HBICG_E_CUDA;
             }
         }
-        if (it == HBICG_OK) it = fused_tail(s, g->k_flushed[slot], &r->launches, &r->flush_ms);
+        if (it == HBICG_OK) it = fused_tail(s, g->k_flushed[slot], &r->launches);
         if (it == HBICG_OK) it = fused_collect(s, r);
         r->shared_ms = g->ms;
         rc = run_end(s, r, it);
