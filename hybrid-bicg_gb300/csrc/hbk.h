@@ -46,6 +46,7 @@ extern "C" {
 #define HBK_HYB_WINDOW 1024  /* rows are sorted by length only inside windows of this many consecutive rows */
 #define HBK_HYB_L4 128       /* long rows up to this length: 4 lanes each, 8 rows per warp */
 #define HBK_HYB_L16 512      /* longer rows up to this length: 16 lanes each, 2 rows per warp; longer: a warp */
+#define HBK_FMT_SELLN 5      /* kernels of a SELL matrix of few entries per row (hbk_matrix.fmt stays HBK_FMT_SELL) */
 #define HBK_FMT_HYBW 4       /* kernels of a HYB matrix with nwide > 0 (hbk_matrix.fmt stays HBK_FMT_HYB) */
 #define HBK_FMT_MERGE 3      /* CSR; rows up to HBK_MERGE_LONG entries in merge-path blocks, longer rows one warp each */
 #define HBK_MERGE_IPT 8      /* merge items (row ends + nonzeros) per lane of a block */

@@ -81,6 +81,26 @@ __global__ void __launch_bounds__(NT, HBK_SELL_MINB) k_spmv<HBK_FMT_SELL>(hbk_ma
     spmv_rows<HBK_FMT_SELL, 7>(A, x, pre, epi);
 }
 
+template <>
+__global__ void __launch_bounds__(NT, HBK_SELL_MINB) k_spmv<HBK_FMT_SELLN>(hbk_matrix A, const double *__restrict__ x,
+                                                                          double *__restrict__ y, double sigma,
+                                                                          int add) {
+    EpiStore epi{y, x, sigma, add};
+    auto pre = [&](unsigned r) { return add ? x[r] : 0.0; };
+    spmv_rows<HBK_FMT_SELLN>(A, x, pre, epi);
+}
+// SELL-32 product of a small matrix: a row or two per thread, so nothing to
+// keep ahead; six blocks per SM (250 k rows of five entries: 6.7 us, 8.2 us
+// with slices ahead; at 1 M rows 16.7 / 16.1; seven entries: the same up to
+// 1 M rows)
+constexpr unsigned SMALL_ROWS = 1u << 19;
+__global__ void __launch_bounds__(NT) k_spmv_small(hbk_matrix A, const double *__restrict__ x, double *__restrict__ y,
+                                                   double sigma, int add) {
+    EpiStore epi{y, x, sigma, add};
+    auto pre = [&](unsigned r) { return add ? x[r] : 0.0; };
+    spmv_rows_sell(A, x, pre, epi, HwGrid());
+}
+
 template <int FMT>
 __global__ void __launch_bounds__(NT) k_spmv_acc(hbk_matrix A, const double *__restrict__ x, double *__restrict__ y) {
     EpiAccum epi{y};
@@ -133,6 +153,12 @@ __global__ void __launch_bounds__(NT, HBK_SELL_MINB) k_true_res<HBK_FMT_SELL>(
     hbk_matrix A, const double *__restrict__ X, size_t ld, const double *__restrict__ b,
     const double *__restrict__ sigma, double *partials, unsigned *counters, double *out) {
     true_res_body<HBK_FMT_SELL>(A, X, ld, b, sigma, partials, counters, out);
+}
+template <>
+__global__ void __launch_bounds__(NT, HBK_SELL_MINB) k_true_res<HBK_FMT_SELLN>(
+    hbk_matrix A, const double *__restrict__ X, size_t ld, const double *__restrict__ b,
+    const double *__restrict__ sigma, double *partials, unsigned *counters, double *out) {
+    true_res_body<HBK_FMT_SELLN>(A, X, ld, b, sigma, partials, counters, out);
 }
 template <>
 __global__ void __launch_bounds__(NT, HBK_HYBW_MINB) k_true_res<HBK_FMT_HYBW>(
@@ -365,6 +391,10 @@ static int product_grid(const hbk_matrix *A) {
 
 int hbk_spmv(const hbk_matrix *A, const double *x, double *y, double sigma, int sigma_add, cudaStream_t st) {
     if (!A->n) return 0;
+    if (A->fmt == HBK_FMT_SELL && A->n < SMALL_ROWS) {
+        k_spmv_small<<<A->grid, NT, 0, st>>>(*A, x, y, sigma, sigma_add);
+        return (int)cudaGetLastError();
+    }
     HBK_LAUNCH_FMT(*A, k_spmv, product_grid(A), NT, st, *A, x, y, sigma, sigma_add);
     return (int)cudaGetLastError();
 }

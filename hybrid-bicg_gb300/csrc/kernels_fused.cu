@@ -287,6 +287,10 @@ __global__ void __launch_bounds__(NT, HBK_SELL_MINB) k_seed_s<HBK_FMT_SELL>(Ctx 
     seed_s_body<HBK_FMT_SELL>(c, HwGrid());
 }
 template <>
+__global__ void __launch_bounds__(NT, HBK_SELL_MINB) k_seed_s<HBK_FMT_SELLN>(Ctx c) {
+    seed_s_body<HBK_FMT_SELLN>(c, HwGrid());
+}
+template <>
 __global__ void __launch_bounds__(NT, HBK_HYBW_MINB) k_seed_s<HBK_FMT_HYBW>(Ctx c) {
     seed_s_body<HBK_FMT_HYBW>(c, HwGrid());
 }
@@ -390,6 +394,10 @@ __global__ void __launch_bounds__(NT) k_seed_y(Ctx c) { seed_y_body<FMT>(c, HwGr
 template <>
 __global__ void __launch_bounds__(NT, HBK_SELL_MINB) k_seed_y<HBK_FMT_SELL>(Ctx c) {
     seed_y_body<HBK_FMT_SELL>(c, HwGrid());
+}
+template <>
+__global__ void __launch_bounds__(NT, HBK_SELL_MINB) k_seed_y<HBK_FMT_SELLN>(Ctx c) {
+    seed_y_body<HBK_FMT_SELLN>(c, HwGrid());
 }
 template <>
 __global__ void __launch_bounds__(NT, HBK_HYBW_MINB) k_seed_y<HBK_FMT_HYBW>(Ctx c) {
@@ -1584,7 +1592,7 @@ static void launch_iteration(Ctx &c, const hbk_matrix *A, int early, cudaStream_
     // that start early would crowd onto the SMs the kernel before leaves free
     // and then run long: the incremental update (FP64-bound; 32^3: 3.4 -> 4.7
     // ms) and the products of the other forms (HYB: 68 -> 75 ms).
-    const bool e = early > 0, es = e && FMT == HBK_FMT_SELL;
+    const bool e = early > 0, es = e && (FMT == HBK_FMT_SELL || FMT == HBK_FMT_SELLN);
     launch(k_seed_s<FMT>, gs, NT, es && early > 1, st, c);
     launch(k_seed_q, q.blocks, q.threads, e, st, c);
     launch(k_seed_y<FMT>, gy, NT, es, st, c);
@@ -1597,7 +1605,8 @@ extern "C" {
 
 int hbk_fused_iteration(const hbk_matrix *A, const hbk_vectors *v, const hbk_shifts *sh, int early, cudaStream_t st) {
     Ctx c = make_ctx(A, v, sh);
-    if (A->fmt == HBK_FMT_SELL) launch_iteration<HBK_FMT_SELL>(c, A, early, st);
+    if (sell_narrow(*A)) launch_iteration<HBK_FMT_SELLN>(c, A, early, st);
+    else if (A->fmt == HBK_FMT_SELL) launch_iteration<HBK_FMT_SELL>(c, A, early, st);
     else if (A->fmt == HBK_FMT_MERGE) launch_iteration<HBK_FMT_MERGE>(c, A, early, st);
     else if (A->fmt == HBK_FMT_HYB && A->nwide) launch_iteration<HBK_FMT_HYBW>(c, A, early, st);
     else if (A->fmt == HBK_FMT_HYB) launch_iteration<HBK_FMT_HYB>(c, A, early, st);

@@ -13,7 +13,8 @@ import pytest
 @pytest.mark.parametrize("dims,m,mode", [
     ((3, 2, 2), 2, "incremental"), ((3, 3, 3), 1, "incremental"), ((9, 8, 7), 65, "incremental"),
     ((8, 8, 8), 130, "incremental"), ((8, 8, 8), 300, "incremental"), ((8, 9, 8), 300, "deferred"),
-    ((31, 30, 29), 5, "incremental"), ((60, 61, 62), 3, "deferred"),
+    ((31, 30, 29), 5, "incremental"), ((60, 61, 62), 3, "deferred"), ((41, 37, 1), 9, "incremental"),
+    ((211, 198, 1), 6, "deferred"),
 ])
 def test_iteration_edges(cuda, pkg, oracle, dims, m, mode):
     a = pkg.workloads.stencil_cd3d(*dims)
@@ -29,7 +30,8 @@ def test_iteration_edges(cuda, pkg, oracle, dims, m, mode):
 @pytest.mark.gpu
 @pytest.mark.parametrize("n,lens", [
     (1, [1]), (31, [7]), (33, [8, 0, 7]), (64, [64]), (255, [9, 1]), (257, [8]), (1000, [0, 3, 15, 16, 17]),
-    (116737, [7, 7, 7, 9]), (250001, [5]),
+    (116737, [7, 7, 7, 9]), (250001, [5]), (524287, [3, 6]), (524288, [5, 5, 6]), (600001, [0, 4, 5, 12]),
+    (700003, [7, 8, 5, 9]),
 ])
 @pytest.mark.parametrize("sigma", [0.0, 0.75])
 def test_sell_product_edges(cuda, pkg, n, lens, sigma):
