@@ -1,58 +1,69 @@
 // Basis flush on the tensor cores: x_j += xi_j Pmat_j + sum_l Xc[j][l] V[l],
-// p_j = rho_j Pmat_j + sum_l Pc[j][l] V[l], with FP64 accuracy from BF16
+// p_j = rho_j Pmat_j + sum_l Pc[j][l] V[l], with FP64 accuracy from FP16
 // tcgen05 MMAs.
 //
 // GB300 runs FP64 at ~1.2 TFLOP/s, so the FP64 form of this product is the
-// solver's bottleneck.  Here each FP64 operand becomes a signed 62-bit fixed
-// point integer against a power-of-two scale — per output row for the
-// coefficients, per vector element for the basis, after normalising every
-// basis slot by a power of two — cut into nine balanced 7-bit digits in
-// [-64, 64], each exact in BF16.  A digit product is at most 2^12, so the sum
-// over K = 64 slots of all pairs of one diagonal (s + t = d, at most nine
-// pairs) stays below 2^22: each diagonal d = 0..8 accumulates exactly in its
-// own FP32 TMEM accumulator and converts to an integer with one FP32 add.
-// Diagonals past 8 are dropped (their total is below 2^-54 of the
-// row/element scale, the accuracy of an FP64 dot product of the same length).
-// The epilogue joins the nine exact diagonal sums in 64-bit integer arithmetic
-// (keeping floor(T / 2^12) of the 75-bit sum T: the dropped bits are below
-// 2^-56 of the row x element scale) and rounds once to FP64; only the
+// solver's bottleneck.  Here each FP64 operand becomes a signed fixed point
+// integer (62 bits for the basis, 63 for the coefficients) against a
+// power-of-two scale — per output row for the coefficients, per vector element
+// for the basis, after normalising every basis slot by a power of two — cut into
+// eight balanced 8-bit digits in [-128, 128], each exact in FP16.  A digit
+// product is at most 2^14, so the sum over K = 64 slots of all pairs of one
+// diagonal (s + t = d, at most eight pairs) stays below 2^23: each diagonal
+// d = 0..7 accumulates exactly in its own FP32 TMEM accumulator.  Diagonals past
+// 7 are dropped (their total is below 2^-54 of the row/element scale, the
+// accuracy of an FP64 dot product of the same length: the coefficients' 63rd bit
+// pays for that; with nine 7-bit digits the bound is the same).
+// The epilogue joins the eight exact diagonal sums in 64-bit integer arithmetic
+// (keeping T / 2^13 of the 75-bit sum T, rounded: a unit is 2^-56 of the row x
+// element scale) and rounds once to FP64; only the
 // own-vector terms use the FP64 pipe.  (The digit splitting is the error-free
 // splitting of Ozaki, Ogita, Oishi and Rump for matrix products, arranged here
 // so that the exact sums fit TMEM.)
 //
-// One CTA per SM (226 KB of shared memory, all 512 TMEM columns), persistent
+// One CTA per SM (166 KB of shared memory, all 512 TMEM columns), persistent
 // over tiles of 48 vector elements (one panel of the panel-major x_j and p_j
 // arrays, whose values for all shifts lie in one contiguous block); 128
 // output rows per group of 64 shifts, ordered so that
 // TMEM lanes 32q..32q+15 hold the x rows of shifts 16q..16q+15 and lanes
 // 32q+16..32q+31 their p rows.  Warps 0-2 make the basis digits of a tile
 // into one of two buffers (tile t+1's while the tensor core reads tile t's);
-// one thread of warp 3 issues its MMAs (M=128, N up to 256, K=16; 52 per
-// tile; coefficient digit slices 0-1 from TMEM, 2-8 from shared memory) into
-// nine accumulators, so that the digit builders never wait behind the MMA
+// one thread of warp 3 issues its MMAs (M=128, N up to 256, K=16; 44 per
+// tile; coefficient digit slices 0-3 from TMEM, 4-7 from shared memory) into
+// eight accumulators, so that the digit builders never wait behind the MMA
 // issue; warps 4-15 empty the accumulators into registers first, so that the
 // next tile's MMAs run while they round, add the own-vector terms and write x
 // and p.  Every wait is bounded: a timeout sets an error flag, the CTA skips
 // its remaining work and still frees its TMEM.
 //
-// What bounds it (clock stamps, n = 2 M, 64 shifts, 59 slots; about 15 k clocks
-// per tile): the epilogue warps are busy for all but 1.5 k of them (rounding,
-// own terms and stores 9.5 k, of which the FP64 pipe 6.1 k, draining 2.1 k,
-// loads 1.8 k) and the builders for nearly all (digits 6.1 k, waiting for
-// their loads 3.5 k); both share the SM quarters' integer pipes, and the tensor
-// core waits 8.5 k.  So instructions count: digits as packed BF16 pairs, basis
-// loads with fewer conditions and a rounding whose rare cases are out of line
-// took a flush from 2.49 to 2.20 ms (256^3, all shifts live: 19.5 to 17.2).  Tried and not kept: x + y of two columns
-// in one FP64 add through shuffles (+3 %), rounding the next columns before
-// each store (+20 %), a fourth builder warp (+7 %), prefetching the basis to
-// L2 (no change).
+// What bounds it (clock stamps, n = 2 M, 64 shifts, 59 slots; 13 k clocks per
+// tile, of which HBM needs 5.6 k and the tensor core 4 to 5 k): two chains of
+// about the same length, both short of issue slots and registers rather than of
+// bandwidth.  A builder warp makes 32 digit rows per thread from values that
+// wait in registers; an epilogue warp drains, rounds and adds for 16 columns,
+// 4.6 k clocks of it the quarter's FP64 pipe.  Each of these shortened a flush
+// (n = 2 M, 64 shifts; 256^3 in brackets):
+//   eight digits instead of nine (fewer digits, MMAs, accumulators to join) and
+//     four coefficient slices in TMEM: 2.21 to 2.17 ms (alone; it frees the
+//     registers for the next two);
+//   the next tile's basis loads one item at a time, as its registers come
+//     free: -5 %;
+//   each x addition issued for two columns at once (below): -6 %;
+//   together 2.21 to 1.99 ms (17.3 to 15.6).
+// The error against quad precision is no larger (rms 5 to 9 % smaller without
+// own terms, from rounding T / 2^13 instead of flooring it).
+// Tried and not kept: basis values by bulk copies to shared memory (2.3 ms: the
+// builders' reads queue behind the MMAs' operands), a sub-tile of 16 columns with
+// barriers of its own per epilogue column group (+20 %: smaller MMAs), a fourth
+// builder warp (+7 %), prefetching the basis to L2 (no change), rounding all 16
+// columns before the first FP64 operation (+25 %).
 //
 // Only the live shifts are formed: a shift that had converged by the previous
 // flush has zero coefficients and own terms (0, 1) since that flush's reset,
 // so its rows would come out unchanged.  The rows of a group are the live
 // shifts in index order; a group without live shifts does nothing, and the
 // epilogue warps of a TMEM quadrant without live rows sit the tiles out.
-#include <cuda_bf16.h>
+#include <cuda_fp16.h>
 #include <math.h>
 #include <stdint.h>
 
@@ -66,18 +77,18 @@ constexpr int TC_M = 128;
 constexpr int TC_N = 48;
 constexpr int TC_K = 64;
 static_assert(TC_N == HBK_PANEL, "a tile is one panel of x_j and p_j");
-constexpr int NDIG = 9;
-constexpr int NDIAG = 9;
+constexpr int NDIG = 8;
+constexpr int NDIAG = 8;
 constexpr int A_SLICE = TC_M * TC_K * 2;  // 16384 B
 constexpr int B_SLICE = TC_N * TC_K * 2;  // 6144 B
-constexpr int A_BYTES = NDIG * A_SLICE;   // 147456 B (a group's coefficient digits in global memory)
-constexpr int B_BYTES = NDIG * B_SLICE;   // 55296 B (one buffer of a tile's basis digits)
-// Coefficient digit slices 0 and 1 live in TMEM (columns after the nine
-// accumulators), the other seven in shared memory: that leaves room for two
-// basis-digit buffers, so the builders write tile t+1's digits while the
-// tensor core works through tile t.
-constexpr int A_TMEM_SLICES = 2;
-constexpr int A_SMEM_BYTES = (NDIG - A_TMEM_SLICES) * A_SLICE;  // 114688 B
+constexpr int A_BYTES = NDIG * A_SLICE;   // 131072 B (a group's coefficient digits in global memory)
+constexpr int B_BYTES = NDIG * B_SLICE;   // 49152 B (one buffer of a tile's basis digits)
+// Coefficient digit slices 0 to 3 live in TMEM (columns after the eight
+// accumulators: all 512 are used), the other four in shared memory: less for the
+// MMAs to read there (2 slices in TMEM: +8 %).  Two basis-digit buffers, so the
+// builders write tile t+1's digits while the tensor core works through tile t.
+constexpr int A_TMEM_SLICES = 4;
+constexpr int A_SMEM_BYTES = (NDIG - A_TMEM_SLICES) * A_SLICE;  // 65536 B
 constexpr int A_TCOL = NDIAG * TC_N;                             // first TMEM column of slice 0 (32 per slice)
 constexpr int NBUF = 2;                                          // basis-digit buffers
 constexpr int BUILD_WARPS = 3;            // warps 0-2: basis digits
@@ -91,18 +102,12 @@ constexpr int ITEMS = (TC_K / 8) * TC_N;          // (slot octet, element) pairs
 constexpr int ITEMS_PER = ITEMS / BUILD_THREADS;  // 4
 constexpr int TMEM_COLS = 512;
 constexpr int SMEM_MISC = 6144;
-constexpr int SMEM_BYTES = A_SMEM_BYTES + NBUF * B_BYTES + SMEM_MISC;  // 231424 B
+constexpr int SMEM_BYTES = A_SMEM_BYTES + NBUF * B_BYTES + SMEM_MISC;  // 169984 B
 constexpr long long WAIT_LIMIT = 1ll << 26;  // polls of an mbarrier before giving up
 constexpr int EXP_NONE = -100000;            // exponent of an all-zero row or column
-// sum_s 64 * 2^(56 - 7 s): adding it to a 62-bit signed value makes every
-// 7-bit field of the sum the balanced digit + 64
-constexpr uint64_t DIGIT_BIAS = 0x4081020408102040ull;
-// magic FP32 1.5 * 2^23: for |D| < 2^22, bits(D + MAGIC) = MAGIC_BITS + D
-constexpr float MAGIC = 12582912.0f;
-constexpr uint32_t MAGIC_BITS = 0x4B400000u;
-constexpr uint64_t HI_BIAS = (uint64_t)MAGIC_BITS * 2113665ull;  // * (2^21 + 2^14 + 2^7 + 1)
-constexpr uint64_t MID_BIAS = (uint64_t)MAGIC_BITS * 66052ull;   // * (2^16 + 2^9 + 2^2)
-constexpr uint64_t T_BIAS = (HI_BIAS << 23) + MID_BIAS;          // (mod 2^64)
+// sum_s 128 * 2^(56 - 8 s): adding it to a 62-bit signed value makes every
+// byte of the sum the balanced digit + 128
+constexpr uint64_t DIGIT_BIAS = 0x8080808080808080ull;
 
 static_assert(ITEMS % BUILD_THREADS == 0, "builder items");
 static_assert(EPI_WARP0 % 4 == 0 && EPI_WARP0 + EPI_WARPS == TC_THREADS / 32, "epilogue warps: whole quadrant sets");
@@ -190,24 +195,25 @@ __device__ __forceinline__ uint64_t biased62(uint64_t bits, int scale) {
     return (q ^ sg) + DIGIT_BIAS + (hi >> 31);            // -q = ~q + 1
 }
 
-// balanced digit s (weight 2^(56 - 7 s)) of a biased value, as an exact float
-template <int S>
-__device__ __forceinline__ float digit(uint64_t U) {
-    const uint32_t e = S == 0 ? (uint32_t)(U >> 56) : ((uint32_t)(U >> (56 - 7 * S)) & 127u);
-    return __uint_as_float(0x4B000000u | e) - 8388672.0f;  // (2^23 + e) - (2^23 + 64)
+// v * 2^(63 - scale) truncated toward zero (|v| < 2^scale, so r >= 1 and the
+// magnitude is below 2^63): a bit more than biased62, for the coefficients,
+// whose digit 0 then reaches 128
+__device__ __forceinline__ int64_t fixed63(uint64_t bits, int scale) {
+    const int eb = (int)((bits >> 52) & 0x7ffu);
+    const uint64_t M = (bits & ((1ull << 52) - 1)) | (eb ? 1ull << 52 : 0ull);
+    const int64_t q = (int64_t)((M << 11) >> min(1023 + scale - max(eb, 1), 63));
+    return (int64_t)bits < 0 ? -q : q;
 }
 
-// the same digits of two values as a BF16 pair: digit + 64 is at most 128, and
-// BF16 0x4300 + e is 128 + e for e = 0..128 (seven fraction bits), so one packed
-// subtraction of 192 leaves the digits, exact
+// balanced digits s (weight 2^(56 - 8 s)) of two biased values as an FP16 pair:
+// FP16 0x6400 + e is 1024 + e for e = 0..255 (ten fraction bits), so one packed
+// subtraction of 1152 leaves the digits e - 128, exact
 template <int S>
 __device__ __forceinline__ uint32_t digit_pair(uint64_t U0, uint64_t U1) {
-    constexpr int sh = 56 - 7 * S;
-    constexpr uint32_t mask = S == 0 ? 0x00ff00ffu : 0x007f007fu;
-    const uint32_t x0 = (uint32_t)(U0 >> sh);
-    const uint32_t x1 = sh >= 16 ? (uint32_t)(U1 >> (sh >= 16 ? sh - 16 : 0)) : (uint32_t)U1 << (sh >= 16 ? 0 : 16 - sh);
-    const uint32_t e = (__byte_perm(x0, x1, 0x7610) & mask) | 0x43004300u;
-    const __nv_bfloat162 h = __hsub2(*reinterpret_cast<const __nv_bfloat162 *>(&e), __nv_bfloat162{192.0f, 192.0f});
+    constexpr uint32_t b = 3 - (S & 3);  // byte of the upper (S < 4) or lower word
+    const uint32_t x0 = (uint32_t)(U0 >> (S < 4 ? 32 : 0)), x1 = (uint32_t)(U1 >> (S < 4 ? 32 : 0));
+    const uint32_t e = (__byte_perm(x0, x1, b | (b << 4) | ((4 + b) << 8) | ((4 + b) << 12)) & 0x00ff00ffu) | 0x64006400u;
+    const __half2 h = __hsub2(*reinterpret_cast<const __half2 *>(&e), __half2half2(__ushort_as_half(0x6480)));
     return *reinterpret_cast<const uint32_t *>(&h);
 }
 
@@ -225,22 +231,33 @@ __device__ __forceinline__ void store_digits(unsigned char *sB, uint32_t off, co
 }
 
 // 32 x 32 + 64 -> 64-bit multiply-add
-__device__ __forceinline__ uint64_t madw(uint32_t a, uint32_t b, uint64_t c) {
-    uint64_t d;
-    asm("mad.wide.u32 %0, %1, %2, %3;" : "=l"(d) : "r"(a), "r"(b), "l"(c));
+__device__ __forceinline__ long long madw(int a, int b, long long c) {
+    long long d;
+    asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(d) : "r"(a), "r"(b), "l"(c));
     return d;
 }
 
-// floor(T / 2^12) of the exact diagonal sum T = sum_d D_d 2^(7 (8 - d)), from
-// the biased FP32 bits B_d = MAGIC_BITS + D_d.  |D_d| <= (d + 1) 64 2^12, so
-// |T| < 2^74.03 and the result fits a signed 64-bit integer; the dropped bits
-// are below 2^-56 of the row x element scale (the dropped diagonals: 2^-54).
-// Arithmetic is modulo 2^64 (the biases cancel exactly).
-__device__ __forceinline__ long long diag_sum(const uint32_t (&B)[NDIAG]) {
-    const uint64_t h = madw(B[0], 1u << 21, madw(B[1], 1u << 14, madw(B[2], 1u << 7, (uint64_t)B[3])));
-    const uint64_t mid = madw(B[4], 1u << 16, madw(B[5], 1u << 9, (uint64_t)B[6] << 2));
-    const int lo = (int)(B[7] * 128u + B[8] - MAGIC_BITS * 129u);  // D_7 2^7 + D_8, |.| < 2^29
-    return (long long)((h << 23) + mid - T_BIAS + (uint64_t)(long long)(lo >> 12));
+// T / 2^13 of the exact diagonal sum T = sum_d D_d 2^(8 (7 - d)), to within 0.54
+// units (rounded: 2048 more halves before the shift).  |D_d| <= (d + 1/2) 2^20 (|digit| <= 128 on both sides, 64 for the
+// basis' digit 0).  Up to D_3 (below 2^22) an FP32 add of 1.5 2^23 leaves the
+// integer in the sum's low bits; the larger ones take 1.5 2^24, which rounds to
+// an even integer: D_4's and D_5's odd unit goes to the next diagonal (256 units
+// there; exact), D_6's and D_7's is dropped (2^-5 of the result's unit, which is
+// 2^-56 of the row x element scale).  Conversion instructions instead: +9 %.
+// Pairs D_2i 2^8 + D_2i+1 fit 32 bits, |T| < 2^75.1 and the result 64.
+constexpr float MAGIC = 12582912.0f, MAGIC2 = 25165824.0f;  // 1.5 2^23, 1.5 2^24
+constexpr uint32_t MAGIC_BITS = 0x4B400000u, MAGIC2_BITS = 0x4BC00000u;
+__device__ __forceinline__ int pair_sum(float a, float b, uint32_t bias, uint32_t more = 0) {
+    return (int)(__float_as_uint(a) * 256u + (__float_as_uint(b) - (bias * 257u - more)));
+}
+__device__ __forceinline__ long long diag_sum(const float (&D)[NDIAG]) {
+    const int h0 = pair_sum(D[0] + MAGIC, D[1] + MAGIC, MAGIC_BITS), h1 = pair_sum(D[2] + MAGIC, D[3] + MAGIC, MAGIC_BITS);
+    const float f4 = D[4] + MAGIC2;
+    const float d5 = fmaf(D[4] - (f4 - MAGIC2), 256.0f, D[5]), f5 = d5 + MAGIC2;
+    const float f6 = fmaf(d5 - (f5 - MAGIC2), 256.0f, D[6]) + MAGIC2, f7 = D[7] + MAGIC2;
+    const int h2 = pair_sum(f4, f5, MAGIC2_BITS), h3 = pair_sum(f6, f7, MAGIC2_BITS, 2048u);  // halves
+    const long long t = madw(h1, 1 << 19, madw(h2, 1 << 4, (long long)(h3 >> 12)));
+    return t + (long long)((unsigned long long)(long long)h0 << 35);
 }
 
 // T 2^k rounded to FP64: round half up on the 64-bit magnitude, whose leading
@@ -270,8 +287,10 @@ __device__ __forceinline__ double join_t(long long T, int k) {
     const int z = __clz((int)ah);
     const int ebm1 = 1085 - z + k;
     if (ah == 0 ? (unsigned)a != 0u : (unsigned)ebm1 > 2044u) return join_rest(T, k);
-    const unsigned long long W = a << z;
-    const unsigned long long mant = (W >> 11) + (((unsigned)W >> 10) & 1u);
+    // (z < 32 where ah is not 0; the shifts of a row of zeros are not used)
+    const unsigned wl = (unsigned)a << (z & 31), wh = __funnelshift_l((unsigned)a, ah, z);
+    const unsigned long long mant =
+        (((unsigned long long)(wh >> 11) << 32) | __funnelshift_r(wl, wh, 11)) + ((wl >> 10) & 1u);
     const unsigned hi = ah ? (unsigned)(mant >> 32) + ((unsigned)ebm1 << 20) : 0u;
     return __hiloint2double((int)(hi | ((unsigned)sg & 0x80000000u)), (int)(unsigned)mant);
 }
@@ -292,7 +311,7 @@ struct TcArgs {
     unsigned n;
     int L;                // slots in use (<= 64)
     const unsigned long long *slot_max;  // bits of max |V[l]| per slot
-    const unsigned char *aimg;           // per group: 9 digit slices of the 128 x 64 coefficient block
+    const unsigned char *aimg;           // per group: 8 digit slices of the 128 x 64 coefficient block
     const int *rowexp;    // per group: [128]
     const double *rown;   // per group: [128] own-term scalar (xi for x rows, rho for p rows)
     double *X, *Pmat;     // panel-major, m systems
@@ -384,14 +403,16 @@ __global__ void __launch_bounds__(TC_K) k_flush_prep(const double *__restrict__ 
     __syncthreads();
     const unsigned long long rmax = s_max[0] > s_max[1] ? s_max[0] : s_max[1];
     const int E = rmax ? exp_of_bits(rmax) : EXP_NONE;
-    const uint64_t U = (rmax && a != 0.0) ? biased62((uint64_t)__double_as_longlong(a), E) : DIGIT_BIAS;
+    int64_t q = (rmax && a != 0.0) ? fixed63((uint64_t)__double_as_longlong(a), E) : 0;
     unsigned char *img = aimg + (size_t)g * A_BYTES;
     const uint32_t off = umma_off(r, l);
-    const float d[NDIG] = {digit<0>(U), digit<1>(U), digit<2>(U), digit<3>(U), digit<4>(U),
-                           digit<5>(U), digit<6>(U), digit<7>(U), digit<8>(U)};
 #pragma unroll
-    for (int s = 0; s < NDIG; ++s)
-        *reinterpret_cast<__nv_bfloat16 *>(img + (size_t)s * A_SLICE + off) = __float2bfloat16_rn(d[s]);
+    for (int s = NDIG - 1; s >= 0; --s) {
+        // balanced digit: the low byte in [-128, 127], its borrow to the next
+        const int d = s ? (int)(signed char)(q & 255) : (int)q;
+        q = (q >> 8) + ((q >> 7) & 1);
+        *reinterpret_cast<__half *>(img + (size_t)s * A_SLICE + off) = __int2half_rn(d);
+    }
     if (l == 0) {
         rowexp[g * TC_M + r] = E;
         rown[g * TC_M + r] = (j >= 0) ? own[2 * (size_t)j + which] : 0.0;
@@ -401,7 +422,7 @@ __global__ void __launch_bounds__(TC_K) k_flush_prep(const double *__restrict__ 
 // ---- the tensor-core flush
 __global__ void __launch_bounds__(TC_THREADS, 1) k_flush_tc(TcArgs a) {
     extern __shared__ __align__(1024) unsigned char smem[];
-    unsigned char *sA = smem;                 // coefficient digit slices 2 .. 8
+    unsigned char *sA = smem;                 // coefficient digit slices 4 .. 7
     unsigned char *sB = smem + A_SMEM_BYTES;  // NBUF basis-digit buffers, tile it in buffer it % 2
     unsigned char *misc = smem + A_SMEM_BYTES + NBUF * B_BYTES;
     // Tiles alternate between the two basis-digit buffers, and the barriers
@@ -460,7 +481,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_flush_tc(TcArgs a) {
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *s_tmem;
-    // coefficient digit slices 0 and 1 into TMEM: lane r holds row r, each
+    // coefficient digit slices 0 .. 3 into TMEM: lane r holds row r, each
     // 32-bit column two consecutive k (the lower k in the low half), slice s
     // at columns A_TCOL + 32 s ..  Warps 4-7 each write their own quadrant.
     if (warp >= EPI_WARP0 && warp < EPI_WARP0 + 4) {
@@ -522,16 +543,16 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_flush_tc(TcArgs a) {
             wmax[u] = (uint32_t)min(7, a.L - 1 - l0);  // (an octet past L: slot L - 1 again, against zero digits)
         }
         const uint32_t ld32 = (uint32_t)ld;
-        auto load_tile = [&](unsigned t) {
+        auto load_item = [&](int u, unsigned t) {
+            const double *p = vcol[u] + min(t * TC_N + ii[u], n - 1);
 #pragma unroll
-            for (int u = 0; u < ITEMS_PER; ++u) {
-                const double *p = vcol[u] + min(t * TC_N + ii[u], n - 1);
-#pragma unroll
-                for (uint32_t w = 0; w < 8; ++w) v[u][w] = w <= wmax[u] ? __ldcs(p + (uint64_t)w * ld32) : 0.0;
-            }
+            for (uint32_t w = 0; w < 8; ++w) v[u][w] = w <= wmax[u] ? __ldcs(p + (uint64_t)w * ld32) : 0.0;
         };
         int it = 0;
-        if (blockIdx.x < ntiles) load_tile(blockIdx.x);
+        if (blockIdx.x < ntiles) {
+#pragma unroll
+            for (int u = 0; u < ITEMS_PER; ++u) load_item(u, blockIdx.x);
+        }
         for (unsigned t = blockIdx.x; t < ntiles; t += gridDim.x, ++it) {
             if (*(volatile int *)s_fail) break;
             // phase A (overlaps the previous tile's MMAs): element exponents;
@@ -586,18 +607,18 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_flush_tc(TcArgs a) {
                     U[w] = biased62((uint64_t)__double_as_longlong(v[u][w]), Fv[u] + se[w]);
                 if (io[u] == 0) s_F[(it & 3) * TC_N + ii[u]] = Fv[u];
                 store_digits<0>(sBt, umma_off(ii[u], 8 * io[u]), U);
+                // the next tile's values take this item's registers
+                if (t + gridDim.x < ntiles) load_item(u, t + gridDim.x);
             }
             // digits written by threads must be visible to the tensor core (async proxy)
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             mbar_arrive(bar_full + (it & 1));
-            // the next tile's basis values are in flight during this tile's MMAs
-            if (t + gridDim.x < ntiles) load_tile(t + gridDim.x);
         }
     } else if (warp == MMA_WARP) {
         // ---- one thread loads the coefficient digits and issues every MMA
         if (lane == 0) {
             // the coefficient digits of this group: one bulk copy per slice
-            // the coefficient digit slices kept in shared memory (2 .. 8)
+            // the coefficient digit slices kept in shared memory (4 .. 7)
             asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar_a)),
                          "r"((uint32_t)A_SMEM_BYTES)
                          : "memory");
@@ -624,9 +645,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_flush_tc(TcArgs a) {
                 tc_fence_after();
                 // diagonal d accumulates in columns [48 d, 48 d + 48).  The basis
                 // digit slices lie one after another along N, so one MMA of
-                // coefficient slice s against basis rows 0 .. 48 (9 - s) - 1,
+                // coefficient slice s against basis rows 0 .. 48 (8 - s) - 1,
                 // written from column 48 s on, adds A_s B_t to diagonal s + t
-                // for every t <= 8 - s (in two MMAs where N would pass 256).
+                // for every t <= 7 - s (in two MMAs where N would pass 256).
 #pragma unroll
                 for (int kk = 0; kk < TC_K / 16; ++kk) {
 #pragma unroll
@@ -635,9 +656,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_flush_tc(TcArgs a) {
 #pragma unroll
                         for (int part = 0; part * 256 < ntot; ++part) {
                             const int nn = ntot - part * 256 < 256 ? ntot - part * 256 : 256;
-                            // kind::f16 instruction descriptor: D = F32, A = B = BF16, both
+                            // kind::f16 instruction descriptor: D = F32, A = B = F16 (0), both
                             // K-major, N >> 3 at bits 17-22, M >> 4 at bits 24-28
-                            const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(nn >> 3) << 17) |
+                            const uint32_t idesc = (1u << 4) | ((uint32_t)(nn >> 3) << 17) |
                                                    ((uint32_t)(TC_M >> 4) << 24);
                             // start-address field: (offset >> 4) adds without carry (smem < 256 KB)
                             const uint64_t bd = bd0 + (uint64_t)((part * 256 / 8 * 1024 + kk * 256) >> 4);
@@ -686,24 +707,40 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_flush_tc(TcArgs a) {
         const int E = s_rowexp[r];
         const double own = s_rown[r];
         const uint32_t tbase = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(cg * EPI_COLS);
-        // this lane's piece of a panel (system j, columns 16 cg .. 16 cg + 15):
-        // x rows in X, p rows in Pmat; consecutive panels m * 48 values apart
-        double *const pbase =
-            live && (which == 0 || a.Pmat) ? (which ? a.Pmat : a.X) + (size_t)j * TC_N + cg * EPI_COLS : nullptr;
+        // A lane pair (u, u + 16) works on one system's piece of a panel
+        // (columns 16 cg .. 16 cg + 15): p row and x row, four 32-byte sectors
+        // each, consecutive panels m * 48 values apart.  Both lanes need the
+        // old p (one load serves both); the additions to x are shared out, the
+        // x lane takes sectors 0 and 2, the p lane 1 and 3, so that an FP64 add
+        // is issued for two columns at a time.
+        const size_t piece = (size_t)j * TC_N + cg * EPI_COLS;
+        const double *const pp = live && a.Pmat ? a.Pmat + piece : nullptr;
+        double *const xp = live ? a.X + piece + 4 * which : nullptr;
         const size_t pstride = (size_t)a.m * TC_N;
         // x and p values of a tile, loaded one tile ahead: the loads are in
         // flight while the warp waits for that tile's MMAs and drains them.
-        // 32-byte sector accesses (pieces are 16 values from a 32-byte aligned base)
-        double pv[EPI_COLS];
+        double pv[EPI_COLS], xv[EPI_COLS / 2];
         auto load_pv = [&](unsigned t) {
             const unsigned c0 = t * TC_N + cg * EPI_COLS;
-            const double *src = pbase ? pbase + (size_t)t * pstride : nullptr;
-            if (src && c0 + EPI_COLS <= n) {
+            const double *ps = pp ? pp + (size_t)t * pstride : nullptr;
+            const double *xs = xp ? xp + (size_t)t * pstride : nullptr;
+            const bool full = c0 + EPI_COLS <= n;
+            if (ps && full) {
 #pragma unroll
-                for (int u = 0; u < EPI_COLS; u += 4) ld_sector(src + u, pv[u], pv[u + 1], pv[u + 2], pv[u + 3]);
+                for (int u = 0; u < EPI_COLS; u += 4) ld_sector(ps + u, pv[u], pv[u + 1], pv[u + 2], pv[u + 3]);
             } else {
 #pragma unroll
-                for (int u = 0; u < EPI_COLS; ++u) pv[u] = (src && c0 + u < n) ? src[u] : 0.0;
+                for (int u = 0; u < EPI_COLS; ++u) pv[u] = (ps && c0 + u < n) ? ps[u] : 0.0;
+            }
+            if (xs && full) {
+#pragma unroll
+                for (int u = 0; u < EPI_COLS / 2; u += 4) ld_sector(xs + 2 * u, xv[u], xv[u + 1], xv[u + 2], xv[u + 3]);
+            } else {
+#pragma unroll
+                for (int u = 0; u < EPI_COLS / 2; ++u) {
+                    const int col = 2 * (u & 4) + (u & 3);
+                    xv[u] = (xs && c0 + 4 * which + col < n) ? xs[col] : 0.0;
+                }
             }
         };
         if (blockIdx.x < ntiles) load_pv(blockIdx.x);
@@ -718,23 +755,23 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_flush_tc(TcArgs a) {
                 break;
             }
             tc_fence_after();
-            // exact diagonal sums -> floor(T / 2^12)
+            // exact diagonal sums -> T / 2^13
             long long T[EPI_COLS];
 #pragma unroll
-            for (int c4 = 0; c4 < EPI_COLS / 4; ++c4) {
-                uint32_t dv[NDIAG][4];
+            for (int c2 = 0; c2 < EPI_COLS; c2 += 2) {
+                float dv[NDIAG][2];
 #pragma unroll
                 for (int d = 0; d < NDIAG; ++d)
-                    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
-                                 : "=r"(dv[d][0]), "=r"(dv[d][1]), "=r"(dv[d][2]), "=r"(dv[d][3])
-                                 : "r"(tbase + (uint32_t)(d * TC_N + 4 * c4)));
+                    asm volatile("tcgen05.ld.sync.aligned.32x32b.x2.b32 {%0,%1}, [%2];"
+                                 : "=f"(dv[d][0]), "=f"(dv[d][1])
+                                 : "r"(tbase + (uint32_t)(d * TC_N + c2)));
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    uint32_t B[NDIAG];
+                for (int u = 0; u < 2; ++u) {
+                    float D[NDIAG];
 #pragma unroll
-                    for (int d = 0; d < NDIAG; ++d) B[d] = __float_as_uint(__uint_as_float(dv[d][u]) + MAGIC);
-                    T[4 * c4 + u] = diag_sum(B);
+                    for (int d = 0; d < NDIAG; ++d) D[d] = dv[d][u];
+                    T[c2 + u] = diag_sum(D);
                 }
             }
             tc_fence_before();
@@ -744,29 +781,33 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_flush_tc(TcArgs a) {
             const unsigned c0 = t * TC_N + cg * EPI_COLS;
             const bool full = c0 + EPI_COLS <= n;
             const int *Fc = s_F + (it & 3) * TC_N + cg * EPI_COLS;
-            double *dst = store && pbase ? pbase + (size_t)t * pstride : nullptr;
-            // one pass per four columns: round, own-vector terms (x lanes take
-            // the old Pmat from their p lane), store
+            double *const pd = store && which && a.Pmat ? a.Pmat + piece + (size_t)t * pstride : nullptr;
+            double *const xd = xp ? xp + (size_t)t * pstride : nullptr;
+            // one pass per two sectors: round, own-vector terms, store
 #pragma unroll
-            for (int u = 0; u < EPI_COLS; u += 4) {
-                double o4[4];
+            for (int u = 0; u < EPI_COLS; u += 8) {
+                double y[8], xn[4];
+#pragma unroll
+                for (int h = 0; h < 8; ++h)  // (a row of zero coefficients has T = 0)
+                    y[h] = fma(own, pv[u + h], join_t(T[u + h], E + Fc[u + h] - 56));
 #pragma unroll
                 for (int h = 0; h < 4; ++h) {
-                    // (a row of zero coefficients has T = 0)
-                    const double G = join_t(T[u + h], E + Fc[u + h] - 56);
-                    const double po = __shfl_xor_sync(0xffffffffu, pv[u + h], 16);
-                    const double pold = which ? pv[u + h] : po;  // (0 without a Pmat: pv is then)
-                    const double y = fma(own, pold, G);
-                    o4[h] = which ? y : pv[u + h] + y;
+                    const double z = __shfl_xor_sync(0xffffffffu, y[4 + h], 16);
+                    xn[h] = xv[u / 2 + h] + (which ? z : y[h]);
                 }
-                if (dst) {
-                    if (full)
-                        st_sector(dst + u, o4[0], o4[1], o4[2], o4[3]);
-                    else {
-#pragma unroll
-                        for (int h = 0; h < 4; ++h)
-                            if (c0 + u + h < n) dst[u + h] = o4[h];
+                if (full) {
+                    if (pd) {
+                        st_sector(pd + u, y[0], y[1], y[2], y[3]);
+                        st_sector(pd + u + 4, y[4], y[5], y[6], y[7]);
                     }
+                    if (xd) st_sector(xd + u, xn[0], xn[1], xn[2], xn[3]);
+                } else {
+#pragma unroll
+                    for (int h = 0; h < 8; ++h)
+                        if (pd && c0 + u + h < n) pd[u + h] = y[h];
+#pragma unroll
+                    for (int h = 0; h < 4; ++h)
+                        if (xd && c0 + u + 4 * which + h < n) xd[u + h] = xn[h];
                 }
             }
             if (t + gridDim.x < ntiles) load_pv(t + gridDim.x);
