@@ -66,6 +66,8 @@ void hbicg__ctx_release(hbicg_context *c);
  * lower list); hwbeg[hnw + 1] list starts, hitem[ni] the lists in order of
  * dealing.  HBICG_OK or HBICG_E_NOMEM. */
 int hbicg__hyb_plan(size_t ni, const unsigned *cost, unsigned hnw, unsigned *hwbeg, unsigned *hitem);
+int hbicg__hyb_plan_after(size_t ni, const unsigned *cost, const unsigned *base, unsigned hnw, unsigned *hwbeg,
+                          unsigned *hitem);
 
 /* positions of A's SELL-32 diagonal entries (computed once per layout) */
 int hbicg__sell_diag(hbicg_matrix *A);

@@ -33,7 +33,23 @@ static int slot_less(const hyb_slot *a, const hyb_slot *b) {
     return a->load < b->load || (a->load == b->load && a->w < b->w);
 }
 
-int hbicg__hyb_plan(size_t ni, const unsigned *cost, unsigned hnw, unsigned *hwbeg, unsigned *hitem) {
+static void slot_sift(hyb_slot *h, unsigned n, size_t p) {
+    for (;;) {
+        const size_t l = 2 * p + 1, r = l + 1;
+        size_t m = p;
+        if (l < n && slot_less(&h[l], &h[m])) m = l;
+        if (r < n && slot_less(&h[r], &h[m])) m = r;
+        if (m == p) return;
+        const hyb_slot t = h[p];
+        h[p] = h[m];
+        h[m] = t;
+        p = m;
+    }
+}
+
+/* base[w]: what list w's warp does before the list, in the items' unit of cost (NULL: nothing) */
+int hbicg__hyb_plan_after(size_t ni, const unsigned *cost, const unsigned *base, unsigned hnw, unsigned *hwbeg,
+                          unsigned *hitem) {
     unsigned long long *key = malloc(sizeof *key * (ni + 1));
     hyb_slot *h = malloc(sizeof *h * hnw);
     unsigned *owner = malloc(sizeof *owner * (ni + 1));
@@ -47,24 +63,15 @@ int hbicg__hyb_plan(size_t ni, const unsigned *cost, unsigned hnw, unsigned *hwb
     }
     for (size_t i = 0; i < ni; ++i) key[i] = ((0xFFFFFFFFull - cost[i]) << 32) | i; /* costliest first, then by item */
     qsort(key, ni, sizeof *key, cmp_u64);
-    for (unsigned w = 0; w < hnw; ++w) h[w] = (hyb_slot){0, w}; /* all zero: a valid heap */
+    for (unsigned w = 0; w < hnw; ++w) h[w] = (hyb_slot){base ? base[w] : 0u, w}; /* all zero: a valid heap */
+    for (unsigned p = base ? hnw / 2 : 0; p-- > 0;) slot_sift(h, hnw, p);
     memset(hwbeg, 0, sizeof *hwbeg * ((size_t)hnw + 1));
     for (size_t k = 0; k < ni; ++k) {
         const unsigned i = (unsigned)(key[k] & 0xFFFFFFFFu);
         owner[i] = h[0].w;
         hwbeg[h[0].w + 1]++;
         h[0].load += 0xFFFFFFFFull - (key[k] >> 32);
-        for (size_t p = 0;;) { /* sift the grown root down */
-            const size_t l = 2 * p + 1, r = l + 1;
-            size_t m = p;
-            if (l < hnw && slot_less(&h[l], &h[m])) m = l;
-            if (r < hnw && slot_less(&h[r], &h[m])) m = r;
-            if (m == p) break;
-            const hyb_slot t = h[p];
-            h[p] = h[m];
-            h[m] = t;
-            p = m;
-        }
+        slot_sift(h, hnw, 0);
     }
     for (unsigned w = 0; w < hnw; ++w) hwbeg[w + 1] += hwbeg[w];
     /* fill each list in the order of dealing */
@@ -80,6 +87,10 @@ int hbicg__hyb_plan(size_t ni, const unsigned *cost, unsigned hnw, unsigned *hwb
     return HBICG_OK;
 }
 
+int hbicg__hyb_plan(size_t ni, const unsigned *cost, unsigned hnw, unsigned *hwbeg, unsigned *hitem) {
+    return hbicg__hyb_plan_after(ni, cost, NULL, hnw, hwbeg, hitem);
+}
+
 /* HYB: rows of at most HBK_HYB_SHORT entries in SELL-32 slices, sorted by
  * length (longest first, stable) inside windows of HBK_HYB_WINDOW consecutive
  * rows, so that the 32 rows of a slice have similar lengths and the rows a
@@ -92,10 +103,14 @@ int hbicg__hyb_plan(size_t ni, const unsigned *cost, unsigned hnw, unsigned *hwb
  * allocation holds each long row's entry range, the long rows, and the warp
  * work lists (hbicg__hyb_plan) for one wave of the kernels that take this form. */
 /* grid of the HYB kernels: one wave of the heaviest, so every warp of a
- * launch runs exactly one list; fewer where rows (with block rows: where
- * nonzeros, 4 per thread) leave blocks without work */
+ * launch runs exactly one list; fewer where rows leave blocks
+ * without work.  With block rows: 12 nonzeros per thread, as each block ends in
+ * the solver's dot products (FP64 adds in every warp) and those matrices fit
+ * half a wave (an iteration with 16 shifts at 4 / 8 / 12 / 16 per thread:
+ * 20 k rows 35.1 / 34.0 / 33.3 / 35.8 us, 40 k 44.0 / 40.9 / 40.6 / 40.3,
+ * 60 k 51.8 / 50.9 / 46.1 / 47.4, 80 k 55.6 / 55.6 / 53.7 / 54.7) */
 static int hyb_grid_for(const unsigned *h_ptr, unsigned n, int wide) {
-    const unsigned by_rows = (n + HBK_THREADS - 1) / HBK_THREADS, by_nnz = h_ptr[n] / (4u * HBK_THREADS) + 1u;
+    const unsigned by_rows = (n + HBK_THREADS - 1) / HBK_THREADS, by_nnz = h_ptr[n] / (12u * HBK_THREADS) + 1u;
     int g = hbk_spmv_grid(wide && by_nnz > by_rows ? by_nnz : by_rows);
     const int wf = hbk_hyb_wave_fused(wide), wb = hbk_hyb_wave_blas(wide);
     if (wf < g) g = wf;
@@ -137,8 +152,8 @@ static int build_hyb(hbicg_matrix *A, const unsigned *h_ptr, unsigned n) {
      * list's (a slice costs about a step per entry of its rows, a long row one
      * per 32 entries): if so, the rows above HBK_HYB_L16 take a block each
      * (spmv_rows_hyb).  Measured, one product of power-law rows, warps only
-     * against block rows: n = 20 k 32.8 / 12.3 us, 60 k 36.9 / 14.4, 300 k
-     * 51.2 / 30.4, 600 k (longest row 1.4 mean lists) 85.7 / 62.5, 1 M (0.8)
+     * against block rows: n = 20 k 32.8 / 10.3 us, 60 k 36.9 / 12.3, 300 k
+     * 51.2 / 30.0, 600 k (longest row 1.4 mean lists) 85.7 / 62.1, 1 M (0.8)
      * 91.8 / 94.5, 2 M (0.4) 152.9 / 175.9. */
     const double mean = ((double)h_ptr[n] / 32.0 + 6.0 * (double)ns + 7.0 * (double)nw) /
                         ((double)hgrid * (HBK_THREADS / 32));
@@ -221,7 +236,22 @@ static int build_hyb(hbicg_matrix *A, const unsigned *h_ptr, unsigned n) {
             }
             cost[k] = 2u + (wrng[2 * first + 1] - wrng[2 * first] + g * batch - 1) / (g * batch) + tree;
         }
-        rc = hbicg__hyb_plan(ni, cost, hnw, wrow + nw, wrow + nw + hnw + 1);
+        /* a block row keeps its block's warps: about 3 steps and one per
+         * batch (1024 entries), as much list less for them.  Without that the
+         * blocks with the longest rows end last (60 k rows, one product:
+         * 14.4 to 12.3 us; 16 shifts, an iteration: 55.0 to 51.8) */
+        unsigned *base = nwide ? calloc(hnw, sizeof *base) : NULL;
+        if (nwide && !base) {
+            rc = HBICG_E_NOMEM;
+            goto done;
+        }
+        for (size_t i = 0; i < nwide; ++i) {
+            const unsigned w0 = (unsigned)(i % (unsigned)hgrid) * (HBK_THREADS / 32);
+            const unsigned len = wrng[2 * i + 1] - wrng[2 * i];
+            for (unsigned w = 0; w < HBK_THREADS / 32; ++w) base[w0 + w] += 3u + (len + 4 * HBK_THREADS - 1) / (4 * HBK_THREADS);
+        }
+        rc = hbicg__hyb_plan_after(ni, cost, base, hnw, wrow + nw, wrow + nw + hnw + 1);
+        free(base);
         if (rc) goto done;
     }
 #define HTRY(call)                                                                               \
