@@ -621,7 +621,9 @@ def run_batch_c4(args, dist: Dist):
     iters = int(sum(r.k for r in res))
     work = lambda f, k: (f.a.nnz + 6.0 * len(f.sigma) * f.a.n) * max(k - 1, 1)
     # the families of the shared persistent launch (incremental shift mode)
-    in_group = lambda f: (not args.no_persistent and (args.persistent_all or (args.shift_mode == "auto"
+    # below 8 workers (with more, these families are too large for it)
+    in_group = lambda f: (not args.no_persistent and (args.persistent_all or (args.workers < 8
+                                                                              and args.shift_mode == "auto"
                                                                               and f.a.n * len(f.sigma) < (1 << 21))))
     line = {"metric": "C4: time to solve 256 uneven shifted families (host arrays in/out), tol 1e-10",
             "value": value, "unit": "s", "n_gpus": 1, "steps": args.steps, "warmup": args.warmup,
@@ -949,7 +951,7 @@ def run_group_kernel(args):
     launch's device time (CUDA events around it) and the whole call's."""
     pkg = graft.load_package()
     fams = [f for f in pkg.workloads.batched_families(256) if f.a.n * len(f.sigma) < (1 << 21)][:args.families]
-    kw = dict(tol=1e-10, max_iter=10000, true_residuals=True, persistent=True, persistent_ctas=args.persistent_ctas)
+    kw = dict(tol=1e-10, max_iter=10000, true_residuals=True, persistent="all", persistent_ctas=args.persistent_ctas)
     for _ in range(args.warmup):
         pkg.batch_solve(fams, workers=args.workers, **kw)
     launch, wall, res = [], [], None

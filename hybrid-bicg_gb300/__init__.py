@@ -372,7 +372,8 @@ def batch_solve(families, workers: int = 8, autotune: bool = False, autotune_cac
     """hbicg_batch_solve_opts over workloads.Family-like objects (a, b,
     sigma, seed): every family solved with the same parameters (kw as
     params()); persistent: the incremental-mode families share one persistent
-    launch ("all": every family, both shift modes; False: none;
+    launch where there are fewer than 8 workers or none of them has more than
+    8192 rows ("all": every family, both shift modes, always; False: none;
     persistent_ctas caps its CTAs, 0 = one wave).
     Returns ([FamilyResult], wall seconds)."""
     p = params(**kw)

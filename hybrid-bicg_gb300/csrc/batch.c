@@ -12,12 +12,13 @@
  * (hbicg_solver_run), with the optional SpMV-form autotuner in front.
  *
  * Small families (incremental shift mode: n m < 2^21 with the automatic mode)
- * are latency-bound when each runs its own short kernels: they instead go to
- * a few host threads that set all of them up and run all their iterations in
- * ONE persistent cooperative launch (hbicg__group_*, hbk_group_run), while
- * the workers take the larger families.  With opts.persistent = 2 every
- * family goes to the shared launch (those in the deferred shift mode pause
- * there at each full basis; the host flushes them between rounds).
+ * can instead go to a few host threads that set all of them up and run all
+ * their iterations in ONE persistent cooperative launch (hbicg__group_*,
+ * hbk_group_run), while the workers take the others: where there are few
+ * workers, or only families of at most GROUP_MOST_ROWS rows.  With
+ * opts.persistent = 2 every family goes to the shared launch (those in the
+ * deferred shift mode pause there at each full basis; the host flushes them
+ * between rounds).
  * Failures are per family (status), never global. */
 #define _GNU_SOURCE
 #include <pthread.h>
@@ -238,6 +239,25 @@ int hbicg_batch_solve(hbicg_family *fams, int count, const hbicg_params *p, int 
     return hbicg_batch_solve_opts(fams, count, p, &o, wall_ms);
 }
 
+/* Shared launch or workers (persistent = 1)?  Eight or more workers overlap the
+ * kernels of as many families, without the shared launch's grid barriers and
+ * with each family's blocks as its own kernels want them; fewer leave the GPU
+ * idle.  Measured (ms; shared launch / 8 workers / 4 / 1): 16 families of 4 k to
+ * 80 k rows 31.3 / 22.7 / 26.7 / 68.7, 48 of them 80.2 / 70.0 / 86.8 / 219, 100 of
+ * 10 k 76.8 / 74.5 / 93.0 / 347, 30 of 9 k to 100 k 75.1 / 61.1 / 69.8 / 160.  A batch
+ * of small families only is left to the shared launch that persistent = 1
+ * names, with its own error (a barrier wait that ran out) and fewest host
+ * threads, although workers are faster there too (2 k to 4 k rows, 3 families
+ * 6.0 / 3.7, 64 families 37.0 / 32.2). */
+#define GROUP_MOST_ROWS 8192
+#define SHARE_BELOW_WORKERS 8
+
+/* whether a family can be solved in the shared launch */
+static int may_join(const hbicg_batch_opts *opts, const hbicg_params *p, const hbicg_family *f) {
+    return opts->persistent && p->form == HBICG_FORM_FUSED && !f->autotune && !f->r && f->m > 0 &&
+           (opts->persistent >= 2 || hbicg__shift_mode_for(p, f->n, f->m) == HBICG_SHIFTS_INCREMENTAL);
+}
+
 int hbicg_batch_solve_opts(hbicg_family *fams, int count, const hbicg_params *p, const hbicg_batch_opts *opts,
                            double *wall_ms) {
     if (count < 0 || (count && !fams) || !opts) return HBICG_E_ARG;
@@ -268,12 +288,14 @@ int hbicg_batch_solve_opts(hbicg_family *fams, int count, const hbicg_params *p,
     qsort(order, (size_t)count, sizeof(int), by_cost_desc);
     pthread_mutex_unlock(&sort_lock);
     /* the families of the persistent launch leave the workers' queue */
+    if (workers < 1) workers = 8;
     int ng = 0, nw = 0;
+    unsigned most = 0; /* rows of the largest family that could join */
+    for (int i = 0; i < count; i++)
+        if (may_join(opts, p, &fams[i]) && fams[i].n > most) most = fams[i].n;
+    const int share = opts->persistent >= 2 || workers < SHARE_BELOW_WORKERS || most <= GROUP_MOST_ROWS;
     for (int i = 0; i < count; i++) {
-        const hbicg_family *f = &fams[order[i]];
-        const int small = opts->persistent && p->form == HBICG_FORM_FUSED && !f->autotune && !f->r && f->m > 0 &&
-                          (opts->persistent >= 2 ||
-                           hbicg__shift_mode_for(p, f->n, f->m) == HBICG_SHIFTS_INCREMENTAL);
+        const int small = share && may_join(opts, p, &fams[order[i]]);
         if (small) grp[ng++] = order[i];
         else order[nw++] = order[i];
     }
@@ -327,7 +349,6 @@ int hbicg_batch_solve_opts(hbicg_family *fams, int count, const hbicg_params *p,
             }
         }
     }
-    if (workers < 1) workers = 8;
     if (workers > count) workers = count > 0 ? count : 1;
     if (workers > 64) workers = 64;
     batch_t b = {fams, order, count, p, autotune_cache, 0, msgs};

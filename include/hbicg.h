@@ -244,10 +244,12 @@ typedef struct {
 int hbicg_batch_solve(hbicg_family *fams, int count, const hbicg_params *p, int workers, const char *autotune_cache,
                       double *wall_ms);
 /* The same with every option.  persistent = 1 (the default of
- * hbicg_batch_solve too): the families that take the incremental shift mode
+ * hbicg_batch_solve too): with fewer than 8 workers, or where none of them has
+ * more than 8192 rows, the families that take the incremental shift mode
  * (n m < 2^21 with shift_mode AUTO; no autotune, no residual output) run all
  * their iterations in one persistent launch on the GPU, set up and finished
- * by a few host threads, while the workers take the other families.
+ * by a few host threads, while the workers take the other families;
+ * otherwise (where that is faster) every family goes to the workers.
  * persistent = 2: every such family whatever its shift mode (deferred-mode
  * families pause in the launch at each full basis and are flushed between
  * rounds of it); 0: every family on the workers. */
