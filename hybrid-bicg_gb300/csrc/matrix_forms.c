@@ -108,10 +108,14 @@ int hbicg__hyb_plan(size_t ni, const unsigned *cost, unsigned hnw, unsigned *hwb
  * the solver's dot products (FP64 adds in every warp) and those matrices fit
  * half a wave (an iteration with 16 shifts at 4 / 8 / 12 / 16 per thread:
  * 20 k rows 35.1 / 34.0 / 33.3 / 35.8 us, 40 k 44.0 / 40.9 / 40.6 / 40.3,
- * 60 k 51.8 / 50.9 / 46.1 / 47.4, 80 k 55.6 / 55.6 / 53.7 / 54.7) */
+ * 60 k 51.8 / 50.9 / 46.1 / 47.4, 80 k 55.6 / 55.6 / 53.7 / 54.7), rounded to the
+ * same number on every SM (at 12: 60 k 46.9 to 45.7, 80 k 53.7 to 53.1) */
 static int hyb_grid_for(const unsigned *h_ptr, unsigned n, int wide) {
     const unsigned by_rows = (n + HBK_THREADS - 1) / HBK_THREADS, by_nnz = h_ptr[n] / (12u * HBK_THREADS) + 1u;
-    int g = hbk_spmv_grid(wide && by_nnz > by_rows ? by_nnz : by_rows);
+    unsigned want = wide && by_nnz > by_rows ? by_nnz : by_rows;
+    const unsigned sms = (unsigned)hbk_device_sm_count();
+    if (wide && sms && want > sms) want = (want + sms / 2) / sms * sms;
+    int g = hbk_spmv_grid(want);
     const int wf = hbk_hyb_wave_fused(wide), wb = hbk_hyb_wave_blas(wide);
     if (wf < g) g = wf;
     if (wb < g) g = wb;
