@@ -203,15 +203,15 @@ def flush_roofline(bytes_per_launch: float, ms_per_launch: float, n: int, m: int
     over its device time per launch (CUDA events around every flush of the
     timed solves, the small live-list, slot-maximum and coefficient-digit
     kernels included).  The tensor-core
-    work behind it is reported beside: 45 digit-pair products over K = 64 per
+    work behind it is reported beside: 36 digit-pair products over K = 64 per
     48-element tile and group of 64 shifts, M = 128."""
     achieved = bytes_per_launch / (ms_per_launch * 1e-3) / 1e9
     tiles = -(-n // 48) * -(-m // 64)
-    tflop = tiles * 2.0 * 128 * 48 * 45 * 64 / 1e12
+    tflop = tiles * 2.0 * 128 * 48 * 36 * 64 / 1e12
     ratio = FLUSH_TRAFFIC_PER_ALGORITHMIC_BYTE
     return {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm,
             "traffic": bytes_per_launch * ratio if ratio else None,
-            "kernel": "k_flush_tc (basis -> x_j, p_j on tcgen05 BF16 digit products)",
+            "kernel": "k_flush_tc (basis -> x_j, p_j on tcgen05 FP16 digit products)",
             "bytes_per_launch": bytes_per_launch, "ms_per_launch": ms_per_launch, "peak_kind": peak_kind,
             "tensor_tflops": tflop / (ms_per_launch * 1e-3), "tensor_peak_tflops": peaks_bf16()}
 

@@ -4,8 +4,8 @@
  * The reference solves one family per program run and sweeps seeds or
  * matrices with hard-coded loops in its drivers (src/main_seed_diff.c:113-155,
  * src/main_repeat.c).  A family of n = 10^4..5*10^5 unknowns fills only a part
- * of GB300 (one SpMV is a few hundred blocks, one iteration is eight short
- * kernels and a few scalar steps), so here a pool of host workers, each with
+ * of GB300 (one SpMV is a few hundred blocks, one iteration is five short
+ * kernels), so here a pool of host workers, each with
  * its own context and CUDA stream, takes families from a shared queue (largest
  * nnz * m first) and runs them concurrently: the GPU interleaves the kernels of
  * several families.  Each family is a complete reference-semantics solve

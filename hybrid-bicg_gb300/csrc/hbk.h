@@ -41,7 +41,7 @@ extern "C" {
 #define HBK_FMT_TILE 0       /* CSR, row blocks staged in shared memory */
 #define HBK_FMT_SELL 1       /* SELL-32: slices of 32 rows, column-major within a slice */
 #define HBK_SELL_MAX_LEN 64  /* longest row the SELL format takes */
-#define HBK_FMT_HYB 2        /* short rows in SELL-32 slices (length-sorted inside windows), long rows one warp each */
+#define HBK_FMT_HYB 2        /* short rows in SELL-32 slices (length-sorted inside windows), long rows in lane groups or blocks */
 #define HBK_HYB_SHORT 32     /* longest row of a HYB slice */
 #define HBK_HYB_WINDOW 1024  /* rows are sorted by length only inside windows of this many consecutive rows */
 #define HBK_HYB_L4 128       /* long rows up to this length: 4 lanes each, 8 rows per warp */
@@ -69,7 +69,7 @@ typedef struct {
     const unsigned *srow;      /* HYB: row of slice s, lane l at 32 s + l (>= n: an empty lane) */
     const unsigned char *slen; /* HYB: length of that row (0: an empty lane) */
     unsigned nslice;           /* HYB: slices of short rows */
-    const unsigned *wrow;      /* HYB: rows longer than HBK_HYB_SHORT, longest first, one warp each */
+    const unsigned *wrow;      /* HYB: rows longer than HBK_HYB_SHORT, longest first */
     unsigned nwrow;
     const unsigned *wrng;      /* HYB: first and end entry of long row i at 2 i, 2 i + 1 */
     const unsigned *hwbeg;     /* HYB: work list of warp w = items hitem[hwbeg[w] .. hwbeg[w + 1]) */

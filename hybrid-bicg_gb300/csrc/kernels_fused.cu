@@ -1,8 +1,7 @@
 // Fused shifted BiCGStab iteration with on-device scalars and seed switching.
 //
-// One iteration is five launches, each reading the
-// device-resident scalars, so an iteration (or a CUDA graph of many) needs no
-// host round trip:
+// One iteration is five launches, each reading the device-resident scalars, so
+// an iteration (or a CUDA graph of many) needs no host round trip:
 //   K1 seed_s     s = (A + sigma_s I) p_s, (r^,s) fused
 //   K2 seed_q     alpha; q = r_{k-1} - alpha s
 //   K3 seed_y     y = (A + sigma_s I) q, (q,q), (q,y) fused
@@ -20,7 +19,6 @@
 #include <vector>
 
 #include "hbk_device.cuh"
-
 
 using namespace hbk;
 
@@ -87,7 +85,8 @@ __device__ __forceinline__ hbk_cur load_cur(const hbk_scalars *sc) {
 // and advances the iteration.  Measured, whole solves, with the slice pipeline
 // of SellRows and early launches: n = 512, 6 shifts 1788 -> 974 us; 32^3, 16
 // shifts 5.61 -> 3.22 ms; 97 k rows, 24 shifts 26.4 -> 18.2 ms; 128^3, 32
-// shifts 72.9 -> 61.1 ms; 256^3, 64 shifts 805 -> 711 ms.
+// shifts 72.9 -> 61.1 ms; 256^3, 64 shifts 805 -> 711 ms (with the changes made
+// elsewhere since: 0.82, 2.9, 16.0, 55.5 and 655 ms).
 
 // The vector kernels (K2, K4, K5) run one block per SM, of as many threads as
 // that takes (blockDim.x, 128..1024): the sums at a block's start then cost an
@@ -1361,10 +1360,10 @@ __global__ void __launch_bounds__(NT) k_panel_to_rows(const double *__restrict__
 // CTAs of one cooperative launch take the virtual blocks of all families in
 // turn (virtual block v goes to CTA v mod grid, so a family's rows stay on
 // the same CTAs from step to step) and run, for every family at once, the
-// same steps as the one-family kernels (K1..K5, and K6, K7 for the families
-// in the deferred mode, with a virtual block in place of the launch's block:
-// same partial sums and, per family, one more entry for the extra block of K4
-// and K5).  A grid-wide barrier separates the steps.  Families stop one by one
+// same steps as the one-family kernels (K1..K5, and the forming of a new
+// seed's p in the deferred mode, with a virtual block in place of the launch's
+// block: same partial sums and, per family, one more entry for the extra block
+// of K4 and K5).  A grid-wide barrier separates the steps.  Families stop one by one
 // (converged, max_iter, breakdown) or pause with a full basis; their virtual
 // blocks then return at once, and the launch ends when every family has
 // stopped or paused (the host flushes the paused ones and launches again).

@@ -95,8 +95,8 @@ int hbicg__hyb_plan(size_t ni, const unsigned *cost, unsigned hnw, unsigned *hwb
  * length (longest first, stable) inside windows of HBK_HYB_WINDOW consecutive
  * rows, so that the 32 rows of a slice have similar lengths and the rows a
  * warp writes stay inside one window; each window's list is padded to whole
- * slices with empty lanes.  Longer rows go to a list, longest first, one warp
- * each.  For power-law row lengths (most rows short, a few thousands long),
+ * slices with empty lanes.  Longer rows go to a list, longest first, for
+ * lane groups or, the longest, blocks (spmv_rows_hyb).  For power-law row lengths (most rows short, a few thousands long),
  * where a thread per row leaves most lanes of a warp idle.  The lengths of the
  * slice rows are kept as bytes after the lane -> row map, so that a warp reads
  * its 32 lengths in one line instead of 64 scattered row pointers.  One

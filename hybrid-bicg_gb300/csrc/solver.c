@@ -906,11 +906,11 @@ static int fused_tail(hbicg_solver *s, int k_flushed, int *launches) {
  * of the shared-launch kernel (hbk_group_run) with this one family, in
  * rounds of one basis block in the deferred mode; its rows are cut into
  * virtual blocks so that about two per SM exist (256..1024 rows each).
- * Measured on GB300 it does not beat the graphs of the default: 5.3 against
- * 5.0 ms on the 32^3 family, 10.3 against 8.4 ms at 48^3, 15.9 against
- * 15.2 ms at 64^3 (deferred): a step's own latency, not the kernel boundary,
- * sets an iteration's length at these sizes, and a grid barrier costs about
- * what a boundary inside a graph does. */
+ * Measured on GB300 it does not beat the graphs of the default: 3.46 against
+ * 2.43 ms on the 32^3 family, 7.22 against 5.78 ms at 48^3, 10.3 against
+ * 9.0 ms at 64^3 (deferred): a step's own latency, not the kernel boundary,
+ * sets an iteration's length at these sizes, and a grid barrier costs more than
+ * a boundary inside a graph does. */
 static int run_persistent(hbicg_solver *s, int *launches, int *flushes, double *flush_ms) {
     cudaStream_t st = s->ctx->stream;
     hbk_scalars *h = s->ctx->h_sc;

@@ -74,7 +74,7 @@ typedef struct {
 typedef enum {
     HBICG_FLUSH_AUTO = 0,   /* tensor cores when the basis block fits one K = 64 operand */
     HBICG_FLUSH_FP64 = 1,   /* FP64 CUDA-core kernel */
-    HBICG_FLUSH_TENSOR = 2  /* tensor cores (BF16 digit products, FP64-accurate) */
+    HBICG_FLUSH_TENSOR = 2  /* tensor cores (FP16 digit products, FP64-accurate) */
 } hbicg_flush_mode;
 
 typedef struct {
@@ -134,8 +134,9 @@ int hbicg_matrix_time_spmv(hbicg_matrix *A, const double *x, double *y, double s
 /* SpMV form of a matrix: CSR row blocks staged in shared memory (TILE);
  * SELL-32, slices of 32 consecutive rows padded to their longest row (rows of
  * at most 64 entries, padding under a third of the nonzeros); HYB, rows of
- * at most 32 entries in SELL-32 slices sorted by length inside windows of 256
- * rows and longer rows one warp each; or MERGE, rows of at most 255 entries in
+ * at most 32 entries in SELL-32 slices sorted by length inside windows of 1024
+ * rows, longer rows in groups of 4, 16 or 32 lanes or in whole blocks; or
+ * MERGE, rows of at most 255 entries in
  * blocks of at most 256 row ends + nonzeros, one warp per block, split evenly
  * among its 32 lanes along the merge path (nonzero-balanced, no copy of the
  * values), longer rows one warp each.  A new matrix takes SELL-32 where it
@@ -288,8 +289,10 @@ int hbicg_solve(unsigned n, unsigned nnz, const unsigned *ptr, const unsigned *c
                 double *r_out, hbicg_stats *stats);
 
 /* Solvers take their device buffers from a library-owned pool that keeps freed
- * memory for the next solver; this returns the memory no live solver uses to
- * the device (call it when the library's solves are done). */
+ * memory for the next solver, and up to 16 contexts that nothing uses any more
+ * are kept with their streams and events; this returns the memory no live
+ * solver uses to the device and frees those contexts (call it when the
+ * library's solves are done). */
 void hbicg_release(void);
 
 #ifdef __cplusplus
