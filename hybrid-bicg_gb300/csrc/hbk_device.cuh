@@ -281,8 +281,8 @@ struct SellRows {
         entries(off, wl, cc, vv);
         head(after(r0), off1, wl1);
     }
-    template <class Pre, class Epi>
-    __device__ __forceinline__ void run(const double *__restrict__ x, const Pre &pre, Epi &epi) {
+    template <class Pre, class Epi, class Turn>
+    __device__ __forceinline__ void run(const double *__restrict__ x, const Pre &pre, Epi &epi, Turn &turn) {
         while (r0 < A.n) {
             const unsigned r = r0 + threadIdx.x, len = wl & 255u;
             double xv[SELL_AHEAD], vn[SELL_AHEAD];
@@ -300,6 +300,7 @@ struct SellRows {
             for (unsigned e = SELL_AHEAD; e < wl >> 8; ++e)
                 if (e < len) acc = fma(__ldg(A.sval + entry(off, e)), __ldg(x + __ldg(A.scol + entry(off, e))), acc);
             if (r < A.n) epi(r, acc, own);
+            turn();
 #pragma unroll
             for (unsigned e = 0; e < SELL_AHEAD; ++e) vv[e] = vn[e];
             off = off1, wl = wl1;
@@ -661,15 +662,21 @@ __device__ __forceinline__ void spmv_rows_merge(const hbk_matrix &A, const doubl
 // Format chosen at compile time so the SELL kernels carry no shared-memory
 // tile (full occupancy); launchers pick the instantiation from A.fmt.
 // (the virtual grids of a persistent launch take the SELL-32 form only)
-// start() reads the matrix alone, so it may run before x is ready.
+// start() reads the matrix alone, so it may run before x is ready.  turns: a
+// block's rows come as NT at a time, all its threads calling turn() after each
+// (SellRows); the other forms have no such steps and never call it.
+struct NoTurn {
+    __device__ __forceinline__ void operator()() const {}
+};
 template <int FMT, class G, int AHEAD = 8>
 struct SpmvRows {
     static_assert(is_hw_grid<G>::value, "virtual grids take the SELL-32 form only");
+    static constexpr bool turns = false;
     const hbk_matrix &A;
     __device__ __forceinline__ SpmvRows(const hbk_matrix &a, const G &) : A(a) {}
     __device__ __forceinline__ void start() {}
-    template <class Pre, class Epi>
-    __device__ __forceinline__ void run(const double *__restrict__ x, const Pre &pre, Epi &epi) {
+    template <class Pre, class Epi, class Turn>
+    __device__ __forceinline__ void run(const double *__restrict__ x, const Pre &pre, Epi &epi, Turn &) {
         if constexpr (FMT == HBK_FMT_HYB || FMT == HBK_FMT_HYBW) {
             spmv_rows_hyb<FMT == HBK_FMT_HYBW>(A, x, pre, epi);
         } else if constexpr (FMT == HBK_FMT_MERGE) {
@@ -683,20 +690,23 @@ struct SpmvRows {
 };
 template <int AHEAD>
 struct SpmvRows<HBK_FMT_SELL, HwGrid, AHEAD> : SellRows<AHEAD> {
+    static constexpr bool turns = true;
     __device__ __forceinline__ SpmvRows(const hbk_matrix &a, const HwGrid &) : SellRows<AHEAD>(a) {}
 };
 template <int AHEAD>
 struct SpmvRows<HBK_FMT_SELLN, HwGrid, AHEAD> : SellRows<5> {
+    static constexpr bool turns = true;
     __device__ __forceinline__ SpmvRows(const hbk_matrix &a, const HwGrid &) : SellRows<5>(a) {}
 };
 template <int AHEAD>
 struct SpmvRows<HBK_FMT_SELL, VGrid, AHEAD> {
+    static constexpr bool turns = false;
     const hbk_matrix &A;
     const VGrid &g;
     __device__ __forceinline__ SpmvRows(const hbk_matrix &a, const VGrid &v) : A(a), g(v) {}
     __device__ __forceinline__ void start() {}
-    template <class Pre, class Epi>
-    __device__ __forceinline__ void run(const double *__restrict__ x, const Pre &pre, Epi &epi) {
+    template <class Pre, class Epi, class Turn>
+    __device__ __forceinline__ void run(const double *__restrict__ x, const Pre &pre, Epi &epi, Turn &) {
         spmv_rows_sell(A, x, pre, epi, g);
     }
 };
@@ -704,7 +714,8 @@ template <int FMT, int AHEAD = 8, class Pre, class Epi>
 __device__ __forceinline__ void spmv_rows(const hbk_matrix &A, const double *__restrict__ x, const Pre &pre, Epi &epi) {
     SpmvRows<FMT, HwGrid, AHEAD> rows(A, HwGrid());
     rows.start();
-    rows.run(x, pre, epi);
+    NoTurn none;
+    rows.run(x, pre, epi, none);
 }
 
 // number of SMs of the current device (cached: one device type per process)

@@ -36,7 +36,7 @@ struct Ctx {
     hbk_matrix A;
     hbk_vectors v;
     hbk_shifts sh;
-    // partial sums that each step leaves behind (the blocks of K1, K3, K4, K5)
+    // partial sums that each step leaves behind (K1, K3, K4; the blocks of K5)
     unsigned np_s, np_y, np_r, np_p;
 };
 
@@ -87,10 +87,23 @@ __device__ __forceinline__ hbk_cur load_cur(const hbk_scalars *sc) {
 // shifts 5.61 -> 3.22 ms; 97 k rows, 24 shifts 26.4 -> 18.2 ms; 128^3, 32
 // shifts 72.9 -> 61.1 ms; 256^3, 64 shifts 805 -> 711 ms (with the changes made
 // elsewhere since: 0.82, 2.9, 16.0, 55.5 and 655 ms).
+//
+// The order of a dot product's sum is part of a solve's outcome: it moves what
+// is left of every residual below the tolerance at which the solve stops, and
+// results that cancel (the shift gradient -w lambda . x: digits lost by the
+// cosine of the two) show that in their ninth digit.  So the order follows from
+// n and the number of SMs alone, not from the blocks a kernel is launched in:
+// NT threads to a set of rows, at most 6 sets per SM for the products of SELL-32
+// matrices and DOT_VEC for K4; a thread adds its rows in ascending order, a tree
+// adds the NT, and NT threads and the same tree add the sets.  Blocks fewer or
+// larger than a set carry several: K1 and K3 (3 blocks per SM) two, their NT-row
+// steps in turn, K4 up to three.  (After a switch (r^, r) is summed once over
+// K5's blocks.)
 
 // The vector kernels (K2, K4, K5) run one block per SM, of as many threads as
-// that takes (blockDim.x, 128..1024): the sums at a block's start then cost an
-// SM one pass, not one per resident block.
+// that takes (blockDim.x, 128..1024; K4: vec_sets): the sums at a block's start
+// then cost an SM one pass, not one per resident block.
+constexpr int DOT_VEC = 4, DOT_ROWS = 512;  // K4: sets per SM at most, rows per set while there are fewer
 
 constexpr int MAXW = 32;  // warps of the largest block
 
@@ -105,7 +118,7 @@ struct PartSum {
     unsigned nw;
     __device__ __forceinline__ void load(const double *p0, const double *p1, unsigned np) {
         const unsigned t = threadIdx.x;
-        nw = min(min(blockDim.x >> 5, 16u), (np + 31) >> 5);
+        nw = min(min(blockDim.x >> 5, (unsigned)NW), (np + 31) >> 5);
         x = y = 0.0;
         if (t < nw * 32 && t < np) {
             x = __ldcg(p0 + t);
@@ -151,20 +164,37 @@ __device__ __forceinline__ void store_part(double v, double *sh, double *out) {
         if (threadIdx.x == 0) *out = t;
     }
 }
-__device__ __forceinline__ void store_part2(double2 v, double *sh, double *out_x, double *out_y) {
-    const unsigned w = threadIdx.x >> 5, l = threadIdx.x & 31, nw = blockDim.x >> 5;
+// Two sums of every 256 threads (NW warps) of the block, where `here`; sh: 2 MAXW
+__device__ __forceinline__ void store_part2(double2 v, double *sh, double *out_x, double *out_y, bool here = true) {
+    const unsigned w = threadIdx.x >> 5, l = threadIdx.x & 31;
     const double x = warp_sum_pair(v.x, v.y);
     if ((l & 15) == 0) sh[(l >> 4) * MAXW + w] = x;
     __syncthreads();
-    if (w == 0) {
-        const double *p = sh + (l >> 4) * MAXW + (l & 15);
-        double t = (l & 15) < nw ? p[0] : 0.0;
-        if (nw > 16) t += (l & 15) + 16 < nw ? p[16] : 0.0;
+    if (w % NW == 0) {
+        double t = (l & 15) < NW ? sh[(l >> 4) * MAXW + w + (l & 15)] : 0.0;
 #pragma unroll
-        for (unsigned k = 8; k; k >>= 1)
-            if (k < nw) t += __shfl_xor_sync(0xffffffffu, t, k);
-        if (l == 0) *out_x = t;
-        if (l == 16) *out_y = t;
+        for (unsigned k = NW / 2; k; k >>= 1) t += __shfl_xor_sync(0xffffffffu, t, k);
+        if (here && l == 0) *out_x = t;
+        if (here && l == 16) *out_y = t;
+    }
+}
+// and two sums each of two sets (v0, v1) of a block of 256 threads, v1's
+// `after` entries behind v0's; sh: 4 MAXW
+__device__ __forceinline__ void store_part4(double2 v0, double2 v1, double *sh, double *out_x, double *out_y,
+                                            unsigned after) {
+    const unsigned w = threadIdx.x >> 5, l = threadIdx.x & 31;
+    const double x = warp_sum_pair(v0.x, v0.y), y = warp_sum_pair(v1.x, v1.y);
+    if ((l & 15) == 0) {
+        sh[(l >> 4) * MAXW + w] = x;
+        sh[(2 + (l >> 4)) * MAXW + w] = y;
+    }
+    __syncthreads();
+    if (w < 2) {
+        double t = (l & 15) < NW ? sh[(2 * w + (l >> 4)) * MAXW + (l & 15)] : 0.0;
+#pragma unroll
+        for (unsigned k = NW / 2; k; k >>= 1) t += __shfl_xor_sync(0xffffffffu, t, k);
+        if (l == 0) out_x[w * after] = t;
+        if (l == 16) out_y[w * after] = t;
     }
 }
 // shared memory of a body is used again by the next virtual block of the CTA
@@ -247,9 +277,10 @@ __global__ void __launch_bounds__(NT) k_init_coef(Ctx c) {
 // ---------------------------------------------------------------------------
 // K1: s = (A + sigma_s I) p_s and (r^, s).  Block 0 copies the scalars that
 // the iteration's other kernels read (hbk_cur).
+// SELL-32: block b carries the sets b and b + (blocks), its NT-row steps in turn.
 template <int FMT, class G>
 __device__ __forceinline__ void seed_s_body(const Ctx &c, const G &g) {
-    __shared__ double red[MAXW];
+    __shared__ double red[2 * MAXW];
     hbk_scalars *sc = c.sh.sc;
     body_begin<G>();
     SpmvRows<FMT, G> rows(c.A, g);
@@ -269,15 +300,26 @@ __device__ __forceinline__ void seed_s_body(const Ctx &c, const G &g) {
     const double *__restrict__ rh = c.v.r_hat;
     double *__restrict__ s = c.v.s;
     const bool folded = c.v.sval_shift != nullptr;  // the product already holds sigma p
-    double acc = 0.0;
+    double acc = 0.0, alt = 0.0;
+    bool odd = false;
     auto pre = [&](unsigned r) { return HBK_LD(G, rh, r); };
     auto epi = [&](unsigned r, double ax, double hr) {
         const double sv = folded ? ax : fma(sig, HBK_LD(G, ps, r), ax);
         s[r] = sv;
         acc = fma(hr, sv, acc);
     };
-    rows.run(ps, pre, epi);
-    store_part(acc, red, parts(c, P_RS) + g.b());
+    auto turn = [&] {
+        const double t = acc;
+        acc = alt, alt = t, odd = !odd;
+    };
+    rows.run(ps, pre, epi, turn);
+    double *out = parts(c, P_RS) + g.b();
+    if constexpr (decltype(rows)::turns) {
+        if (odd) turn();
+        store_part2(make_double2(acc, alt), red, out, out + g.nb());
+    } else {
+        store_part(acc, red, out);
+    }
 }
 template <int FMT>
 __global__ void __launch_bounds__(NT) k_seed_s(Ctx c) { seed_s_body<FMT>(c, HwGrid()); }
@@ -363,12 +405,14 @@ __device__ __forceinline__ void seed_q_body(const Ctx &c, const G &g) {
 }
 __global__ void __launch_bounds__(1024) k_seed_q(Ctx c) { seed_q_body(c, HwGrid()); }
 
-// K3: y = (A + sigma_s I) q, (q,q) and (q,y)
+// K3: y = (A + sigma_s I) q, (q,q) and (q,y).  SELL-32: the sums of two sets take
+// the registers of an eighth entry ahead (256^3: 295 us; with it they spill, 367;
+// the other set's in shared memory 321, with seven ahead 340).
 template <int FMT, class G>
 __device__ __forceinline__ void seed_y_body(const Ctx &c, const G &g) {
-    __shared__ double red[2 * MAXW];
+    __shared__ double red[4 * MAXW];
     body_begin<G>();
-    SpmvRows<FMT, G> rows(c.A, g);
+    SpmvRows<FMT, G, 7> rows(c.A, g);
     rows.start();
     body_ready<G>();
     const hbk_cur u = load_cur(c.sh.sc);
@@ -377,7 +421,9 @@ __device__ __forceinline__ void seed_y_body(const Ctx &c, const G &g) {
     const double *__restrict__ q = vec_q(c, u);
     double *__restrict__ y = c.v.y;
     const bool folded = c.v.sval_shift != nullptr;  // the product already holds sigma q
-    double2 acc = make_double2(0.0, 0.0);
+    constexpr bool turns = decltype(rows)::turns;
+    double2 acc = make_double2(0.0, 0.0), alt = acc;
+    bool odd = false;
     auto pre = [&](unsigned r) { return HBK_LD(G, q, r); };
     auto epi = [&](unsigned r, double ax, double qr) {
         const double yv = folded ? ax : fma(sig, qr, ax);
@@ -385,8 +431,16 @@ __device__ __forceinline__ void seed_y_body(const Ctx &c, const G &g) {
         acc.x = fma(qr, qr, acc.x);
         acc.y = fma(qr, yv, acc.y);
     };
-    rows.run(q, pre, epi);
-    store_part2(acc, red, parts(c, P_QQ) + g.b(), parts(c, P_QY) + g.b());
+    auto turn = [&] {
+        const double2 t = alt;
+        alt = acc;
+        acc = t, odd = !odd;
+    };
+    rows.run(q, pre, epi, turn);
+    double *qq = parts(c, P_QQ) + g.b(), *qy = parts(c, P_QY) + g.b();
+    if (turns && odd) turn();
+    if (turns && c.np_y > g.nb()) store_part4(acc, alt, red, qq, qy, g.nb());
+    else store_part2(acc, red, qq, qy);
 }
 template <int FMT>
 __global__ void __launch_bounds__(NT) k_seed_y(Ctx c) { seed_y_body<FMT>(c, HwGrid()); }
@@ -524,7 +578,10 @@ __device__ __forceinline__ void seed_update_body(const Ctx &c, const G &g) {
     const double *__restrict__ y = c.v.y;
     const double *__restrict__ rh = c.v.r_hat;
     const bool extra = g.extra();
-    size_t i = extra ? (size_t)n : g.b() * (size_t)blockDim.x + threadIdx.x;
+    // 256 threads per set of rows
+    const unsigned set = g.b() * (blockDim.x / NT) + threadIdx.x / NT, nset = c.np_r;
+    const bool here = !extra && set < nset;
+    size_t i = here ? set * (size_t)NT + threadIdx.x % NT : (size_t)n;
     double hi = i < n ? HBK_LD(G, rh, i) : 0.0;
     body_ready<G>();
     const hbk_cur u = load_cur(sc);
@@ -564,7 +621,7 @@ __device__ __forceinline__ void seed_update_body(const Ctx &c, const G &g) {
     }
     double2 acc = make_double2(0.0, 0.0);
     unsigned long long mx = 0;
-    const size_t step = (size_t)g.nb() * blockDim.x;
+    const size_t step = (size_t)nset * NT;
     while (i < n) {
         const size_t in = i + step;  // the next element's loads go before this one's store
         const double yn = in < n ? HBK_LD(G, y, in) : 0.0, hn = in < n ? HBK_LD(G, rh, in) : 0.0;
@@ -578,9 +635,10 @@ __device__ __forceinline__ void seed_update_body(const Ctx &c, const G &g) {
         yi = yn, hi = hn, qi = qn, i = in;
     }
     if (c.v.slot_max) block_max_to(mx, smx, c.v.slot_max + (size_t)(u.slots + 1) * HBK_SLOT_SPREAD);  // r_k
-    store_part2(acc, sh, parts(c, P_RR) + g.b(), parts(c, P_RRH) + g.b());
+    store_part2(acc, sh, parts(c, P_RR) + set, parts(c, P_RRH) + set, here);
 }
-__global__ void __launch_bounds__(1024) k_seed_update(Ctx c) { seed_update_body(c, HwGridX{1}); }
+template <int PER_SM>
+__global__ void __launch_bounds__(2 * NT, PER_SM) k_seed_update(Ctx c) { seed_update_body(c, HwGridX{1}); }
 
 // ---------------------------------------------------------------------------
 // Argmax of |1/(zeta_j pi_j)| over the systems still running after this
@@ -1557,6 +1615,19 @@ static VecGrid vec_grid(unsigned n, int extra) {
     const unsigned need = n ? (n + t - 1) / t : 1;
     return {need < (unsigned)most ? (int)need : most, (int)t};
 }
+// K4's: all its sets of rows resident at once, beside the extra block: one block
+// per SM with 64 registers while two sets fill it; two blocks and 40 registers
+// (a third fits) where there are more, as then the scalars in the extra block
+// need not be fast (their spills cost 1.6 us, K4 8.5 instead of 6.9 us at n = 512).
+static int vec_sets(unsigned n) {
+    const int most = DOT_VEC * sm_count();
+    const unsigned want = n ? (n + DOT_ROWS - 1) / DOT_ROWS : 1;
+    return want < (unsigned)most ? (int)want : most;
+}
+static VecGrid set_grid(int sets) {
+    const int per = sets <= sm_count() ? 1 : 2;
+    return {(sets + per - 1) / per, per * NT};
+}
 
 // kernel<<<...>>>, allowed to start before the stream's previous kernel ends
 // (the kernel waits for it before it reads anything the iteration writes)
@@ -1578,24 +1649,24 @@ template <int FMT>
 static void launch_iteration(Ctx &c, const hbk_matrix *A, int early, cudaStream_t st) {
     // the products are grid-stride loops: at most one wave of them
     const int gs = wave_grid<k_seed_s<FMT>>(A->grid), gy = wave_grid<k_seed_y<FMT>>(A->grid);
-    // (K4 leaves two SMs: the grid also fixes the order of its dot products' sums,
-    // and with the order, all being equally accurate, the 256^3 family's solve
-    // takes 413..457 iterations; with 150 blocks it takes 415, as the
-    // reference's own 414 does to within 2 %)
-    const VecGrid q = vec_grid(c.v.n, 0), r = vec_grid(c.v.n, 2);
+    constexpr bool sell = FMT == HBK_FMT_SELL || FMT == HBK_FMT_SELLN;
+    const VecGrid q = vec_grid(c.v.n, 0), r = set_grid(vec_sets(c.v.n));
     const unsigned ncoef = !c.v.deferred ? 0 : ((unsigned)(c.sh.m < 256 ? c.sh.m : 256) * 64u + q.threads - 1) / q.threads;
     const VecGrid p = vec_grid(c.v.n, 1 + (int)ncoef);
-    c.np_s = (unsigned)gs, c.np_y = (unsigned)gy, c.np_r = (unsigned)r.blocks, c.np_p = (unsigned)p.blocks;
+    // (SELL-32: a set for every NT rows up to two per block)
+    const auto sets = [&](int blocks) { return (unsigned)(sell && A->grid < 2 * blocks ? A->grid : sell ? 2 * blocks : blocks); };
+    c.np_s = sets(gs), c.np_y = sets(gy);
+    c.np_r = (unsigned)vec_sets(c.v.n), c.np_p = (unsigned)p.blocks;
     // Early starts: measured on whole solves, SELL-32, n = 512: 1163 -> 1061 us;
     // 97 k rows: 20.1 -> 18.5 ms; 128^3: 64.2 -> 63.0 ms.  Not where blocks
     // that start early would crowd onto the SMs the kernel before leaves free
     // and then run long: the incremental update (FP64-bound; 32^3: 3.4 -> 4.7
     // ms) and the products of the other forms (HYB: 68 -> 75 ms).
-    const bool e = early > 0, es = e && (FMT == HBK_FMT_SELL || FMT == HBK_FMT_SELLN);
+    const bool e = early > 0, es = e && sell;
     launch(k_seed_s<FMT>, gs, NT, es && early > 1, st, c);
     launch(k_seed_q, q.blocks, q.threads, e, st, c);
     launch(k_seed_y<FMT>, gy, NT, es, st, c);
-    launch(k_seed_update, r.blocks + 1, r.threads, e, st, c);
+    launch(r.blocks <= sm_count() ? k_seed_update<2> : k_seed_update<3>, r.blocks + 1, r.threads, e, st, c);
     if (!c.v.deferred) launch(k_shift_update<64>, p.blocks + 1, p.threads, false, st, c);
     else launch(k_seed_p_deferred, p.blocks + 1 + (int)ncoef, p.threads, e, st, c, ncoef);
 }
