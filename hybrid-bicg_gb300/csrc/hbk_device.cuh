@@ -310,7 +310,8 @@ struct SellRows {
 };
 // The same one slice at a time: on a virtual grid (a persistent launch's
 // families are small and their matrices in L2; the x may have been written by
-// the same launch), and for the plain product of a small matrix (k_spmv_small)
+// the same launch), and for the plain products that slices ahead do not make
+// faster (k_spmv_slices)
 template <class G, class Pre, class Epi>
 __device__ __forceinline__ void spmv_rows_sell(const hbk_matrix &A, const double *__restrict__ x, const Pre &pre,
                                                Epi &epi, const G &g) {
@@ -328,13 +329,15 @@ __device__ __forceinline__ void spmv_rows_sell(const hbk_matrix &A, const double
         const unsigned len = r < n ? __ldg(A.ptr + r + 1) - __ldg(A.ptr + r) : 0;
         const double *__restrict__ vv = A.sval + base + lane;
         const unsigned *__restrict__ cc = A.scol + base + lane;
-        const double own = r < n ? pre(r) : 0.0;
+        // (a launch's own grid: read behind the sum; 20 k rows of 40 entries, one product: 10.3
+        // against 12.4 us)
+        const double own = !G::hw && r < n ? pre(r) : 0.0;
         double acc = 0.0;
 #pragma unroll 4
         for (unsigned e = 0; e < w; ++e) {
             if (e < len) acc = fma(G::ldv(vv + 32 * (size_t)e), G::ldx(x + __ldg(cc + 32 * (size_t)e)), acc);
         }
-        if (r < n) epi(r, acc, own);
+        if (r < n) epi(r, acc, G::hw ? pre(r) : own);
     }
 }
 
@@ -749,12 +752,17 @@ inline int wave_grid(int want) {
 // 128^3 257 / 278.
 inline bool sell_narrow(const hbk_matrix &A) { return A.fmt == HBK_FMT_SELL && (double)A.nnz <= 5.5 * A.n; }
 
-// launch helper: kernel<FMT> for the matrix's format
+// launch helpers: kernel<FMT> for the matrix's format
 #define HBK_LAUNCH_FMT(A, kern, grid, block, stream, ...)                                   \
     do {                                                                                    \
         if (sell_narrow(A)) kern<HBK_FMT_SELLN><<<grid, block, 0, stream>>>(__VA_ARGS__);   \
         else if ((A).fmt == HBK_FMT_SELL) kern<HBK_FMT_SELL><<<grid, block, 0, stream>>>(__VA_ARGS__); \
-        else if ((A).fmt == HBK_FMT_HYB && (A).nwide) kern<HBK_FMT_HYBW><<<grid, block, 0, stream>>>(__VA_ARGS__); \
+        else HBK_LAUNCH_CSR(A, kern, grid, block, stream, __VA_ARGS__);                     \
+    } while (0)
+// the same for the forms other than SELL-32
+#define HBK_LAUNCH_CSR(A, kern, grid, block, stream, ...)                                   \
+    do {                                                                                    \
+        if ((A).fmt == HBK_FMT_HYB && (A).nwide) kern<HBK_FMT_HYBW><<<grid, block, 0, stream>>>(__VA_ARGS__); \
         else if ((A).fmt == HBK_FMT_HYB) kern<HBK_FMT_HYB><<<grid, block, 0, stream>>>(__VA_ARGS__); \
         else if ((A).fmt == HBK_FMT_MERGE) kern<HBK_FMT_MERGE><<<grid, block, 0, stream>>>(__VA_ARGS__); \
         else kern<HBK_FMT_TILE><<<grid, block, 0, stream>>>(__VA_ARGS__);                  \

@@ -3,6 +3,8 @@
 // host exactly in the reference's order (src/solver_dynamic.c:156-256).
 #include <stdio.h>
 
+#include <math.h>
+
 #include "hbk_device.cuh"
 
 using namespace hbk;
@@ -89,15 +91,18 @@ __global__ void __launch_bounds__(NT, HBK_SELL_MINB) k_spmv<HBK_FMT_SELLN>(hbk_m
     auto pre = [&](unsigned r) { return add ? x[r] : 0.0; };
     spmv_rows<HBK_FMT_SELLN>(A, x, pre, epi);
 }
-// SELL-32 product of a small matrix: a row or two per thread, so nothing to
-// keep ahead; six blocks per SM (250 k rows of five entries: 6.7 us, 8.2 us
-// with slices ahead; at 1 M rows 16.7 / 16.1; seven entries: the same up to
-// 1 M rows)
-constexpr unsigned SMALL_ROWS = 1u << 19;
-__global__ void __launch_bounds__(NT) k_spmv_small(hbk_matrix A, const double *__restrict__ x, double *__restrict__ y,
-                                                   double sigma, int add) {
+// SELL-32 product, one slice at a time (eight blocks per SM): where there is
+// nothing to gain from slices ahead (slices_ahead)
+__global__ void __launch_bounds__(NT) k_spmv_slices(hbk_matrix A, const double *__restrict__ x, double *__restrict__ y,
+                                                    double sigma, int add) {
     EpiStore epi{y, x, sigma, add};
     auto pre = [&](unsigned r) { return add ? x[r] : 0.0; };
+    spmv_rows_sell(A, x, pre, epi, HwGrid());
+}
+__global__ void __launch_bounds__(NT) k_spmv_acc_slices(hbk_matrix A, const double *__restrict__ x,
+                                                        double *__restrict__ y) {
+    EpiAccum epi{y};
+    auto pre = [&](unsigned r) { return y[r]; };
     spmv_rows_sell(A, x, pre, epi, HwGrid());
 }
 
@@ -383,25 +388,45 @@ int hbk_merge_grid(unsigned units) {
     return g < 1 ? 1 : g;
 }
 
-// blocks of a product: SELL-32 at most one wave (a second, partial wave cost
-// 340 against 261 us on the 256^3 stencil), the other forms as planned
+// blocks of a product with slices ahead: at most one wave (a second, partial wave cost
+// 340 against 261 us on the 256^3 stencil); the other forms as planned
 static int product_grid(const hbk_matrix *A) {
     return A->fmt == HBK_FMT_SELL ? wave_grid<k_spmv<HBK_FMT_SELL>>(A->grid) : A->grid;
 }
 
+// Does a SELL-32 product keep slices ahead (three blocks per SM) or take them
+// one at a time (eight)?  Banded matrices of w entries per row, us, one at a
+// time / ahead:
+//   below half a million rows a thread has a row or two, nothing to keep ahead: 250 k rows,
+//     w = 5 6.7 / 8.2; 500 k, w = 1 6.2 / 10.3, w = 13 18.5 / 20.5
+//   w up to 4: the rows' own latency is short and the warps count: 3 M rows, w = 1
+//     16.8 / 36.9, w = 3 35.0 / 40.7, w = 4 41.0 / 41.5
+//   w = 5..8, longer than its chain of loads, all of it ahead: 3 M rows, w = 5 47.7 / 44.1,
+//     w = 7 57.4 / 53.0 (10 M: 174 / 158)
+//   wider rows have enough loads of their own: 3 M rows, w = 9 72.1 / 79.1, w = 20
+//     139.6 / 143.5; 600 k, w = 40 57.8 / 64.2; but from w = 16 on, where the last wave of
+//     eight blocks per SM would be nearly empty and that of three is not: 1 M, w = 20
+//     58.2 / 53.7, w = 27 73.5 / 65.5, w = 40 104 / 95
+static bool slices_ahead(const hbk_matrix *A) {
+    if (A->n < (1u << 19) || A->nnz <= 4.5 * A->n) return false;
+    if (A->nnz <= 8.0 * A->n) return true;
+    if (A->nnz < 16.0 * A->n) return false;
+    const double blocks = (A->n + NT - 1) / NT;
+    const auto waves = [&](int grid) { return ceil(blocks / grid) * grid / blocks; };
+    return waves(A->grid) > 1.1 * waves(product_grid(A));
+}
+
 int hbk_spmv(const hbk_matrix *A, const double *x, double *y, double sigma, int sigma_add, cudaStream_t st) {
     if (!A->n) return 0;
-    if (A->fmt == HBK_FMT_SELL && A->n < SMALL_ROWS) {
-        k_spmv_small<<<A->grid, NT, 0, st>>>(*A, x, y, sigma, sigma_add);
-        return (int)cudaGetLastError();
-    }
-    HBK_LAUNCH_FMT(*A, k_spmv, product_grid(A), NT, st, *A, x, y, sigma, sigma_add);
+    if (A->fmt == HBK_FMT_SELL && !slices_ahead(A)) k_spmv_slices<<<A->grid, NT, 0, st>>>(*A, x, y, sigma, sigma_add);
+    else HBK_LAUNCH_FMT(*A, k_spmv, product_grid(A), NT, st, *A, x, y, sigma, sigma_add);
     return (int)cudaGetLastError();
 }
 
 int hbk_spmv_accumulate(const hbk_matrix *A, const double *x, double *y, cudaStream_t st) {
     if (!A->n) return 0;
-    HBK_LAUNCH_FMT(*A, k_spmv_acc, product_grid(A), NT, st, *A, x, y);
+    if (A->fmt == HBK_FMT_SELL) k_spmv_acc_slices<<<A->grid, NT, 0, st>>>(*A, x, y);
+    else HBK_LAUNCH_CSR(*A, k_spmv_acc, A->grid, NT, st, *A, x, y);
     return (int)cudaGetLastError();
 }
 
