@@ -67,35 +67,67 @@ __global__ void __launch_bounds__(NT) k_grad_b(unsigned n, int m, const double *
 // read once and coalesced, and two shifts have their loads in flight together
 // (one or four: 2 % slower; more than two blocks per SM: up to 5 %).  128^3,
 // 32 shifts: 2062 -> 1110 us, without the map from entries to rows (47 us);
-// floor 740 us (one FMA per entry and shift).
+// floor 740 us (one FMA per entry and shift).  An operation that no lane needs
+// costs the pipe as much as any other, so a warp runs the code for the longest
+// of its rows (with that for GRAD_E always, 1 M rows and 32 shifts took 785 us
+// at one, two or three entries per row; k_grad_val 435, 548, 689).
 constexpr int GRAD_E = 8;
+struct GradRow {
+    unsigned e0, cnt;  // the row's next entries
+    size_t row;
+    int m;
+    const unsigned *__restrict__ col;
+    const double *__restrict__ X, *__restrict__ Y, *__restrict__ w;
+    size_t ldx, ldy;
+    double *__restrict__ dval;
+    template <int E>
+    __device__ __forceinline__ void part() const {
+        unsigned c[E];
+        double s[E];
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+            c[e] = (unsigned)e < cnt ? col[e0 + e] : 0u;
+            s[e] = 0.0;
+        }
+        const double *xj = X, *yj = Y + row;
+#pragma unroll 2
+        for (int j = 0; j < m; ++j, xj += ldx, yj += ldy) {
+            const double y = (w ? w[j] : 1.0) * *yj;
+#pragma unroll
+            for (int e = 0; e < E; ++e)
+                if ((unsigned)e < cnt) s[e] = fma(y, xj[c[e]], s[e]);
+        }
+#pragma unroll
+        for (int e = 0; e < E; ++e)
+            if ((unsigned)e < cnt) dval[e0 + e] = -s[e];
+    }
+    // most: of cnt over the warp
+    template <int E>
+    __device__ __forceinline__ void parts(unsigned most) const {
+        if constexpr (E > 1) {
+            if (most < E) {
+                parts<E - 1>(most);
+                return;
+            }
+        }
+        part<E>();
+    }
+};
 __global__ void __launch_bounds__(NT, 2) k_grad_val_rows(unsigned n, const unsigned *__restrict__ ptr,
                                                       const unsigned *__restrict__ col, int m,
                                                       const double *__restrict__ X, size_t ldx,
                                                       const double *__restrict__ Y, size_t ldy,
                                                       const double *__restrict__ w, double *__restrict__ dval) {
-    for (size_t i = blockIdx.x * (size_t)NT + threadIdx.x; i < n; i += (size_t)gridDim.x * NT) {
-        const unsigned e1 = ptr[i + 1];
-        for (unsigned e0 = ptr[i]; e0 < e1; e0 += GRAD_E) {
-            const unsigned cnt = e1 - e0;
-            unsigned c[GRAD_E];
-            double s[GRAD_E];
-#pragma unroll
-            for (int e = 0; e < GRAD_E; ++e) {
-                c[e] = (unsigned)e < cnt ? col[e0 + e] : 0u;
-                s[e] = 0.0;
-            }
-            const double *xj = X, *yj = Y + i;
-#pragma unroll 2
-            for (int j = 0; j < m; ++j, xj += ldx, yj += ldy) {
-                const double y = (w ? w[j] : 1.0) * *yj;
-#pragma unroll
-                for (int e = 0; e < GRAD_E; ++e)
-                    if ((unsigned)e < cnt) s[e] = fma(y, xj[c[e]], s[e]);
-            }
-#pragma unroll
-            for (int e = 0; e < GRAD_E; ++e)
-                if ((unsigned)e < cnt) dval[e0 + e] = -s[e];
+    for (size_t i0 = blockIdx.x * (size_t)NT + (threadIdx.x & ~31u); i0 < n; i0 += (size_t)gridDim.x * NT) {
+        const size_t i = i0 + (threadIdx.x & 31);
+        GradRow g{0u, 0u, i < n ? i : n - 1, m, col, X, Y, w, ldx, ldy, dval};
+        if (i < n) g.e0 = ptr[i], g.cnt = ptr[i + 1] - g.e0;
+        for (;;) {  // (whole warps)
+            const unsigned most = __reduce_max_sync(0xffffffffu, g.cnt);
+            if (!most) break;
+            g.parts<GRAD_E>(most);
+            const unsigned done = g.cnt < GRAD_E ? g.cnt : GRAD_E;
+            g.e0 += done, g.cnt -= done;
         }
     }
 }

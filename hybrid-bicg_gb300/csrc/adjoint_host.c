@@ -51,6 +51,22 @@ int hbicg_matrix_transpose(hbicg_matrix *A, hbicg_matrix **At) {
     return transpose_into(A, hbicg__matrix_context(A), At);
 }
 
+/* Gradients of the values: a thread per row where rows are short and alike
+ * (the matrices that take SELL-32: at most 64 entries, little padding), else a
+ * thread per entry, in us at 32 shifts (row / entry): 1 M rows, w = 1 397 /
+ * 435, w = 3 474 / 695, w = 7 676 / 1334, w = 60 4064 / 10191.  But not
+ *   for few long rows, whose threads walk w m products one after another:
+ *     w = 60, 2 k rows 263 / 223, 8 k 263 / 267; w = 33, 500 rows 198 / 197;
+ *   for millions of rows of one entry (two, at one or two shifts), which wait
+ *     for memory, with more of it in flight per entry: w = 1, 3 M rows 978 / 916,
+ *     10 M and one shift 354 / 269; w = 2 there 376 / 327 */
+static int row_threads(const hbk_matrix *k, int m) {
+    const double n = k->n, nnz = k->nnz;
+    if (k->fmt != HBK_FMT_SELL) return 0;
+    if (n < 8000.0 && nnz * m > 1150.0 * n) return 0;
+    return !(n > 2097152.0 && nnz <= (m <= 2 ? 2.5 : 1.5) * n);
+}
+
 int hbicg_adjoint_gradients(hbicg_matrix *A, int m, const double *X, unsigned long long ldx, const double *Lam,
                             unsigned long long ldl, const double *w, double *dJ_dval, double *dJ_db,
                             double *dJ_dsigma) {
@@ -71,9 +87,7 @@ int hbicg_adjoint_gradients(hbicg_matrix *A, int m, const double *X, unsigned lo
         CK((cudaError_t)hbk_shift_dots(k->n, m, X, ldx, Lam, ldl, 0, w, -1.0, dJ_dsigma, tmp, sb));
     }
     if (dJ_db) CK((cudaError_t)hbk_grad_b(k->n, m, Lam, ldl, w, dJ_db, sb));
-    /* a thread per row where rows are short and alike (the matrices that take
-     * SELL-32: at most 64 entries, little padding), else a thread per entry */
-    if (dJ_dval && k->fmt == HBK_FMT_SELL) {
+    if (dJ_dval && row_threads(k, m)) {
         CK((cudaError_t)hbk_grad_val_rows(k->n, k->ptr, k->col, m, X, ldx, Lam, ldl, w, dJ_dval, st));
     } else if (dJ_dval) {
         CK(hbicg__dev_alloc((void **)&rows, sizeof(unsigned) * ((size_t)k->nnz + 1), st));
