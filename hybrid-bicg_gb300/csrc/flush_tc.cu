@@ -840,6 +840,9 @@ size_t hbk_flush_tc_workspace_bytes(int m) {
 
 int hbk_flush_tc_max_slots(void) { return TC_K; }
 
+static int g_test_error = 0;
+void hbk_flush_tc_test_error(int on) { g_test_error = on ? 1 : 0; }
+
 // x_j (and p_j when keep_p) from the first L basis slots on the tensor cores,
 // for the live shifts only: conv_k[j] == 0 or conv_k[j] > k_last (conv_k
 // NULL: every shift).  slot_max: bits of each slot's max |value| (NULL:
@@ -883,7 +886,12 @@ int hbk_flush_tc_run_live(const double *V, size_t ld, unsigned n, int L, const d
     const unsigned gx = ntiles < (unsigned)sms ? ntiles : (unsigned)sms;
     TcArgs args{V, ld, n, L, slot_max, aimg, rowexp, rown, X, Pmat, m, keep_p, live, err};
     k_flush_tc<<<dim3(gx, groups), TC_THREADS, SMEM_BYTES, st>>>(args);
-    return (int)cudaGetLastError();
+    if ((e = cudaGetLastError())) return (int)e;
+    if (g_test_error) {
+        g_test_error = 0;
+        e = cudaMemsetAsync(err, 1, sizeof(int), st);
+    }
+    return (int)e;
 }
 
 // device address of the live-shift count of the last hbk_flush_tc_run_live on ws

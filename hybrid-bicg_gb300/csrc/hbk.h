@@ -288,6 +288,8 @@ int hbk_grad_val_rows(unsigned n, const unsigned *ptr, const unsigned *col, int 
                       const double *Y, size_t ldy, const double *w, double *dval, cudaStream_t st);
 size_t hbk_flush_tc_workspace_bytes(int m);
 int hbk_flush_tc_max_slots(void);
+/* the next flush sets its error flag (one shot; for the test of a failed flush) */
+void hbk_flush_tc_test_error(int on);
 int hbk_flush_tc_run(const double *V, size_t ld, unsigned n, int L, const double *Xc, const double *Pc, int cap,
                      const double *own, int m, double *X, double *Pmat, int keep_p, void *ws, int *err,
                      cudaStream_t st);
@@ -301,8 +303,9 @@ int hbk_flush_tc_run_live(const double *V, size_t ld, unsigned n, int L, const d
 const int *hbk_flush_tc_live_count(const void *ws, int m); /* device int: live shifts of the last run on ws */
 /* x[i] = element i of system j of the panel-major Xp (m systems), i < n */
 int hbk_panel_row(const double *Xp, int m, unsigned n, int j, double *x, cudaStream_t st);
-/* X[j][i] (leading dimension ld) = Xp in panel layout with m systems, i < n */
-int hbk_panel_to_rows(const double *Xp, int m, unsigned n, double *X, size_t ld, cudaStream_t st);
+/* X[j][i] (leading dimension ld) = Xp in panel layout with m systems, i < n;
+ * X stays as it is where *err (device, may be NULL) is set when the stream gets there */
+int hbk_panel_to_rows(const double *Xp, int m, unsigned n, double *X, size_t ld, const int *err, cudaStream_t st);
 /* after a flush: zero the coefficients, own = (0, keep_p), basis slot 0 = r_{k-1};
  * live: device count of the shifts it formed (added to the scalars' flush_rows), or NULL */
 int hbk_deferred_reset(const hbk_vectors *v, const hbk_shifts *sh, int keep_p, const int *live, cudaStream_t st);

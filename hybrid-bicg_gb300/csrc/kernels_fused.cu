@@ -1396,9 +1396,12 @@ __global__ void __launch_bounds__(NT) k_panel_row(const double *__restrict__ Xp,
 }
 
 // X[j][i] = element i of system j of the panel-major Xp: one block per panel
-// (m * HBK_PANEL values read contiguously, written as runs of HBK_PANEL)
+// (m * HBK_PANEL values read contiguously, written as runs of HBK_PANEL);
+// nothing where *err says that a flush failed
 __global__ void __launch_bounds__(NT) k_panel_to_rows(const double *__restrict__ Xp, int m, unsigned n,
-                                                      double *__restrict__ X, size_t ld) {
+                                                      double *__restrict__ X, size_t ld,
+                                                      const int *__restrict__ err) {
+    if (err && *err) return;
     const unsigned per = (unsigned)m * HBK_PANEL;
     const size_t np = ((size_t)n + HBK_PANEL - 1) / HBK_PANEL;
     for (size_t p = blockIdx.x; p < np; p += gridDim.x) {
@@ -1542,10 +1545,10 @@ int hbk_panel_row(const double *Xp, int m, unsigned n, int j, double *x, cudaStr
     return (int)cudaGetLastError();
 }
 
-int hbk_panel_to_rows(const double *Xp, int m, unsigned n, double *X, size_t ld, cudaStream_t st) {
+int hbk_panel_to_rows(const double *Xp, int m, unsigned n, double *X, size_t ld, const int *err, cudaStream_t st) {
     if (m <= 0 || n == 0) return 0;
     const size_t np = ((size_t)n + HBK_PANEL - 1) / HBK_PANEL;
-    k_panel_to_rows<<<(unsigned)(np < 4864 ? np : 4864), NT, 0, st>>>(Xp, m, n, X, ld);
+    k_panel_to_rows<<<(unsigned)(np < 4864 ? np : 4864), NT, 0, st>>>(Xp, m, n, X, ld, err);
     return (int)cudaGetLastError();
 }
 

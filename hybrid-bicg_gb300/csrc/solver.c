@@ -217,7 +217,7 @@ struct hbicg_solver {
     double flush_bytes; /* compulsory HBM bytes of this solve's basis flushes */
     int flush_timed;    /* evf0, evf1 hold a flush whose time has not been read */
     /* where this solve's x_j end up, rows xld apart: the workspace's X, or the
-     * caller's device array (the deferred mode writes rows straight into it) */
+     * caller's device array (the deferred mode without corrections writes rows straight into it) */
     double *xrows;
     size_t xld;
     /* deferred mode, pinned host x: solutions that became final at a flush
@@ -897,7 +897,7 @@ static int fused_tail(hbicg_solver *s, int k_flushed, int *launches) {
         CUDA_TRY(cudaEventRecord(s->ctx->cev, s->ctx->cstream));
         CUDA_TRY(cudaStreamWaitEvent(st, s->ctx->cev, 0));
     }
-    HBK_TRY(hbk_panel_to_rows(s->v.Xp, s->v.pm, s->A->k.n, s->xrows, s->xld, st));
+    HBK_TRY(hbk_panel_to_rows(s->v.Xp, s->v.pm, s->A->k.n, s->xrows, s->xld, s->d_tc_err, st));
     ++*launches;
     return HBICG_OK;
 }
@@ -1227,7 +1227,8 @@ static int run_begin(hbicg_solver *s, const double *b, const double *sigma, run_
     int *act = hb->act = calloc((size_t)s->kcap + 1, sizeof(int));
     int *sw_k = hb->sw_k = calloc(m > 0 ? m : 1, sizeof(int)), *sw_seed = hb->sw_seed = calloc(m > 0 ? m : 1, sizeof(int));
     int *conv = hb->conv = calloc(m > 0 ? m : 1, sizeof(int));
-    if (!h_sigma || !act || !sw_k || !sw_seed || !conv) {
+    if (s->p.form != HBICG_FORM_PLAIN) hb->pack = malloc(s->pack_bytes);
+    if (!h_sigma || !act || !sw_k || !sw_seed || !conv || (s->p.form != HBICG_FORM_PLAIN && !hb->pack)) {
         set_msg("host scratch of %d shifts and %d iterations", m, s->kcap);
         return HBICG_E_NOMEM;
     }
@@ -1269,9 +1270,12 @@ static int run_begin(hbicg_solver *s, const double *b, const double *sigma, run_
     s->early = NULL;
     if (s->p.form != HBICG_FORM_PLAIN && s->v.deferred && x_pinned && (s->early = calloc((size_t)m, 1)) != NULL)
         s->early_x = x;
+    /* a failed solve leaves x alone: straight there only where nothing but a
+     * flush can still fail, which the writing kernel sees (with refine the
+     * rows may be corrected first) */
     s->xrows = s->v.X;
     s->xld = s->ld;
-    if (s->p.form != HBICG_FORM_PLAIN && s->v.deferred && out_where == HBICG_DEVICE && x) {
+    if (s->p.form != HBICG_FORM_PLAIN && s->v.deferred && out_where == HBICG_DEVICE && x && !s->p.refine) {
         s->xrows = x;
         s->xld = n;
     }
@@ -1305,11 +1309,7 @@ static int fused_collect(hbicg_solver *s, run_t *r) {
     CUDA_TRY(cudaEventRecord(s->ctx->ev1, st));
     const int nk = r->k < s->kcap ? r->k : s->kcap;
     const size_t bytes = hbk_pack_bytes(m, nk);
-    char *p = r->hb.pack = malloc(bytes);
-    if (!p) {
-        set_msg("host scratch of %zu bytes", bytes);
-        return HBICG_E_NOMEM;
-    }
+    char *p = r->hb.pack;
     HBK_TRY(hbk_pack(&s->sh, nk, s->d_res, s->d_tc_err, s->d_pack, st));
     CUDA_TRY(cudaMemcpyAsync(p, s->d_pack, bytes, cudaMemcpyDeviceToHost, st));
     CUDA_TRY(cudaStreamSynchronize(st));

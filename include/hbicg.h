@@ -194,7 +194,9 @@ int hbicg_solver_create(hbicg_context *ctx, hbicg_matrix *A, int m, const hbicg_
 void hbicg_solver_destroy(hbicg_solver *s);
 /* Solve.  b [n], sigma [m] and x [m*n, shift-major, leading dimension n] are
  * host or device pointers per in_where / out_where; r_out [n] (optional)
- * receives the final seed residual.  Returns hbicg_status; stats optional. */
+ * receives the final seed residual.  Returns hbicg_status; stats optional.  A
+ * solve that fails (any status but breakdown and max_iter) leaves a device x as
+ * it was; host memory may hold rows copied out, or zeros, by then. */
 int hbicg_solver_run(hbicg_solver *s, const double *b, const double *sigma, int seed, int in_where, double *x,
                      double *r_out, int out_where, hbicg_stats *stats);
 
