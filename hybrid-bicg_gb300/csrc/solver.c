@@ -214,6 +214,7 @@ struct hbicg_solver {
     void *tc_ws;      /* tensor-core flush workspace (deferred mode) */
     int *d_tc_err;    /* set by the tensor-core flush on a bounded-wait timeout */
     int launches_per_iter;
+    int nested;         /* corrects another solver's run: the context's ev0 and ev1 are that run's */
     double flush_bytes; /* compulsory HBM bytes of this solve's basis flushes */
     int flush_timed;    /* evf0, evf1 hold a flush whose time has not been read */
     /* where this solve's x_j end up, rows xld apart: the workspace's X, or the
@@ -1150,6 +1151,7 @@ static int refine_shifts(hbicg_solver *s, run_t *rn, int *refined, unsigned char
                 p1.true_residuals = 0;
                 p1.shift_mode = HBICG_SHIFTS_INCREMENTAL;
                 if ((rc = hbicg_solver_create(s->ctx, s->A, 1, &p1, &sub)) != HBICG_OK) break;
+                sub->nested = 1;
             }
             double *xj = s->xrows + (size_t)j * s->xld;
             HBK_GOTO(hbk_spmv(&s->A->k, xj, e, h_sigma[j], 1, st)); /* e = (A + sigma_j I) x_j */
@@ -1279,7 +1281,7 @@ static int run_begin(hbicg_solver *s, const double *b, const double *sigma, run_
         s->xrows = x;
         s->xld = n;
     }
-    CUDA_TRY(cudaEventRecord(ctx->ev0, st));
+    if (!s->nested) CUDA_TRY(cudaEventRecord(ctx->ev0, st));
     s->flush_bytes = 0.0;
     s->flush_timed = 0;
     r->k = 1;
@@ -1306,7 +1308,7 @@ static int fused_collect(hbicg_solver *s, run_t *r) {
     if (check)
         HBK_TRY(hbk_true_residuals_ld(&s->A->k, s->xrows, s->xld, s->d_b, s->d_sigma, m, HBK_MAX_GRID, s->sh.partials,
                                       s->sh.counters + 16, s->d_res, st));
-    CUDA_TRY(cudaEventRecord(s->ctx->ev1, st));
+    if (!s->nested) CUDA_TRY(cudaEventRecord(s->ctx->ev1, st));
     const int nk = r->k < s->kcap ? r->k : s->kcap;
     const size_t bytes = hbk_pack_bytes(m, nk);
     char *p = r->hb.pack;
@@ -1375,7 +1377,7 @@ static int run_end(hbicg_solver *s, run_t *r, int rc) {
     const int k = r->k, n_sw = r->n_sw, final_seed = r->final_seed;
     int status = r->status;
     const double *r_final = r->r_final;
-    if (s->p.form == HBICG_FORM_PLAIN) CUDA_TRY(cudaEventRecord(ctx->ev1, st));
+    if (s->p.form == HBICG_FORM_PLAIN && !s->nested) CUDA_TRY(cudaEventRecord(ctx->ev1, st));
     /* copies issued during the solve finish before anything rewrites X */
     if (s->early_pending) CUDA_TRY(cudaStreamSynchronize(ctx->cstream));
     int refined = 0;
