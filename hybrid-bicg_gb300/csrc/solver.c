@@ -966,17 +966,13 @@ static int run_fused(hbicg_solver *s, int seed, int *launches, int *flushes, dou
     if (rc0) return rc0;
     if (persistent) return run_persistent(s, launches, flushes, flush_ms);
     const int use_graph = s->p.use_graph;
-    /* every launch of a chunk advances k by chunk unless the solve ends or
-     * the basis pauses it; bound the host loop all the same */
-    long guard = 0;
-    const long guard_max = 4L * s->kcap / s->chunk + 64 + s->m; /* (a pause per seed switch) */
+    /* every launch advances k, by a chunk or up to a full basis, a seed switch
+     * or the end; bound the host loop all the same */
+    const int idle_max = 64; /* launches without an iteration, one after the other */
+    int k_seen = 0, idle = 0;
     int k_flushed = 0; /* last iteration covered by a flush */
     int loops_seen = 0; /* loop-graph bodies counted so far (k_init zeroes the device count) */
     for (;;) {
-        if (++guard > guard_max) {
-            set_msg("fused loop made no progress after %ld chunks", guard_max);
-            return HBICG_E_TIMEOUT;
-        }
         int looped = 0;
         if (use_graph) {
             if (!s->graph) {
@@ -996,6 +992,12 @@ static int run_fused(hbicg_solver *s, int seed, int *launches, int *flushes, dou
             loops_seen = h->loops;
         } else {
             *launches += s->chunk * s->launches_per_iter;
+        }
+        idle = h->k > k_seen ? 0 : idle + 1;
+        k_seen = h->k;
+        if (idle > idle_max) {
+            set_msg("fused loop made no progress in %d chunks", idle);
+            return HBICG_E_TIMEOUT;
         }
         if (!h->finished) continue;
         const int over = (h->status & HBK_ST_BREAKDOWN) || h->n_done >= h->m || h->k >= h->kcap;
