@@ -118,9 +118,24 @@ struct HwGridX {
     __device__ __forceinline__ unsigned cb() const { return blockIdx.x - 1; }
     __device__ __forceinline__ unsigned ncb() const { return x - 1; }
 };
-// element i of a vector the launch also writes (p indexed directly in a
-// one-step kernel, so its code is what it was without grid views)
-#define HBK_LD(G, p, i) ((G::hw) ? (p)[i] : __ldcg((p) + (i)))
+// Element i of a vector that this launch, or a kernel before it that may still
+// be running when this one starts early, also writes.  An explicit ordinary
+// load: what the compiler makes of an index into a const __restrict__ pointer
+// (and __ldg) may be the read-only one, whose data nothing may write while the
+// kernel is resident, and griddepcontrol.wait orders ordinary loads only.
+#define HBK_LD(G, p, i) ((G::hw) ? __ldca((p) + (i)) : __ldcg((p) + (i)))
+// The same for vectors that the launch only reads: the compiler may order these
+// loads as it likes, but behind the point where settle() gave it the pointer
+// (behind the wait).
+__device__ __forceinline__ double ld_settled(const double *p) {
+    double v;
+    asm("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ const double *settle(const double *p) {
+    asm volatile("" : "+l"(p)::"memory");
+    return p;
+}
 
 template <class G>
 struct is_hw_grid {
@@ -233,7 +248,8 @@ struct SpmvSmem {
 // way, up to SELL_AHEAD entries per row ahead (7 or 8: a seven-point stencil's
 // whole row), and `pre(row)` loads what the row's epilogue needs beside the x.
 // start() issues the first slice's loads, so that a caller can wait for x to
-// be ready behind them.  256^3 stencil, measured alone: y = A x 300 -> 261 us
+// be ready behind them; x itself, which the kernel before may still be writing
+// then, is read by ordinary loads (ld_settled).  256^3 stencil, measured alone: y = A x 300 -> 261 us
 // (6.7 TB/s) with 7 ahead (8: 275 us), with a dot product 330 -> 312 us; the
 // 256^3 solve 765 ms with 7 ahead in its products, 755 ms with 8; at 80
 // registers, three blocks per SM (64 registers, four blocks: 597 us).  Values and columns through
@@ -282,12 +298,13 @@ struct SellRows {
         head(after(r0), off1, wl1);
     }
     template <class Pre, class Epi, class Turn>
-    __device__ __forceinline__ void run(const double *__restrict__ x, const Pre &pre, Epi &epi, Turn &turn) {
+    __device__ __forceinline__ void run(const double *x_ready, const Pre &pre, Epi &epi, Turn &turn) {
+        const double *const x = settle(x_ready);
         while (r0 < A.n) {
             const unsigned r = r0 + threadIdx.x, len = wl & 255u;
             double xv[SELL_AHEAD], vn[SELL_AHEAD];
 #pragma unroll
-            for (unsigned e = 0; e < SELL_AHEAD; ++e) xv[e] = e < len ? __ldg(x + cc[e]) : 0.0;
+            for (unsigned e = 0; e < SELL_AHEAD; ++e) xv[e] = e < len ? ld_settled(x + cc[e]) : 0.0;
             const double own = r < A.n ? pre(r) : 0.0;
             entries(off1, wl1, cc, vn);
             r0 = after(r0);
@@ -298,7 +315,7 @@ struct SellRows {
             for (unsigned e = 0; e < SELL_AHEAD; ++e)
                 if (e < wl >> 8 && e < len) acc = fma(vv[e], xv[e], acc);
             for (unsigned e = SELL_AHEAD; e < wl >> 8; ++e)
-                if (e < len) acc = fma(__ldg(A.sval + entry(off, e)), __ldg(x + __ldg(A.scol + entry(off, e))), acc);
+                if (e < len) acc = fma(__ldg(A.sval + entry(off, e)), ld_settled(x + __ldg(A.scol + entry(off, e))), acc);
             if (r < A.n) epi(r, acc, own);
             turn();
 #pragma unroll

@@ -94,7 +94,7 @@ __device__ __forceinline__ hbk_cur load_cur(const hbk_scalars *sc) {
 // cosine of the two) show that in their ninth digit.  So the order follows from
 // n and the number of SMs alone, not from the blocks a kernel is launched in:
 // NT threads to a set of rows, at most 6 sets per SM for the products of SELL-32
-// matrices and DOT_VEC for K4; a thread adds its rows in ascending order, a tree
+// matrices (TILE 6, MERGE 4, HYB its lists' grid) and DOT_VEC for K4; a thread adds its rows in ascending order, a tree
 // adds the NT, and NT threads and the same tree add the sets.  Blocks fewer or
 // larger than a set carry several: K1 and K3 (3 blocks per SM) two, their NT-row
 // steps in turn, K4 up to three.  (After a switch (r^, r) is summed once over
@@ -424,7 +424,9 @@ __device__ __forceinline__ void seed_y_body(const Ctx &c, const G &g) {
     constexpr bool turns = decltype(rows)::turns;
     double2 acc = make_double2(0.0, 0.0), alt = acc;
     bool odd = false;
-    auto pre = [&](unsigned r) { return HBK_LD(G, q, r); };
+    // (as HBK_LD: 327 us at 256^3)
+    const double *const own = G::hw ? settle(q) : q;
+    auto pre = [&](unsigned r) { return G::hw ? ld_settled(own + r) : __ldcg(q + r); };
     auto epi = [&](unsigned r, double ax, double qr) {
         const double yv = folded ? ax : fma(sig, qr, ax);
         y[r] = yv;
@@ -1650,8 +1652,11 @@ static void launch(void (*kernel)(P...), int blocks, int threads, bool early, cu
 
 template <int FMT>
 static void launch_iteration(Ctx &c, const hbk_matrix *A, int early, cudaStream_t st) {
-    // the products are grid-stride loops: at most one wave of them
-    const int gs = wave_grid<k_seed_s<FMT>>(A->grid), gy = wave_grid<k_seed_y<FMT>>(A->grid);
+    // the products are grid-stride loops: at most one wave of them, and of the
+    // forms whose blocks are the sets, a number that registers do not move
+    const int most = FMT == HBK_FMT_MERGE ? 4 * sm_count() : FMT == HBK_FMT_TILE ? 6 * sm_count() : HBK_MAX_GRID;
+    const int want = A->grid < most ? A->grid : most;
+    const int gs = wave_grid<k_seed_s<FMT>>(want), gy = wave_grid<k_seed_y<FMT>>(want);
     constexpr bool sell = FMT == HBK_FMT_SELL || FMT == HBK_FMT_SELLN;
     const VecGrid q = vec_grid(c.v.n, 0), r = set_grid(vec_sets(c.v.n));
     const unsigned ncoef = !c.v.deferred ? 0 : ((unsigned)(c.sh.m < 256 ? c.sh.m : 256) * 64u + q.threads - 1) / q.threads;
