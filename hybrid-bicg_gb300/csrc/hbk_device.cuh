@@ -57,22 +57,6 @@ __device__ __forceinline__ double block_sum(double v, double *sh) {
     return warp_sum(t);
 }
 
-__device__ __forceinline__ double2 block_sum2(double2 v, double *sh) {
-    v.x = warp_sum(v.x);
-    v.y = warp_sum(v.y);
-    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    __syncthreads();
-    if (l == 0) {
-        sh[w] = v.x;
-        sh[NW + w] = v.y;
-    }
-    __syncthreads();
-    double2 t;
-    t.x = warp_sum((l < NW) ? sh[l] : 0.0);
-    t.y = warp_sum((l < NW) ? sh[NW + l] : 0.0);
-    return t;
-}
-
 // Writes this block's partial(s) and takes a ticket; returns true in every
 // thread of the block that arrives last of `nb` blocks (the launch's grid by
 // default).  That block then sums the partials in block-index order (fixed
@@ -98,8 +82,6 @@ struct HwGrid {
     static constexpr bool hw = true;
     __device__ __forceinline__ unsigned b() const { return blockIdx.x; }
     __device__ __forceinline__ unsigned nb() const { return gridDim.x; }
-    template <class T>
-    __device__ static __forceinline__ T ld(const T *p) { return *p; }
     template <class T>
     __device__ static __forceinline__ T ldx(const T *p) { return __ldg(p); }
     template <class T>
@@ -156,8 +138,6 @@ struct VGrid {
     __device__ __forceinline__ bool does_coef() const { return true; }
     __device__ __forceinline__ unsigned cb() const { return vb; }
     __device__ __forceinline__ unsigned ncb() const { return vnb; }
-    template <class T>
-    __device__ static __forceinline__ T ld(const T *p) { return __ldcg(p); }
     template <class T>
     __device__ static __forceinline__ T ldx(const T *p) { return __ldcg(p); }
     // matrix values: the seed's private SELL-32 copy gets a new diagonal after

@@ -1104,7 +1104,7 @@ __device__ __forceinline__ void coef_update(const Ctx &c, const hbk_cur &u, doub
 }
 
 // K5 (deferred): x_s and p_s, the coefficient update (in a one-family launch
-// by g.ncoef() extra blocks, else by every block), on a switch the rescaled
+// by g.ncb() extra blocks, else by every block), on a switch the rescaled
 // r_k in a new slot
 template <class G>
 __device__ __forceinline__ void seed_p_deferred_body(const Ctx &c, const G &g) {
