@@ -94,14 +94,14 @@ __device__ __forceinline__ hbk_cur load_cur(const hbk_scalars *sc) {
 // cosine of the two) show that in their ninth digit.  So the order follows from
 // n and the number of SMs alone, not from the blocks a kernel is launched in:
 // NT threads to a set of rows, at most 6 sets per SM for the products of SELL-32
-// matrices (TILE 6, MERGE 4, HYB its lists' grid) and DOT_VEC for K4; a thread adds its rows in ascending order, a tree
-// adds the NT, and NT threads and the same tree add the sets.  Blocks fewer or
-// larger than a set carry several: K1 and K3 (3 blocks per SM) two, their NT-row
-// steps in turn, K4 up to three.  (After a switch (r^, r) is summed once over
-// K5's blocks.)
+// matrices (TILE 6, MERGE 4, HYB its lists' grid) and DOT_VEC for K4; a thread
+// adds its rows in ascending order, a tree adds the NT, and NT threads and the
+// same tree add the sets.  Blocks fewer or larger than a set carry several: K1
+// and K3 (3 blocks per SM) two, their NT-row steps in turn, K4 up to four.
+// (After a switch (r^, r) is summed once over K5's blocks.)
 
 // The vector kernels (K2, K4, K5) run one block per SM, of as many threads as
-// that takes (blockDim.x, 128..1024; K4: vec_sets): the sums at a block's start
+// that takes (blockDim.x, 128..1024; K4: set_grid): the sums at a block's start
 // then cost an SM one pass, not one per resident block.
 constexpr int DOT_VEC = 4, DOT_ROWS = 512;  // K4: sets per SM at most, rows per set while there are fewer
 
@@ -640,7 +640,9 @@ __device__ __forceinline__ void seed_update_body(const Ctx &c, const G &g) {
     store_part2(acc, sh, parts(c, P_RR) + set, parts(c, P_RRH) + set, here);
 }
 template <int PER_SM>
-__global__ void __launch_bounds__(2 * NT, PER_SM) k_seed_update(Ctx c) { seed_update_body(c, HwGridX{1}); }
+__global__ void __launch_bounds__(PER_SM == 1 ? DOT_VEC * NT : 2 * NT, PER_SM) k_seed_update(Ctx c) {
+    seed_update_body(c, HwGridX{1});
+}
 
 // ---------------------------------------------------------------------------
 // Argmax of |1/(zeta_j pi_j)| over the systems still running after this
@@ -1620,18 +1622,31 @@ static VecGrid vec_grid(unsigned n, int extra) {
     const unsigned need = n ? (n + t - 1) / t : 1;
     return {need < (unsigned)most ? (int)need : most, (int)t};
 }
-// K4's: all its sets of rows resident at once, beside the extra block: one block
-// per SM with 64 registers while two sets fill it; two blocks and 40 registers
-// (a third fits) where there are more, as then the scalars in the extra block
-// need not be fast (their spills cost 1.6 us, K4 8.5 instead of 6.9 us at n = 512).
+// K4's: all its sets of rows resident at once beside the extra block, in one block
+// per SM and 64 registers where that leaves the extra one an SM; else (the most
+// sets, DOT_VEC per SM) two blocks per SM and 40 registers, so that a third fits
+// (their spills are the scalars' in the extra block, which need not be fast then;
+// n = 512 would take 8.5 instead of 6.3 us).
 static int vec_sets(unsigned n) {
     const int most = DOT_VEC * sm_count();
     const unsigned want = n ? (n + DOT_ROWS - 1) / DOT_ROWS : 1;
     return want < (unsigned)most ? (int)want : most;
 }
-static VecGrid set_grid(int sets) {
-    const int per = sets <= sm_count() ? 1 : 2;
-    return {(sets + per - 1) / per, per * NT};
+struct SetGrid {
+    int blocks, threads;
+    bool one;    // one block per SM
+    bool early;  // may start early
+};
+// Early only where blocks cannot crowd onto the SMs that the kernel before
+// leaves first: blocks that fill an SM's registers, or few small ones.  Measured, an
+// iteration, early / not: 256^3, 2 shifts 1010 / 950 us, 128^3 172 / 163, 80 k power-law
+// rows 47.9 / 46.4, 42^3 34.1 / 31.9; blocks of 1024: 64^3 61.6 / 63.0; 36^3 26.5 both.
+static SetGrid set_grid(int sets) {
+    const int sms = sm_count();
+    if (sets <= sms) return {sets, NT, true, sets <= sms * 4 / 5};
+    for (int per = 2; per <= DOT_VEC; ++per)
+        if (sets <= per * (sms - 1)) return {(sets + per - 1) / per, per * NT, true, per == DOT_VEC};
+    return {(sets + 1) / 2, 2 * NT, false, false};
 }
 
 // kernel<<<...>>>, allowed to start before the stream's previous kernel ends
@@ -1658,7 +1673,8 @@ static void launch_iteration(Ctx &c, const hbk_matrix *A, int early, cudaStream_
     const int want = A->grid < most ? A->grid : most;
     const int gs = wave_grid<k_seed_s<FMT>>(want), gy = wave_grid<k_seed_y<FMT>>(want);
     constexpr bool sell = FMT == HBK_FMT_SELL || FMT == HBK_FMT_SELLN;
-    const VecGrid q = vec_grid(c.v.n, 0), r = set_grid(vec_sets(c.v.n));
+    const VecGrid q = vec_grid(c.v.n, 0);
+    const SetGrid r = set_grid(vec_sets(c.v.n));
     const unsigned ncoef = !c.v.deferred ? 0 : ((unsigned)(c.sh.m < 256 ? c.sh.m : 256) * 64u + q.threads - 1) / q.threads;
     const VecGrid p = vec_grid(c.v.n, 1 + (int)ncoef);
     // (SELL-32: a set for every NT rows up to two per block)
@@ -1669,12 +1685,13 @@ static void launch_iteration(Ctx &c, const hbk_matrix *A, int early, cudaStream_
     // 97 k rows: 20.1 -> 18.5 ms; 128^3: 64.2 -> 63.0 ms.  Not where blocks
     // that start early would crowd onto the SMs the kernel before leaves free
     // and then run long: the incremental update (FP64-bound; 32^3: 3.4 -> 4.7
-    // ms) and the products of the other forms (HYB: 68 -> 75 ms).
+    // ms), the products of the other forms (HYB, an iteration with 16 shifts, 20 k
+    // rows 34.6 -> 34.0 us, but 60 k 49.1 -> 56.8, 1 M 294 -> 303), K4 by set_grid.
     const bool e = early > 0, es = e && sell;
     launch(k_seed_s<FMT>, gs, NT, es && early > 1, st, c);
     launch(k_seed_q, q.blocks, q.threads, e, st, c);
     launch(k_seed_y<FMT>, gy, NT, es, st, c);
-    launch(r.blocks <= sm_count() ? k_seed_update<2> : k_seed_update<3>, r.blocks + 1, r.threads, e, st, c);
+    launch(r.one ? k_seed_update<1> : k_seed_update<3>, r.blocks + 1, r.threads, e && r.early, st, c);
     if (!c.v.deferred) launch(k_shift_update<64>, p.blocks + 1, p.threads, false, st, c);
     else launch(k_seed_p_deferred, p.blocks + 1 + (int)ncoef, p.threads, e, st, c, ncoef);
 }
