@@ -1614,10 +1614,10 @@ int hbk_hyb_wave_fused(int wide) {
 struct VecGrid {
     int blocks, threads;
 };
-static VecGrid vec_grid(unsigned n, int extra) {
+static VecGrid vec_grid(unsigned n, int extra, unsigned least = 128) {
     const int sms = sm_count();
     const unsigned per = (n / (unsigned)sms + 64) / 64 * 64;
-    const unsigned t = per < 128 ? 128 : (per > 1024 ? 1024 : per);
+    const unsigned t = per < least ? least : (per > 1024 ? 1024 : per);
     const int most = t <= 512 ? sms : (sms > 2 * extra ? sms - extra : 1);
     const unsigned need = n ? (n + t - 1) / t : 1;
     return {need < (unsigned)most ? (int)need : most, (int)t};
@@ -1673,7 +1673,9 @@ static void launch_iteration(Ctx &c, const hbk_matrix *A, int early, cudaStream_
     const int want = A->grid < most ? A->grid : most;
     const int gs = wave_grid<k_seed_s<FMT>>(want), gy = wave_grid<k_seed_y<FMT>>(want);
     constexpr bool sell = FMT == HBK_FMT_SELL || FMT == HBK_FMT_SELLN;
-    const VecGrid q = vec_grid(c.v.n, 0);
+    // (K2 adds K1's sums with NT threads, or fewer where there are no more sums
+    // than these, as a few rows leave of SELL-32 only)
+    const VecGrid q = vec_grid(c.v.n, 0, sell ? 128 : NT);
     const SetGrid r = set_grid(vec_sets(c.v.n));
     const unsigned ncoef = !c.v.deferred ? 0 : ((unsigned)(c.sh.m < 256 ? c.sh.m : 256) * 64u + q.threads - 1) / q.threads;
     const VecGrid p = vec_grid(c.v.n, 1 + (int)ncoef);

@@ -77,8 +77,8 @@ WIDE = ((-7, -2, -1, 0, 1, 2, 7), (-0.7, -0.3, -1.1, 4.6, -0.9, -0.4, -0.6))
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("band", [NARROW, WIDE], ids=["narrow", "wide"])
-# one set; a few; around 3 and 6 sets of 256 rows and 4 of 512 per SM of 152
-@pytest.mark.parametrize("n", [200, 700, 40001, 116800, 130000, 233500, 300001, 311300, 400000])
+# one set; a few; around 3 and 6 sets of 256 rows and 1, 2, 3 and 4 of 512 per SM of 152
+@pytest.mark.parametrize("n", [200, 700, 40001, 77825, 116800, 130000, 154625, 233500, 300001, 311300, 400000])
 def test_one_iteration_bit_for_bit(cuda, pkg, band, n):
     import torch
 
@@ -109,3 +109,39 @@ def test_one_iteration_bit_for_bit(cuda, pkg, band, n):
     r = _fma(-omega, y, q)
     assert h["rr"][1] == _dot(r, r, by_vec)
     assert h["beta"][1] == (alpha / omega) * (_dot(b, r, by_vec) / bb)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [3000, 3100, 4000, 5000, 22222])
+def test_sums_of_many_blocks(cuda, pkg, n):
+    """TILE products of few rows with many entries leave more sums than K2 has threads for its rows: alpha of the first
+    iteration in the order that NT threads add them."""
+    rng = np.random.default_rng(n)
+    lens = np.full(n, 3)
+    lens[::7] = 300  # a row of over 256 entries is a block of its own, as is every run of rows between
+    ptr = np.zeros(n + 1, dtype=np.uint32)
+    np.cumsum(lens, out=ptr[1:])
+    row = np.repeat(np.arange(n), lens)
+    col = ((row + np.arange(len(row)) - ptr[:-1].astype(np.int64)[row]) % n).astype(np.uint32)
+    val = np.where(rng.random(len(row)) < 0.5, -0.125, 0.125)  # every product and sum of a row is exact
+    b = np.where(rng.random(n) < 0.5, -1.0, 1.0) * (1.0 + rng.integers(0, 2**10, n) * 2.0**-10)  # (b, b) too
+    A = pkg.Matrix(pkg.Context(), ptr, col, val)
+    A.set_format("tile")
+    sg = 0.00371  # (the sum cancels: another order shows)
+    h = pkg.Solver(A, 1, max_iter=2, shift_mode="incremental", refine=False).run(b, np.array([sg])).extra["hist"]
+    y = np.zeros(n)
+    np.add.at(y, row, val * b[col])
+    s = _fma(sg, b, y)
+    # blocks of rows: 6 consecutive rows of 3 entries, one long row, in turn from row 0 (long)
+    bounds = np.unique(np.concatenate([np.arange(0, n, 7), np.arange(1, n, 7), [n]]))
+    blocks = len(bounds) - 1
+    sets = min(blocks, 6 * 152, 8 * 152)
+    acc = np.zeros((sets, NT))
+    for k, (lo, hi) in enumerate(zip(bounds[:-1], bounds[1:])):
+        acc[k % sets, :hi - lo] = _fma(b[lo:hi], s[lo:hi], acc[k % sets, :hi - lo])
+    part = np.array([_tree(a) for a in acc])
+    thread = np.zeros(NT)
+    for i in range(0, sets, NT):
+        p = part[i:i + NT]
+        thread[:len(p)] = thread[:len(p)] + p
+    assert h["alpha"][1] == np.sum(b * b) / _tree(thread)
