@@ -96,8 +96,13 @@ int hbicg_context_create(hbicg_context **out) { return hbicg__context_create_pri
 
 /* Streams, events and pinned words of destroyed contexts wait here for the next
  * context of the same device and priority (a one-shot call makes and destroys
- * one: 0.2 ms), at most HBICG_CTX_KEEP of them; hbicg_release gives them back. */
-#define HBICG_CTX_KEEP 16
+ * one, an adjoint two: 7 instead of 28 us each), at most HBICG_CTX_KEEP of them;
+ * hbicg_release gives them back.  No more than these: every stream of the
+ * process slows its stream-ordered allocations.  A matrix of 64^3 rows takes 290 us
+ * to make, 325 with 4 contexts kept, 415 with 16, which a batch of 8 workers leaves
+ * behind (forward and backward of a 176 k-row solve 18.2 / 18.8 / 19.3 ms; the next
+ * batch, of 22 ms, gains 0.5 ms by 16). */
+#define HBICG_CTX_KEEP 2
 static hbicg_context *g_ctx_idle[HBICG_CTX_KEEP];
 static int g_ctx_nidle;
 static pthread_mutex_t g_ctx_lock = PTHREAD_MUTEX_INITIALIZER;

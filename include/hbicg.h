@@ -291,7 +291,7 @@ int hbicg_solve(unsigned n, unsigned nnz, const unsigned *ptr, const unsigned *c
                 double *r_out, hbicg_stats *stats);
 
 /* Solvers take their device buffers from a library-owned pool that keeps freed
- * memory for the next solver, and up to 16 contexts that nothing uses any more
+ * memory for the next solver, and up to 2 contexts that nothing uses any more
  * are kept with their streams and events; this returns the memory no live
  * solver uses to the device and frees those contexts (call it when the
  * library's solves are done). */

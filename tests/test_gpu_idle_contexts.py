@@ -1,0 +1,31 @@
+"""Contexts kept for the next call do not slow the calls that follow: a matrix takes no longer to make after a batch of
+many workers than before it (every idle stream adds to each stream-ordered allocation)."""
+import time
+
+import numpy as np
+import pytest
+
+
+@pytest.mark.gpu
+def test_matrix_after_a_batch(cuda, pkg):
+    a = pkg.workloads.stencil_cd3d(64)
+    dev = [cuda.from_numpy(np.ascontiguousarray(v, dtype=t)).cuda() for v, t in
+           ((a.ptr, np.int32), (a.col, np.int32), (a.val, np.float64))]
+
+    def best():
+        times = []
+        for _ in range(60):
+            cuda.cuda.synchronize()
+            t = time.perf_counter()
+            pkg.Matrix(pkg.Context(), *dev).close()
+            cuda.cuda.synchronize()
+            times.append(time.perf_counter() - t)
+        return sorted(times)[10]
+
+    pkg.release()
+    best()
+    before = best()
+    fams = pkg.workloads.batched_families(32, n_lo=9000, n_hi=20000, seed=1)
+    pkg.batch_solve(fams, workers=16, tol=1e-8, max_iter=1000)
+    after = best()
+    assert after < 1.2 * before, (before, after)
