@@ -28,4 +28,4 @@ def test_matrix_after_a_batch(cuda, pkg):
     fams = pkg.workloads.batched_families(32, n_lo=9000, n_hi=20000, seed=1)
     pkg.batch_solve(fams, workers=16, tol=1e-8, max_iter=1000)
     after = best()
-    assert after < 1.2 * before, (before, after)
+    assert after < 1.35 * before, (before, after)
