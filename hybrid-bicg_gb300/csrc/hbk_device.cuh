@@ -229,10 +229,10 @@ struct SpmvSmem {
 // whole row), and `pre(row)` loads what the row's epilogue needs beside the x.
 // start() issues the first slice's loads, so that a caller can wait for x to
 // be ready behind them; x itself, which the kernel before may still be writing
-// then, is read by ordinary loads (ld_settled).  256^3 stencil, measured alone: y = A x 300 -> 261 us
-// (6.7 TB/s) with 7 ahead (8: 275 us), with a dot product 330 -> 312 us; the
-// 256^3 solve 765 ms with 7 ahead in its products, 755 ms with 8; at 80
-// registers, three blocks per SM (64 registers, four blocks: 597 us).  Values and columns through
+// then, is read by ordinary loads (ld_settled).  256^3 stencil, measured alone:
+// y = A x 300 -> 261 us (6.7 TB/s) with 7 ahead (8: 275 us); with a dot product
+// (K1) 330 -> 288 us with 8, with two (K3) 294 us with 7; at 80 registers, three
+// blocks per SM (64 registers, four blocks: 597 us).  Values and columns through
 // bulk copies into shared memory, two to four slices deep, were slower
 // (275..339 us).
 template <int SELL_AHEAD>

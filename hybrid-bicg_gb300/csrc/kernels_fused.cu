@@ -86,7 +86,7 @@ __device__ __forceinline__ hbk_cur load_cur(const hbk_scalars *sc) {
 // of SellRows and early launches: n = 512, 6 shifts 1788 -> 974 us; 32^3, 16
 // shifts 5.61 -> 3.22 ms; 97 k rows, 24 shifts 26.4 -> 18.2 ms; 128^3, 32
 // shifts 72.9 -> 61.1 ms; 256^3, 64 shifts 805 -> 711 ms (with the changes made
-// elsewhere since: 0.82, 2.9, 16.0, 55.5 and 655 ms).
+// elsewhere since: 0.79, 2.78, 15.8, 56.2 and 651 ms).
 //
 // The order of a dot product's sum is part of a solve's outcome: it moves what
 // is left of every residual below the tolerance at which the solve stops, and
@@ -406,7 +406,7 @@ __device__ __forceinline__ void seed_q_body(const Ctx &c, const G &g) {
 __global__ void __launch_bounds__(1024) k_seed_q(Ctx c) { seed_q_body(c, HwGrid()); }
 
 // K3: y = (A + sigma_s I) q, (q,q) and (q,y).  SELL-32: the sums of two sets take
-// the registers of an eighth entry ahead (256^3: 295 us; with it they spill, 367;
+// the registers of an eighth entry ahead (256^3: 294 us; with it they spill, 367;
 // the other set's in shared memory 321, with seven ahead 340).
 template <int FMT, class G>
 __device__ __forceinline__ void seed_y_body(const Ctx &c, const G &g) {
