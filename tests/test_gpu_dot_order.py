@@ -135,7 +135,7 @@ def test_sums_of_many_blocks(cuda, pkg, n):
     # blocks of rows: 6 consecutive rows of 3 entries, one long row, in turn from row 0 (long)
     bounds = np.unique(np.concatenate([np.arange(0, n, 7), np.arange(1, n, 7), [n]]))
     blocks = len(bounds) - 1
-    sets = min(blocks, 6 * 152, 8 * 152)
+    sets = min(blocks, 6 * cuda.cuda.get_device_properties(0).multi_processor_count)
     acc = np.zeros((sets, NT))
     for k, (lo, hi) in enumerate(zip(bounds[:-1], bounds[1:])):
         acc[k % sets, :hi - lo] = _fma(b[lo:hi], s[lo:hi], acc[k % sets, :hi - lo])
